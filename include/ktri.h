@@ -50,8 +50,9 @@ extern "C" {
 typedef struct ktri_opts {
     uint32_t struct_size;          /* sizeof(ktri_opts); 0 is read as "all defaults" */
     int32_t intersection_method;   /* KTRI_METHOD_* */
-    uint32_t small_outdegree;      /* owners with out-degree <= this use the tile kernel: 1..48 (0 = default 32;
-                                      bounds above 32 pay off on graphs of average degree above ~40) */
+    uint32_t small_outdegree;      /* edges between out-degrees <= this are counted at their tail by the small
+                                      kernel, the rest by owner tiles: 1..48 (0 = default: 48, or medium_outdegree
+                                      where that is set lower) */
     uint32_t collect_stats;        /* 1: also compute wedge_checks / intersection work counters */
     uint64_t binary_intersection_cutoff; /* Config::binary_intersection_cutoff (config.h:173), default 1000 */
     double hybrid_cutoff_scale;    /* Config::hybrid_cutoff_scale (config.h:174), default 1.0 */
@@ -59,7 +60,7 @@ typedef struct ktri_opts {
                                       graphs with nnz + 3n > 2^32 take; exposed for testing) */
     uint32_t medium_outdegree;     /* owners above small_outdegree and at most this use the warp-per-tile
                                       kernel, larger ones the block-per-tile kernel: small_outdegree..256
-                                      (0 = default 256) */
+                                      (0 = default 256; at least 32 with small_outdegree 0) */
     uint32_t segment;              /* adjacency slots per owner tile of those two kernels: a power of two
                                       in 64..1024 (0 = default 1024) */
     uint32_t copy_wait_polls;      /* bound on the polls of the large-owner kernel's first wait for each

@@ -79,7 +79,7 @@ u64 isqrt_ceil(u64 x) {
 
 // Workspace of one count.  num_sms = 0 sizes the grids for the largest supported part.
 Layout make_layout(u64 n, u64 nnz, int32_t method, int num_sms, bool with_inputs, bool internal_cnt,
-                   bool force_wide = false, u32 small_d = (u32)ktri::SMALL_D_LOW, u32 seg = ktri::LARGE_SEG) {
+                   bool force_wide = false, u32 small_d = 32, u32 seg = ktri::LARGE_SEG) {
     Layout L;
     const u64 cap = ktri::oriented_capacity(n, nnz);
     L.wide = force_wide || cap > ktri::NARROW_CAPACITY;
@@ -147,12 +147,14 @@ ktri::Options resolve(const ktri_opts* o) {
     ktri::Options r;
     if (!o || o->struct_size == 0) return r;
     r.method = o->intersection_method;
-    if (o->small_outdegree) r.small_outdegree = o->small_outdegree;
     r.collect_stats = o->collect_stats != 0;
     if (o->binary_intersection_cutoff) r.binary_cutoff = o->binary_intersection_cutoff;
     if (o->hybrid_cutoff_scale > 0) r.hybrid_scale = o->hybrid_cutoff_scale;
     r.force_wide = o->force_wide_offsets != 0;
     if (o->medium_outdegree) r.medium_outdegree = o->medium_outdegree;
+    // the default lies at the largest bound, or at a medium bound the caller set below it (32 at least)
+    if (o->small_outdegree) r.small_outdegree = o->small_outdegree;
+    else r.small_outdegree = std::max(32u, std::min(r.small_outdegree, r.medium_outdegree));
     if (o->segment) r.segment = o->segment;
     r.copy_wait_polls = o->copy_wait_polls;
     r.tile_order = o->tile_order;
@@ -362,8 +364,7 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     const u64 tcap = ktri::large_tile_capacity(n, nnz, opt.small_outdegree, opt.segment);
     auto* ltiles = autom ? mtiles + tcap : nullptr;
     ktri::launch_desc<OffT>(fo, n, dplus, vdesc, mtiles, ltiles, autom ? opt.small_outdegree : 0xFFFFFFFFu,
-                            opt.medium_outdegree, opt.segment,
-                            autom ? ktri::SMALL_WARP_DEG : 0xFFFFFFFFu, ctl, sms, st);
+                            opt.medium_outdegree, opt.segment, ctl, sms, st);
     // Tile orders (large tiles by the vertex range they stream, for L2 reuse; medium tiles
     // longest owner first, so the warps' last tiles are short).  Below 2^20 adjacency entries
     // everything fits L2 and the few tiles are not worth the four extra launches.
@@ -389,7 +390,8 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     }
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[1], st));
     if (opt.collect_stats)
-        ktri::launch_stats<OffT>(fo, head, n, vdesc, headp, autom ? opt.medium_outdegree : 0xFFFFFFFFu, ctl, sms, st);
+        ktri::launch_stats<OffT>(fo, head, n, vdesc, headp, opt.small_outdegree,
+                                 autom ? opt.medium_outdegree : 0xFFFFFFFFu, ctl, sms, st);
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[2], st));
     if (sort_all) {
         // orientation export only: no counting
@@ -402,7 +404,7 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
                                                    opt.segment, cnt, partials, ctl, sms, st,
                                                    events ? ctx->ev[4] : nullptr, events ? ctx->ev[5] : nullptr,
                                                    first_wait_polls(opt.copy_wait_polls)));
-        ktri::launch_final_auto<OffT>(partials, n, opt.small_outdegree, sms, d_total, ctl, st);
+        ktri::launch_final_auto<OffT>(partials, n, sms, d_total, ctl, st);
     } else {
         const int grid = ktri::count_grid_edges(sms);
         ktri::launch_count_edges<OffT>(n, vdesc, headp, opt.method, opt.binary_cutoff, opt.hybrid_scale, cnt, partials,
@@ -1471,10 +1473,8 @@ int ktri_plan_create_batch(ktri_ctx* ctx, const uint64_t* d_first_out, const uin
         return cuda_fail(ctx, e, "cudaMalloc(plan workspace)");
     }
     // occupancy queries happen once, outside the capture
-    for (u32 sd : {(u32)ktri::SMALL_D_LOW, (u32)ktri::SMALL_D}) {
-        (void)ktri::count_grid_auto<u32>(ctx->num_sms, sd);
-        (void)ktri::count_grid_auto<u64>(ctx->num_sms, sd);
-    }
+    (void)ktri::count_grid_auto<u32>(ctx->num_sms);
+    (void)ktri::count_grid_auto<u64>(ctx->num_sms);
     cudaStream_t cs = nullptr;
     cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
     char* base = static_cast<char*>(p->ws);

@@ -3,26 +3,21 @@
 //
 // Every undirected edge {x,y} contributes |N+(x) ∩ N+(y)| triangles, where N+ is the
 // out-list after orientation by (degree, id); the sum over all edges is the triangle total,
-// exactly as the reference's sum over oriented edges (v,u) of |N+(v) ∩ N+(u)|.  The edge is
-// evaluated once, at its "owner": the endpoint whose (out-degree, id) is larger.  The owner's
-// out-list sits in a shared-memory hash table and the other endpoint's (shorter) out-list
-// is streamed through it, so the work of an edge is min(|N+(x)|, |N+(y)|) probes.
+// exactly as the reference's sum over oriented edges (v,u) of |N+(v) ∩ N+(u)|.  Each edge is
+// evaluated once: one endpoint's out-list sits in a shared-memory hash table and the other's is
+// streamed through it.  Edges between two out-degrees of at most small_outdegree are evaluated
+// at their tail; the others at their "owner", the endpoint whose (out-degree, id) is larger, so
+// that their work is min(|N+(x)|, |N+(y)|) probes.
 //
 // Per-vertex counts: a hit w of edge {x,y} is the triangle {x,y,w}.  w is a key of the
-// owner's table: its hits accumulate in a shared-memory counter next to the key and are
-// flushed once per table.  y gets one atomic per edge, x one per tile.
+// table: its hits accumulate in a shared-memory counter next to the key and are flushed once per
+// table.  The streamed endpoint gets its list's hits, the other one its table's total.
 //
-// Three kernels split the owners by out-degree (the bounds are runtime options, at most
-// SMALL_D and MEDIUM_D):
-//   k_count_small: owners with out-degree <= small_outdegree and degree <= SMALL_WARP_DEG
-//     (instantiated for bounds up to SMALL_D_LOW and up to SMALL_D).  A warp takes 32
-//     consecutive vertices and counts their owners in groups of up to eight that share its
-//     slice of shared memory: tables side by side, one flattened pass over all their keys, one
-//     over all their adjacency slots (queueing the lower neighbours' lists), a counting sort of
-//     the queue by list length, then one list per lane with uint4 loads.  No block barrier.
-//   k_count_medium: owners up to medium_outdegree (and small-out-degree owners of larger
-//     degree), one warp per (owner, segment) tile with the warp's own table, filter and
-//     survivor buffer, so tiles need no block barrier.
+// Three kernels (the bounds are runtime options, at most SMALL_D and MEDIUM_D):
+//   k_count_small: the edges between out-degrees of at most small_outdegree, groups of tails per
+//     warp, one streamed list per lane.  No block barrier.
+//   k_count_medium: owners up to medium_outdegree, one warp per (owner, segment) tile with the
+//     warp's own table, filter and survivor buffer, so tiles need no block barrier.
 //   k_count_large: larger owners, one (owner, segment) tile per block iteration.  Short
 //     streamed lists are handled one per thread while the segment is scanned; longer ones are
 //     queued and taken one at a time by whole warps (one entry per lane, eight loads in
@@ -143,234 +138,276 @@ __device__ __forceinline__ u32 bucket_probe16_flat(const u32* keys, u32* hits32,
     return slot < 4u ? 1u : 0u;
 }
 
-// Small owners (k_count_small), warp-granular.  A warp takes
-// 32 consecutive vertices at a time and counts their owners (out-degree 1..small_outdegree,
-// degree at most SMALL_WARP_DEG; owners of larger degree go to the medium kernel's tiles) in
-// groups: up to GROUP owners whose tables fit TAB slots and whose adjacency fits QCAP slots
-// share the warp's slice of shared memory.  Each phase runs over the whole group at once (all
-// keys, then all adjacency slots, then all queued lists), so one round of global loads serves
-// every owner of the group; the queue is counting-sorted by list length and streamed one list
-// per lane, longest first.  Only __syncwarp orders the phases: the warps of a block never wait
-// for one another.
-template <int SD, typename OffT>
+// Small edges (k_count_small), warp-granular: the edges (v, u) whose endpoints both have an
+// out-degree of at most small_outdegree, each counted at its tail v.  A warp takes a few
+// consecutive vertices and counts their out-lists in groups of up to GROUP tails that hold up to
+// QCAP keys together.  A key is both an entry of its tail's table and an edge whose head's list
+// is streamed through that table, so one pass over the keys builds the tables and the queue, and
+// neither the input adjacency nor the lower neighbours are read.  The queue is counting-sorted
+// by list length and streamed one list per lane, longest first.  Only __syncwarp orders the
+// phases: the warps of a block never wait for one another.
+//
+// What bounds it: instruction issue and shared-memory wavefronts of the lookups.  A lookup reads
+// one bucket of two keys (8 bytes) and never walks: a table of 3 d buckets for d keys is rebuilt
+// with another multiplier until no bucket holds more than two (about 0.013 d overfull buckets
+// expected, so most tables of d <= 32 succeed at once), and a table that never does is searched
+// entry by entry.  Against one table per owner in buckets of four with early exits, streamed over
+// the whole adjacency (the form before), 1.0x to 1.05x the entries are streamed on uniform and
+// geometric graphs (the head's list instead of the shorter one) at a quarter of the instructions.
+template <typename OffT>
 struct SmallWarpLayout {
-    static constexpr int GROUP = 8;      // owners per group
-    static constexpr int TAB = 256;      // table slots of a group (each table a power of two >= 2 d+)
-    static constexpr int QCAP = 256;     // adjacency slots of a group (the queue's capacity)
-    static constexpr int NBIN = SD + 2;  // list lengths 0..SD
-    static constexpr int OW = 10;        // words per owner record
+    static constexpr int GROUP = 16;             // tails per group
+    static constexpr int QCAP = 128;             // keys (and queued lists) of a group
+    static constexpr int ROWS = QCAP / 32;       // keys per lane
+    static constexpr int NB = 3 * QCAP;          // buckets: three per key
+    static constexpr int MAX_TRIES = 16;         // multipliers tried per table
     // u32 words per warp
-    static constexpr int W_KEYS = 0;
-    static constexpr int W_HITS = W_KEYS + TAB;                         // two 16-bit counters per word
-    static constexpr int W_QY = W_HITS + TAB / 2;
-    static constexpr int W_QS = W_QY + QCAP;                            // list starts (OffT)
-    static constexpr int W_QM = W_QS + QCAP * (int)(sizeof(OffT) / 4);  // (owner << 8) | length
-    static constexpr int W_ORD = W_QM + QCAP;                           // queue order by length (u16)
-    static constexpr int W_BIN = W_ORD + QCAP / 2;                      // 64 length bins
-    static constexpr int W_OWN = W_BIN + 64;
-    static constexpr int PER_WARP = (W_OWN + OW * GROUP + 3) & ~3;
+    static constexpr int W_KEYS = 0;                                    // two keys per bucket
+    static constexpr int W_HITS = W_KEYS + 2 * NB;                      // two 16-bit counters per bucket
+    static constexpr int W_REC = W_HITS + NB;                           // tail records (uint4)
+    static constexpr int W_QS = W_REC + 4 * GROUP;                      // list starts (OffT), by key
+    static constexpr int W_OS = W_QS + QCAP * (int)(sizeof(OffT) / 4);  // tails' list starts (OffT)
+    static constexpr int W_QM = W_OS + GROUP * (int)(sizeof(OffT) / 4); // (slot << 11) | (tail << 7) | length, by key
+    static constexpr int W_TOT = W_QM + QCAP;                           // tails' hit totals
+    static constexpr int W_VTX = W_TOT + GROUP;                         // tails' vertices
+    static constexpr int W_BIN = W_VTX + GROUP;                         // lists by length in 16-byte groups
+    static constexpr int W_ORD = W_BIN + 32;                            // queue order (u16)
+    static constexpr int PER_WARP = (W_ORD + QCAP / 2 + 3) & ~3;
     static constexpr size_t bytes(int warps) { return sizeof(u32) * PER_WARP * warps; }
 };
 
-// One batch of 32 consecutive vertices (bi), counted by one warp in its slice of shared
-// memory: the owners among them, in groups.
-template <int SD, typename OffT, bool CG = false>
-__device__ __forceinline__ void small_batch(u32* base, u64 bi, const u64* __restrict__ fo,
-                                            const u32* __restrict__ head, u64 n,
-                                            const Desc<OffT>* __restrict__ vdesc, const u32* __restrict__ headp,
-                                            u32 sd, u64* __restrict__ cnt, u64& local_total, u32& dup) {
-    using L = SmallWarpLayout<SD, OffT>;
-    constexpr int OW = L::OW;
-    static_assert(2 * SD <= L::TAB / 2, "two owners of the largest out-degree fit a group's tables");
-    static_assert(SMALL_WARP_DEG <= (u32)L::QCAP, "one owner's adjacency fits the queue");
-    static_assert(SD < 256 && L::NBIN <= 64, "list length is packed in 8 bits, bins two per lane");
+constexpr u32 NO_SLOT = 1023;  // a key without a table slot (its tail's table could not be built)
+
+// A warp's tables are empty between groups: keys and counters are cleared as they are flushed.
+template <typename OffT>
+__device__ __forceinline__ void small_init(u32* base) {
+    using L = SmallWarpLayout<OffT>;
     const int lane = threadIdx.x & 31;
-    const u32 lt_mask = (1u << lane) - 1;
+    for (int i = lane; i < 2 * L::NB; i += 32) base[L::W_KEYS + i] = EMPTY_KEY;
+    for (int i = lane; i < L::NB; i += 32) base[L::W_HITS + i] = 0;
+    __syncwarp();
+}
+
+// One batch: the tails among the vertices [bi * vb, (bi + 1) * vb), vb <= 32, counted by one warp in
+// its slice of shared memory.
+template <typename OffT, bool CG = false>
+__device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, const Desc<OffT>* __restrict__ vdesc,
+                                            const u32* __restrict__ headp, u32 sd, u64* __restrict__ cnt,
+                                            u64& local_total, u32& dup) {
+    using L = SmallWarpLayout<OffT>;
+    constexpr u32 FULL = 0xFFFFFFFFu;
+    static_assert(SMALL_D < 128 && SMALL_D <= L::QCAP && L::GROUP <= 16, "field widths of the queue entries");
+    static_assert(2 * L::NB <= (int)NO_SLOT && (SMALL_D + 3) / 4 < 32, "slots and length bins");
+    const u32 lane = threadIdx.x & 31;
+    const u32 lt_mask = (1u << lane) - 1, le_mask = lt_mask | (1u << lane);
     u32* keys = base + L::W_KEYS;
-    u32* hitc = base + L::W_HITS;
-    u32* q_y = base + L::W_QY;
+    u32* hits = base + L::W_HITS;
+    unsigned short* hits16 = reinterpret_cast<unsigned short*>(hits);
+    uint4* rec = reinterpret_cast<uint4*>(base + L::W_REC);  // x: first key, y: out-degree, z: multiplier
     OffT* q_s = reinterpret_cast<OffT*>(base + L::W_QS);
+    OffT* o_s = reinterpret_cast<OffT*>(base + L::W_OS);
     u32* q_m = base + L::W_QM;
-    unsigned short* q_ord = reinterpret_cast<unsigned short*>(base + L::W_ORD);
+    u32* tot = base + L::W_TOT;
+    u32* vtx = base + L::W_VTX;
     u32* bins = base + L::W_BIN;
-    // owner gi at own + OW * gi: [0] vertex, [1] (table offset << 5) | lg, [2] out-degree,
-    // [3] key prefix, [4] adjacency prefix, [5] hit total, [6..7] first adjacency slot (u64),
-    // [8..9] out-list start (u64)
-    u32* own = base + L::W_OWN;
+    unsigned short* q_ord = reinterpret_cast<unsigned short*>(base + L::W_ORD);
     const uint4* headp4 = reinterpret_cast<const uint4*>(headp);
-    const u64 v = bi * 32 + lane;
+    const u64 v = bi * vb + lane;
     Desc<OffT> dv;
     dv.start = 0;
     dv.d = 0;
-    u64 a = 0;
-    u32 deg = 0;
-    bool is_owner = false;
-    if (v < n) {
-        dv = ld_desc<CG>(vdesc + v);
-        a = ld_in<CG>(fo + v);
-        const u64 b = ld_in<CG>(fo + v + 1);
-        is_owner = dv.d > 0 && dv.d <= sd && b - a <= (u64)SMALL_WARP_DEG;
-        deg = (u32)(b - a);
-    }
-    u32 lg = 0, tsz = 0;
-    if (is_owner) {
-        lg = ceil_log2(2 * dv.d);
-        if (lg < 2) lg = 2;
-        tsz = 1u << lg;
-    }
-    u32 todo = __ballot_sync(0xFFFFFFFFu, is_owner);
+    if (lane < vb && v < n) dv = ld_desc<CG>(vdesc + v);
+    u32 todo = __ballot_sync(FULL, dv.d >= 2 && dv.d <= sd);  // a tail needs two out-neighbours
     while (todo) {
-        // the group: the next owners in lane order while their tables and adjacency fit
+        // the group: the next tails in lane order while their keys fit
         const bool cand = (todo >> lane) & 1u;
-        u32 pk = cand ? (tsz << 16) | deg : 0u;  // inclusive prefix of (table slots, adjacency)
+        u32 pk = cand ? dv.d : 0u;  // inclusive prefix of the tails' out-degrees
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const u32 y = __shfl_up_sync(0xFFFFFFFFu, pk, o);
-            if (lane >= o) pk += y;
+            const u32 y = __shfl_up_sync(FULL, pk, o);
+            if (lane >= (u32)o) pk += y;
         }
         const u32 rank = __popc(todo & lt_mask);
-        const bool in = cand && (pk >> 16) <= (u32)L::TAB && (pk & 0xFFFFu) <= (u32)L::QCAP &&
-                        rank < (u32)L::GROUP;
-        const u32 gmask = __ballot_sync(0xFFFFFFFFu, in);
+        const bool in = cand && pk <= (u32)L::QCAP && rank < (u32)L::GROUP;
+        const u32 gmask = __ballot_sync(FULL, in);
         todo &= ~gmask;
         const u32 G = __popc(gmask);
-        const u32 last = 31 - __clz(gmask);  // the group's last member holds its totals
-        const u32 tot_pk = __shfl_sync(0xFFFFFFFFu, pk, last);
-        const u32 T = tot_pk >> 16, D = tot_pk & 0xFFFFu;
-        u32 kk = in ? dv.d : 0u;  // inclusive prefix of the members' out-degrees
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const u32 y = __shfl_up_sync(0xFFFFFFFFu, kk, o);
-            if (lane >= o) kk += y;
-        }
-        const u32 K = __shfl_sync(0xFFFFFFFFu, kk, last);
+        const u32 K = __shfl_sync(FULL, pk, 31 - __clz(gmask));
         if (in) {
-            const u32 gi = __popc(gmask & lt_mask);
-            u32* o = own + OW * gi;
-            const u64 ls = list_start(dv);
-            o[0] = (u32)v;
-            o[1] = (((pk >> 16) - tsz) << 5) | lg;
-            o[2] = dv.d;
-            o[3] = kk - dv.d;
-            o[4] = (pk & 0xFFFFu) - deg;
-            o[5] = 0;
-            o[6] = (u32)a;
-            o[7] = (u32)(a >> 32);
-            o[8] = (u32)ls;
-            o[9] = (u32)(ls >> 32);
+            rec[rank] = make_uint4(pk - dv.d, dv.d, 0x9E3779B1u, 0u);
+            o_s[rank] = (OffT)list_group(dv);
+            tot[rank] = 0;
+            vtx[rank] = (u32)v;
         }
-        for (u32 i = lane; i < T; i += 32) keys[i] = EMPTY_KEY;
-        for (u32 i = lane; i < T / 2; i += 32) hitc[i] = 0;
-        for (u32 i = lane; i < 64; i += 32) bins[i] = 0;
+        bins[lane] = 0;
         __syncwarp();
-        // member lane (< G) holds its key and adjacency prefixes: owners of items by start masks
-        const u32 le_mask = lt_mask | (1u << lane);
-        const bool mem = (u32)lane < G;
-        const u32 kst = mem ? own[OW * lane + 3] : 0u, ast = mem ? own[OW * lane + 4] : 0u;
-        // keys of every owner of the group
-        for (u32 q0 = 0; q0 < K; q0 += 32) {
-            const u32 before = __popc(__ballot_sync(0xFFFFFFFFu, mem && kst <= q0));
-            const u32 starts = __reduce_or_sync(0xFFFFFFFFu, start_bit(mem, kst, q0));
-            const u32 q = q0 + lane;
-            if (q >= K) continue;
-            const u32* o = own + OW * segment_of(before, starts, le_mask);
-            const u64 xs = (u64)o[8] | ((u64)o[9] << 32);
-            if (!bucket_insert(keys + (o[1] >> 5), o[1] & 31u, ld_in<CG>(headp + xs + (q - o[3])))) dup = 1;
-        }
-        // adjacency of every owner: queue the lower neighbours' lists (four slots in flight)
-        u32 qn = 0;
-        for (u32 e0 = 0; e0 < D; e0 += 128) {
-            u32 yv[4], gv[4];
+        // this lane's keys (one per row): the tail by start masks, the key, its out-list
+        const bool mem = lane < G;
+        const u32 kst = mem ? rec[lane].x : 0u;
+        u32 w[L::ROWS], gi[L::ROWS], slot[L::ROWS];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const u32 eb = e0 + 32 * u;
-                const u32 before = __popc(__ballot_sync(0xFFFFFFFFu, mem && ast <= eb));
-                const u32 starts = __reduce_or_sync(0xFFFFFFFFu, start_bit(mem, ast, eb));
-                const u32 e = eb + lane;
-                yv[u] = NONE;
-                gv[u] = 0;
-                if (e < D) {
-                    const u32 gi = segment_of(before, starts, le_mask);
-                    const u64 xa = (u64)own[OW * gi + 6] | ((u64)own[OW * gi + 7] << 32);
-                    gv[u] = gi;
-                    yv[u] = ld_in<CG>(head + xa + (e - own[OW * gi + 4]));
-                }
-            }
-            Desc<OffT> dyv[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                dyv[u].start = 0;
-                dyv[u].d = 0;
-                if (yv[u] < n) dyv[u] = ld_desc<CG>(vdesc + yv[u]);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const u32 gi = gv[u], dy = dyv[u].d;
-                const bool sel = yv[u] < n && dy > 0 && key_less(dy, yv[u], own[OW * gi + 2], own[OW * gi]);
-                const u32 ball = __ballot_sync(0xFFFFFFFFu, sel);
-                if (sel) {
-                    const u32 qi = qn + __popc(ball & lt_mask);
-                    q_y[qi] = yv[u];
-                    q_s[qi] = (OffT)list_group(dyv[u]);
-                    q_m[qi] = (gi << 8) | dy;
-                    atomicAdd(&bins[dy], 1u);
-                }
-                qn += __popc(ball);
+        for (int r = 0; r < L::ROWS; ++r) {
+            w[r] = EMPTY_KEY;
+            gi[r] = 0;
+            slot[r] = NO_SLOT;
+            const u32 q0 = 32 * r;
+            if (q0 >= K) continue;
+            const u32 before = __popc(__ballot_sync(FULL, mem && kst <= q0));
+            const u32 starts = __reduce_or_sync(FULL, start_bit(mem, kst, q0));
+            if (q0 + lane < K) {
+                gi[r] = segment_of(before, starts, le_mask);
+                w[r] = ld_in<CG>(headp + 4 * (u64)o_s[gi[r]] + (q0 + lane - rec[gi[r]].x));
             }
         }
-        __syncwarp();
-        // counting sort of the queue by list length (bins 2 lane and 2 lane + 1 in each lane)
+        Desc<OffT> dw[L::ROWS];
+#pragma unroll
+        for (int r = 0; r < L::ROWS; ++r) {
+            dw[r].start = 0;
+            dw[r].d = 0;
+            if (w[r] != EMPTY_KEY) dw[r] = ld_desc<CG>(vdesc + w[r]);
+        }
+        // the tables: a tail whose keys overfill a bucket starts over with another multiplier
+        u32 brute = 0;  // tails without a table
         {
-            const u32 c0 = bins[2 * lane], c1 = bins[2 * lane + 1];
-            u32 x = c0 + c1;
+            u32 need = 0;
+#pragma unroll
+            for (int r = 0; r < L::ROWS; ++r) need |= (w[r] != EMPTY_KEY ? 1u : 0u) << r;
+            for (int attempt = 0;; ++attempt) {
+                u32 failed = 0;
+#pragma unroll
+                for (int r = 0; r < L::ROWS; ++r) {
+                    if (!((need >> r) & 1u)) continue;
+                    const uint4 t = rec[gi[r]];
+                    const u32 at = 2 * (3 * t.x + __umulhi(w[r] * t.z, 3 * t.y));
+                    u32 prev = atomicCAS(&keys[at], EMPTY_KEY, w[r]);
+                    slot[r] = at;
+                    if (prev != EMPTY_KEY && prev != w[r]) {
+                        prev = atomicCAS(&keys[at + 1], EMPTY_KEY, w[r]);
+                        slot[r] = at + 1;
+                        if (prev != EMPTY_KEY && prev != w[r]) {
+                            slot[r] = NO_SLOT;
+                            failed |= 1u << gi[r];
+                        }
+                    }
+                    if (prev == w[r]) dup = 1;
+                }
+                const u32 fmask = __reduce_or_sync(FULL, failed);
+                if (!fmask) break;
+                need = 0;
+#pragma unroll
+                for (int r = 0; r < L::ROWS; ++r) {
+                    if (w[r] == EMPTY_KEY || !((fmask >> gi[r]) & 1u)) continue;
+                    if (slot[r] != NO_SLOT) keys[slot[r]] = EMPTY_KEY;
+                    slot[r] = NO_SLOT;
+                    need |= 1u << r;
+                }
+                if (attempt + 1 == L::MAX_TRIES) {
+                    brute = fmask;
+                    break;
+                }
+                if ((fmask >> lane) & 1u) rec[lane].z = rec[lane].z * 0x2C1B3C6Du + 2u;  // stays odd
+                __syncwarp();
+            }
+        }
+        // the queue: heads with a small out-list, binned by length
+#pragma unroll
+        for (int r = 0; r < L::ROWS; ++r) {
+            const u32 d = dw[r].d;
+            if (d == 0 || d > sd) continue;
+            const u32 q = 32 * r + lane;
+            q_s[q] = (OffT)list_group(dw[r]);
+            q_m[q] = (slot[r] << 11) | (gi[r] << 7) | d;
+            atomicAdd(&bins[(d + 3) >> 2], 1u);
+        }
+        __syncwarp();
+        u32 qn;
+        {
+            // exclusive sums from the longest bin down
+            const u32 c = bins[31 - lane];
+            u32 x = c;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const u32 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-                if (lane >= o) x += y;
+                const u32 y = __shfl_up_sync(FULL, x, o);
+                if (lane >= (u32)o) x += y;
             }
-            bins[2 * lane] = x - c0 - c1;
-            bins[2 * lane + 1] = x - c1;
+            bins[31 - lane] = x - c;
+            qn = __shfl_sync(FULL, x, 31);
         }
         __syncwarp();
-        for (u32 qi = lane; qi < qn; qi += 32) q_ord[atomicAdd(&bins[q_m[qi] & 0xFFu], 1u)] = (unsigned short)qi;
-        __syncwarp();
-        // stream the queued lists, one per lane, longest first
-        for (u32 r = lane; r < qn; r += 32) {
-            const u32 qi = q_ord[qn - 1 - r];
-            const u32 meta = q_m[qi];
-            const u32 gi = meta >> 8, dy = meta & 0xFFu;
-            const u32 tb = own[OW * gi + 1];
-            const u32* tk = keys + (tb >> 5);
-            u32* th = hitc + ((tb >> 5) >> 1);  // table offsets are multiples of 4 slots
-            const u32 tl = tb & 31u;
-            const u64 q0 = (u64)q_s[qi];
-            u32 hits = 0;
-            // one 16-byte group of the list per iteration (groups are padded, so the load stays
-            // inside the list's slots): four groups per iteration, loaded together, measured
-            // slower, the loop body then holding sixteen inlined probes
-            for (u32 g0 = 0; 4 * g0 < dy; ++g0) {
-                const uint4 qv = ld_in<CG>(headp4 + q0 + g0);
-                const u32 e = 4 * g0;
-                hits += bucket_probe16(tk, th, tl, qv.x);
-                if (e + 1 < dy) hits += bucket_probe16(tk, th, tl, qv.y);
-                if (e + 2 < dy) hits += bucket_probe16(tk, th, tl, qv.z);
-                if (e + 3 < dy) hits += bucket_probe16(tk, th, tl, qv.w);
-            }
-            if (hits) {
-                atomicAdd(&cnt[q_y[qi]], (u64)hits);
-                atomicAdd(&own[OW * gi + 5], hits);
-            }
+#pragma unroll
+        for (int r = 0; r < L::ROWS; ++r) {
+            const u32 d = dw[r].d;
+            if (d != 0 && d <= sd) q_ord[atomicAdd(&bins[(d + 3) >> 2], 1u)] = (unsigned short)(32 * r + lane);
         }
         __syncwarp();
-        // flush: every key's hits, then the owners' totals
-        for (u32 i = lane; i < T; i += 32) {
-            const u32 h = read16(hitc, i);
-            if (h) atomicAdd(&cnt[keys[i]], (u64)h);
+        // stream the queued lists, one per lane, longest first; the next 16-byte group of a list is
+        // in flight while the current one is looked up (groups are padded, so the load stays inside
+        // the list's slots)
+        for (u32 i = lane; i < qn; i += 32) {
+            const u32 q = q_ord[i];
+            const u32 m = q_m[q];
+            const u32 g = (m >> 7) & 15u;
+            const uint4* lp = headp4 + (u64)q_s[q];
+            const uint4 t = rec[g];
+            int rem = (int)(m & 127u);
+            u32 found = 0;
+            if ((brute >> g) & 1u) {
+                const u32* lst = reinterpret_cast<const u32*>(lp);
+                const u32* own = headp + 4 * (u64)o_s[g];
+                for (int e = 0; e < rem; ++e) {
+                    const u32 z = ld_in<CG>(lst + e);
+                    for (u32 k = 0; k < t.y; ++k)
+                        if (ld_in<CG>(own + k) == z) {
+                            atomicAdd(&cnt[z], 1ull);
+                            ++found;
+                        }
+                }
+                if (found) atomicAdd(&cnt[ld_in<CG>(own + (q - t.x))], (u64)found);
+            } else {
+                const u32 nb = 3 * t.y, mult = t.z;
+                const uint2* tk = reinterpret_cast<const uint2*>(keys) + 3 * t.x;
+                u32* th = hits + 3 * t.x;
+                uint4 cur = ld_in<CG>(lp);
+                while (true) {
+                    uint4 nxt = cur;
+                    if (rem > 4) nxt = ld_in<CG>(++lp);
+                    const u32 z[4] = {cur.x, cur.y, cur.z, cur.w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const u32 b = __umulhi(z[k] * mult, nb);
+                        const uint2 kk = tk[b];
+                        const bool h0 = kk.x == z[k], h1 = kk.y == z[k];
+                        if ((h0 | h1) & (k < rem)) {
+                            atomicAdd(&th[b], h1 ? 0x10000u : 1u);
+                            ++found;
+                        }
+                    }
+                    rem -= 4;
+                    if (rem <= 0) break;
+                    cur = nxt;
+                }
+                if (found) {
+                    const u32 s = m >> 11;
+                    atomicAdd(&hits[s >> 1], found << ((s & 1u) << 4));  // the edge's head
+                }
+            }
+            if (found) atomicAdd(&tot[g], found);
         }
-        if ((u32)lane < G) {
-            const u32 t = own[OW * lane + 5];
+        __syncwarp();
+        // flush and clear: every key's hits (as the third corner and as the head of its edge), then
+        // the tails' totals
+#pragma unroll
+        for (int r = 0; r < L::ROWS; ++r) {
+            if (slot[r] == NO_SLOT) continue;
+            const u32 h = hits16[slot[r]];
+            keys[slot[r]] = EMPTY_KEY;
+            hits16[slot[r]] = 0;
+            if (h) atomicAdd(&cnt[w[r]], (u64)h);
+        }
+        if (mem) {
+            const u32 t = tot[lane];
             if (t) {
-                atomicAdd(&cnt[own[OW * lane]], (u64)t);
+                atomicAdd(&cnt[vtx[lane]], (u64)t);
                 local_total += t;
             }
         }
@@ -378,20 +415,20 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, const u64* __rest
     }
 }
 
-template <int BLOCK, int SD, typename OffT>
-__global__ void __launch_bounds__(BLOCK, 4) k_count_small(const u64* __restrict__ fo, const u32* __restrict__ head,
-                                                          u64 n, const Desc<OffT>* __restrict__ vdesc,
+template <int BLOCK, typename OffT>
+__global__ void __launch_bounds__(BLOCK, 4) k_count_small(u64 n, u32 vb, const Desc<OffT>* __restrict__ vdesc,
                                                           const u32* __restrict__ headp, u32 sd,
                                                           u64* __restrict__ cnt, u64* __restrict__ partials,
                                                           Control* ctl) {
-    using L = SmallWarpLayout<SD, OffT>;
+    using L = SmallWarpLayout<OffT>;
     constexpr int NW = BLOCK / 32;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ u64 s_red[NW];
     if (ctl->err & DEV_ERR_MASK) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     u32* base = reinterpret_cast<u32*>(smem) + warp * L::PER_WARP;
-    const u64 nbatch = (n + 31) / 32;
+    small_init<OffT>(base);
+    const u64 nbatch = (n + vb - 1) / vb;
     u64 local_total = 0;
     u32 dup = 0;
     while (true) {
@@ -399,7 +436,7 @@ __global__ void __launch_bounds__(BLOCK, 4) k_count_small(const u64* __restrict_
         if (lane == 0) bi = atomicAdd(&ctl->small_next, 1ull);
         bi = __shfl_sync(0xFFFFFFFFu, bi, 0);
         if (bi >= nbatch) break;
-        small_batch<SD, OffT>(base, bi, fo, head, n, vdesc, headp, sd, cnt, local_total, dup);
+        small_batch<OffT>(base, bi, vb, n, vdesc, headp, sd, cnt, local_total, dup);
     }
     if (dup) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
     const u64 bt = block_sum_u64<BLOCK>(local_total, s_red);
@@ -868,7 +905,7 @@ __global__ void __launch_bounds__(256) k_graph_totals(const u64* __restrict__ cn
 // chunk and stream their segment once per chunk).
 template <typename OffT>
 __global__ void k_stats(const u64* __restrict__ fo, const u32* __restrict__ head, u64 n,
-                        const Desc<OffT>* __restrict__ vdesc, const u32* __restrict__ headp, u32 medium_d,
+                        const Desc<OffT>* __restrict__ vdesc, const u32* __restrict__ headp, u32 small_d, u32 medium_d,
                         Control* ctl) {
     if (ctl->err & DEV_ERR_MASK) return;
     const int lane = threadIdx.x & 31;
@@ -884,11 +921,15 @@ __global__ void k_stats(const u64* __restrict__ fo, const u32* __restrict__ head
             const u32 du = load_desc(vdesc + u).d;
             wedge += du;
             isz += (u64)dv.d + du;
+            if (dv.d >= 2 && dv.d <= small_d && du <= small_d) {  // counted at the tail
+                streamed += du;
+                chunked += du;
+            }
         }
         for (u64 e = fo[v] + lane; e < fo[v + 1]; e += 32) {
             const u32 y = head[e];
             const u32 dy = load_desc(vdesc + y).d;
-            if (dy > 0 && key_less(dy, y, dv.d, v)) {
+            if (dy > 0 && dv.d > small_d && key_less(dy, y, dv.d, v)) {
                 streamed += dy;
                 chunked += dy * chunks;
             }
@@ -913,8 +954,7 @@ __global__ void k_stats(const u64* __restrict__ fo, const u32* __restrict__ head
 
 // ---- the serving engine ----------------------------------------------------------------
 
-constexpr int ENGINE_SD = SMALL_D;  // the small-owner layout for any small_outdegree bound
-using EngineSmallL = SmallWarpLayout<ENGINE_SD, u32>;
+using EngineSmallL = SmallWarpLayout<u32>;
 using EngineMediumL = MediumLayout<ENGINE_BLOCK>;
 using EngineLargeL = LargeLayout<ENGINE_BLOCK, LARGE_CAP, u32>;
 constexpr size_t cmax(size_t a, size_t b) { return a > b ? a : b; }
@@ -1074,12 +1114,13 @@ __global__ void __launch_bounds__(ENGINE_BLOCK, 4) k_engine(EngineJob* jobs, u32
         bool timed_out = false;
         if (u < jb->units_small) {
             const u64 nb = (jb->n + 31) / 32;
+            u32* slice = reinterpret_cast<u32*>(smem) + warp * EngineSmallL::PER_WARP;
+            small_init<u32>(slice);  // other kinds of unit use the same shared memory
             for (u32 r = 0; r < ENGINE_REPS; ++r) {
                 const u64 bi = (u * (ENGINE_BLOCK / 32) + warp) * ENGINE_REPS + r;
                 if (bi < nb)
-                    small_batch<ENGINE_SD, u32, true>(reinterpret_cast<u32*>(smem) + warp * EngineSmallL::PER_WARP, bi,
-                                                      jb->fo, jb->head, jb->n, vd, jb->headp, jb->small_d, jb->cnt,
-                                                      unused_total, dup);
+                    small_batch<u32, true>(slice, bi, 32, jb->n, vd, jb->headp, jb->small_d, jb->cnt, unused_total,
+                                           dup);
             }
         } else if (u < jb->units_small + jb->units_medium) {
             const u64 nt = *(volatile unsigned long long*)&ctl->medium_tiles;
@@ -1150,12 +1191,12 @@ template <typename OffT>
 using LargeL = LargeLayout<LARGE_BLOCK, LARGE_CAP, OffT>;
 using MediumL = MediumLayout<MEDIUM_BLOCK>;
 
-template <int SD, typename OffT>
+template <typename OffT>
 int occupancy_small() {
     static int occ = -1;
     if (occ < 0) {
-        auto kern = k_count_small<SMALL_BLOCK, SD, OffT>;
-        const size_t bytes = SmallWarpLayout<SD, OffT>::bytes(SMALL_BLOCK / 32);
+        auto kern = k_count_small<SMALL_BLOCK, OffT>;
+        const size_t bytes = SmallWarpLayout<OffT>::bytes(SMALL_BLOCK / 32);
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         int o = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, SMALL_BLOCK, bytes);
@@ -1190,9 +1231,8 @@ int occupancy_large() {
 }  // namespace
 
 template <typename OffT>
-int count_grid_small(int num_sms, u32 small_d) {
-    return num_sms * (small_d <= (u32)SMALL_D_LOW ? occupancy_small<SMALL_D_LOW, OffT>()
-                                                  : occupancy_small<SMALL_D, OffT>());
+int count_grid_small(int num_sms) {
+    return num_sms * occupancy_small<OffT>();
 }
 template <typename OffT>
 int count_grid_medium(int num_sms) {
@@ -1202,17 +1242,24 @@ template <typename OffT>
 int count_grid_large(int num_sms) {
     return num_sms * occupancy_large<OffT>();
 }
-// Blocks the small-owner kernel is launched with: enough for one vertex batch per warp, at most
-// its resident grid (a small graph does not start hundreds of warps that find no batch).
+// Vertices per batch of the small kernel: 32, or fewer where the graph does not hold a batch of 32
+// for every resident warp (a power of two, at least 4: a warp's serial chain is then shorter).
+static u32 small_batch_vertices(u64 n, int cap) {
+    u32 vb = 32;
+    while (vb > 4 && n < (u64)cap * (SMALL_BLOCK / 32) * vb) vb >>= 1;
+    return vb;
+}
+// Blocks the small kernel is launched with: enough for one vertex batch per warp, at most its
+// resident grid (a small graph does not start hundreds of warps that find no batch).
 int small_grid_launched(u64 n, int cap) {
-    const u64 need = ((n + 31) / 32 + SMALL_BLOCK / 32 - 1) / (SMALL_BLOCK / 32);
+    const u32 vb = small_batch_vertices(n, cap);
+    const u64 need = ((n + vb - 1) / vb + SMALL_BLOCK / 32 - 1) / (SMALL_BLOCK / 32);
     return (int)(need < 1 ? 1 : (need < (u64)cap ? need : (u64)cap));
 }
 
 template <typename OffT>
-int count_grid_auto(int num_sms, u32 small_d) {
-    return count_grid_small<OffT>(num_sms, small_d) + count_grid_medium<OffT>(num_sms) +
-           count_grid_large<OffT>(num_sms);
+int count_grid_auto(int num_sms) {
+    return count_grid_small<OffT>(num_sms) + count_grid_medium<OffT>(num_sms) + count_grid_large<OffT>(num_sms);
 }
 
 template <typename OffT>
@@ -1221,19 +1268,13 @@ cudaError_t launch_count_auto(const u64* fo, const u32* head, u64 n, u64 nnz, co
                               Control* ctl, int num_sms, cudaStream_t st, cudaEvent_t after_small,
                               cudaEvent_t after_large, u32 copy_wait_polls) {
     (void)nnz;
-    const int cap = count_grid_small<OffT>(num_sms, small_d);
+    const int cap = count_grid_small<OffT>(num_sms);
     const int gs = small_grid_launched(n, cap);
     const int gm = count_grid_medium<OffT>(num_sms);
     const int gl = count_grid_large<OffT>(num_sms);
     const auto* vd = reinterpret_cast<const Desc<OffT>*>(vdesc);
-    if (small_d <= (u32)SMALL_D_LOW)
-        k_count_small<SMALL_BLOCK, SMALL_D_LOW, OffT>
-            <<<gs, SMALL_BLOCK, SmallWarpLayout<SMALL_D_LOW, OffT>::bytes(SMALL_BLOCK / 32), st>>>(
-                fo, head, n, vd, headp, small_d, cnt, partials, ctl);
-    else
-        k_count_small<SMALL_BLOCK, SMALL_D, OffT>
-            <<<gs, SMALL_BLOCK, SmallWarpLayout<SMALL_D, OffT>::bytes(SMALL_BLOCK / 32), st>>>(
-                fo, head, n, vd, headp, small_d, cnt, partials, ctl);
+    k_count_small<SMALL_BLOCK, OffT><<<gs, SMALL_BLOCK, SmallWarpLayout<OffT>::bytes(SMALL_BLOCK / 32), st>>>(
+        n, small_batch_vertices(n, cap), vd, headp, small_d, cnt, partials, ctl);
     if (after_small) cudaEventRecord(after_small, st);
     k_count_medium<MEDIUM_BLOCK, OffT>
         <<<gm, MEDIUM_BLOCK, MediumL::bytes, st>>>(fo, head, n, vd, headp, mtiles, seg, cnt, partials + cap, ctl);
@@ -1256,40 +1297,39 @@ void launch_final(const u64* partials, u32 np, u64* total, Control* ctl, cudaStr
 }
 
 template <typename OffT>
-void launch_final_auto(const u64* partials, u64 n, u32 small_d, int num_sms, u64* total, Control* ctl,
-                       cudaStream_t st) {
-    const int cap = count_grid_small<OffT>(num_sms, small_d);
-    k_final<<<1, 1024, 0, st>>>(partials, (u32)count_grid_auto<OffT>(num_sms, small_d), (u32)small_grid_launched(n, cap),
+void launch_final_auto(const u64* partials, u64 n, int num_sms, u64* total, Control* ctl, cudaStream_t st) {
+    const int cap = count_grid_small<OffT>(num_sms);
+    k_final<<<1, 1024, 0, st>>>(partials, (u32)count_grid_auto<OffT>(num_sms), (u32)small_grid_launched(n, cap),
                                 (u32)cap, total, ctl);
 }
 
 template <typename OffT>
-void launch_stats(const u64* fo, const u32* head, u64 n, const void* vdesc, const u32* headp, u32 medium_d,
-                  Control* ctl, int num_sms, cudaStream_t st) {
+void launch_stats(const u64* fo, const u32* head, u64 n, const void* vdesc, const u32* headp, u32 small_d,
+                  u32 medium_d, Control* ctl, int num_sms, cudaStream_t st) {
     if (n == 0) return;
     k_stats<OffT><<<num_sms * 8, 256, 0, st>>>(fo, head, n, reinterpret_cast<const Desc<OffT>*>(vdesc), headp,
-                                               medium_d, ctl);
+                                               small_d, medium_d, ctl);
 }
 
-template void launch_final_auto<u32>(const u64*, u64, u32, int, u64*, Control*, cudaStream_t);
-template void launch_final_auto<u64>(const u64*, u64, u32, int, u64*, Control*, cudaStream_t);
-template int count_grid_small<u32>(int, u32);
-template int count_grid_small<u64>(int, u32);
+template void launch_final_auto<u32>(const u64*, u64, int, u64*, Control*, cudaStream_t);
+template void launch_final_auto<u64>(const u64*, u64, int, u64*, Control*, cudaStream_t);
+template int count_grid_small<u32>(int);
+template int count_grid_small<u64>(int);
 template int count_grid_large<u32>(int);
 template int count_grid_large<u64>(int);
 template int count_grid_medium<u32>(int);
 template int count_grid_medium<u64>(int);
-template int count_grid_auto<u32>(int, u32);
-template int count_grid_auto<u64>(int, u32);
+template int count_grid_auto<u32>(int);
+template int count_grid_auto<u64>(int);
 template cudaError_t launch_count_auto<u32>(const u64*, const u32*, u64, u64, const void*, const u32*, const uint2*,
                                             const uint2*, u32, u32, u64*, u64*, Control*, int, cudaStream_t,
                                             cudaEvent_t, cudaEvent_t, u32);
 template cudaError_t launch_count_auto<u64>(const u64*, const u32*, u64, u64, const void*, const u32*, const uint2*,
                                             const uint2*, u32, u32, u64*, u64*, Control*, int, cudaStream_t,
                                             cudaEvent_t, cudaEvent_t, u32);
-template void launch_stats<u32>(const u64*, const u32*, u64, const void*, const u32*, u32, Control*, int,
+template void launch_stats<u32>(const u64*, const u32*, u64, const void*, const u32*, u32, u32, Control*, int,
                                 cudaStream_t);
-template void launch_stats<u64>(const u64*, const u32*, u64, const void*, const u32*, u32, Control*, int,
+template void launch_stats<u64>(const u64*, const u32*, u64, const void*, const u32*, u32, u32, Control*, int,
                                 cudaStream_t);
 
 }  // namespace ktri

@@ -18,7 +18,7 @@ namespace ktri {
 // Resolved options (defaults filled in).
 struct Options {
     int32_t method = KTRI_METHOD_AUTO;
-    uint32_t small_outdegree = 32;   // owner bins and tile segment of the AUTO kernels
+    uint32_t small_outdegree = 48;   // owner bins and tile segment of the AUTO kernels
     uint32_t medium_outdegree = 256;
     uint32_t segment = 1024;
     bool collect_stats = false;

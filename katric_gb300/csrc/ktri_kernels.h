@@ -15,9 +15,7 @@ using u64 = unsigned long long;
 constexpr int ORIENT_BLOCK = 256;   // 8 warps, one merge-path tile each
 constexpr int ORIENT_IPT = 8;       // slots per lane of a tile: tiles of 256 diagonals
 constexpr int SMALL_BLOCK = 256;
-constexpr int SMALL_D = 48;          // largest out-degree bound of the small-owner kernel's owners
-constexpr int SMALL_D_LOW = 32;      // bounds up to this run the small-owner kernel's instantiation for
-                                     // 32, the others the one for SMALL_D (more table and bin space)
+constexpr int SMALL_D = 48;          // largest (and default) out-degree bound of the small kernel's edges
 constexpr int MEDIUM_D = 256;        // out-degree bound of the warp-per-tile kernel's owners
 constexpr int MEDIUM_BLOCK = 256;
 constexpr int LARGE_BLOCK = 256;
@@ -26,8 +24,6 @@ constexpr u32 LARGE_SEG = 1024;      // most adjacency slots per (owner, segment
 constexpr u32 MIN_SEG = 64;          // fewest adjacency slots per (owner, segment) tile
 constexpr int LONG_LIST = 16;        // lists longer than this are streamed by a whole warp
 constexpr u32 COPY_WAIT_POLLS = 1u << 22;  // polls of a bounded wait for a bulk copy into shared memory
-constexpr u32 SMALL_WARP_DEG = 256;  // the small-owner kernel takes owners up to this degree; owners of
-                                     // larger degree (and small out-degree) go to the medium kernel's tiles
 
 // Merge-path tile boundaries are tabulated once per call at this granularity: entry k holds
 // the vertex where diagonal k * TILE_BASE crosses the path.  One warp orients one base tile.
@@ -35,10 +31,10 @@ constexpr u64 TILE_BASE = 32ull * ORIENT_IPT;
 inline u64 base_tiles(u64 n, u64 nnz) { return (n + nnz + TILE_BASE - 1) / TILE_BASE; }
 // Each base tile records at most one split list (the one that starts in it and ends past it).
 inline u64 spanning_capacity(u64 n, u64 nnz) { return base_tiles(n, nnz) + 2; }
-// Owners above small_d hold more than small_d adjacency entries each, and owners routed to the
-// tiles for their degree more than SMALL_WARP_DEG; every owner has at most deg / seg + 1 tiles.
+// Owners above small_d hold more than small_d adjacency entries each; every owner has at most
+// deg / seg + 1 tiles.
 inline u64 large_tile_capacity(u64 n, u64 nnz, u32 small_d, u32 seg) {
-    u64 owners = nnz / ((u64)small_d + 1) + nnz / ((u64)SMALL_WARP_DEG + 1) + 1;
+    u64 owners = nnz / ((u64)small_d + 1) + 1;
     if (owners > n) owners = n;
     return owners + nnz / seg + 1;
 }
@@ -85,11 +81,9 @@ void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* de
                    u64 tile_end = ~0ull);
 // Owner tiles: medium owners' tiles are written to mtiles, large owners' to ltiles (each
 // array holds large_tile_capacity entries).
-// small_deg_max: owners up to small_d whose degree exceeds it get medium tiles too (the
-// small-owner kernel's bound, SMALL_WARP_DEG).
 template <typename OffT>
 void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, uint2* mtiles, uint2* ltiles, u32 small_d,
-                 u32 medium_d, u32 seg, u32 small_deg_max, Control* ctl, int num_sms, cudaStream_t st);
+                 u32 medium_d, u32 seg, Control* ctl, int num_sms, cudaStream_t st);
 
 // Owner tiles reordered (*count tiles on the device) by a counting sort on a 12-bit key:
 // TILE_BY_VERTEX, the first vertex each segment streams (tiles that run together then stream
@@ -106,24 +100,23 @@ void launch_order_tiles(const u64* fo, const u32* head, const u32* dplus, u64 n,
 
 // Owner-side hash counting (KTRI_METHOD_AUTO).  partials needs small_grid + large_grid entries.
 template <typename OffT>
-int count_grid_small(int num_sms, u32 small_d);
+int count_grid_small(int num_sms);
 template <typename OffT>
 int count_grid_medium(int num_sms);
 template <typename OffT>
 int count_grid_large(int num_sms);
 template <typename OffT>
-int count_grid_auto(int num_sms, u32 small_d);  // small + medium + large, for this small-owner bound
+int count_grid_auto(int num_sms);  // small + medium + large
 template <typename OffT>
 cudaError_t launch_count_auto(const u64* fo, const u32* head, u64 n, u64 nnz, const void* vdesc, const u32* headp,
                               const uint2* mtiles, const uint2* ltiles, u32 small_d, u32 seg, u64* cnt, u64* partials,
                               Control* ctl, int num_sms, cudaStream_t st, cudaEvent_t after_small,
                               cudaEvent_t after_large, u32 copy_wait_polls = COPY_WAIT_POLLS);
 void launch_final(const u64* partials, u32 np, u64* total, Control* ctl, cudaStream_t st);
-// The total of an AUTO count (the small-owner kernel's grid depends on n).
+// The total of an AUTO count (the small kernel's grid depends on n).
 int small_grid_launched(u64 n, int cap);
 template <typename OffT>
-void launch_final_auto(const u64* partials, u64 n, u32 small_d, int num_sms, u64* total, Control* ctl,
-                       cudaStream_t st);
+void launch_final_auto(const u64* partials, u64 n, int num_sms, u64* total, Control* ctl, cudaStream_t st);
 
 // ---- the serving engine ------------------------------------------------------------------
 // A prepared batch (orientation, descriptors and owner tiles done on its slot's stream) is
@@ -199,8 +192,8 @@ void launch_graph_totals(const u64* cnt, const u64* graph_first, u64 num_graphs,
 // Work counters of the reference (wedge_checks, intersection_size_local) and of the AUTO
 // kernels, accumulated into the control block.
 template <typename OffT>
-void launch_stats(const u64* fo, const u32* head, u64 n, const void* vdesc, const u32* headp, u32 medium_d,
-                  Control* ctl, int num_sms, cudaStream_t st);
+void launch_stats(const u64* fo, const u32* head, u64 n, const void* vdesc, const u32* headp, u32 small_d,
+                  u32 medium_d, Control* ctl, int num_sms, cudaStream_t st);
 
 // Sorted-list strategies (merge, binary search, binary, hybrid): sort out-lists by id, then
 // one warp per oriented edge.

@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(BLOCK) k_orient(const u64* __restrict__ fo, co
 template <typename OffT>
 __global__ void k_desc(const u64* __restrict__ fo, u64 n, const u32* __restrict__ dplus, Desc<OffT>* __restrict__ vdesc,
                        uint2* __restrict__ mtiles, uint2* __restrict__ ltiles, u32 small_d, u32 medium_d, u32 seg,
-                       u32 small_deg_max, Control* ctl) {
+                       Control* ctl) {
     if (ctl->err & DEV_ERR_MASK) return;
     const int lane = threadIdx.x & 31;
     const u64 warp_global = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -239,7 +239,7 @@ __global__ void k_desc(const u64* __restrict__ fo, u64 n, const u32* __restrict_
             if constexpr (sizeof(OffT) == 8) ds.pad = 0;
             vdesc[v] = ds;
             // no tiles at all without tile arrays (the reference strategies pass none)
-            const bool tiled = mtiles && ltiles && (d > small_d || (d > 0 && b - a > small_deg_max));
+            const bool tiled = mtiles && ltiles && d > small_d;
             const u32 nt = tiled ? (u32)((b - a + seg - 1) / seg) : 0u;
             if (d > medium_d) nl = nt;
             else nm = nt;
@@ -449,18 +449,17 @@ void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* de
 
 template <typename OffT>
 void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, uint2* mtiles, uint2* ltiles, u32 small_d,
-                 u32 medium_d, u32 seg, u32 small_deg_max, Control* ctl, int num_sms, cudaStream_t st) {
+                 u32 medium_d, u32 seg, Control* ctl, int num_sms, cudaStream_t st) {
     if (n == 0) return;
     u64 blocks = (n + 255) / 256;
     u64 cap = (u64)num_sms * 8;
     k_desc<OffT><<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(
-        fo, n, dplus, reinterpret_cast<Desc<OffT>*>(vdesc), mtiles, ltiles, small_d, medium_d, seg, small_deg_max,
-        ctl);
+        fo, n, dplus, reinterpret_cast<Desc<OffT>*>(vdesc), mtiles, ltiles, small_d, medium_d, seg, ctl);
 }
 
-template void launch_desc<u32>(const u64*, u64, const u32*, void*, uint2*, uint2*, u32, u32, u32, u32, Control*,
-                               int, cudaStream_t);
-template void launch_desc<u64>(const u64*, u64, const u32*, void*, uint2*, uint2*, u32, u32, u32, u32, Control*,
-                               int, cudaStream_t);
+template void launch_desc<u32>(const u64*, u64, const u32*, void*, uint2*, uint2*, u32, u32, u32, Control*, int,
+                               cudaStream_t);
+template void launch_desc<u64>(const u64*, u64, const u32*, void*, uint2*, uint2*, u32, u32, u32, Control*, int,
+                               cudaStream_t);
 
 }  // namespace ktri

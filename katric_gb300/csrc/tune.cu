@@ -4,7 +4,7 @@
 // per shape class in a JSON-lines cache file, so later runs on inputs of the same class read
 // it back without timing.
 //
-// Search: the library default (KTRI_METHOD_AUTO with bins 32 / 256, segment 1024) is timed
+// Search: the library default (KTRI_METHOD_AUTO with bins 48 / 256, segment 1024) is timed
 // first; then the reference's strategies (hybrid first; merge, binary search and binary only
 // when hybrid comes within 1.5x of the best); then, if an AUTO configuration is best, one pass
 // of coordinate descent over small_outdegree, medium_outdegree and segment, and last the tile
@@ -53,7 +53,7 @@ int floor_log2(u64 x) {
 
 struct Cand {
     int32_t method = KTRI_METHOD_AUTO;
-    uint32_t small = 32, medium = 256, seg = 1024, order = 0;
+    uint32_t small = 48, medium = 256, seg = 1024, order = 0;
     bool operator==(const Cand& o) const {
         return method == o.method && small == o.small && medium == o.medium && seg == o.seg && order == o.order;
     }
