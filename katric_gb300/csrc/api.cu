@@ -15,6 +15,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "ktri.h"
@@ -52,6 +53,7 @@ struct ktri_ctx {
     bool have_events = false;
     int32_t last_method = KTRI_METHOD_AUTO;
     bool last_collect = false;
+    bool hubs = true;          // counts may split their out-lists (more workspace than ktri_workspace_bytes)
 };
 
 namespace {
@@ -63,8 +65,10 @@ struct Layout {
     size_t ctl = 0, deg = 0, dplus = 0, tile_i0 = 0, vdesc = 0, headp = 0, ltiles = 0, thist = 0, tkeys = 0,
            spanning = 0,
            partials = 0, cnt = 0,
-           total = 0, mid = 0, big = 0, scratch = 0, in_fo = 0, in_head = 0, bytes = 0;
+           total = 0, mid = 0, big = 0, scratch = 0, in_fo = 0, in_head = 0, hub_bins = 0, hub_tmp = 0,
+           hub_ids = 0, hub_lists = 0, bytes = 0;
     bool wide = false;
+    bool hub = false;  // split out-lists (AUTO with 32-bit descriptors)
     u64 scratch_per_block = 0;
     int big_grid = 0;
     u32 npartials = 0;
@@ -77,9 +81,11 @@ u64 isqrt_ceil(u64 x) {
     return r;
 }
 
+constexpr size_t HUB_WORKSPACE_BYTES = size_t(64) << 20;
+
 // Workspace of one count.  num_sms = 0 sizes the grids for the largest supported part.
 Layout make_layout(u64 n, u64 nnz, int32_t method, int num_sms, bool with_inputs, bool internal_cnt,
-                   bool force_wide = false, u32 small_d = 32, u32 seg = ktri::LARGE_SEG) {
+                   bool force_wide = false, u32 small_d = 32, u32 seg = ktri::LARGE_SEG, bool hub = false) {
     Layout L;
     const u64 cap = ktri::oriented_capacity(n, nnz);
     L.wide = force_wide || cap > ktri::NARROW_CAPACITY;
@@ -122,6 +128,16 @@ Layout make_layout(u64 n, u64 nnz, int32_t method, int num_sms, bool with_inputs
     if (with_inputs) {
         L.in_fo = take(sizeof(u64) * (n + 1));
         L.in_head = take(sizeof(u32) * (nnz + 1));
+    }
+    // Hubs pay from the size on where the lists leave L1 and the choice of hubs (three short
+    // launches) is small; every graph the no-allocation array holds stays below the line.
+    if (hub && method == KTRI_METHOD_AUTO && !L.wide && off > HUB_WORKSPACE_BYTES && n < ktri::HUB_MAX_N &&
+        nnz <= ktri::HUB_MAX_NNZ) {
+        L.hub = true;
+        L.hub_bins = take(sizeof(u32) * ktri::hub_bins_words());
+        L.hub_tmp = take(sizeof(uint2) * ktri::HUB_H);
+        L.hub_ids = take(sizeof(u32) * ktri::HUB_H);
+        L.hub_lists = take(sizeof(ktri::u16) * ktri::hub_capacity(n, nnz));
     }
     L.bytes = off;
     return L;
@@ -207,6 +223,31 @@ int ensure_ws(ktri_ctx* ctx, size_t bytes) {
     }
     ctx->ws_bytes = grow;
     return KTRI_OK;
+}
+
+// The layout of a count on a context, with extra bytes behind it: split out-lists (hubs) where the
+// larger workspace is within the memory budget and, when the workspace has to grow, within what
+// the device has free; otherwise the plain one, which any accepted call can have.
+template <class Extra>
+Layout pick_layout(ktri_ctx* ctx, u64 n, u64 nnz, const ktri::Options& opt, bool with_inputs, bool internal_cnt,
+                   Extra extra) {
+    const Layout L = make_layout(n, nnz, opt.method, ctx->num_sms, with_inputs, internal_cnt, opt.force_wide,
+                                 opt.small_outdegree, opt.segment, ctx->hubs);
+    if (L.hub) {
+        const size_t bytes = extra(L.bytes);
+        bool fits = !ctx->budget || bytes <= ctx->budget;
+        if (fits && bytes > ctx->ws_bytes) {
+            size_t free_bytes = 0, total_bytes = 0;
+            fits = cudaMemGetInfo(&free_bytes, &total_bytes) == cudaSuccess && bytes <= free_bytes + ctx->ws_bytes;
+        }
+        if (!fits)
+            return make_layout(n, nnz, opt.method, ctx->num_sms, with_inputs, internal_cnt, opt.force_wide,
+                               opt.small_outdegree, opt.segment, false);
+    }
+    return L;
+}
+Layout pick_layout(ktri_ctx* ctx, u64 n, u64 nnz, const ktri::Options& opt, bool with_inputs, bool internal_cnt) {
+    return pick_layout(ctx, n, nnz, opt, with_inputs, internal_cnt, [](size_t b) { return b; });
 }
 
 struct DeviceGuard {
@@ -323,7 +364,7 @@ u32 first_wait_polls(uint32_t opt) {
 
 // The launch sequence of one count on the workspace at base.  ctx may be NULL (the
 // no-allocation entry point): errors then carry no message and no events are recorded.
-template <typename OffT>
+template <typename OffT, bool HUB>
 int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const u64* fo, const u32* head, u64 n,
                      u64 nnz, u64* d_total, u64* cnt, const ktri::Options& opt, cudaStream_t st, bool sort_all,
                      bool events, ktri::TriangleSink sink = ktri::TriangleSink{}, const HeadChunks* chunks = nullptr,
@@ -337,6 +378,13 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     auto* spanning = reinterpret_cast<u32*>(base + L.spanning);
     auto* partials = reinterpret_cast<u64*>(base + L.partials);
     auto* tile_i0 = reinterpret_cast<u32*>(base + L.tile_i0);
+    ktri::HubState hub;
+    if (HUB) {
+        hub.bins = reinterpret_cast<u32*>(base + L.hub_bins);
+        hub.tmp = reinterpret_cast<uint2*>(base + L.hub_tmp);
+        hub.ids = reinterpret_cast<u32*>(base + L.hub_ids);
+        hub.lists = reinterpret_cast<ktri::u16*>(base + L.hub_lists);
+    }
 
     // an error a caller's own failed runtime call left in this thread must not be taken for a
     // failed launch of ours below (errors of kernels that faulted are sticky and stay visible)
@@ -344,9 +392,9 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     KTRI_CK(ctx, cudaMemsetAsync(ctl, 0, sizeof(Control), st));
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[0], st));
     const bool autom = opt.method == KTRI_METHOD_AUTO && !sort_all;
-    ktri::launch_prep(fo, n, nnz, deg, dplus, cnt, tile_i0, ctl, sms, st);
+    ktri::launch_prep(fo, n, nnz, deg, dplus, cnt, tile_i0, hub, ctl, sms, st);
     if (!chunks) {
-        ktri::launch_orient(fo, head, n, nnz, deg, tile_i0, headp, dplus, spanning, ctl, st);
+        ktri::launch_orient(fo, head, n, nnz, deg, tile_i0, headp, hub, dplus, spanning, ctl, st);
     } else {
         // tile t reads slots below (t + 1) * ORIENT_TILE + 1: launch each tile once its slots are in
         u64 done = 0;
@@ -355,7 +403,7 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
             const u64 upto = c + 1 == chunks->count ? ktri::orient_tiles(n, nnz)
                                                     : (chunks->ends[c] - 1) / ktri::ORIENT_TILE;
             if (upto > done) {
-                ktri::launch_orient(fo, head, n, nnz, deg, tile_i0, headp, dplus, spanning, ctl, st, done, upto);
+                ktri::launch_orient(fo, head, n, nnz, deg, tile_i0, headp, hub, dplus, spanning, ctl, st, done, upto);
                 done = upto;
             }
         }
@@ -363,7 +411,7 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     auto* mtiles = autom ? reinterpret_cast<uint2*>(base + L.ltiles) : nullptr;
     const u64 tcap = ktri::large_tile_capacity(n, nnz, opt.small_outdegree, opt.segment);
     auto* ltiles = autom ? mtiles + tcap : nullptr;
-    ktri::launch_desc<OffT>(fo, n, dplus, vdesc, mtiles, ltiles, autom ? opt.small_outdegree : 0xFFFFFFFFu,
+    ktri::launch_desc<OffT, HUB>(fo, n, dplus, vdesc, hub, mtiles, ltiles, autom ? opt.small_outdegree : 0xFFFFFFFFu,
                             opt.medium_outdegree, opt.segment, ctl, sms, st);
     // Tile orders (large tiles by the vertex range they stream, for L2 reuse; medium tiles
     // longest owner first, so the warps' last tiles are short).  Below 2^20 adjacency entries
@@ -377,10 +425,10 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
         const bool by_cost = opt.tile_order == KTRI_TILE_ORDER_COST;
         auto* keys = reinterpret_cast<u32*>(base + L.tkeys);
         ktri::launch_order_tiles(fo, head, dplus, n, ltiles, &ctl->large_tiles, opt.segment,
-                                 by_cost ? ktri::TILE_BY_COST : ktri::TILE_BY_VERTEX, keys,
+                                 by_cost ? ktri::TILE_BY_COST : ktri::TILE_BY_VERTEX, HUB, keys,
                                  reinterpret_cast<u32*>(base + L.thist), lrun, ctl, sms, st);
         ktri::launch_order_tiles(fo, head, dplus, n, mtiles, &ctl->medium_tiles, opt.segment,
-                                 by_cost ? ktri::TILE_BY_COST : ktri::TILE_BY_DEGREE, keys,
+                                 by_cost ? ktri::TILE_BY_COST : ktri::TILE_BY_DEGREE, HUB, keys,
                                  reinterpret_cast<u32*>(base + L.thist), mrun, ctl, sms, st);
     }
     if (!autom) {
@@ -390,7 +438,7 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     }
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[1], st));
     if (opt.collect_stats)
-        ktri::launch_stats<OffT>(fo, head, n, vdesc, headp, opt.small_outdegree,
+        ktri::launch_stats<OffT, HUB>(fo, head, n, vdesc, headp, hub, opt.small_outdegree,
                                  autom ? opt.medium_outdegree : 0xFFFFFFFFu, ctl, sms, st);
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[2], st));
     if (sort_all) {
@@ -400,11 +448,11 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
         ktri::launch_publish(publish->job, publish->seq, fo, head, n, vdesc, headp, mrun, lrun, cnt, ctl,
                              opt.small_outdegree, opt.segment, publish->done_word, st);
     } else if (autom) {
-        KTRI_CK(ctx, ktri::launch_count_auto<OffT>(fo, head, n, nnz, vdesc, headp, mrun, lrun, opt.small_outdegree,
-                                                   opt.segment, cnt, partials, ctl, sms, st,
-                                                   events ? ctx->ev[4] : nullptr, events ? ctx->ev[5] : nullptr,
-                                                   first_wait_polls(opt.copy_wait_polls)));
-        ktri::launch_final_auto<OffT>(partials, n, sms, d_total, ctl, st);
+        const cudaError_t e = ktri::launch_count_auto<OffT, HUB>(
+            fo, head, n, nnz, vdesc, headp, hub, mrun, lrun, opt.small_outdegree, opt.segment, cnt, partials, ctl, sms,
+            st, events ? ctx->ev[4] : nullptr, events ? ctx->ev[5] : nullptr, first_wait_polls(opt.copy_wait_polls));
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "launch of the counting kernels");
+        ktri::launch_final_auto<OffT, HUB>(partials, n, sms, d_total, ctl, st);
     } else {
         const int grid = ktri::count_grid_edges(sms);
         ktri::launch_count_edges<OffT>(n, vdesc, headp, opt.method, opt.binary_cutoff, opt.hybrid_scale, cnt, partials,
@@ -416,14 +464,21 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     return KTRI_OK;
 }
 
+// enqueue_pipeline for the layout's kind of descriptors and lists.
+template <class... Args>
+int enqueue_layout(ktri_ctx* ctx, int sms, char* base, const Layout& L, Args&&... args) {
+    if (L.wide) return enqueue_pipeline<u64, false>(ctx, sms, base, L, std::forward<Args>(args)...);
+    if (L.hub) return enqueue_pipeline<u32, true>(ctx, sms, base, L, std::forward<Args>(args)...);
+    return enqueue_pipeline<u32, false>(ctx, sms, base, L, std::forward<Args>(args)...);
+}
+
 // Enqueue a count on the context's workspace and remember it for ktri_ctx_check / stats.
-template <typename OffT>
 int run_pipeline(ktri_ctx* ctx, const Layout& L, const u64* fo, const u32* head, u64 n, u64 nnz, u64* d_total,
                  u64* cnt, const ktri::Options& opt, cudaStream_t st, bool sort_all,
                  ktri::TriangleSink sink = ktri::TriangleSink{}, const HeadChunks* chunks = nullptr) {
     char* base = static_cast<char*>(ctx->ws);
-    const int rc = enqueue_pipeline<OffT>(ctx, ctx->num_sms, base, L, fo, head, n, nnz, d_total, cnt, opt, st, sort_all,
-                                          true, sink, chunks);
+    const int rc =
+        enqueue_layout(ctx, ctx->num_sms, base, L, fo, head, n, nnz, d_total, cnt, opt, st, sort_all, true, sink, chunks);
     if (rc) return rc;
     ctx->ctl = reinterpret_cast<Control*>(base + L.ctl);
     ctx->last_stream = st;
@@ -589,12 +644,10 @@ int noalloc_scratch(int device, void** out) {
 // The AUTO pipeline of ktri_count_csr_device (the same launch sequence, default options) on
 // the fixed scratch array.  enqueue_pipeline zeroes the control block; k_prep zeroes the
 // out-degrees and per-vertex counts; every other region is fully written before it is read.
-template <typename OffT>
 int run_noalloc(char* base, const Layout& L, const u64* fo, const u32* head, u64 n, u64 nnz, u64* d_total, u64* cnt,
                 int sms, cudaStream_t st) {
     const ktri::Options opt;  // AUTO, default owner bins and segment (the layout is sized for them)
-    if (enqueue_pipeline<OffT>(nullptr, sms, base, L, fo, head, n, nnz, d_total, cnt, opt, st, false, false) !=
-        KTRI_OK)
+    if (enqueue_layout(nullptr, sms, base, L, fo, head, n, nnz, d_total, cnt, opt, st, false, false) != KTRI_OK)
         return KTRI_ERR_CUDA;
     auto* ctl = reinterpret_cast<Control*>(base + L.ctl);
     u32 herr = 0;
@@ -607,6 +660,8 @@ int run_noalloc(char* base, const Layout& L, const u64* fo, const u32* head, u64
 }  // namespace
 
 int ktri::ctx_device(const ktri_ctx* ctx) { return ctx->device; }
+
+void ktri::ctx_plain_lists(ktri_ctx* ctx) { ctx->hubs = false; }
 
 int ktri::ctx_num_sms(const ktri_ctx* ctx) { return ctx->num_sms; }
 
@@ -630,7 +685,7 @@ int ktri::engine_prepare_batch(ktri_ctx* ctx, const uint64_t* d_first_out, const
     pub.job = job;
     pub.seq = seq;
     pub.done_word = done_word;
-    rc = enqueue_pipeline<u32>(ctx, ctx->num_sms, base, L, reinterpret_cast<const u64*>(d_first_out), d_head, n_total,
+    rc = enqueue_pipeline<u32, false>(ctx, ctx->num_sms, base, L, reinterpret_cast<const u64*>(d_first_out), d_head, n_total,
                                nnz_total, reinterpret_cast<u64*>(base + L.total), reinterpret_cast<u64*>(d_per_vertex),
                                opt, st, false, false, ktri::TriangleSink{}, nullptr, &pub);
     if (rc) return rc;
@@ -749,16 +804,14 @@ int ktri_count_csr_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint
         ctx->stats = ktri_run_stats{};
         return KTRI_OK;
     }
-    const Layout L = make_layout(n, nnz, opt.method, ctx->num_sms, false, d_per_vertex == nullptr,
-                                 opt.force_wide, opt.small_outdegree, opt.segment);
+    const Layout L = pick_layout(ctx, n, nnz, opt, false, d_per_vertex == nullptr);
     rc = ensure_ws(ctx, L.bytes);
     if (rc) return rc;
     u64* cnt = d_per_vertex ? reinterpret_cast<u64*>(d_per_vertex)
                             : reinterpret_cast<u64*>(static_cast<char*>(ctx->ws) + L.cnt);
     auto* fo = reinterpret_cast<const u64*>(d_first_out);
     auto* tot = reinterpret_cast<u64*>(d_total);
-    if (L.wide) return run_pipeline<u64>(ctx, L, fo, d_head, n, nnz, tot, cnt, opt, st, false);
-    return run_pipeline<u32>(ctx, L, fo, d_head, n, nnz, tot, cnt, opt, st, false);
+    return run_pipeline(ctx, L, fo, d_head, n, nnz, tot, cnt, opt, st, false);
 }
 
 int ktri_count_csr_device_noalloc(const uint64_t* d_first_out, const uint32_t* d_head, uint64_t n, uint64_t nnz,
@@ -791,8 +844,7 @@ int ktri_count_csr_device_noalloc(const uint64_t* d_first_out, const uint32_t* d
     auto* fo = reinterpret_cast<const u64*>(d_first_out);
     auto* tot = reinterpret_cast<u64*>(d_total);
     auto* cnt = reinterpret_cast<u64*>(d_per_vertex);
-    if (L.wide) return run_noalloc<u64>(base, L, fo, d_head, n, nnz, tot, cnt, sms, st);
-    return run_noalloc<u32>(base, L, fo, d_head, n, nnz, tot, cnt, sms, st);
+    return run_noalloc(base, L, fo, d_head, n, nnz, tot, cnt, sms, st);
 }
 
 int ktri_count_csr_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t* head, uint64_t n, uint64_t nnz,
@@ -809,8 +861,7 @@ int ktri_count_csr_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t*
     }
     if (first_out[0] != 0 || first_out[n] != nnz)
         return set_error(ctx, KTRI_ERR_INVALID_CSR, "first_out[0] must be 0 and first_out[n] must equal nnz");
-    const Layout L = make_layout(n, nnz, opt.method, ctx->num_sms, true, true,
-                                 opt.force_wide, opt.small_outdegree, opt.segment);
+    const Layout L = pick_layout(ctx, n, nnz, opt, true, true);
     rc = ensure_ws(ctx, L.bytes);
     if (rc) return rc;
     char* base = static_cast<char*>(ctx->ws);
@@ -849,10 +900,7 @@ int ktri_count_csr_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t*
         if (nnz) KTRI_CK(ctx, copy_host(ctx, d_head, head, head_bytes, true, st));
         KTRI_CK(ctx, cudaEventRecord(ctx->ev_io[1], st));
     }
-    rc = L.wide ? run_pipeline<u64>(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, false, {},
-                                    chunks.count ? &chunks : nullptr)
-                : run_pipeline<u32>(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, false, {},
-                                    chunks.count ? &chunks : nullptr);
+    rc = run_pipeline(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, false, {}, chunks.count ? &chunks : nullptr);
     if (rc) return rc;
     KTRI_CK(ctx, cudaEventRecord(ctx->ev_io[2], st));
     KTRI_CK(ctx, copy_host(ctx, total_out, d_total, sizeof(u64), false, st));
@@ -943,8 +991,7 @@ int ktri_count_binary_file(ktri_ctx* ctx, const char* stem, uint64_t* total_out,
         *total_out = 0;
         return cleanup(nnz ? set_error(ctx, KTRI_ERR_INVALID_CSR, "edges without vertices") : KTRI_OK);
     }
-    Layout L = make_layout(n, nnz, opt.method, ctx->num_sms, true, true, opt.force_wide, opt.small_outdegree,
-                           opt.segment);
+    Layout L = pick_layout(ctx, n, nnz, opt, true, true, [&](size_t b) { return align_up(b + 2 * chunk_bytes); });
     // two device staging chunks for u64 ids follow the count's workspace
     const size_t x_stage = L.bytes;
     L.bytes = align_up(x_stage + 2 * chunk_bytes);
@@ -1001,8 +1048,7 @@ int ktri_count_binary_file(ktri_ctx* ctx, const char* stem, uint64_t* total_out,
     rc = pump(fhd, 8 * nnz, reinterpret_cast<char*>(d_head), true);
     if (rc) return cleanup(rc);
     KTRI_CK(ctx, cudaGetLastError());
-    rc = L.wide ? run_pipeline<u64>(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, false)
-                : run_pipeline<u32>(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, false);
+    rc = run_pipeline(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, false);
     if (rc) return cleanup(rc);
     KTRI_CK(ctx, copy_host(ctx, total_out, d_total, sizeof(u64), false, st));
     bool staged = false;
@@ -1134,10 +1180,7 @@ int ktri_partition_cost(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t
     KTRI_CK(ctx, cudaMemcpyAsync(d_fo, first_out, 8 * (n + 1), cudaMemcpyHostToDevice, st));
     if (nnz) KTRI_CK(ctx, cudaMemcpyAsync(d_head, head, 4 * nnz, cudaMemcpyHostToDevice, st));
     // degrees and out-degrees come from the orientation stage of the pipeline
-    rc = L.wide ? run_pipeline<u64>(ctx, L, d_fo, d_head, n, nnz, reinterpret_cast<u64*>(base + L.total),
-                                    reinterpret_cast<u64*>(base + L.cnt), opt, st, true)
-                : run_pipeline<u32>(ctx, L, d_fo, d_head, n, nnz, reinterpret_cast<u64*>(base + L.total),
-                                    reinterpret_cast<u64*>(base + L.cnt), opt, st, true);
+    rc = run_pipeline(ctx, L, d_fo, d_head, n, nnz, reinterpret_cast<u64*>(base + L.total), reinterpret_cast<u64*>(base + L.cnt), opt, st, true);
     if (rc) return rc;
     ktri::launch_cost_partition(d_fo, d_head, n, reinterpret_cast<const u32*>(base + L.deg),
                                 reinterpret_cast<const u32*>(base + L.dplus), cost_function, parts, d_cost,
@@ -1189,8 +1232,7 @@ int ktri_list_triangles(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t
     KTRI_CK(ctx, cudaMemsetAsync(sink.pos, 0, sizeof(u64), st));
     KTRI_CK(ctx, cudaMemcpyAsync(d_fo, first_out, sizeof(u64) * (n + 1), cudaMemcpyHostToDevice, st));
     if (nnz) KTRI_CK(ctx, cudaMemcpyAsync(d_head, head, sizeof(u32) * nnz, cudaMemcpyHostToDevice, st));
-    rc = L.wide ? run_pipeline<u64>(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, false, sink)
-                : run_pipeline<u32>(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, false, sink);
+    rc = run_pipeline(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, false, sink);
     if (rc) return rc;
     u64 total = 0;
     KTRI_CK(ctx, cudaMemcpyAsync(&total, d_total, sizeof(u64), cudaMemcpyDeviceToHost, st));
@@ -1222,8 +1264,7 @@ int ktri_count_dag_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint
         return KTRI_OK;
     }
     const u64 nnz = 2 * m;
-    const Layout L = make_layout(n, nnz, opt.method, ctx->num_sms, true, d_per_vertex == nullptr, opt.force_wide,
-                                 opt.small_outdegree, opt.segment);
+    const Layout L = pick_layout(ctx, n, nnz, opt, true, d_per_vertex == nullptr);
     rc = ensure_ws(ctx, L.bytes);
     if (rc) return rc;
     char* base = static_cast<char*>(ctx->ws);
@@ -1238,8 +1279,7 @@ int ktri_count_dag_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint
     KTRI_CK(ctx, cudaGetLastError());
     u64* cnt = d_per_vertex ? reinterpret_cast<u64*>(d_per_vertex) : reinterpret_cast<u64*>(base + L.cnt);
     auto* tot = reinterpret_cast<u64*>(d_total);
-    return L.wide ? run_pipeline<u64>(ctx, L, fs, hs, n, nnz, tot, cnt, opt, st, false)
-                  : run_pipeline<u32>(ctx, L, fs, hs, n, nnz, tot, cnt, opt, st, false);
+    return run_pipeline(ctx, L, fs, hs, n, nnz, tot, cnt, opt, st, false);
 }
 
 int ktri_count_dag_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t* head, uint64_t n, uint64_t m,
@@ -1260,8 +1300,10 @@ int ktri_count_dag_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t*
             return set_error(ctx, KTRI_ERR_INVALID_CSR, "first_out is not monotone");
     if (m > (1ull << 62)) return set_error(ctx, KTRI_ERR_UNSUPPORTED, "too many edges");
     const u64 nnz = 2 * m;
-    Layout L = make_layout(n, nnz, opt.method, ctx->num_sms, true, true, opt.force_wide, opt.small_outdegree,
-                           opt.segment);
+    Layout L = pick_layout(ctx, n, nnz, opt, true, true, [&](size_t b) {
+        return align_up(align_up(align_up(b + sizeof(u64) * (n + 1)) + sizeof(u32) * m) +
+                        sizeof(u64) * (ktri::dag_scan_chunks(n) + 1));
+    });
     // the caller's lists and the scan sums follow the count's workspace
     const size_t x_fo = L.bytes, x_head = align_up(x_fo + sizeof(u64) * (n + 1)),
                  x_sums = align_up(x_head + sizeof(u32) * m);
@@ -1282,8 +1324,7 @@ int ktri_count_dag_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t*
     if (m) KTRI_CK(ctx, copy_host(ctx, dhead, head, sizeof(u32) * m, true, st));
     ktri::launch_dag_symmetrize(dfo, dhead, n, fs, hs, cursor, sums, ctx->num_sms, st);
     KTRI_CK(ctx, cudaGetLastError());
-    rc = L.wide ? run_pipeline<u64>(ctx, L, fs, hs, n, nnz, d_total, d_cnt, opt, st, false)
-                : run_pipeline<u32>(ctx, L, fs, hs, n, nnz, d_total, d_cnt, opt, st, false);
+    rc = run_pipeline(ctx, L, fs, hs, n, nnz, d_total, d_cnt, opt, st, false);
     if (rc) return rc;
     KTRI_CK(ctx, copy_host(ctx, total_out, d_total, sizeof(u64), false, st));
     bool staged = false;
@@ -1312,13 +1353,11 @@ int check_batch(ktri_ctx* ctx, const void* fo, const void* head, u64 n, u64 nnz,
     return KTRI_OK;
 }
 
-template <typename OffT>
 int enqueue_batch(ktri_ctx* ctx, char* base, const Layout& L, const u64* fo, const u32* head, u64 n, u64 nnz,
                   const u64* graph_first, u64 num_graphs, u64* totals, u64* cnt, const ktri::Options& opt,
                   cudaStream_t st, bool events) {
     auto* d_total = reinterpret_cast<u64*>(base + L.total);
-    int rc = enqueue_pipeline<OffT>(ctx, ctx->num_sms, base, L, fo, head, n, nnz, d_total, cnt, opt, st, false,
-                                    events);
+    int rc = enqueue_layout(ctx, ctx->num_sms, base, L, fo, head, n, nnz, d_total, cnt, opt, st, false, events);
     if (rc) return rc;
     ktri::launch_graph_totals(cnt, graph_first, num_graphs, n, totals, reinterpret_cast<Control*>(base + L.ctl),
                               ctx->num_sms, st);
@@ -1359,8 +1398,7 @@ int ktri_count_batch_device(ktri_ctx* ctx, const uint64_t* d_first_out, const ui
         ctx->pending = false;
         return KTRI_OK;
     }
-    const Layout L = make_layout(n_total, nnz_total, opt.method, ctx->num_sms, false, true,
-                                 opt.force_wide, opt.small_outdegree, opt.segment);
+    const Layout L = pick_layout(ctx, n_total, nnz_total, opt, false, true);
     rc = ensure_ws(ctx, L.bytes);
     if (rc) return rc;
     char* base = static_cast<char*>(ctx->ws);
@@ -1368,10 +1406,7 @@ int ktri_count_batch_device(ktri_ctx* ctx, const uint64_t* d_first_out, const ui
     auto* fo = reinterpret_cast<const u64*>(d_first_out);
     auto* gf = reinterpret_cast<const u64*>(d_graph_first);
     auto* tot = reinterpret_cast<u64*>(d_totals);
-    rc = L.wide ? enqueue_batch<u64>(ctx, base, L, fo, d_head, n_total, nnz_total, gf, num_graphs, tot, cnt, opt, st,
-                                     true)
-                : enqueue_batch<u32>(ctx, base, L, fo, d_head, n_total, nnz_total, gf, num_graphs, tot, cnt, opt, st,
-                                     true);
+    rc = enqueue_batch(ctx, base, L, fo, d_head, n_total, nnz_total, gf, num_graphs, tot, cnt, opt, st, true);
     if (rc) return rc;
     note_pending(ctx, L, base, st, n_total, nnz_total, opt);
     return KTRI_OK;
@@ -1396,8 +1431,9 @@ int ktri_count_batch_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_
     }
     if (first_out[0] != 0 || first_out[n_total] != nnz_total)
         return set_error(ctx, KTRI_ERR_INVALID_CSR, "first_out[0] must be 0 and first_out[n] must equal nnz");
-    const Layout L = make_layout(n_total, nnz_total, opt.method, ctx->num_sms, true, true,
-                                 opt.force_wide, opt.small_outdegree, opt.segment);
+    const Layout L = pick_layout(ctx, n_total, nnz_total, opt, true, true, [&](size_t b) {
+        return align_up(align_up(b + sizeof(u64) * (num_graphs + 1)) + sizeof(u64) * (num_graphs + 1));
+    });
     const size_t off_gf = L.bytes, off_tot = align_up(off_gf + sizeof(u64) * (num_graphs + 1));
     const size_t total_bytes = align_up(off_tot + sizeof(u64) * (num_graphs + 1));
     rc = ensure_ws(ctx, total_bytes);
@@ -1412,10 +1448,7 @@ int ktri_count_batch_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_
     KTRI_CK(ctx, copy_host(ctx, d_fo, first_out, sizeof(u64) * (n_total + 1), true, st));
     if (nnz_total) KTRI_CK(ctx, copy_host(ctx, d_head, head, sizeof(u32) * nnz_total, true, st));
     KTRI_CK(ctx, copy_host(ctx, d_gf, graph_first, sizeof(u64) * (num_graphs + 1), true, st));
-    rc = L.wide ? enqueue_batch<u64>(ctx, base, L, d_fo, d_head, n_total, nnz_total, d_gf, num_graphs, d_tot, d_cnt,
-                                     opt, st, true)
-                : enqueue_batch<u32>(ctx, base, L, d_fo, d_head, n_total, nnz_total, d_gf, num_graphs, d_tot, d_cnt,
-                                     opt, st, true);
+    rc = enqueue_batch(ctx, base, L, d_fo, d_head, n_total, nnz_total, d_gf, num_graphs, d_tot, d_cnt, opt, st, true);
     if (rc) return rc;
     note_pending(ctx, L, base, st, n_total, nnz_total, opt);
     if (num_graphs) KTRI_CK(ctx, copy_host(ctx, totals_out, d_tot, sizeof(u64) * num_graphs, false, st));
@@ -1458,8 +1491,12 @@ int ktri_plan_create_batch(ktri_ctx* ctx, const uint64_t* d_first_out, const uin
     if (n_total == 0) return set_error(ctx, KTRI_ERR_INVALID_ARGUMENT, "a plan needs at least one vertex");
     DeviceGuard g(ctx->device);
     if (ctx->pending) device_status(ctx);
-    const Layout L = make_layout(n_total, nnz_total, opt.method, ctx->num_sms, false, true,
-                                 opt.force_wide, opt.small_outdegree, opt.segment);
+    auto layout = [&](bool hub) {
+        return make_layout(n_total, nnz_total, opt.method, ctx->num_sms, false, true, opt.force_wide,
+                           opt.small_outdegree, opt.segment, hub);
+    };
+    Layout L = layout(ctx->hubs);
+    if (L.hub && ctx->budget && L.bytes > ctx->budget) L = layout(false);
     if (ctx->budget && L.bytes > ctx->budget)
         return set_error(ctx, KTRI_ERR_OUT_OF_MEMORY, "plan workspace exceeds the memory budget");
     ktri_plan* p = new (std::nothrow) ktri_plan();
@@ -1467,14 +1504,20 @@ int ktri_plan_create_batch(ktri_ctx* ctx, const uint64_t* d_first_out, const uin
     p->ctx = ctx;
     p->device = ctx->device;
     cudaError_t e = cudaMalloc(&p->ws, L.bytes);
+    if (e != cudaSuccess && L.hub) {
+        cudaGetLastError();
+        L = layout(false);
+        e = cudaMalloc(&p->ws, L.bytes);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         delete p;
         return cuda_fail(ctx, e, "cudaMalloc(plan workspace)");
     }
     // occupancy queries happen once, outside the capture
-    (void)ktri::count_grid_auto<u32>(ctx->num_sms);
-    (void)ktri::count_grid_auto<u64>(ctx->num_sms);
+    (void)ktri::count_grid_auto<u32, false>(ctx->num_sms);
+    (void)ktri::count_grid_auto<u32, true>(ctx->num_sms);
+    (void)ktri::count_grid_auto<u64, false>(ctx->num_sms);
     cudaStream_t cs = nullptr;
     cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
     char* base = static_cast<char*>(p->ws);
@@ -1484,10 +1527,7 @@ int ktri_plan_create_batch(ktri_ctx* ctx, const uint64_t* d_first_out, const uin
     auto* tot = reinterpret_cast<u64*>(d_totals);
     e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        rc = L.wide ? enqueue_batch<u64>(ctx, base, L, fo, d_head, n_total, nnz_total, gf, num_graphs, tot, cnt, opt, cs,
-                                         false)
-                    : enqueue_batch<u32>(ctx, base, L, fo, d_head, n_total, nnz_total, gf, num_graphs, tot, cnt, opt, cs,
-                                         false);
+        rc = enqueue_batch(ctx, base, L, fo, d_head, n_total, nnz_total, gf, num_graphs, tot, cnt, opt, cs, false);
         cudaGraph_t graph = nullptr;
         const cudaError_t e2 = cudaStreamEndCapture(cs, &graph);
         if (rc == KTRI_OK && e2 != cudaSuccess) rc = cuda_fail(ctx, e2, "cudaStreamEndCapture");
@@ -1578,8 +1618,7 @@ int ktri_orient_csr(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t* he
     cudaStream_t st = ctx->stream;
     KTRI_CK(ctx, cudaMemcpyAsync(d_fo, first_out, sizeof(u64) * (n + 1), cudaMemcpyHostToDevice, st));
     if (nnz) KTRI_CK(ctx, cudaMemcpyAsync(d_head, head, sizeof(u32) * nnz, cudaMemcpyHostToDevice, st));
-    rc = L.wide ? run_pipeline<u64>(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, true)
-                : run_pipeline<u32>(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, true);
+    rc = run_pipeline(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, true);
     if (rc) return rc;
     if (L.wide) ktri::launch_outdeg<u64>(n, base + L.vdesc, d_cnt, ctx->num_sms, st);
     else ktri::launch_outdeg<u32>(n, base + L.vdesc, d_cnt, ctx->num_sms, st);

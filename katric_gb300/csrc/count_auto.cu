@@ -154,7 +154,7 @@ __device__ __forceinline__ u32 bucket_probe16_flat(const u32* keys, u32* hits32,
 // entry by entry.  Against one table per owner in buckets of four with early exits, streamed over
 // the whole adjacency (the form before), 1.0x to 1.05x the entries are streamed on uniform and
 // geometric graphs (the head's list instead of the shorter one) at a quarter of the instructions.
-template <typename OffT>
+template <typename OffT, bool HUB>
 struct SmallWarpLayout {
     static constexpr int GROUP = 16;             // tails per group
     static constexpr int QCAP = 128;             // keys (and queued lists) of a group
@@ -167,8 +167,9 @@ struct SmallWarpLayout {
     static constexpr int W_REC = W_HITS + NB;                           // tail records (uint4)
     static constexpr int W_QS = W_REC + 4 * GROUP;                      // list starts (OffT), by key
     static constexpr int W_OS = W_QS + QCAP * (int)(sizeof(OffT) / 4);  // tails' list starts (OffT)
-    static constexpr int W_QM = W_OS + GROUP * (int)(sizeof(OffT) / 4); // (slot << 11) | (tail << 7) | length, by key
-    static constexpr int W_TOT = W_QM + QCAP;                           // tails' hit totals
+    static constexpr int W_QM = W_OS + GROUP * (int)(sizeof(OffT) / 4); // by key: slot << 16 | tail << 12 | hubs << 6 | others
+    static constexpr int W_QH = W_QM + QCAP;                            // HUB: hub list starts (16-byte groups), by key
+    static constexpr int W_TOT = W_QH + (HUB ? QCAP : 0);                         // tails' hit totals
     static constexpr int W_VTX = W_TOT + GROUP;                         // tails' vertices
     static constexpr int W_BIN = W_VTX + GROUP;                         // lists by length in 16-byte groups
     static constexpr int W_ORD = W_BIN + 32;                            // queue order (u16)
@@ -179,9 +180,9 @@ struct SmallWarpLayout {
 constexpr u32 NO_SLOT = 1023;  // a key without a table slot (its tail's table could not be built)
 
 // A warp's tables are empty between groups: keys and counters are cleared as they are flushed.
-template <typename OffT>
+template <typename OffT, bool HUB>
 __device__ __forceinline__ void small_init(u32* base) {
-    using L = SmallWarpLayout<OffT>;
+    using L = SmallWarpLayout<OffT, HUB>;
     const int lane = threadIdx.x & 31;
     for (int i = lane; i < 2 * L::NB; i += 32) base[L::W_KEYS + i] = EMPTY_KEY;
     for (int i = lane; i < L::NB; i += 32) base[L::W_HITS + i] = 0;
@@ -189,14 +190,15 @@ __device__ __forceinline__ void small_init(u32* base) {
 }
 
 // One batch: the tails among the vertices [bi * vb, (bi + 1) * vb), vb <= 32, counted by one warp in
-// its slice of shared memory.
-template <typename OffT, bool CG = false>
+// its slice of shared memory.  HUB: lists are split, and hub i is the key n + i of a table.
+template <typename OffT, bool HUB, bool CG = false>
 __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, const Desc<OffT>* __restrict__ vdesc,
-                                            const u32* __restrict__ headp, u32 sd, u64* __restrict__ cnt,
+                                            const u32* __restrict__ headp, const u16* __restrict__ hubp,
+                                            const u32* __restrict__ hub_ids, u32 sd, u64* __restrict__ cnt,
                                             u64& local_total, u32& dup) {
-    using L = SmallWarpLayout<OffT>;
+    using L = SmallWarpLayout<OffT, HUB>;
     constexpr u32 FULL = 0xFFFFFFFFu;
-    static_assert(SMALL_D < 128 && SMALL_D <= L::QCAP && L::GROUP <= 16, "field widths of the queue entries");
+    static_assert(SMALL_D < 64 && SMALL_D <= L::QCAP && L::GROUP <= 16, "field widths of the queue entries");
     static_assert(2 * L::NB <= (int)NO_SLOT && (SMALL_D + 3) / 4 < 32, "slots and length bins");
     const u32 lane = threadIdx.x & 31;
     const u32 lt_mask = (1u << lane) - 1, le_mask = lt_mask | (1u << lane);
@@ -207,21 +209,26 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
     OffT* q_s = reinterpret_cast<OffT*>(base + L::W_QS);
     OffT* o_s = reinterpret_cast<OffT*>(base + L::W_OS);
     u32* q_m = base + L::W_QM;
+    u32* q_h = base + L::W_QH;
     u32* tot = base + L::W_TOT;
     u32* vtx = base + L::W_VTX;
     u32* bins = base + L::W_BIN;
     unsigned short* q_ord = reinterpret_cast<unsigned short*>(base + L::W_ORD);
     const uint4* headp4 = reinterpret_cast<const uint4*>(headp);
+    const uint4* hubp8 = reinterpret_cast<const uint4*>(hubp);
+    const u32 n32 = (u32)n;
+    auto vertex_of = [&](u32 key) { return HUB && key >= n32 ? ld_in<CG>(hub_ids + (key - n32)) : key; };
     const u64 v = bi * vb + lane;
     Desc<OffT> dv;
     dv.start = 0;
     dv.d = 0;
     if (lane < vb && v < n) dv = ld_desc<CG>(vdesc + v);
-    u32 todo = __ballot_sync(FULL, dv.d >= 2 && dv.d <= sd);  // a tail needs two out-neighbours
+    const u32 len_v = list_len<HUB>(dv.d);
+    u32 todo = __ballot_sync(FULL, len_v >= 2 && len_v <= sd);  // a tail needs two out-neighbours
     while (todo) {
         // the group: the next tails in lane order while their keys fit
         const bool cand = (todo >> lane) & 1u;
-        u32 pk = cand ? dv.d : 0u;  // inclusive prefix of the tails' out-degrees
+        u32 pk = cand ? len_v : 0u;  // inclusive prefix of the tails' out-degrees
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const u32 y = __shfl_up_sync(FULL, pk, o);
@@ -234,7 +241,7 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
         const u32 G = __popc(gmask);
         const u32 K = __shfl_sync(FULL, pk, 31 - __clz(gmask));
         if (in) {
-            rec[rank] = make_uint4(pk - dv.d, dv.d, 0x9E3779B1u, 0u);
+            rec[rank] = make_uint4(pk - len_v, len_v, 0x9E3779B1u, rest_len<HUB>(dv.d));
             o_s[rank] = (OffT)list_group(dv);
             tot[rank] = 0;
             vtx[rank] = (u32)v;
@@ -256,7 +263,11 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
             const u32 starts = __reduce_or_sync(FULL, start_bit(mem, kst, q0));
             if (q0 + lane < K) {
                 gi[r] = segment_of(before, starts, le_mask);
-                w[r] = ld_in<CG>(headp + 4 * (u64)o_s[gi[r]] + (q0 + lane - rec[gi[r]].x));
+                const uint4 t = rec[gi[r]];
+                const u64 s = 4 * (u64)o_s[gi[r]];
+                const u32 k = q0 + lane - t.x;
+                if (!HUB || k < t.w) w[r] = ld_in<CG>(headp + s + k);
+                else w[r] = n32 + ld_in<CG>(hubp + hub_start(s, vtx[gi[r]]) + (k - t.w));
             }
         }
         Desc<OffT> dw[L::ROWS];
@@ -264,7 +275,7 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
         for (int r = 0; r < L::ROWS; ++r) {
             dw[r].start = 0;
             dw[r].d = 0;
-            if (w[r] != EMPTY_KEY) dw[r] = ld_desc<CG>(vdesc + w[r]);
+            if (w[r] != EMPTY_KEY) dw[r] = ld_desc<CG>(vdesc + vertex_of(w[r]));
         }
         // the tables: a tail whose keys overfill a bucket starts over with another multiplier
         u32 brute = 0;  // tails without a table
@@ -312,12 +323,13 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
         // the queue: heads with a small out-list, binned by length
 #pragma unroll
         for (int r = 0; r < L::ROWS; ++r) {
-            const u32 d = dw[r].d;
+            const u32 d = list_len<HUB>(dw[r].d);
             if (d == 0 || d > sd) continue;
-            const u32 q = 32 * r + lane;
+            const u32 q = 32 * r + lane, dr = rest_len<HUB>(dw[r].d), dh = hub_len<HUB>(dw[r].d);
             q_s[q] = (OffT)list_group(dw[r]);
-            q_m[q] = (slot[r] << 11) | (gi[r] << 7) | d;
-            atomicAdd(&bins[(d + 3) >> 2], 1u);
+            if constexpr (HUB) q_h[q] = (u32)(hub_start(list_start(dw[r]), vertex_of(w[r])) >> 3);
+            q_m[q] = (slot[r] << 16) | (gi[r] << 12) | (dh << 6) | dr;
+            atomicAdd(&bins[(dr + 3) / 4 + (dh + 7) / 8], 1u);
         }
         __syncwarp();
         u32 qn;
@@ -336,8 +348,9 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
         __syncwarp();
 #pragma unroll
         for (int r = 0; r < L::ROWS; ++r) {
-            const u32 d = dw[r].d;
-            if (d != 0 && d <= sd) q_ord[atomicAdd(&bins[(d + 3) >> 2], 1u)] = (unsigned short)(32 * r + lane);
+            const u32 d = list_len<HUB>(dw[r].d), dr = rest_len<HUB>(dw[r].d), dh = hub_len<HUB>(dw[r].d);
+            if (d != 0 && d <= sd)
+                q_ord[atomicAdd(&bins[(dr + 3) / 4 + (dh + 7) / 8], 1u)] = (unsigned short)(32 * r + lane);
         }
         __syncwarp();
         // stream the queued lists, one per lane, longest first; the next 16-byte group of a list is
@@ -346,48 +359,67 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
         for (u32 i = lane; i < qn; i += 32) {
             const u32 q = q_ord[i];
             const u32 m = q_m[q];
-            const u32 g = (m >> 7) & 15u;
+            const u32 g = (m >> 12) & 15u;
             const uint4* lp = headp4 + (u64)q_s[q];
             const uint4 t = rec[g];
-            int rem = (int)(m & 127u);
+            int rem = (int)(m & 63u), hrem = HUB ? (int)((m >> 6) & 63u) : 0;
             u32 found = 0;
             if ((brute >> g) & 1u) {
-                const u32* lst = reinterpret_cast<const u32*>(lp);
-                const u32* own = headp + 4 * (u64)o_s[g];
-                for (int e = 0; e < rem; ++e) {
-                    const u32 z = ld_in<CG>(lst + e);
+                const u64 own = 4 * (u64)o_s[g], hown = hub_start(own, vtx[g]);
+                auto own_key = [&](u32 k) {
+                    return !HUB || k < t.w ? ld_in<CG>(headp + own + k) : n32 + ld_in<CG>(hubp + hown + (k - t.w));
+                };
+                for (int e = 0; e < rem + hrem; ++e) {
+                    const u32 z = e < rem ? ld_in<CG>(reinterpret_cast<const u32*>(lp) + e)
+                                          : n32 + ld_in<CG>(reinterpret_cast<const u16*>(hubp8 + q_h[q]) + (e - rem));
                     for (u32 k = 0; k < t.y; ++k)
-                        if (ld_in<CG>(own + k) == z) {
-                            atomicAdd(&cnt[z], 1ull);
+                        if (own_key(k) == z) {
+                            atomicAdd(&cnt[vertex_of(z)], 1ull);
                             ++found;
                         }
                 }
-                if (found) atomicAdd(&cnt[ld_in<CG>(own + (q - t.x))], (u64)found);
+                if (found) atomicAdd(&cnt[vertex_of(own_key(q - t.x))], (u64)found);
             } else {
                 const u32 nb = 3 * t.y, mult = t.z;
                 const uint2* tk = reinterpret_cast<const uint2*>(keys) + 3 * t.x;
                 u32* th = hits + 3 * t.x;
-                uint4 cur = ld_in<CG>(lp);
-                while (true) {
-                    uint4 nxt = cur;
-                    if (rem > 4) nxt = ld_in<CG>(++lp);
-                    const u32 z[4] = {cur.x, cur.y, cur.z, cur.w};
+                auto look = [&](u32 z, bool valid) {
+                    const u32 b = __umulhi(z * mult, nb);
+                    const uint2 kk = tk[b];
+                    const bool h0 = kk.x == z, h1 = kk.y == z;
+                    if ((h0 | h1) & valid) {
+                        atomicAdd(&th[b], h1 ? 0x10000u : 1u);
+                        ++found;
+                    }
+                };
+                if (!HUB || rem > 0) {
+                    uint4 cur = ld_in<CG>(lp);
+                    while (true) {
+                        uint4 nxt = cur;
+                        if (rem > 4) nxt = ld_in<CG>(++lp);
+                        look(cur.x, true);
+                        look(cur.y, rem > 1);
+                        look(cur.z, rem > 2);
+                        look(cur.w, rem > 3);
+                        rem -= 4;
+                        if (rem <= 0) break;
+                        cur = nxt;
+                    }
+                }
+                if constexpr (HUB) {
+                    const uint4* hp = hubp8 + q_h[q];
+                    for (; hrem > 0; hrem -= 8) {
+                        const uint4 cur = ld_in<CG>(hp++);
+                        const u32 pair[4] = {cur.x, cur.y, cur.z, cur.w};
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const u32 b = __umulhi(z[k] * mult, nb);
-                        const uint2 kk = tk[b];
-                        const bool h0 = kk.x == z[k], h1 = kk.y == z[k];
-                        if ((h0 | h1) & (k < rem)) {
-                            atomicAdd(&th[b], h1 ? 0x10000u : 1u);
-                            ++found;
+                        for (int k = 0; k < 4; ++k) {
+                            look(n32 + (pair[k] & 0xFFFFu), 2 * k < hrem);
+                            look(n32 + (pair[k] >> 16), 2 * k + 1 < hrem);
                         }
                     }
-                    rem -= 4;
-                    if (rem <= 0) break;
-                    cur = nxt;
                 }
                 if (found) {
-                    const u32 s = m >> 11;
+                    const u32 s = m >> 16;
                     atomicAdd(&hits[s >> 1], found << ((s & 1u) << 4));  // the edge's head
                 }
             }
@@ -402,7 +434,7 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
             const u32 h = hits16[slot[r]];
             keys[slot[r]] = EMPTY_KEY;
             hits16[slot[r]] = 0;
-            if (h) atomicAdd(&cnt[w[r]], (u64)h);
+            if (h) atomicAdd(&cnt[vertex_of(w[r])], (u64)h);
         }
         if (mem) {
             const u32 t = tot[lane];
@@ -415,19 +447,21 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
     }
 }
 
-template <int BLOCK, typename OffT>
+template <int BLOCK, typename OffT, bool HUB>
 __global__ void __launch_bounds__(BLOCK, 4) k_count_small(u64 n, u32 vb, const Desc<OffT>* __restrict__ vdesc,
-                                                          const u32* __restrict__ headp, u32 sd,
+                                                          const u32* __restrict__ headp, const u16* __restrict__ hubp,
+                                                          const u32* __restrict__ hub_ids, u32 sd,
                                                           u64* __restrict__ cnt, u64* __restrict__ partials,
                                                           Control* ctl) {
-    using L = SmallWarpLayout<OffT>;
+    using L = SmallWarpLayout<OffT, HUB>;
     constexpr int NW = BLOCK / 32;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ u64 s_red[NW];
     if (ctl->err & DEV_ERR_MASK) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     u32* base = reinterpret_cast<u32*>(smem) + warp * L::PER_WARP;
-    small_init<OffT>(base);
+    small_init<OffT, HUB>(base);
+    const bool split = HUB && ctl->hubs != 0;  // without hubs the plain body reads the same lists
     const u64 nbatch = (n + vb - 1) / vb;
     u64 local_total = 0;
     u32 dup = 0;
@@ -436,7 +470,10 @@ __global__ void __launch_bounds__(BLOCK, 4) k_count_small(u64 n, u32 vb, const D
         if (lane == 0) bi = atomicAdd(&ctl->small_next, 1ull);
         bi = __shfl_sync(0xFFFFFFFFu, bi, 0);
         if (bi >= nbatch) break;
-        small_batch<OffT>(base, bi, vb, n, vdesc, headp, sd, cnt, local_total, dup);
+        if (split)
+            small_batch<OffT, HUB>(base, bi, vb, n, vdesc, headp, hubp, hub_ids, sd, cnt, local_total, dup);
+        else
+            small_batch<OffT, false>(base, bi, vb, n, vdesc, headp, nullptr, nullptr, sd, cnt, local_total, dup);
     }
     if (dup) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
     const u64 bt = block_sum_u64<BLOCK>(local_total, s_red);
@@ -552,7 +589,7 @@ __device__ __forceinline__ void chunk_sizes(u32 klen, u32 max_lg, u32 max_fl, u3
 // One (owner, segment) tile of a large owner, counted by the whole block.  bar is the block's
 // bulk-copy mbarrier, initialised once and kept where no other use of shared memory reaches.
 // Returns true when a bounded wait for a bulk copy ran out (inflight: the second wait ran out too).
-template <int BLOCK, int CAP, typename OffT, bool CG = false>
+template <int BLOCK, int CAP, typename OffT, bool HUB, bool CG = false>
 __device__ __forceinline__ bool large_tile(unsigned char* smem, unsigned long long* bar, uint2 tl,
                                            const u64* __restrict__ fo,
                                            const u32* __restrict__ head, u64 n, const Desc<OffT>* __restrict__ vdesc,
@@ -581,7 +618,7 @@ __device__ __forceinline__ bool large_tile(unsigned char* smem, unsigned long lo
     bool timed_out = false;
     const u64 x = tl.x;
     const Desc<OffT> dxd = ld_desc<CG>(vdesc + x);
-    const u32 dx = dxd.d;
+    const u32 dx = rest_len<HUB>(dxd.d), dxt = list_len<HUB>(dxd.d);
     const u64 fx1 = ld_in<CG>(fo + x + 1);
     const u64 a = ld_in<CG>(fo + x) + (u64)tl.y * seg;
     const u64 b = a + seg < fx1 ? a + seg : fx1;
@@ -640,8 +677,9 @@ __device__ __forceinline__ bool large_tile(unsigned char* smem, unsigned long lo
             if (e < b) {
                 y = ld_in<CG>(head + e);
                 if (y < n) vy = ld_desc<CG>(vdesc + y);
-                const u32 dy = vy.d;
-                if (dy > 0 && key_less(dy, y, dx, x)) {
+                const u32 dyt = list_len<HUB>(vy.d), dy = rest_len<HUB>(vy.d);
+                vy.d = dy;
+                if (dy > 0 && key_less(dyt, y, dxt, x)) {
                     if (dy <= (u32)LONG_LIST) {
                         const u32 hits = lane_stream_short<OffT, CG>(headp4, vy, keys, hitc, lg, filt, fl);
                         if (hits) {
@@ -698,7 +736,7 @@ __device__ __forceinline__ bool large_tile(unsigned char* smem, unsigned long lo
     return timed_out;
 }
 
-template <int BLOCK, int CAP, typename OffT>
+template <int BLOCK, int CAP, typename OffT, bool HUB>
 __global__ void __launch_bounds__(BLOCK) k_count_large(const u64* __restrict__ fo, const u32* __restrict__ head,
                                                        u64 n, const Desc<OffT>* __restrict__ vdesc,
                                                        const u32* __restrict__ headp,
@@ -724,7 +762,7 @@ __global__ void __launch_bounds__(BLOCK) k_count_large(const u64* __restrict__ f
         __syncthreads();
         const u64 t = s_t;
         if (t >= ntiles) break;
-        timed_out = large_tile<BLOCK, CAP, OffT>(smem, s_bar, ltiles[t], fo, head, n, vdesc, headp, seg, cnt,
+        timed_out = large_tile<BLOCK, CAP, OffT, HUB>(smem, s_bar, ltiles[t], fo, head, n, vdesc, headp, seg, cnt,
                                                  first_wait_polls, phase, inflight, local_total, dup);
         if (timed_out) break;
     }
@@ -748,7 +786,7 @@ struct MediumLayout {
 
 // One (owner, segment) tile of a medium owner, counted by one warp in its slice of shared
 // memory (keys at `keys`, then the hit counters, the filter and the survivor buffer).
-template <int BLOCK, typename OffT, bool CG = false>
+template <int BLOCK, typename OffT, bool HUB, bool CG = false>
 __device__ __forceinline__ void medium_tile(u32* keys, uint2 tl, const u64* __restrict__ fo,
                                             const u32* __restrict__ head, const Desc<OffT>* __restrict__ vdesc,
                                             const u32* __restrict__ headp, u32 seg, u64* __restrict__ cnt,
@@ -763,7 +801,8 @@ __device__ __forceinline__ void medium_tile(u32* keys, uint2 tl, const u64* __re
     const uint4* headp4 = reinterpret_cast<const uint4*>(headp);
     const u64 x = tl.x;
     const Desc<OffT> dxd = ld_desc<CG>(vdesc + x);
-    const u32 dx = dxd.d;
+    const u32 dx = rest_len<HUB>(dxd.d), dxt = list_len<HUB>(dxd.d);
+    if (HUB && dx == 0) return;
     const u64 fx1 = ld_in<CG>(fo + x + 1);
     const u64 a = ld_in<CG>(fo + x) + (u64)tl.y * seg;
     const u64 b = a + seg < fx1 ? a + seg : fx1;
@@ -792,8 +831,9 @@ __device__ __forceinline__ void medium_tile(u32* keys, uint2 tl, const u64* __re
         if (e < b) {
             y = ld_in<CG>(head + e);
             vy = ld_desc<CG>(vdesc + y);
-            const u32 dy = vy.d;
-            if (dy > 0 && key_less(dy, y, dx, x)) {
+            const u32 dyt = list_len<HUB>(vy.d), dy = rest_len<HUB>(vy.d);
+            vy.d = dy;
+            if (dy > 0 && key_less(dyt, y, dxt, x)) {
                 if (dy <= (u32)LONG_LIST) {
                     const u32 hits = lane_stream_short<OffT, CG>(headp4, vy, keys, hitc, lg, filt, fl);
                     if (hits) {
@@ -833,7 +873,7 @@ __device__ __forceinline__ void medium_tile(u32* keys, uint2 tl, const u64* __re
     __syncwarp();
 }
 
-template <int BLOCK, typename OffT>
+template <int BLOCK, typename OffT, bool HUB>
 __global__ void __launch_bounds__(BLOCK)
     k_count_medium(const u64* __restrict__ fo, const u32* __restrict__ head, u64 n,
                    const Desc<OffT>* __restrict__ vdesc, const u32* __restrict__ headp,
@@ -854,11 +894,209 @@ __global__ void __launch_bounds__(BLOCK)
         if (lane == 0) t = atomicAdd(&ctl->medium_next, 1ull);
         t = __shfl_sync(0xFFFFFFFFu, t, 0);
         if (t >= ntiles) break;
-        medium_tile<BLOCK, OffT>(keys, mtiles[t], fo, head, vdesc, headp, seg, cnt, local_total, dup);
+        medium_tile<BLOCK, OffT, HUB>(keys, mtiles[t], fo, head, vdesc, headp, seg, cnt, local_total, dup);
     }
     if (dup) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
     const u64 bt = block_sum_u64<BLOCK>(local_total, s_red);
     if (threadIdx.x == 0) partials[blockIdx.x] = bt;
+}
+
+// The hub part of the owner tiles (k_count_hub): for every edge {x, y} of an owner x, the hubs that
+// both out-lists hold.  Hubs are the few thousand vertices of highest degree, which most entries of
+// a skewed graph's out-lists name (80 % of the entries RMAT-24 streams are among its first 2^15,
+// 98 % of RMAT-20's), and a hub list holds 16-bit indices.  So an owner's table is a bitmap of HUB_H
+// bits: a lookup is one 4-byte shared-memory read without hash, filter or walk, and a streamed
+// entry costs two bytes of L2 traffic instead of four.
+// A block holds one counter per hub for its whole life and flushes them once, so a tile clears
+// nothing but its bitmap.  Each warp takes its own (owner, segment) tiles and has its own bitmap.
+// Lists above HUB_LANE entries are streamed by the whole warp, four consecutive entries per lane (so
+// that a sorted list's lanes read neighbouring words), the shorter ones one per lane.
+struct HubLayout {
+    static constexpr u32 BITS = HUB_H / 32;  // bitmap words of a warp
+    static constexpr u32 off_bits = 0;       // the warps' bitmaps, each aligned to its own size
+    static constexpr u32 off_cnt = sizeof(u32) * BITS * HUB_WARPS;  // u32 counter per hub
+    static constexpr u32 align = sizeof(u32) * BITS;
+    static constexpr size_t bytes = off_cnt + sizeof(u32) * HUB_H;
+};
+constexpr size_t HUB_SMEM = HubLayout::bytes + HubLayout::align;  // room to align the bitmaps
+constexpr u32 HUB_LANE = 16;                       // hub lists up to this length are streamed by one lane
+constexpr u32 HUB_PAD2 = HUB_PAD | (HUB_PAD << 16);  // two entries that hit nothing
+
+// Two entries of a hub list looked up in the bitmap at shared address `bits` (aligned to its size):
+// counts the hits at the hubs' counters (shared address cnt) and returns their number.  A miss
+// counts at the spare word instead: a predicated reduction becomes a branch around it (four more
+// instructions per entry, and with a hit in almost every row it skips nothing; 2.12 against 1.90 ms
+// on RMAT n = 10^6).
+__device__ __forceinline__ u32 hub_probe2(u32 pair, u32 bits, u32 cnt, u32 spare) {
+    u32 found;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        ".reg .u32 a, b, h, k, v, w;\n\t"
+        "and.b32 h, %1, 0xFFFF;\n\t"
+        "shr.u32 k, %1, 16;\n\t"
+        "shr.u32 a, %1, 3;\n\t"
+        "shr.u32 b, %1, 19;\n\t"
+        "lop3.b32 a, a, %4, %2, 0xEA;\n\t"  // (a & mask) | bits
+        "lop3.b32 b, b, %4, %2, 0xEA;\n\t"
+        "ld.shared.u32 v, [a];\n\t"
+        "ld.shared.u32 w, [b];\n\t"
+        "shf.r.wrap.b32 v, v, v, h;\n\t"
+        "shf.r.wrap.b32 w, w, w, k;\n\t"
+        "and.b32 v, v, 1;\n\t"
+        "and.b32 w, w, 1;\n\t"
+        "setp.ne.u32 p, v, 0;\n\t"
+        "setp.ne.u32 q, w, 0;\n\t"
+        "mad.lo.u32 h, h, 4, %3;\n\t"
+        "mad.lo.u32 k, k, 4, %3;\n\t"
+        "selp.u32 h, h, %5, p;\n\t"
+        "selp.u32 k, k, %5, q;\n\t"
+        "red.shared.add.u32 [h], 1;\n\t"
+        "red.shared.add.u32 [k], 1;\n\t"
+        "add.u32 %0, v, w;\n\t"
+        "}"
+        : "=r"(found)
+        : "r"(pair), "r"(bits), "r"(cnt), "n"(HUB_H / 8 - 4), "r"(spare)
+        : "memory");
+    return found;
+}
+
+__global__ void __launch_bounds__(32 * HUB_WARPS, 1)
+    k_count_hub(const u64* __restrict__ fo, const u32* __restrict__ head, const Desc<u32>* __restrict__ vdesc,
+                const u16* __restrict__ hubp, const u32* __restrict__ hub_ids, const uint2* __restrict__ mtiles,
+                const uint2* __restrict__ ltiles, u32 seg, u64* __restrict__ cnt, u64* __restrict__ partials,
+                Control* ctl) {
+    using L = HubLayout;
+    constexpr u32 FULL = 0xFFFFFFFFu;
+    constexpr u32 ROWS = 2;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ u64 s_red[HUB_WARPS];
+    if (ctl->err & DEV_ERR_MASK) return;
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const u32 nh = ctl->hubs;
+    const u64 nl = *(volatile unsigned long long*)&ctl->large_tiles;
+    const u64 nt = nh ? nl + *(volatile unsigned long long*)&ctl->medium_tiles : 0;
+    unsigned char* sbase = smem + ((L::align - (smem_u32(smem) & (L::align - 1))) & (L::align - 1));
+    u32* hcnt = reinterpret_cast<u32*>(sbase + L::off_cnt);
+    u32* bits = reinterpret_cast<u32*>(sbase + L::off_bits) + warp * L::BITS;
+    const u32 bits_at = smem_u32(bits), cnt_at = smem_u32(hcnt);
+    const u32 spare_at = cnt_at + sizeof(u32) * HUB_PAD;  // no hub's counter
+    for (u32 i = threadIdx.x; i < nh; i += 32 * HUB_WARPS) hcnt[i] = 0;
+    for (u32 i = lane; i < L::BITS; i += 32) bits[i] = 0;
+    __syncthreads();
+    u64 total = 0;
+    u32 dup = 0;
+    while (true) {
+        unsigned long long t = 0;
+        if (lane == 0) t = atomicAdd(&ctl->hub_next, 1ull);
+        t = __shfl_sync(FULL, t, 0);
+        if (t >= nt) break;
+        const uint2 tl = t < nl ? ltiles[t] : mtiles[t - nl];
+        const u32 x = tl.x;
+        const Desc<u32> dx = load_desc(vdesc + x);
+        const u32 xh = hub_len<true>(dx.d), xt = list_len<true>(dx.d);
+        if (xh == 0) continue;
+        const u16* own = hubp + hub_start(list_start(dx), x);
+        for (u32 k = lane; k < xh; k += 32) {
+            const u32 h = __ldg(own + k), bit = 1u << (h & 31u);
+            if (atomicOr(&bits[h >> 5], bit) & bit) dup = 1;
+        }
+        const u64 a = fo[x] + (u64)tl.y * seg, fx1 = fo[x + 1];
+        const u32 ns = (u32)(a + seg < fx1 ? (u64)seg : fx1 - a);
+        __syncwarp();
+        u32 T = 0;
+        // neighbours of the next 32 slots are in flight while the current ones are counted
+        u32 y = lane < ns ? __ldg(head + a + lane) : x;
+        for (u32 e0 = 0; e0 < ns; e0 += 32) {
+            const u32 yc = y;
+            const bool have = e0 + lane < ns;
+            const Desc<u32> vy = load_desc(vdesc + yc);
+            y = e0 + 32 + lane < ns ? __ldg(head + a + e0 + 32 + lane) : x;
+            const u32 yh = hub_len<true>(vy.d);
+            const bool sel = have && yh > 0 && key_less(list_len<true>(vy.d), yc, xt, x);
+            const u32 ys = (u32)(hub_start(list_start(vy), yc) >> 3);  // in 16-byte groups
+            u32 hits = 0;
+            u32 longs = __ballot_sync(FULL, sel && yh > HUB_LANE);
+            if (sel && yh <= HUB_LANE) {
+                const uint4* lp = reinterpret_cast<const uint4*>(hubp) + ys;
+                const uint4 g0 = __ldg(lp), g1 = yh > 8 ? __ldg(lp + 1) : g0;
+                hits = hub_probe2(g0.x, bits_at, cnt_at, spare_at);
+                if (yh > 2) hits += hub_probe2(g0.y, bits_at, cnt_at, spare_at);
+                if (yh > 4) hits += hub_probe2(g0.z, bits_at, cnt_at, spare_at);
+                if (yh > 6) hits += hub_probe2(g0.w, bits_at, cnt_at, spare_at);
+                if (yh > 8) hits += hub_probe2(g1.x, bits_at, cnt_at, spare_at);
+                if (yh > 10) hits += hub_probe2(g1.y, bits_at, cnt_at, spare_at);
+                if (yh > 12) hits += hub_probe2(g1.z, bits_at, cnt_at, spare_at);
+                if (yh > 14) hits += hub_probe2(g1.w, bits_at, cnt_at, spare_at);
+            }
+            __syncwarp();
+            // the long lists one after the other, in blocks of ROWS x 128 entries: the next block, of
+            // this list or the next one, is in flight while the current one is looked up
+            uint2 nb[ROWS];
+            u32 nq = 0;  // quadruples of entries left from the next block on
+            const uint2* np = nullptr;
+            auto load_block = [&]() {
+#pragma unroll
+                for (u32 r = 0; r < ROWS; ++r) {
+                    nb[r] = make_uint2(HUB_PAD2, HUB_PAD2);
+                    if (lane + 32 * r < nq) nb[r] = __ldg(np + 32 * r);
+                }
+            };
+            auto next_list = [&](int src) {
+                nq = (__shfl_sync(FULL, yh, src) + 3) / 4;
+                np = reinterpret_cast<const uint2*>(hubp) + (u64)__shfl_sync(FULL, ys, src) * 2 + lane;
+                load_block();
+            };
+            if (longs) next_list(__ffs(longs) - 1);
+            while (longs) {
+                const u32 src = __ffs(longs) - 1;
+                longs &= longs - 1;
+                u32 f = 0;
+                while (true) {
+                    uint2 cb[ROWS];
+#pragma unroll
+                    for (u32 r = 0; r < ROWS; ++r) cb[r] = nb[r];
+                    const u32 left = nq;
+                    const bool more = left > 32 * ROWS;
+                    if (more) {
+                        nq = left - 32 * ROWS;
+                        np += 32 * ROWS;
+                        load_block();
+                    } else if (longs) {
+                        next_list(__ffs(longs) - 1);
+                    }
+#pragma unroll
+                    for (u32 r = 0; r < ROWS; ++r) {
+                        if (32 * r >= left) break;
+                        f += hub_probe2(cb[r].x, bits_at, cnt_at, spare_at);
+                        f += hub_probe2(cb[r].y, bits_at, cnt_at, spare_at);
+                    }
+                    if (!more) break;
+                }
+                f = __reduce_add_sync(FULL, f);
+                if (lane == src) hits = f;
+            }
+            if (hits) {
+                atomicAdd(&cnt[yc], (u64)hits);
+                T += hits;
+            }
+        }
+        const u32 wt = __reduce_add_sync(FULL, T);
+        if (lane == 0 && wt) {
+            atomicAdd(&cnt[x], (u64)wt);
+            total += wt;
+        }
+        __syncwarp();
+        for (u32 k = lane; k < xh; k += 32) bits[__ldg(own + k) >> 5] = 0;
+        __syncwarp();
+    }
+    if (dup) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
+    const u64 bt = block_sum_u64<32 * HUB_WARPS>(total, s_red);  // also orders the counters' last hits
+    if (threadIdx.x == 0) partials[blockIdx.x] = bt;
+    for (u32 i = threadIdx.x; i < nh; i += 32 * HUB_WARPS) {
+        const u32 c = hcnt[i];
+        if (c) atomicAdd(&cnt[hub_ids[i]], (u64)c);
+    }
 }
 
 // Sum of the per-block partial totals (a u64 tree reduction in one block), without the slots
@@ -903,9 +1141,10 @@ __global__ void __launch_bounds__(256) k_graph_totals(const u64* __restrict__ cn
 // (cetric_edge_iterator.h:279-281), plus the entries streamed by the AUTO kernels, also counted
 // once per table chunk of their owner (owners above medium_d keep at most LARGE_CAP keys per
 // chunk and stream their segment once per chunk).
-template <typename OffT>
+template <typename OffT, bool HUB>
 __global__ void k_stats(const u64* __restrict__ fo, const u32* __restrict__ head, u64 n,
-                        const Desc<OffT>* __restrict__ vdesc, const u32* __restrict__ headp, u32 small_d, u32 medium_d,
+                        const Desc<OffT>* __restrict__ vdesc, const u32* __restrict__ headp,
+                        const u16* __restrict__ hubp, const u32* __restrict__ hub_ids, u32 small_d, u32 medium_d,
                         Control* ctl) {
     if (ctl->err & DEV_ERR_MASK) return;
     const int lane = threadIdx.x & 31;
@@ -914,24 +1153,26 @@ __global__ void k_stats(const u64* __restrict__ fo, const u32* __restrict__ head
     u64 wedge = 0, isz = 0, streamed = 0, oriented = 0, chunked = 0;
     for (u64 v = gw; v < n; v += nwarps) {
         const Desc<OffT> dv = load_desc(vdesc + v);
-        const u64 chunks = dv.d > medium_d ? (dv.d + LARGE_CAP - 1) / LARGE_CAP : 1;
-        if (lane == 0) oriented += dv.d;
-        for (u32 k = lane; k < dv.d; k += 32) {
-            const u32 u = headp[list_start(dv) + k];
-            const u32 du = load_desc(vdesc + u).d;
+        const u32 lv = list_len<HUB>(dv.d), rv = rest_len<HUB>(dv.d);
+        const u64 chunks = lv > medium_d ? (rv + LARGE_CAP - 1) / LARGE_CAP : 1;
+        if (lane == 0) oriented += lv;
+        for (u32 k = lane; k < lv; k += 32) {
+            const u32 u = k < rv ? headp[list_start(dv) + k]
+                                 : hub_ids[hubp[hub_start(list_start(dv), v) + (k - rv)]];
+            const u32 du = list_len<HUB>(load_desc(vdesc + u).d);
             wedge += du;
-            isz += (u64)dv.d + du;
-            if (dv.d >= 2 && dv.d <= small_d && du <= small_d) {  // counted at the tail
+            isz += (u64)lv + du;
+            if (lv >= 2 && lv <= small_d && du <= small_d) {  // counted at the tail
                 streamed += du;
                 chunked += du;
             }
         }
         for (u64 e = fo[v] + lane; e < fo[v + 1]; e += 32) {
             const u32 y = head[e];
-            const u32 dy = load_desc(vdesc + y).d;
-            if (dy > 0 && dv.d > small_d && key_less(dy, y, dv.d, v)) {
+            const u32 word = load_desc(vdesc + y).d, dy = list_len<HUB>(word);
+            if (dy > 0 && lv > small_d && key_less(dy, y, lv, v)) {
                 streamed += dy;
-                chunked += dy * chunks;
+                chunked += hub_len<HUB>(word) + rest_len<HUB>(word) * (chunks ? chunks : 1);
             }
         }
     }
@@ -954,7 +1195,7 @@ __global__ void k_stats(const u64* __restrict__ fo, const u32* __restrict__ head
 
 // ---- the serving engine ----------------------------------------------------------------
 
-using EngineSmallL = SmallWarpLayout<u32>;
+using EngineSmallL = SmallWarpLayout<u32, false>;
 using EngineMediumL = MediumLayout<ENGINE_BLOCK>;
 using EngineLargeL = LargeLayout<ENGINE_BLOCK, LARGE_CAP, u32>;
 constexpr size_t cmax(size_t a, size_t b) { return a > b ? a : b; }
@@ -1115,25 +1356,25 @@ __global__ void __launch_bounds__(ENGINE_BLOCK, 4) k_engine(EngineJob* jobs, u32
         if (u < jb->units_small) {
             const u64 nb = (jb->n + 31) / 32;
             u32* slice = reinterpret_cast<u32*>(smem) + warp * EngineSmallL::PER_WARP;
-            small_init<u32>(slice);  // other kinds of unit use the same shared memory
+            small_init<u32, false>(slice);  // other kinds of unit use the same shared memory
             for (u32 r = 0; r < ENGINE_REPS; ++r) {
                 const u64 bi = (u * (ENGINE_BLOCK / 32) + warp) * ENGINE_REPS + r;
                 if (bi < nb)
-                    small_batch<u32, true>(slice, bi, 32, jb->n, vd, jb->headp, jb->small_d, jb->cnt, unused_total,
-                                           dup);
+                    small_batch<u32, false, true>(slice, bi, 32, jb->n, vd, jb->headp, nullptr, nullptr, jb->small_d,
+                                                  jb->cnt, unused_total, dup);
             }
         } else if (u < jb->units_small + jb->units_medium) {
             const u64 nt = *(volatile unsigned long long*)&ctl->medium_tiles;
             for (u32 r = 0; r < ENGINE_REPS; ++r) {
                 const u64 t = ((u - jb->units_small) * (ENGINE_BLOCK / 32) + warp) * ENGINE_REPS + r;
                 if (t < nt)
-                    medium_tile<BLOCK, u32, true>(reinterpret_cast<u32*>(smem) + warp * EngineMediumL::PER_WARP,
+                    medium_tile<BLOCK, u32, false, true>(reinterpret_cast<u32*>(smem) + warp * EngineMediumL::PER_WARP,
                                                   __ldcg(jb->mtiles + t), jb->fo, jb->head, vd, jb->headp, jb->seg,
                                                   jb->cnt, unused_total, dup);
             }
         } else {
             const u64 t = u - jb->units_small - jb->units_medium;
-            timed_out = large_tile<BLOCK, LARGE_CAP, u32, true>(smem, s_bar, __ldcg(jb->ltiles + t), jb->fo, jb->head,
+            timed_out = large_tile<BLOCK, LARGE_CAP, u32, false, true>(smem, s_bar, __ldcg(jb->ltiles + t), jb->fo, jb->head,
                                                                 jb->n, vd, jb->headp,
                                                           jb->seg, jb->cnt, COPY_WAIT_POLLS, phase, inflight,
                                                           unused_total, dup);
@@ -1191,56 +1432,37 @@ template <typename OffT>
 using LargeL = LargeLayout<LARGE_BLOCK, LARGE_CAP, OffT>;
 using MediumL = MediumLayout<MEDIUM_BLOCK>;
 
-template <typename OffT>
-int occupancy_small() {
-    static int occ = -1;
-    if (occ < 0) {
-        auto kern = k_count_small<SMALL_BLOCK, OffT>;
-        const size_t bytes = SmallWarpLayout<OffT>::bytes(SMALL_BLOCK / 32);
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        int o = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, SMALL_BLOCK, bytes);
-        occ = o > 0 ? o : 1;
-    }
-    return occ;
-}
-template <typename OffT>
-int occupancy_medium() {
-    static int occ = -1;
-    if (occ < 0) {
-        auto kern = k_count_medium<MEDIUM_BLOCK, OffT>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MediumL::bytes);
-        int o = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, MEDIUM_BLOCK, MediumL::bytes);
-        occ = o > 0 ? o : 1;
-    }
-    return occ;
-}
-template <typename OffT>
-int occupancy_large() {
-    static int occ = -1;
-    if (occ < 0) {
-        auto kern = k_count_large<LARGE_BLOCK, LARGE_CAP, OffT>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LargeL<OffT>::bytes);
-        int o = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, LARGE_BLOCK, LargeL<OffT>::bytes);
-        occ = o > 0 ? o : 1;
-    }
-    return occ;
+// Resident blocks per SM of a kernel, looked up once; also allows it its dynamic shared memory.
+template <typename Kernel>
+int occupancy_of(Kernel kern, int block, size_t bytes) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    int o = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, block, bytes);
+    return o > 0 ? o : 1;
 }
 }  // namespace
 
-template <typename OffT>
+template <typename OffT, bool HUB>
 int count_grid_small(int num_sms) {
-    return num_sms * occupancy_small<OffT>();
+    static const int occ = occupancy_of(k_count_small<SMALL_BLOCK, OffT, HUB>, SMALL_BLOCK,
+                                        SmallWarpLayout<OffT, HUB>::bytes(SMALL_BLOCK / 32));
+    return num_sms * occ;
 }
-template <typename OffT>
+template <typename OffT, bool HUB>
 int count_grid_medium(int num_sms) {
-    return num_sms * occupancy_medium<OffT>();
+    static const int occ = occupancy_of(k_count_medium<MEDIUM_BLOCK, OffT, HUB>, MEDIUM_BLOCK, MediumL::bytes);
+    return num_sms * occ;
 }
-template <typename OffT>
+template <typename OffT, bool HUB>
 int count_grid_large(int num_sms) {
-    return num_sms * occupancy_large<OffT>();
+    static const int occ = occupancy_of(k_count_large<LARGE_BLOCK, LARGE_CAP, OffT, HUB>, LARGE_BLOCK, LargeL<OffT>::bytes);
+    return num_sms * occ;
+}
+template <bool HUB>
+int count_grid_hub(int num_sms) {
+    if constexpr (!HUB) return 0;
+    static const int occ = occupancy_of(k_count_hub, 32 * HUB_WARPS, HUB_SMEM);
+    return num_sms * occ;
 }
 // Vertices per batch of the small kernel: 32, or fewer where the graph does not hold a batch of 32
 // for every resident warp (a power of two, at least 4: a warp's serial chain is then shorter).
@@ -1257,28 +1479,32 @@ int small_grid_launched(u64 n, int cap) {
     return (int)(need < 1 ? 1 : (need < (u64)cap ? need : (u64)cap));
 }
 
-template <typename OffT>
+template <typename OffT, bool HUB>
 int count_grid_auto(int num_sms) {
-    return count_grid_small<OffT>(num_sms) + count_grid_medium<OffT>(num_sms) + count_grid_large<OffT>(num_sms);
+    return count_grid_small<OffT, HUB>(num_sms) + count_grid_medium<OffT, HUB>(num_sms) +
+           count_grid_large<OffT, HUB>(num_sms) + count_grid_hub<HUB>(num_sms);
 }
 
-template <typename OffT>
+template <typename OffT, bool HUB>
 cudaError_t launch_count_auto(const u64* fo, const u32* head, u64 n, u64 nnz, const void* vdesc, const u32* headp,
-                              const uint2* mtiles, const uint2* ltiles, u32 small_d, u32 seg, u64* cnt, u64* partials,
+                              const HubState& hub, const uint2* mtiles, const uint2* ltiles, u32 small_d, u32 seg, u64* cnt, u64* partials,
                               Control* ctl, int num_sms, cudaStream_t st, cudaEvent_t after_small,
                               cudaEvent_t after_large, u32 copy_wait_polls) {
     (void)nnz;
-    const int cap = count_grid_small<OffT>(num_sms);
+    const int cap = count_grid_small<OffT, HUB>(num_sms);
     const int gs = small_grid_launched(n, cap);
-    const int gm = count_grid_medium<OffT>(num_sms);
-    const int gl = count_grid_large<OffT>(num_sms);
+    const int gm = count_grid_medium<OffT, HUB>(num_sms);
+    const int gl = count_grid_large<OffT, HUB>(num_sms);
     const auto* vd = reinterpret_cast<const Desc<OffT>*>(vdesc);
-    k_count_small<SMALL_BLOCK, OffT><<<gs, SMALL_BLOCK, SmallWarpLayout<OffT>::bytes(SMALL_BLOCK / 32), st>>>(
-        n, small_batch_vertices(n, cap), vd, headp, small_d, cnt, partials, ctl);
+    k_count_small<SMALL_BLOCK, OffT, HUB><<<gs, SMALL_BLOCK, SmallWarpLayout<OffT, HUB>::bytes(SMALL_BLOCK / 32), st>>>(
+        n, small_batch_vertices(n, cap), vd, headp, hub.lists, hub.ids, small_d, cnt, partials, ctl);
     if (after_small) cudaEventRecord(after_small, st);
-    k_count_medium<MEDIUM_BLOCK, OffT>
+    if constexpr (HUB)
+        k_count_hub<<<count_grid_hub<HUB>(num_sms), 32 * HUB_WARPS, HUB_SMEM, st>>>(
+            fo, head, vd, hub.lists, hub.ids, mtiles, ltiles, seg, cnt, partials + cap + gm + gl, ctl);
+    k_count_medium<MEDIUM_BLOCK, OffT, HUB>
         <<<gm, MEDIUM_BLOCK, MediumL::bytes, st>>>(fo, head, n, vd, headp, mtiles, seg, cnt, partials + cap, ctl);
-    k_count_large<LARGE_BLOCK, LARGE_CAP, OffT>
+    k_count_large<LARGE_BLOCK, LARGE_CAP, OffT, HUB>
         <<<gl, LARGE_BLOCK, LargeL<OffT>::bytes, st>>>(fo, head, n, vd, headp, ltiles, seg, cnt, partials + cap + gm,
                                                        ctl, copy_wait_polls);
     if (after_large) cudaEventRecord(after_large, st);
@@ -1296,40 +1522,33 @@ void launch_final(const u64* partials, u32 np, u64* total, Control* ctl, cudaStr
     k_final<<<1, 1024, 0, st>>>(partials, np, 0, 0, total, ctl);
 }
 
-template <typename OffT>
+template <typename OffT, bool HUB>
 void launch_final_auto(const u64* partials, u64 n, int num_sms, u64* total, Control* ctl, cudaStream_t st) {
-    const int cap = count_grid_small<OffT>(num_sms);
-    k_final<<<1, 1024, 0, st>>>(partials, (u32)count_grid_auto<OffT>(num_sms), (u32)small_grid_launched(n, cap),
+    const int cap = count_grid_small<OffT, HUB>(num_sms);
+    k_final<<<1, 1024, 0, st>>>(partials, (u32)count_grid_auto<OffT, HUB>(num_sms), (u32)small_grid_launched(n, cap),
                                 (u32)cap, total, ctl);
 }
 
-template <typename OffT>
-void launch_stats(const u64* fo, const u32* head, u64 n, const void* vdesc, const u32* headp, u32 small_d,
-                  u32 medium_d, Control* ctl, int num_sms, cudaStream_t st) {
+template <typename OffT, bool HUB>
+void launch_stats(const u64* fo, const u32* head, u64 n, const void* vdesc, const u32* headp, const HubState& hub,
+                  u32 small_d, u32 medium_d, Control* ctl, int num_sms, cudaStream_t st) {
     if (n == 0) return;
-    k_stats<OffT><<<num_sms * 8, 256, 0, st>>>(fo, head, n, reinterpret_cast<const Desc<OffT>*>(vdesc), headp,
-                                               small_d, medium_d, ctl);
+    k_stats<OffT, HUB><<<num_sms * 8, 256, 0, st>>>(fo, head, n, reinterpret_cast<const Desc<OffT>*>(vdesc), headp,
+                                                    hub.lists, hub.ids, small_d, medium_d, ctl);
 }
 
-template void launch_final_auto<u32>(const u64*, u64, int, u64*, Control*, cudaStream_t);
-template void launch_final_auto<u64>(const u64*, u64, int, u64*, Control*, cudaStream_t);
-template int count_grid_small<u32>(int);
-template int count_grid_small<u64>(int);
-template int count_grid_large<u32>(int);
-template int count_grid_large<u64>(int);
-template int count_grid_medium<u32>(int);
-template int count_grid_medium<u64>(int);
-template int count_grid_auto<u32>(int);
-template int count_grid_auto<u64>(int);
-template cudaError_t launch_count_auto<u32>(const u64*, const u32*, u64, u64, const void*, const u32*, const uint2*,
-                                            const uint2*, u32, u32, u64*, u64*, Control*, int, cudaStream_t,
-                                            cudaEvent_t, cudaEvent_t, u32);
-template cudaError_t launch_count_auto<u64>(const u64*, const u32*, u64, u64, const void*, const u32*, const uint2*,
-                                            const uint2*, u32, u32, u64*, u64*, Control*, int, cudaStream_t,
-                                            cudaEvent_t, cudaEvent_t, u32);
-template void launch_stats<u32>(const u64*, const u32*, u64, const void*, const u32*, u32, u32, Control*, int,
-                                cudaStream_t);
-template void launch_stats<u64>(const u64*, const u32*, u64, const void*, const u32*, u32, u32, Control*, int,
-                                cudaStream_t);
+#define KTRI_INST(OffT, HUB)                                                                                        \
+    template void launch_final_auto<OffT, HUB>(const u64*, u64, int, u64*, Control*, cudaStream_t);                 \
+    template int count_grid_auto<OffT, HUB>(int);                                                                   \
+    template cudaError_t launch_count_auto<OffT, HUB>(const u64*, const u32*, u64, u64, const void*, const u32*,    \
+                                                      const HubState&, const uint2*, const uint2*, u32, u32, u64*,  \
+                                                      u64*, Control*, int, cudaStream_t, cudaEvent_t, cudaEvent_t,  \
+                                                      u32);                                                         \
+    template void launch_stats<OffT, HUB>(const u64*, const u32*, u64, const void*, const u32*, const HubState&,    \
+                                          u32, u32, Control*, int, cudaStream_t);
+KTRI_INST(u32, false)
+KTRI_INST(u32, true)
+KTRI_INST(u64, false)
+#undef KTRI_INST
 
 }  // namespace ktri

@@ -9,6 +9,7 @@
 
 namespace ktri {
 
+using u16 = uint16_t;
 using u32 = uint32_t;
 using u64 = unsigned long long;
 
@@ -65,6 +66,34 @@ template <>
 __device__ __forceinline__ Desc<u64> load_desc<u64>(const Desc<u64>* p) {
     uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
     return Desc<u64>{(u64)v.x | ((u64)v.y << 32), v.z, 0};
+}
+
+// Split out-lists (hubs).  With hubs, an out-list is kept in two parts: the entries that are
+// not hubs (u32 ids, in the gapped array above) and the hubs (u16 hub indices, in a gapped array
+// of their own whose lists start on 16-byte boundaries).  The length word of a descriptor then
+// packs both: hubs in the high half, the others in the low half (both below 2^16, see HUB_MAX_NNZ).
+// The region of x in the hub array starts at align8(oriented start + 4x) and has room for deg(x)
+// entries; the array holds nnz + 7n + 32 entries.  A list is filled up to a
+// multiple of four entries with HUB_PAD, an index no hub has, so it can be read four at a time.
+constexpr u32 HUB_H = 32768;          // hub indices: 0 .. HUB_H - 2
+constexpr u32 HUB_PAD = HUB_H - 1;
+constexpr u32 HUB_MIN_DEGREE = 128;   // a hub's degree is at least this
+constexpr u32 HUB_BINS = 4096;        // degree bins of the hub choice: 7 fractional bits of log2
+constexpr u32 HUB_FLAG = 0x80000000u; // orientation key of a hub: HUB_FLAG | (HUB_H - 1 - index)
+constexpr u64 HUB_MAX_N = 1ull << 30;
+constexpr u64 HUB_MAX_NNZ = (1ull << 32) - 1;  // 2^16 or more out-neighbours need 2^32 adjacency entries
+template <bool HUB>
+__host__ __device__ __forceinline__ u32 rest_len(u32 d) { return HUB ? d & 0xFFFFu : d; }
+template <bool HUB>
+__host__ __device__ __forceinline__ u32 hub_len(u32 d) { return HUB ? d >> 16 : 0u; }
+template <bool HUB>
+__host__ __device__ __forceinline__ u32 list_len(u32 d) { return HUB ? (d & 0xFFFFu) + (d >> 16) : d; }
+__host__ __device__ __forceinline__ u64 hub_start(u64 list_start, u64 x) { return (list_start + 4 * x + 7) & ~7ull; }
+__host__ __device__ __forceinline__ u64 hub_capacity(u64 n, u64 nnz) { return nnz + 7 * n + 32; }
+// Degree bin: 128 bins per power of two (d > 0).
+__device__ __forceinline__ u32 degree_bin(u32 d) {
+    const u32 lg = 31 - __clz(d);
+    return lg * 128 + (lg >= 7 ? (d >> (lg - 7)) & 0x7Fu : (d << (7 - lg)) & 0x7Fu);
 }
 
 // Total order of the orientation, node_ordering::degree_outward: (deg, id).

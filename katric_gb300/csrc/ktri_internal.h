@@ -32,6 +32,8 @@ struct Options {
 // The device a context was created on, and its SM count.
 int ctx_device(const ktri_ctx* ctx);
 int ctx_num_sms(const ktri_ctx* ctx);
+// Keep a context's workspaces at what ktri_workspace_bytes reports (no split out-lists).
+void ctx_plain_lists(ktri_ctx* ctx);
 
 struct Control;
 struct EngineJob;
@@ -75,7 +77,11 @@ struct Control {
     unsigned long long medium_tiles;     // number of (owner, segment) tiles for medium owners
     unsigned long long medium_next;      // dynamic tile cursor of the medium-owner kernel
     unsigned long long stat_chunked;     // collect_stats: streamed entries times the owner's table chunks
-    unsigned long long pad[1];
+    unsigned long long hub_next;         // dynamic tile cursor of the hub kernel
+    uint32_t hubs;                       // number of hubs
+    uint32_t hub_bin;                    // smallest degree bin of the hubs
+    uint32_t prep_blocks;                // blocks of k_prep that have finished
+    uint32_t pad1;
 };
 
 }  // namespace ktri

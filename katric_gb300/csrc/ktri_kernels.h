@@ -9,6 +9,7 @@
 
 namespace ktri {
 
+using u16 = uint16_t;
 using u32 = uint32_t;
 using u64 = unsigned long long;
 
@@ -69,21 +70,33 @@ struct TriangleSink {
 #endif
 };
 
-void launch_prep(const u64* fo, u64 n, u64 nnz, u32* deg, u32* dplus, u64* cnt, u32* tile_i0, Control* ctl,
-                 int num_sms, cudaStream_t st);
+// Hubs of a count (see HUB_H): bins holds hub_bins_words() u32, tmp and ids HUB_H entries (ids[i] =
+// the vertex of hub i), lists hub_capacity(n, nnz) u16.  All null without hubs.
+struct HubState {
+    u32* bins = nullptr;
+    uint2* tmp = nullptr;
+    u32* ids = nullptr;
+    u16* lists = nullptr;
+    explicit operator bool() const { return lists != nullptr; }
+};
+u64 hub_bins_words();
+
+// Degrees, tile boundaries and, with hubs, the hub choice (deg then holds orientation keys).
+void launch_prep(const u64* fo, u64 n, u64 nnz, u32* deg, u32* dplus, u64* cnt, u32* tile_i0, const HubState& hub,
+                 Control* ctl, int num_sms, cudaStream_t st);
 // Orientation over the blocks [tile_begin, tile_end) of ORIENT_TILE diagonals (all by
 // default; a block holds ORIENT_BLOCK / 32 base tiles).  Block t reads adjacency slots below
 // (t + 1) * ORIENT_TILE + 1 only, so it may run as soon as that prefix of head is on the device.
 constexpr u64 ORIENT_TILE = (u64)ORIENT_BLOCK * ORIENT_IPT;
 u64 orient_tiles(u64 n, u64 nnz);
 void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* deg, const u32* tile_i0, u32* headp,
-                   u32* dplus, u32* spanning, Control* ctl, cudaStream_t st, u64 tile_begin = 0,
+                   const HubState& hub, u32* dplus, u32* spanning, Control* ctl, cudaStream_t st, u64 tile_begin = 0,
                    u64 tile_end = ~0ull);
 // Owner tiles: medium owners' tiles are written to mtiles, large owners' to ltiles (each
 // array holds large_tile_capacity entries).
-template <typename OffT>
-void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, uint2* mtiles, uint2* ltiles, u32 small_d,
-                 u32 medium_d, u32 seg, Control* ctl, int num_sms, cudaStream_t st);
+template <typename OffT, bool HUB>
+void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, const HubState& hub, uint2* mtiles,
+                 uint2* ltiles, u32 small_d, u32 medium_d, u32 seg, Control* ctl, int num_sms, cudaStream_t st);
 
 // Owner tiles reordered (*count tiles on the device) by a counting sort on a 12-bit key:
 // TILE_BY_VERTEX, the first vertex each segment streams (tiles that run together then stream
@@ -95,27 +108,29 @@ void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, uint2* mti
 enum : u32 { TILE_BY_VERTEX = 0, TILE_BY_DEGREE = 1, TILE_BY_COST = 2 };
 u64 tile_order_scratch_words();
 void launch_order_tiles(const u64* fo, const u32* head, const u32* dplus, u64 n, const uint2* tiles,
-                        const unsigned long long* count, u32 seg, u32 mode, u32* keys, u32* hist, uint2* sorted,
-                        Control* ctl, int num_sms, cudaStream_t st);
+                        const unsigned long long* count, u32 seg, u32 mode, bool hub, u32* keys, u32* hist,
+                        uint2* sorted, Control* ctl, int num_sms, cudaStream_t st);
 
-// Owner-side hash counting (KTRI_METHOD_AUTO).  partials needs small_grid + large_grid entries.
-template <typename OffT>
+// The counting kernels of KTRI_METHOD_AUTO.  partials needs count_grid_auto entries.  The hub
+// kernel runs where hub is set (HUB, 32-bit descriptors only).
+constexpr int HUB_WARPS = 23;        // warps of a hub kernel block (one block per SM)
+template <typename OffT, bool HUB>
 int count_grid_small(int num_sms);
-template <typename OffT>
+template <typename OffT, bool HUB>
 int count_grid_medium(int num_sms);
-template <typename OffT>
+template <typename OffT, bool HUB>
 int count_grid_large(int num_sms);
-template <typename OffT>
-int count_grid_auto(int num_sms);  // small + medium + large
-template <typename OffT>
+template <typename OffT, bool HUB>
+int count_grid_auto(int num_sms);  // small + medium + large + hub
+template <typename OffT, bool HUB>
 cudaError_t launch_count_auto(const u64* fo, const u32* head, u64 n, u64 nnz, const void* vdesc, const u32* headp,
-                              const uint2* mtiles, const uint2* ltiles, u32 small_d, u32 seg, u64* cnt, u64* partials,
-                              Control* ctl, int num_sms, cudaStream_t st, cudaEvent_t after_small,
-                              cudaEvent_t after_large, u32 copy_wait_polls = COPY_WAIT_POLLS);
+                              const HubState& hub, const uint2* mtiles, const uint2* ltiles, u32 small_d, u32 seg,
+                              u64* cnt, u64* partials, Control* ctl, int num_sms, cudaStream_t st,
+                              cudaEvent_t after_small, cudaEvent_t after_large, u32 copy_wait_polls = COPY_WAIT_POLLS);
 void launch_final(const u64* partials, u32 np, u64* total, Control* ctl, cudaStream_t st);
 // The total of an AUTO count (the small kernel's grid depends on n).
 int small_grid_launched(u64 n, int cap);
-template <typename OffT>
+template <typename OffT, bool HUB>
 void launch_final_auto(const u64* partials, u64 n, int num_sms, u64* total, Control* ctl, cudaStream_t st);
 
 // ---- the serving engine ------------------------------------------------------------------
@@ -191,9 +206,9 @@ void launch_graph_totals(const u64* cnt, const u64* graph_first, u64 num_graphs,
 
 // Work counters of the reference (wedge_checks, intersection_size_local) and of the AUTO
 // kernels, accumulated into the control block.
-template <typename OffT>
-void launch_stats(const u64* fo, const u32* head, u64 n, const void* vdesc, const u32* headp, u32 small_d,
-                  u32 medium_d, Control* ctl, int num_sms, cudaStream_t st);
+template <typename OffT, bool HUB>
+void launch_stats(const u64* fo, const u32* head, u64 n, const void* vdesc, const u32* headp, const HubState& hub,
+                  u32 small_d, u32 medium_d, Control* ctl, int num_sms, cudaStream_t st);
 
 // Sorted-list strategies (merge, binary search, binary, hybrid): sort out-lists by id, then
 // one warp per oriented edge.

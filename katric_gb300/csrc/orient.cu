@@ -18,8 +18,21 @@ namespace ktri {
 // Also tabulates the merge-path tile boundaries: vertex v covers the diagonals
 // [first_out[v] + v, first_out[v+1] + v] (its slots and its end event), so every boundary
 // k * TILE_BASE in that range crosses the path at vertex v.
-__global__ void k_prep(const u64* __restrict__ fo, u64 n, u64 nnz, u32* __restrict__ deg, u32* __restrict__ dplus,
-                       u64* __restrict__ cnt, u32* __restrict__ tile_i0, Control* ctl) {
+// HUB: also a histogram of the degrees from HUB_MIN_DEGREE on (hub_bins[0, HUB_BINS), zeroed by the
+// caller).  The block that finishes last turns it into the hub choice: the hubs are the vertices
+// of the highest bins that together hold fewer than HUB_H; hub_bins[HUB_BINS + b] receives the number
+// of hubs above bin b (the scatter's cursor) and hub_bins[2 * HUB_BINS + b] the same for the ranking.
+constexpr int PREP_BLOCK = 256;
+template <bool HUB>
+__global__ void __launch_bounds__(PREP_BLOCK) k_prep(const u64* __restrict__ fo, u64 n, u64 nnz, u32* __restrict__ deg,
+                                                     u32* __restrict__ dplus, u64* __restrict__ cnt,
+                                                     u32* __restrict__ tile_i0, u32* __restrict__ hub_bins,
+                                                     Control* ctl) {
+    __shared__ u32 s_bins[HUB ? HUB_BINS : 1];
+    if constexpr (HUB) {
+        for (u32 b = threadIdx.x; b < HUB_BINS; b += PREP_BLOCK) s_bins[b] = 0;
+        __syncthreads();
+    }
     const u64 stride = (u64)gridDim.x * blockDim.x;
     const u64 nt = (n + nnz + TILE_BASE - 1) / TILE_BASE;
     u32 err = 0;
@@ -36,12 +49,95 @@ __global__ void k_prep(const u64* __restrict__ fo, u64 n, u64 nnz, u32* __restri
         deg[v] = d;
         dplus[v] = 0;
         if (cnt) cnt[v] = 0;
+        if constexpr (HUB) {
+            if (d >= HUB_MIN_DEGREE) atomicAdd(&s_bins[degree_bin(d)], 1u);
+        }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         tile_i0[nt] = (u32)n;
         if (fo[0] != 0 || fo[n] != nnz) err |= DEV_ERR_DEGREE;
     }
     if (err) atomicOr(&ctl->err, err);
+    if constexpr (HUB) {
+        __shared__ u32 s_last;
+        __shared__ u32 s_warp[PREP_BLOCK / 32];
+        __shared__ u32 s_bin, s_hubs;
+        __syncthreads();
+        for (u32 b = threadIdx.x; b < HUB_BINS; b += PREP_BLOCK)
+            if (s_bins[b]) atomicAdd(&hub_bins[b], s_bins[b]);
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) s_last = atomicAdd(&ctl->prep_blocks, 1u) + 1 == gridDim.x;
+        __syncthreads();
+        if (!s_last) return;
+        // vertices above each bin, from the highest bin down (thread t holds PER bins)
+        constexpr int PER = HUB_BINS / PREP_BLOCK;
+        if (threadIdx.x == 0) {
+            s_bin = HUB_BINS;
+            s_hubs = 0;
+        }
+        u32 c[PER];
+        unsigned long long sum = 0;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            c[k] = __ldcg(&hub_bins[HUB_BINS - 1 - (threadIdx.x * PER + k)]);
+            sum += c[k];
+        }
+        // counts above 2 HUB_H do not matter: saturate, so that 32 bits hold every prefix
+        u32 total;
+        u32 run = block_exclusive_scan<PREP_BLOCK>(sum > 2 * HUB_H ? 2 * HUB_H : (u32)sum, s_warp, &total);
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const u32 b = HUB_BINS - 1 - (threadIdx.x * PER + k);
+            hub_bins[HUB_BINS + b] = run;
+            hub_bins[2 * HUB_BINS + b] = run;
+            const u32 next = run + (c[k] > 2 * HUB_H ? 2 * HUB_H : c[k]);
+            if (next < HUB_H) {
+                atomicMin(&s_bin, b);
+                atomicMax(&s_hubs, next);
+            }
+            run = next < 4 * HUB_H ? next : 4 * HUB_H;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            ctl->hub_bin = s_bin;
+            ctl->hubs = s_hubs;
+        }
+    }
+}
+
+// The hubs' vertices by bin, unordered inside a bin (with their degrees: the ranking below
+// overwrites deg).
+__global__ void k_hub_place(u64 n, const u32* __restrict__ deg, u32* __restrict__ hub_bins, uint2* __restrict__ hub_tmp,
+                            const Control* ctl) {
+    if (ctl->hubs == 0 || (ctl->err & DEV_ERR_MASK)) return;
+    const u32 low = ctl->hub_bin;
+    const u64 stride = (u64)gridDim.x * blockDim.x;
+    for (u64 v = (u64)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
+        const u32 d = deg[v];
+        if (d < HUB_MIN_DEGREE) continue;
+        const u32 b = degree_bin(d);
+        if (b >= low) hub_tmp[atomicAdd(&hub_bins[HUB_BINS + b], 1u)] = make_uint2((u32)v, d);
+    }
+}
+
+// Hub index = rank by (degree, id) from the top: the hubs above the bin plus those of the bin that
+// order higher.  key[v] (the degree of every other vertex) becomes the hub's orientation key, so
+// one gather gives a neighbour's place in the order and its hub index.
+__global__ void k_hub_rank(const u32* __restrict__ hub_bins, const uint2* __restrict__ hub_tmp, u32* __restrict__ hub_ids,
+                           u32* __restrict__ key, const Control* ctl) {
+    const u32 p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= ctl->hubs || (ctl->err & DEV_ERR_MASK)) return;
+    const uint2 me = hub_tmp[p];
+    const u32 b = degree_bin(me.y);
+    const u32 first = hub_bins[2 * HUB_BINS + b], count = hub_bins[b];
+    u32 r = first;
+    for (u32 q = first; q < first + count; ++q) {
+        const uint2 o = hub_tmp[q];
+        if (o.y > me.y || (o.y == me.y && o.x > me.x)) ++r;
+    }
+    hub_ids[r] = me.x;
+    key[me.x] = HUB_FLAG | (HUB_H - 1 - r);
 }
 
 // Orientation of one merge-path tile of W = 32 * IPT diagonals per warp.  The tile holds the
@@ -61,21 +157,18 @@ __global__ void k_prep(const u64* __restrict__ fo, u64 n, u64 nnz, u32* __restri
 // A list held by one tile keeps its input order.  A split list's pieces reserve their ranges
 // with one atomic each and are recorded in the spanning list by the tile that holds the list's
 // start.
-template <int BLOCK, int IPT>
-__global__ void __launch_bounds__(BLOCK) k_orient(const u64* __restrict__ fo, const u32* __restrict__ head, u64 n,
-                                                  u64 nnz, const u32* __restrict__ deg,
-                                                  const u32* __restrict__ tile_i0, u32* __restrict__ headp,
-                                                  u32* __restrict__ dplus, u32* __restrict__ spanning,
-                                                  Control* ctl, u64 tile_begin) {
+// HUB: deg holds orientation keys (the degree, or a hub's key above every degree), a kept entry that
+// is a hub goes to the hub array as its index and the others to headp, so a piece has two ranks
+// and two shares of its out-list's length word (hubs << 16 | others, as everywhere with hubs).
+template <int BLOCK, int IPT, bool HUB>
+__device__ __forceinline__ void orient_tile(uint2 (*s_info_all)[32 * IPT], u64 (*s_base_all)[32 * IPT],
+                                            const u64* __restrict__ fo, const u32* __restrict__ head, u64 n, u64 nnz,
+                                            const u32* __restrict__ deg, const u32* __restrict__ tile_i0,
+                                            u32* __restrict__ headp, u16* __restrict__ hubp, u32* __restrict__ dplus,
+                                            u32* __restrict__ spanning, Control* ctl, u64 tile_begin) {
     constexpr int W = 32 * IPT;
     constexpr int WARPS = BLOCK / 32;
     constexpr u32 FULL = 0xFFFFFFFFu;
-    __shared__ uint2 s_info_all[WARPS][W];  // at a piece's first slot: (window index + 1, degree)
-    // at a piece's first slot: the tile ranks (at its first slot, past its last slot), then the
-    // headp index of tile rank 0 for its entries
-    __shared__ u64 s_base_all[WARPS][W];
-
-    if (ctl->err & DEV_ERR_MASK) return;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const u64 total = n + nnz;
     const u64 tile = (tile_begin + blockIdx.x) * WARPS + wid;
@@ -111,29 +204,28 @@ __global__ void __launch_bounds__(BLOCK) k_orient(const u64* __restrict__ fo, co
     // tile); their bounds stay in registers for the piece pass
     const bool have0 = (u32)lane < nwin;
     const u64 a0 = have0 ? fo[i0 + lane] : 0, b0 = have0 ? fo[i0 + lane + 1] : 0;
-    const u64 fo_i0 = __shfl_sync(FULL, a0, 0), fo_i0_end = __shfl_sync(FULL, b0, 0);
     if (have0 && b0 > a0 && a0 < j1 && b0 > j0)
-        s_info[a0 > j0 ? a0 - j0 : 0] = make_uint2((u32)lane + 1, (u32)(b0 - a0));
+        s_info[a0 > j0 ? a0 - j0 : 0] = make_uint2((u32)lane + 1, HUB ? __ldg(deg + i0 + lane) : (u32)(b0 - a0));
     for (u32 k = 32 + lane; k < nwin; k += 32) {
         const u64 v = i0 + k;
         const u64 a = fo[v], b = fo[v + 1];
-        if (b > a && a < j1 && b > j0) s_info[a - j0] = make_uint2(k + 1, (u32)(b - a));
+        if (b > a && a < j1 && b > j0) s_info[a - j0] = make_uint2(k + 1, HUB ? __ldg(deg + v) : (u32)(b - a));
     }
     __syncwarp();
-    const bool first_before = fo_i0 < j0;  // the first piece continues a list begun before the tile
-    // the first vertex's list continues past the tile
-    const bool first_past = fo_i0_end > j1;
+    // the tile's last list continues past the tile
+    const bool last_past = fo[last_v] < j1 && fo[last_v + 1] > j1;
     const u32 lt = (1u << lane) - 1u, le = lt | (1u << lane);
     const u32 i0_32 = (u32)i0;
 
-    u32 s0_r[IPT], km_r[IPT];
-    u32 rank = 0;                // kept entries of the tile before this iteration
+    u32 s0_r[IPT], km_r[IPT], hm_r[HUB ? IPT : 1];
+    u32 rank = 0;                // kept entries of the tile before this iteration (HUB: hubs << 16 | others)
     u32 s0c = 0, kc = 0, dc = 0;  // the piece open at the end of the previous iteration
     bool bad_id = false, self_loop = false, dup = false, unsorted = false;
 #pragma unroll
     for (int it = 0; it < IPT; ++it) {
         s0_r[it] = 0;
         km_r[it] = 0;
+        if constexpr (HUB) hm_r[it] = 0;
         if ((u32)it * 32 >= ns) continue;
         const u32 s = (u32)it * 32 + lane;
         const bool valid = s < ns;
@@ -154,20 +246,24 @@ __global__ void __launch_bounds__(BLOCK) k_orient(const u64* __restrict__ fo, co
         self_loop |= valid && in_range && y == x;
         const u32 dy = dy_r[it];
         const bool kept = valid && in_range && y != x && (dx < dy || (dx == dy && x < y));
-        const u32 km = __ballot_sync(FULL, kept);
+        u32 km = __ballot_sync(FULL, kept), hm = 0;
+        if constexpr (HUB) {
+            hm = __ballot_sync(FULL, kept && dy >= HUB_FLAG);
+            km &= ~hm;
+        }
         const bool last_slot = s + 1 == ns;
         bool next_start;
         if (lane < 31) next_start = (starts >> (lane + 1)) & 1u;
         else next_start = valid && !last_slot && s_info[s + 1].x != 0;
         // tile ranks at the piece's first slot and past its last slot
-        if (valid && info.x != 0) s_rank[s].x = rank + __popc(km & lt);
-        if (valid && (last_slot || next_start)) s_rank[s0].y = rank + __popc(km & le);
+        if (valid && info.x != 0) s_rank[s].x = rank + __popc(km & lt) + (HUB ? __popc(hm & lt) << 16 : 0u);
+        if (valid && (last_slot || next_start))
+            s_rank[s0].y = rank + __popc(km & le) + (HUB ? __popc(hm & le) << 16 : 0u);
         // the next slot's neighbour (the next lane's, or lane 0's of the next iteration) when it
         // belongs to the same list: adjacent duplicates and order
         const u32 nd = __shfl_down_sync(FULL, y, 1);
         const u32 nn = __shfl_sync(FULL, y_r[it + 1 < IPT ? it + 1 : it], 0);
-        const bool past = (k1 == 1 && first_before) ? first_past : dx > ns - s0;
-        const bool same = valid && (last_slot ? past : !next_start);
+        const bool same = valid && (last_slot ? last_past : !next_start);
         if (same) {
             const u32 nx = last_slot ? __ldcs(head + j1) : (lane < 31 ? nd : nn);
             unsorted |= nx < y;
@@ -176,9 +272,10 @@ __global__ void __launch_bounds__(BLOCK) k_orient(const u64* __restrict__ fo, co
         s0c = __shfl_sync(FULL, s0, 31);
         kc = __shfl_sync(FULL, k1, 31);
         dc = __shfl_sync(FULL, dx, 31);
-        rank += __popc(km);
+        rank += __popc(km) + (HUB ? __popc(hm) << 16 : 0u);
         s0_r[it] = s0;
         km_r[it] = km;
+        if constexpr (HUB) hm_r[it] = hm;
     }
     const u32 err = (bad_id ? DEV_ERR_ID_RANGE : 0u) | (self_loop ? DEV_ERR_SELF_LOOP : 0u) |
                     (dup ? DEV_ERR_DUPLICATE : 0u);
@@ -186,6 +283,7 @@ __global__ void __launch_bounds__(BLOCK) k_orient(const u64* __restrict__ fo, co
     if (unsorted) atomicOr(&ctl->err, DEV_FLAG_UNSORTED);
     __syncwarp();
     // piece pass: out-degree shares and where each piece's kept entries go
+    const u64 ref = oriented_start(j0, i0), href = hub_start(ref, i0);  // HUB: origins of the 32-bit indices
     {
         auto settle = [&](u64 v, u64 a, u64 b) {
             if (!(b > a && a < j1 && b > j0)) return;
@@ -199,7 +297,15 @@ __global__ void __launch_bounds__(BLOCK) k_orient(const u64* __restrict__ fo, co
             } else {
                 dplus[v] = cnt;
             }
-            s_base[s0] = oriented_start(a, v) + carry - rk.x;
+            const u64 start = oriented_start(a, v);
+            if constexpr (HUB) {
+                // differences stay below 2^31: a list begins at most its degree before the tile
+                const u32 to = (u32)(start - ref) + (carry & 0xFFFFu) - (rk.x & 0xFFFFu);
+                const u32 hto = (u32)(hub_start(start, v) - href) + (carry >> 16) - (rk.x >> 16);
+                s_base[s0] = (u64)to | ((u64)hto << 32);
+            } else {
+                s_base[s0] = start + carry - rk.x;
+            }
         };
         if (have0) settle(i0 + lane, a0, b0);
         for (u32 k = 32 + lane; k < nwin; k += 32) {
@@ -212,15 +318,54 @@ __global__ void __launch_bounds__(BLOCK) k_orient(const u64* __restrict__ fo, co
 #pragma unroll
     for (int it = 0; it < IPT; ++it) {
         const u32 km = km_r[it];
-        if ((km >> lane) & 1u) __stcs(headp + s_base[s0_r[it]] + rank + __popc(km & lt), y_r[it]);
-        rank += __popc(km);
+        if constexpr (HUB) {
+            const u32 hm = hm_r[it];
+            if (((km | hm) >> lane) & 1u) {
+                const u64 base = s_base[s0_r[it]];
+                if ((km >> lane) & 1u) {
+                    const u32 at = (u32)base + (rank & 0xFFFFu) + __popc(km & lt);
+                    __stcs(headp + ref + (long long)(int)at, y_r[it]);
+                } else {
+                    const u32 at = (u32)(base >> 32) + (rank >> 16) + __popc(hm & lt);
+                    __stcs(hubp + href + (long long)(int)at, (u16)(HUB_H - 1 - (dy_r[it] & ~HUB_FLAG)));
+                }
+            }
+            rank += __popc(km) + (__popc(hm) << 16);
+        } else {
+            if ((km >> lane) & 1u) __stcs(headp + s_base[s0_r[it]] + rank + __popc(km & lt), y_r[it]);
+            rank += __popc(km);
+        }
     }
+}
+
+// One tile per warp.  HUB: a graph without hubs (hubs = 0) runs the plain body, whose lists and
+// length words are then the same.
+template <int BLOCK, int IPT, bool HUB>
+__global__ void __launch_bounds__(BLOCK, 4) k_orient(const u64* __restrict__ fo, const u32* __restrict__ head, u64 n,
+                                                     u64 nnz, const u32* __restrict__ deg,
+                                                     const u32* __restrict__ tile_i0, u32* __restrict__ headp,
+                                                     u16* __restrict__ hubp, u32* __restrict__ dplus,
+                                                     u32* __restrict__ spanning, Control* ctl, u64 tile_begin) {
+    // at a piece's first slot: (window index + 1, key)
+    __shared__ uint2 s_info_all[BLOCK / 32][32 * IPT];
+    // at a piece's first slot: the tile ranks (at its first slot, past its last slot), then the
+    // headp index of tile rank 0 for its entries (HUB: the indices in both arrays relative to where
+    // the tile's first vertex would start, 32 bits each)
+    __shared__ u64 s_base_all[BLOCK / 32][32 * IPT];
+    if (ctl->err & DEV_ERR_MASK) return;
+    if (HUB && ctl->hubs)
+        orient_tile<BLOCK, IPT, true>(s_info_all, s_base_all, fo, head, n, nnz, deg, tile_i0, headp, hubp, dplus,
+                                      spanning, ctl, tile_begin);
+    else
+        orient_tile<BLOCK, IPT, false>(s_info_all, s_base_all, fo, head, n, nnz, deg, tile_i0, headp, nullptr, dplus,
+                                       spanning, ctl, tile_begin);
 }
 
 // Out-list descriptors, and the (owner, segment) tiles of owners above the small
 // out-degree threshold.
-template <typename OffT>
+template <typename OffT, bool HUB>
 __global__ void k_desc(const u64* __restrict__ fo, u64 n, const u32* __restrict__ dplus, Desc<OffT>* __restrict__ vdesc,
+                       u16* __restrict__ hubp,
                        uint2* __restrict__ mtiles, uint2* __restrict__ ltiles, u32 small_d, u32 medium_d, u32 seg,
                        Control* ctl) {
     if (ctl->err & DEV_ERR_MASK) return;
@@ -238,10 +383,14 @@ __global__ void k_desc(const u64* __restrict__ fo, u64 n, const u32* __restrict_
             ds.d = d;
             if constexpr (sizeof(OffT) == 8) ds.pad = 0;
             vdesc[v] = ds;
+            if constexpr (HUB) {
+                const u64 hs = hub_start(list_start(ds), v);
+                for (u32 k = hub_len<HUB>(d); k & 3u; ++k) hubp[hs + k] = (u16)HUB_PAD;
+            }
             // no tiles at all without tile arrays (the reference strategies pass none)
-            const bool tiled = mtiles && ltiles && d > small_d;
+            const bool tiled = mtiles && ltiles && list_len<HUB>(d) > small_d;
             const u32 nt = tiled ? (u32)((b - a + seg - 1) / seg) : 0u;
-            if (d > medium_d) nl = nt;
+            if (list_len<HUB>(d) > medium_d) nl = nt;
             else nm = nt;
         }
         // warp-aggregated reservation of tile slots, one list per owner class
@@ -275,12 +424,12 @@ constexpr u32 TILE_BUCKETS = 4096;
 // streams; (TILE_BY_DEGREE): the owner's out-degree, largest first (longest tiles first);
 // (TILE_BY_COST): the key k_tile_cost left in keys[t].
 __device__ __forceinline__ u32 tile_key(const u64* fo, const u32* head, const u32* dplus, uint2 tl, u32 seg,
-                                        u32 shift, u32 mode, const u32* keys, u64 t) {
+                                        u32 shift, u32 mode, bool hub, const u32* keys, u64 t) {
     u32 key;
     if (mode == TILE_BY_COST) {
         key = keys[t];
     } else if (mode == TILE_BY_DEGREE) {
-        const u32 d = dplus[tl.x];
+        const u32 d = hub ? list_len<true>(dplus[tl.x]) : dplus[tl.x];
         key = d >= TILE_BUCKETS ? 0u : TILE_BUCKETS - 1 - d;
     } else {
         key = __ldg(head + fo[tl.x] + (u64)tl.y * seg) >> shift;
@@ -295,7 +444,7 @@ __device__ __forceinline__ u32 tile_key(const u64* fo, const u32* head, const u3
 // log scale (7 fractional bits).
 __global__ void k_tile_cost(const u64* __restrict__ fo, const u32* __restrict__ head, const u32* __restrict__ dplus,
                             const uint2* __restrict__ tiles, const unsigned long long* count, u32 seg,
-                            u32* __restrict__ keys, Control* ctl) {
+                            bool hub, u32* __restrict__ keys, Control* ctl) {
     if (ctl->err & DEV_ERR_MASK) return;
     const u64 nt = *(volatile const unsigned long long*)count;
     const int lane = threadIdx.x & 31;
@@ -303,12 +452,12 @@ __global__ void k_tile_cost(const u64* __restrict__ fo, const u32* __restrict__ 
     for (u64 t = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += nwarps) {
         const uint2 tl = tiles[t];
         const u64 x = tl.x;
-        const u32 dx = dplus[x];
+        const u32 dx = hub ? list_len<true>(dplus[x]) : dplus[x];
         const u64 a = fo[x] + (u64)tl.y * seg, e1 = fo[x + 1], b = a + seg < e1 ? a + seg : e1;
         u64 cost = 0;
         for (u64 e = a + lane; e < b; e += 32) {
             const u32 y = __ldg(head + e);
-            const u32 dy = __ldg(dplus + y);
+            const u32 word = __ldg(dplus + y), dy = hub ? list_len<true>(word) : word;
             if (dy > 0 && key_less(dy, y, dx, x)) cost += dy;
         }
 #pragma unroll
@@ -341,7 +490,7 @@ __global__ void __launch_bounds__(TILE_ORDER_BLOCK) k_tile_hist(const u64* __res
                                                                 const u32* __restrict__ dplus,
                                                                 const uint2* __restrict__ tiles,
                                                                 const unsigned long long* count, u32 seg, u32 shift,
-                                                                u32 mode, u32* __restrict__ keys, u32* hist,
+                                                                u32 mode, bool hub, u32* __restrict__ keys, u32* hist,
                                                                 Control* ctl) {
     __shared__ u32 s_cnt[TILE_BUCKETS];
     if (ctl->err & DEV_ERR_MASK) return;
@@ -352,7 +501,7 @@ __global__ void __launch_bounds__(TILE_ORDER_BLOCK) k_tile_hist(const u64* __res
     for (u32 k = threadIdx.x; k < TILE_BUCKETS; k += TILE_ORDER_BLOCK) s_cnt[k] = 0;
     __syncthreads();
     for (u64 t = t0 + threadIdx.x; t < t1; t += TILE_ORDER_BLOCK) {
-        const u32 key = tile_key(fo, head, dplus, tiles[t], seg, shift, mode, keys, t);
+        const u32 key = tile_key(fo, head, dplus, tiles[t], seg, shift, mode, hub, keys, t);
         if (mode != TILE_BY_COST) keys[t] = key;
         atomicAdd(&s_cnt[key], 1u);
     }
@@ -412,54 +561,73 @@ __global__ void __launch_bounds__(TILE_ORDER_BLOCK) k_tile_scatter(const uint2* 
 u64 tile_order_scratch_words() { return TILE_BUCKETS; }
 
 void launch_order_tiles(const u64* fo, const u32* head, const u32* dplus, u64 n, const uint2* tiles,
-                        const unsigned long long* count, u32 seg, u32 mode, u32* keys, u32* hist, uint2* sorted,
-                        Control* ctl, int num_sms, cudaStream_t st) {
+                        const unsigned long long* count, u32 seg, u32 mode, bool hub, u32* keys, u32* hist,
+                        uint2* sorted, Control* ctl, int num_sms, cudaStream_t st) {
     if (n == 0) return;
     u32 bits = 0;
     while ((1ull << bits) < n) ++bits;
     const u32 shift = bits > 12 ? bits - 12 : 0;
     cudaMemsetAsync(hist, 0, sizeof(u32) * TILE_BUCKETS, st);
     if (mode == TILE_BY_COST)
-        k_tile_cost<<<num_sms * 8, 256, 0, st>>>(fo, head, dplus, tiles, count, seg, keys, ctl);
-    k_tile_hist<<<num_sms * 4, TILE_ORDER_BLOCK, 0, st>>>(fo, head, dplus, tiles, count, seg, shift, mode, keys, hist,
-                                                          ctl);
+        k_tile_cost<<<num_sms * 8, 256, 0, st>>>(fo, head, dplus, tiles, count, seg, hub, keys, ctl);
+    k_tile_hist<<<num_sms * 4, TILE_ORDER_BLOCK, 0, st>>>(fo, head, dplus, tiles, count, seg, shift, mode, hub, keys,
+                                                          hist, ctl);
     k_tile_scan<<<1, TILE_SCAN_BLOCK, 0, st>>>(hist, ctl);
     k_tile_scatter<<<num_sms * 4, TILE_ORDER_BLOCK, 0, st>>>(tiles, count, keys, hist, sorted, ctl);
 }
 
-void launch_prep(const u64* fo, u64 n, u64 nnz, u32* deg, u32* dplus, u64* cnt, u32* tile_i0, Control* ctl,
-                 int num_sms, cudaStream_t st) {
+void launch_prep(const u64* fo, u64 n, u64 nnz, u32* deg, u32* dplus, u64* cnt, u32* tile_i0, const HubState& hub,
+                 Control* ctl, int num_sms, cudaStream_t st) {
     if (n == 0) return;
-    u64 blocks = (n + 255) / 256;
-    u64 cap = (u64)num_sms * 8;
-    k_prep<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(fo, n, nnz, deg, dplus, cnt, tile_i0, ctl);
+    const u64 blocks = (n + PREP_BLOCK - 1) / PREP_BLOCK;
+    const u64 cap = (u64)num_sms * 8;
+    const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
+    if (!hub) {
+        k_prep<false><<<grid, PREP_BLOCK, 0, st>>>(fo, n, nnz, deg, dplus, cnt, tile_i0, nullptr, ctl);
+        return;
+    }
+    cudaMemsetAsync(hub.bins, 0, sizeof(u32) * HUB_BINS, st);
+    k_prep<true><<<grid, PREP_BLOCK, 0, st>>>(fo, n, nnz, deg, dplus, cnt, tile_i0, hub.bins, ctl);
+    k_hub_place<<<grid, 256, 0, st>>>(n, deg, hub.bins, hub.tmp, ctl);
+    k_hub_rank<<<HUB_H / 128, 128, 0, st>>>(hub.bins, hub.tmp, hub.ids, deg, ctl);
 }
+
+u64 hub_bins_words() { return 3ull * HUB_BINS; }
 
 u64 orient_tiles(u64 n, u64 nnz) { return (n + nnz + ORIENT_TILE - 1) / ORIENT_TILE; }
 
 void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* deg, const u32* tile_i0, u32* headp,
-                   u32* dplus, u32* spanning, Control* ctl, cudaStream_t st, u64 tile_begin, u64 tile_end) {
+                   const HubState& hub, u32* dplus, u32* spanning, Control* ctl, cudaStream_t st, u64 tile_begin,
+                   u64 tile_end) {
     constexpr int BLOCK = ORIENT_BLOCK, IPT = ORIENT_IPT;
     const u64 tiles = orient_tiles(n, nnz);
     if (tile_end > tiles) tile_end = tiles;
     if (tile_begin >= tile_end) return;
-    k_orient<BLOCK, IPT><<<(unsigned)(tile_end - tile_begin), BLOCK, 0, st>>>(fo, head, n, nnz, deg, tile_i0, headp,
-                                                                             dplus, spanning, ctl, tile_begin);
+    const unsigned grid = (unsigned)(tile_end - tile_begin);
+    if (hub)
+        k_orient<BLOCK, IPT, true><<<grid, BLOCK, 0, st>>>(fo, head, n, nnz, deg, tile_i0, headp, hub.lists, dplus,
+                                                           spanning, ctl, tile_begin);
+    else
+        k_orient<BLOCK, IPT, false><<<grid, BLOCK, 0, st>>>(fo, head, n, nnz, deg, tile_i0, headp, nullptr, dplus,
+                                                            spanning, ctl, tile_begin);
 }
 
-template <typename OffT>
-void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, uint2* mtiles, uint2* ltiles, u32 small_d,
+template <typename OffT, bool HUB>
+void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, const HubState& hub, uint2* mtiles, uint2* ltiles, u32 small_d,
                  u32 medium_d, u32 seg, Control* ctl, int num_sms, cudaStream_t st) {
     if (n == 0) return;
     u64 blocks = (n + 255) / 256;
     u64 cap = (u64)num_sms * 8;
-    k_desc<OffT><<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(
-        fo, n, dplus, reinterpret_cast<Desc<OffT>*>(vdesc), mtiles, ltiles, small_d, medium_d, seg, ctl);
+    k_desc<OffT, HUB><<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(
+        fo, n, dplus, reinterpret_cast<Desc<OffT>*>(vdesc), hub.lists, mtiles, ltiles, small_d, medium_d, seg, ctl);
 }
 
-template void launch_desc<u32>(const u64*, u64, const u32*, void*, uint2*, uint2*, u32, u32, u32, Control*, int,
-                               cudaStream_t);
-template void launch_desc<u64>(const u64*, u64, const u32*, void*, uint2*, uint2*, u32, u32, u32, Control*, int,
-                               cudaStream_t);
+#define KTRI_INST(OffT, HUB)                                                                                     \
+    template void launch_desc<OffT, HUB>(const u64*, u64, const u32*, void*, const HubState&, uint2*, uint2*,    \
+                                         u32, u32, u32, Control*, int, cudaStream_t);
+KTRI_INST(u32, false)
+KTRI_INST(u32, true)
+KTRI_INST(u64, false)
+#undef KTRI_INST
 
 }  // namespace ktri

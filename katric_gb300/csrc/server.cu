@@ -916,6 +916,7 @@ int ktri_server_create(int device, const ktri_server_opts* opts, ktri_server** o
     int rc = KTRI_OK;
     for (Slot& sl : s->slots) {
         rc = ktri_ctx_create(device, &sl.ctx);
+        if (rc == KTRI_OK) ktri::ctx_plain_lists(sl.ctx);  // the budget counts ktri_workspace_bytes per batch
         if (rc) break;
         cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking);
         cudaEventCreate(&sl.start);
