@@ -66,7 +66,7 @@ struct Layout {
            spanning = 0,
            partials = 0, cnt = 0,
            total = 0, mid = 0, big = 0, scratch = 0, in_fo = 0, in_head = 0, hub_bins = 0, hub_tmp = 0,
-           hub_ids = 0, hub_lists = 0, bytes = 0;
+           hub_ids = 0, hub_lists = 0, top_info = 0, top_long = 0, top_bits = 0, bytes = 0;
     bool wide = false;
     bool hub = false;  // split out-lists (AUTO with 32-bit descriptors)
     u64 scratch_per_block = 0;
@@ -138,6 +138,9 @@ Layout make_layout(u64 n, u64 nnz, int32_t method, int num_sms, bool with_inputs
         L.hub_tmp = take(sizeof(uint2) * ktri::HUB_H);
         L.hub_ids = take(sizeof(u32) * ktri::HUB_H);
         L.hub_lists = take(sizeof(ktri::u16) * ktri::hub_capacity(n, nnz));
+        L.top_info = take(sizeof(u32) * n);
+        L.top_long = take(sizeof(u32) * ktri::hub_long_capacity(nnz));
+        L.top_bits = take(ktri::HUB_TOP / 8 * ktri::hub_top_capacity(nnz));
     }
     L.bytes = off;
     return L;
@@ -384,6 +387,10 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
         hub.tmp = reinterpret_cast<uint2*>(base + L.hub_tmp);
         hub.ids = reinterpret_cast<u32*>(base + L.hub_ids);
         hub.lists = reinterpret_cast<ktri::u16*>(base + L.hub_lists);
+        hub.top_info = reinterpret_cast<u32*>(base + L.top_info);
+        hub.top_long = reinterpret_cast<u32*>(base + L.top_long);
+        hub.top_bits = reinterpret_cast<uint2*>(base + L.top_bits);
+        hub.top_cap = (u32)ktri::hub_top_capacity(nnz);
     }
 
     // an error a caller's own failed runtime call left in this thread must not be taken for a
@@ -441,6 +448,7 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
         ktri::launch_stats<OffT, HUB>(fo, head, n, vdesc, headp, hub, opt.small_outdegree,
                                  autom ? opt.medium_outdegree : 0xFFFFFFFFu, ctl, sms, st);
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[2], st));
+    if (HUB) ktri::launch_hub_tops(vdesc, hub, ctl, sms, st);  // after the work counters, which read whole lists
     if (sort_all) {
         // orientation export only: no counting
     } else if (autom && publish) {

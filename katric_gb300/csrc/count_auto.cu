@@ -909,66 +909,122 @@ __global__ void __launch_bounds__(BLOCK)
 // entry costs two bytes of L2 traffic instead of four.
 // A block holds one counter per hub for its whole life and flushes them once, so a tile clears
 // nothing but its bitmap.  Each warp takes its own (owner, segment) tiles and has its own bitmap.
-// Lists above HUB_LANE entries are streamed by the whole warp, four consecutive entries per lane (so
-// that a sorted list's lanes read neighbouring words), the shorter ones one per lane.
+// Lists above HUB_LANE entries are streamed in units of 64 entries by eight lanes each, eight
+// consecutive entries per lane, the shorter ones one per lane.  The densest part of the lists, the
+// first HUB_TOP hubs, does not go through the lists where that pays: half of the streamed lists of
+// RMAT-24 keep 45 % of the streamed hub entries in bitmaps of 256 bytes (81 MB in all), and one
+// AND, a population count and 3.5 additions per word count 32 of them (TopCounters).
+// Measured (medium and large tiles, RMAT n = 10^6 / RMAT-24): ids through filters and hash tables
+// 4.31 / 119.4 ms; hub lists, one list per warp 1.90 / 74.7 ms; with the top bitmaps and units
+// 1.50 / 71.6 ms, of which this kernel takes 1.4 / 43 ms.  What is left: on RMAT-24 the lists'
+// reads (2.9 TB/s from L2 at a 70 % hit rate, 22 warps per SM beside 128 KB of counters), on
+// smaller graphs instruction issue.
 struct HubLayout {
     static constexpr u32 BITS = HUB_H / 32;  // bitmap words of a warp
     static constexpr u32 off_bits = 0;       // the warps' bitmaps, each aligned to its own size
     static constexpr u32 off_cnt = sizeof(u32) * BITS * HUB_WARPS;  // u32 counter per hub
+    static constexpr u32 off_queue = off_cnt + sizeof(u32) * HUB_H;  // the warps' top bitmaps of a chunk
     static constexpr u32 align = sizeof(u32) * BITS;
-    static constexpr size_t bytes = off_cnt + sizeof(u32) * HUB_H;
+    static constexpr size_t bytes = off_queue + sizeof(u32) * 32 * HUB_WARPS;
 };
 constexpr size_t HUB_SMEM = HubLayout::bytes + HubLayout::align;  // room to align the bitmaps
-constexpr u32 HUB_LANE = 16;                       // hub lists up to this length are streamed by one lane
+constexpr u32 HUB_LANE = 8;                        // hub lists up to this length are streamed by one lane
 constexpr u32 HUB_PAD2 = HUB_PAD | (HUB_PAD << 16);  // two entries that hit nothing
 
-// Two entries of a hub list looked up in the bitmap at shared address `bits` (aligned to its size):
-// counts the hits at the hubs' counters (shared address cnt) and returns their number.  A miss
-// counts at the spare word instead: a predicated reduction becomes a branch around it (four more
-// instructions per entry, and with a hit in almost every row it skips nothing; 2.12 against 1.90 ms
-// on RMAT n = 10^6).
-__device__ __forceinline__ u32 hub_probe2(u32 pair, u32 bits, u32 cnt, u32 spare) {
-    u32 found;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, q;\n\t"
-        ".reg .u32 a, b, h, k, v, w;\n\t"
-        "and.b32 h, %1, 0xFFFF;\n\t"
-        "shr.u32 k, %1, 16;\n\t"
-        "shr.u32 a, %1, 3;\n\t"
-        "shr.u32 b, %1, 19;\n\t"
-        "lop3.b32 a, a, %4, %2, 0xEA;\n\t"  // (a & mask) | bits
-        "lop3.b32 b, b, %4, %2, 0xEA;\n\t"
-        "ld.shared.u32 v, [a];\n\t"
-        "ld.shared.u32 w, [b];\n\t"
-        "shf.r.wrap.b32 v, v, v, h;\n\t"
-        "shf.r.wrap.b32 w, w, w, k;\n\t"
-        "and.b32 v, v, 1;\n\t"
-        "and.b32 w, w, 1;\n\t"
-        "setp.ne.u32 p, v, 0;\n\t"
-        "setp.ne.u32 q, w, 0;\n\t"
-        "mad.lo.u32 h, h, 4, %3;\n\t"
-        "mad.lo.u32 k, k, 4, %3;\n\t"
-        "selp.u32 h, h, %5, p;\n\t"
-        "selp.u32 k, k, %5, q;\n\t"
-        "red.shared.add.u32 [h], 1;\n\t"
-        "red.shared.add.u32 [k], 1;\n\t"
-        "add.u32 %0, v, w;\n\t"
-        "}"
-        : "=r"(found)
-        : "r"(pair), "r"(bits), "r"(cnt), "n"(HUB_H / 8 - 4), "r"(spare)
-        : "memory");
+// Eight entries of a hub list looked up in the bitmap at shared address `bits` (aligned to its
+// size): counts the hits at the hubs' counters (shared address spare + base4) and returns their
+// number.  A miss counts at the spare word: a predicated reduction becomes a branch around it (four
+// more instructions per entry, and with a hit in almost every row it skips nothing; 2.12 against
+// 1.90 ms on RMAT n = 10^6), and the address comes from a multiplication by the bit, since the
+// logic units are the busiest (72 % with compares and selects).  All reads go out before the
+// first test.
+__device__ __forceinline__ u32 hub_probe8(const uint4& w, u32 bits, u32 base4, u32 spare) {
+    const u32 pair[4] = {w.x, w.y, w.z, w.w};
+    u32 h[8], v[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        h[2 * i] = pair[i] & 0xFFFFu;
+        h[2 * i + 1] = pair[i] >> 16;
+        const u32 a0 = ((pair[i] >> 3) & (HUB_H / 8 - 4)) | bits;
+        const u32 a1 = ((pair[i] >> 19) & (HUB_H / 8 - 4)) | bits;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v[2 * i]) : "r"(a0) : "memory");
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v[2 * i + 1]) : "r"(a1) : "memory");
+    }
+    u32 found = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const u32 hit = __funnelshift_r(v[i], v[i], h[i]) & 1u;
+        const u32 at = (h[i] * 4 + base4) * hit + spare;
+        asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(at) : "memory");
+        found += hit;
+    }
     return found;
 }
 
+// A warp's hit counts of the first HUB_TOP hubs, bit-sliced: lane l holds the words 2 l and 2 l + 1,
+// plane p the bits of weight 2^p of 64 counters.  Four masks are added by carry-save adders, so a
+// mask costs about 3.5 logic instructions per word instead of one atomic per hit.
+struct TopCounters {
+    static constexpr int PLANES = 11;
+    u32 c[PLANES][2];
+    u32 pend[2];     // a carry of weight 4 not yet added
+    u32 added, odd;  // masks since the last flush; whether pend holds one
+    static __device__ __forceinline__ u32 csa(u32& a, u32 b, u32 d) {  // a + b + d: sum bit to a, carry returned
+        const u32 carry = (a & b) | (a & d) | (b & d);
+        a = a ^ b ^ d;
+        return carry;
+    }
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int p = 0; p < PLANES; ++p) c[p][0] = c[p][1] = 0;
+        pend[0] = pend[1] = 0;
+        added = odd = 0;
+    }
+    __device__ __forceinline__ void add4(const uint2 (&m)[4], u32* hcnt, u32 lane) {
+        u32 four[2];
+        four[0] = csa(c[1][0], csa(c[0][0], m[0].x, m[1].x), csa(c[0][0], m[2].x, m[3].x));
+        four[1] = csa(c[1][1], csa(c[0][1], m[0].y, m[1].y), csa(c[0][1], m[2].y, m[3].y));
+        if (odd) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                u32 carry = csa(c[2][k], pend[k], four[k]);
+#pragma unroll
+                for (int p = 3; p < PLANES; ++p) {
+                    const u32 next = c[p][k] & carry;
+                    c[p][k] ^= carry;
+                    carry = next;
+                }
+            }
+            odd = 0;
+        } else {
+            pend[0] = four[0];
+            pend[1] = four[1];
+            odd = 1;
+        }
+        added += 4;
+        if (added + 4 >= (1u << PLANES)) flush(hcnt, lane);
+    }
+    // Adds the counters to the block's (lanes start at different bits: no two in one bank).
+    __device__ __forceinline__ void flush(u32* hcnt, u32 lane) {
+        for (u32 i = 0; i < 64; ++i) {
+            const u32 k = i >> 5, b = (i + lane) & 31u;
+            u32 v = odd ? ((k ? pend[1] : pend[0]) >> b & 1u) << 2 : 0u;
+#pragma unroll
+            for (int p = 0; p < PLANES; ++p) v += ((k ? c[p][1] : c[p][0]) >> b & 1u) << p;
+            if (v) atomicAdd(&hcnt[(2 * lane + k) * 32 + b], v);
+        }
+        clear();
+    }
+};
+
 __global__ void __launch_bounds__(32 * HUB_WARPS, 1)
     k_count_hub(const u64* __restrict__ fo, const u32* __restrict__ head, const Desc<u32>* __restrict__ vdesc,
-                const u16* __restrict__ hubp, const u32* __restrict__ hub_ids, const uint2* __restrict__ mtiles,
+                const u16* __restrict__ hubp, const u32* __restrict__ hub_ids, const u32* __restrict__ top_info,
+                const uint2* __restrict__ top_bits, const uint2* __restrict__ mtiles,
                 const uint2* __restrict__ ltiles, u32 seg, u64* __restrict__ cnt, u64* __restrict__ partials,
                 Control* ctl) {
     using L = HubLayout;
     constexpr u32 FULL = 0xFFFFFFFFu;
-    constexpr u32 ROWS = 2;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ u64 s_red[HUB_WARPS];
     if (ctl->err & DEV_ERR_MASK) return;
@@ -979,13 +1035,17 @@ __global__ void __launch_bounds__(32 * HUB_WARPS, 1)
     unsigned char* sbase = smem + ((L::align - (smem_u32(smem) & (L::align - 1))) & (L::align - 1));
     u32* hcnt = reinterpret_cast<u32*>(sbase + L::off_cnt);
     u32* bits = reinterpret_cast<u32*>(sbase + L::off_bits) + warp * L::BITS;
-    const u32 bits_at = smem_u32(bits), cnt_at = smem_u32(hcnt);
-    const u32 spare_at = cnt_at + sizeof(u32) * HUB_PAD;  // no hub's counter
-    for (u32 i = threadIdx.x; i < nh; i += 32 * HUB_WARPS) hcnt[i] = 0;
+    const u32 bits_at = smem_u32(bits);
+    u32* queue = reinterpret_cast<u32*>(sbase + L::off_queue) + warp * 32;
+    const u32 spare_at = smem_u32(hcnt + HUB_PAD);  // no hub's counter
+    const u32 base4 = 0u - (u32)sizeof(u32) * HUB_PAD;  // the counters from there
+    for (u32 i = threadIdx.x; i < HUB_H; i += 32 * HUB_WARPS) hcnt[i] = 0;
     for (u32 i = lane; i < L::BITS; i += 32) bits[i] = 0;
     __syncthreads();
     u64 total = 0;
     u32 dup = 0;
+    TopCounters tops;
+    tops.clear();
     while (true) {
         unsigned long long t = 0;
         if (lane == 0) t = atomicAdd(&ctl->hub_next, 1ull);
@@ -997,84 +1057,116 @@ __global__ void __launch_bounds__(32 * HUB_WARPS, 1)
         const u32 xh = hub_len<true>(dx.d), xt = list_len<true>(dx.d);
         if (xh == 0) continue;
         const u16* own = hubp + hub_start(list_start(dx), x);
-        for (u32 k = lane; k < xh; k += 32) {
+        const u32 xinfo = __ldg(top_info + x), xo = xh - (xinfo & 0xFFFu);
+        uint2* top_words = reinterpret_cast<uint2*>(bits) + lane;  // this lane's two words of the top bits
+        if (xinfo) *top_words = __ldg(top_bits + (u64)(xinfo >> 12) * 32 + lane);
+        __syncwarp();
+        for (u32 k = lane; k < xo; k += 32) {
             const u32 h = __ldg(own + k), bit = 1u << (h & 31u);
             if (atomicOr(&bits[h >> 5], bit) & bit) dup = 1;
         }
         const u64 a = fo[x] + (u64)tl.y * seg, fx1 = fo[x + 1];
         const u32 ns = (u32)(a + seg < fx1 ? (u64)seg : fx1 - a);
         __syncwarp();
+        const uint2 xtop = *top_words;
         u32 T = 0;
-        // neighbours of the next 32 slots are in flight while the current ones are counted
-        u32 y = lane < ns ? __ldg(head + a + lane) : x;
+        // two chunks ahead the neighbours, one chunk ahead their descriptors are in flight
+        auto neighbour = [&](u32 e) { return e + lane < ns ? __ldg(head + a + e + lane) : x; };
+        u32 y0 = neighbour(0), y1 = neighbour(32);
+        Desc<u32> v0 = load_desc(vdesc + y0);
+        u32 i0 = __ldg(top_info + y0);
         for (u32 e0 = 0; e0 < ns; e0 += 32) {
-            const u32 yc = y;
+            const u32 yc = y0, info0 = i0;
+            const Desc<u32> vy = v0;
             const bool have = e0 + lane < ns;
-            const Desc<u32> vy = load_desc(vdesc + yc);
-            y = e0 + 32 + lane < ns ? __ldg(head + a + e0 + 32 + lane) : x;
+            y0 = y1;
+            v0 = load_desc(vdesc + y0);
+            i0 = __ldg(top_info + y0);
+            y1 = neighbour(e0 + 64);
             const u32 yh = hub_len<true>(vy.d);
             const bool sel = have && yh > 0 && key_less(list_len<true>(vy.d), yc, xt, x);
             const u32 ys = (u32)(hub_start(list_start(vy), yc) >> 3);  // in 16-byte groups
+            const u32 info = sel ? info0 : 0u;
+            const u32 yo = yh - (info & 0xFFFu);  // entries left in the list
             u32 hits = 0;
-            u32 longs = __ballot_sync(FULL, sel && yh > HUB_LANE);
-            if (sel && yh <= HUB_LANE) {
+            // top bitmaps, four at a time: one AND for 32 entries, counted per bit position
+            const u32 with_top = __ballot_sync(FULL, info != 0);
+            if (with_top) {
+                const u32 rank = __popc(with_top & ((1u << lane) - 1));
+                queue[lane] = 0;
+                __syncwarp();
+                if (info) queue[rank] = info >> 12;
+                __syncwarp();
+                u32 v = 0;  // lane r: the hits of the chunk's r-th bitmap
+                const u32 nb = __popc(with_top);
+                for (u32 r = 0; r < nb; r += 4) {
+                    const uint4 at = *reinterpret_cast<const uint4*>(queue + r);
+                    uint2 m[4];
+                    m[0] = __ldg(top_bits + (u64)at.x * 32 + lane);
+                    m[1] = __ldg(top_bits + (u64)at.y * 32 + lane);
+                    m[2] = __ldg(top_bits + (u64)at.z * 32 + lane);
+                    m[3] = __ldg(top_bits + (u64)at.w * 32 + lane);
+                    u32 p[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        m[j].x &= xtop.x;
+                        m[j].y &= xtop.y;
+                        p[j] = __popc(m[j].x) + __popc(m[j].y);
+                    }
+                    const u32 r01 = __reduce_add_sync(FULL, p[0] | (p[1] << 16));
+                    const u32 r23 = __reduce_add_sync(FULL, p[2] | (p[3] << 16));
+                    const u32 mine = lane - r;  // 0..3: one of these four is this lane's
+                    if (mine < 4) v = ((mine & 2u ? r23 : r01) >> (16 * (mine & 1u))) & 0xFFFFu;
+                    tops.add4(m, hcnt, lane);
+                }
+                v = __shfl_sync(FULL, v, rank & 31);
+                if (info) hits = v;
+            }
+            if (sel && yo > 0 && yo <= HUB_LANE) {
                 const uint4* lp = reinterpret_cast<const uint4*>(hubp) + ys;
-                const uint4 g0 = __ldg(lp), g1 = yh > 8 ? __ldg(lp + 1) : g0;
-                hits = hub_probe2(g0.x, bits_at, cnt_at, spare_at);
-                if (yh > 2) hits += hub_probe2(g0.y, bits_at, cnt_at, spare_at);
-                if (yh > 4) hits += hub_probe2(g0.z, bits_at, cnt_at, spare_at);
-                if (yh > 6) hits += hub_probe2(g0.w, bits_at, cnt_at, spare_at);
-                if (yh > 8) hits += hub_probe2(g1.x, bits_at, cnt_at, spare_at);
-                if (yh > 10) hits += hub_probe2(g1.y, bits_at, cnt_at, spare_at);
-                if (yh > 12) hits += hub_probe2(g1.z, bits_at, cnt_at, spare_at);
-                if (yh > 14) hits += hub_probe2(g1.w, bits_at, cnt_at, spare_at);
+                const uint4 g0 = __ldg(lp);
+                hits += hub_probe8(g0, bits_at, base4, spare_at);
             }
             __syncwarp();
-            // the long lists one after the other, in blocks of ROWS x 128 entries: the next block, of
-            // this list or the next one, is in flight while the current one is looked up
-            uint2 nb[ROWS];
-            u32 nq = 0;  // quadruples of entries left from the next block on
-            const uint2* np = nullptr;
-            auto load_block = [&]() {
+            // the longer lists, cut into units of 64 entries: eight lanes take a unit, four units
+            // (of one list or of several) a row.  The next row is in flight while the current one
+            // is looked up.
+            const u32 yq = (yo + 7) / 8;  // 16-byte groups
+            const u32 units = sel && yo > HUB_LANE ? (yq + 7) / 8 : 0u;
+            u32 P = units;
 #pragma unroll
-                for (u32 r = 0; r < ROWS; ++r) {
-                    nb[r] = make_uint2(HUB_PAD2, HUB_PAD2);
-                    if (lane + 32 * r < nq) nb[r] = __ldg(np + 32 * r);
-                }
+            for (int o = 1; o < 32; o <<= 1) {
+                const u32 z = __shfl_up_sync(FULL, P, o);
+                if (lane >= (u32)o) P += z;
+            }
+            const u32 U = __shfl_sync(FULL, P, 31);
+            P = units ? P - units : 0xFFFFFFFFu;  // the list's first unit
+            uint4 nw = make_uint4(HUB_PAD2, HUB_PAD2, HUB_PAD2, HUB_PAD2);
+            int n0 = 0, n1 = 0, n2 = 0, n3 = 0;  // the lanes whose lists the row's units belong to
+            auto fetch = [&](u32 u) {
+                n0 = 31 - __clz(__ballot_sync(FULL, P <= u));
+                n1 = 31 - __clz(__ballot_sync(FULL, P <= u + 1));
+                n2 = 31 - __clz(__ballot_sync(FULL, P <= u + 2));
+                n3 = 31 - __clz(__ballot_sync(FULL, P <= u + 3));
+                const int k = lane < 16 ? (lane < 8 ? n0 : n1) : (lane < 24 ? n2 : n3);
+                const u32 o = (u + (lane >> 3) - __shfl_sync(FULL, P, k)) * 8 + (lane & 7u);
+                const bool in = o < __shfl_sync(FULL, yq, k);
+                const uint4* lp = reinterpret_cast<const uint4*>(hubp) + __shfl_sync(FULL, ys, k);
+                nw = make_uint4(HUB_PAD2, HUB_PAD2, HUB_PAD2, HUB_PAD2);
+                if (in) nw = __ldg(lp + o);
             };
-            auto next_list = [&](int src) {
-                nq = (__shfl_sync(FULL, yh, src) + 3) / 4;
-                np = reinterpret_cast<const uint2*>(hubp) + (u64)__shfl_sync(FULL, ys, src) * 2 + lane;
-                load_block();
-            };
-            if (longs) next_list(__ffs(longs) - 1);
-            while (longs) {
-                const u32 src = __ffs(longs) - 1;
-                longs &= longs - 1;
-                u32 f = 0;
-                while (true) {
-                    uint2 cb[ROWS];
-#pragma unroll
-                    for (u32 r = 0; r < ROWS; ++r) cb[r] = nb[r];
-                    const u32 left = nq;
-                    const bool more = left > 32 * ROWS;
-                    if (more) {
-                        nq = left - 32 * ROWS;
-                        np += 32 * ROWS;
-                        load_block();
-                    } else if (longs) {
-                        next_list(__ffs(longs) - 1);
-                    }
-#pragma unroll
-                    for (u32 r = 0; r < ROWS; ++r) {
-                        if (32 * r >= left) break;
-                        f += hub_probe2(cb[r].x, bits_at, cnt_at, spare_at);
-                        f += hub_probe2(cb[r].y, bits_at, cnt_at, spare_at);
-                    }
-                    if (!more) break;
-                }
-                f = __reduce_add_sync(FULL, f);
-                if (lane == src) hits = f;
+            if (U) fetch(0);
+            for (u32 u = 0; u < U; u += 4) {
+                const uint4 w = nw;
+                const int k0 = n0, k1 = n1, k2 = n2, k3 = n3;
+                if (u + 4 < U) fetch(u + 4);
+                const u32 f = hub_probe8(w, bits_at, base4, spare_at);
+                // the four units' hits (at most 64 each) side by side in one sum
+                const u32 s4 = __reduce_add_sync(FULL, f << (lane & 24u));
+                if ((int)lane == k0) hits += s4 & 0xFFu;
+                if ((int)lane == k1) hits += (s4 >> 8) & 0xFFu;
+                if ((int)lane == k2) hits += (s4 >> 16) & 0xFFu;
+                if ((int)lane == k3) hits += s4 >> 24;
             }
             if (hits) {
                 atomicAdd(&cnt[yc], (u64)hits);
@@ -1087,9 +1179,11 @@ __global__ void __launch_bounds__(32 * HUB_WARPS, 1)
             total += wt;
         }
         __syncwarp();
-        for (u32 k = lane; k < xh; k += 32) bits[__ldg(own + k) >> 5] = 0;
+        *top_words = make_uint2(0, 0);
+        for (u32 k = lane; k < xo; k += 32) bits[__ldg(own + k) >> 5] = 0;
         __syncwarp();
     }
+    tops.flush(hcnt, lane);
     if (dup) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
     const u64 bt = block_sum_u64<32 * HUB_WARPS>(total, s_red);  // also orders the counters' last hits
     if (threadIdx.x == 0) partials[blockIdx.x] = bt;
@@ -1501,7 +1595,7 @@ cudaError_t launch_count_auto(const u64* fo, const u32* head, u64 n, u64 nnz, co
     if (after_small) cudaEventRecord(after_small, st);
     if constexpr (HUB)
         k_count_hub<<<count_grid_hub<HUB>(num_sms), 32 * HUB_WARPS, HUB_SMEM, st>>>(
-            fo, head, vd, hub.lists, hub.ids, mtiles, ltiles, seg, cnt, partials + cap + gm + gl, ctl);
+            fo, head, vd, hub.lists, hub.ids, hub.top_info, hub.top_bits, mtiles, ltiles, seg, cnt, partials + cap + gm + gl, ctl);
     k_count_medium<MEDIUM_BLOCK, OffT, HUB>
         <<<gm, MEDIUM_BLOCK, MediumL::bytes, st>>>(fo, head, n, vd, headp, mtiles, seg, cnt, partials + cap, ctl);
     k_count_large<LARGE_BLOCK, LARGE_CAP, OffT, HUB>

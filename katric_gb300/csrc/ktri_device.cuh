@@ -74,12 +74,23 @@ __device__ __forceinline__ Desc<u64> load_desc<u64>(const Desc<u64>* p) {
 // packs both: hubs in the high half, the others in the low half (both below 2^16, see HUB_MAX_NNZ).
 // The region of x in the hub array starts at align8(oriented start + 4x) and has room for deg(x)
 // entries; the array holds nnz + 7n + 32 entries.  A list is filled up to a
-// multiple of four entries with HUB_PAD, an index no hub has, so it can be read four at a time.
+// multiple of eight entries with HUB_PAD, an index no hub has, so it can be read eight at a time.
 constexpr u32 HUB_H = 32768;          // hub indices: 0 .. HUB_H - 2
 constexpr u32 HUB_PAD = HUB_H - 1;
 constexpr u32 HUB_MIN_DEGREE = 128;   // a hub's degree is at least this
 constexpr u32 HUB_BINS = 4096;        // degree bins of the hub choice: 7 fractional bits of log2
 constexpr u32 HUB_FLAG = 0x80000000u; // orientation key of a hub: HUB_FLAG | (HUB_H - 1 - index)
+// Top bitmaps: a hub list of more than HUB_TOP_LIST entries with at least HUB_TOP_MIN among the
+// first HUB_TOP hubs keeps those as a bitmap of HUB_TOP bits and only the others in the list
+// (the descriptor still counts all).  top_info[x] = bitmap index << 12 | entries in the bitmap, 0
+// without one; bitmap 0 is empty.  Above the small kernel's bound, which reads whole hub lists.
+constexpr u32 HUB_TOP = 2048;
+constexpr u32 HUB_TOP_LIST = 48;
+constexpr u32 HUB_TOP_MIN = 32;
+__host__ __device__ __forceinline__ u64 hub_top_capacity(u64 nnz) {  // bitmaps; lists beyond it stay whole
+    return 1 + (nnz / 256 < (1u << 20) - 2 ? nnz / 256 : (1u << 20) - 2);
+}
+__host__ __device__ __forceinline__ u64 hub_long_capacity(u64 nnz) { return nnz / HUB_TOP_LIST + 1; }
 constexpr u64 HUB_MAX_N = 1ull << 30;
 constexpr u64 HUB_MAX_NNZ = (1ull << 32) - 1;  // 2^16 or more out-neighbours need 2^32 adjacency entries
 template <bool HUB>

@@ -81,6 +81,8 @@ struct Control {
     uint32_t hubs;                       // number of hubs
     uint32_t hub_bin;                    // smallest degree bin of the hubs
     uint32_t prep_blocks;                // blocks of k_prep that have finished
+    uint32_t hub_long;                   // vertices with a hub list above HUB_TOP_LIST
+    uint32_t hub_tops;                   // hub lists whose top entries became bitmaps
     uint32_t pad1;
 };
 

@@ -77,9 +77,15 @@ struct HubState {
     uint2* tmp = nullptr;
     u32* ids = nullptr;
     u16* lists = nullptr;
+    u32* top_info = nullptr;   // n entries
+    u32* top_long = nullptr;   // hub_long_capacity(nnz): vertices whose lists may get a bitmap
+    uint2* top_bits = nullptr; // hub_top_capacity(nnz) bitmaps of HUB_TOP bits
+    u32 top_cap = 0;
     explicit operator bool() const { return lists != nullptr; }
 };
 u64 hub_bins_words();
+// Top entries of long hub lists into bitmaps (after launch_desc; the lists then hold the others).
+void launch_hub_tops(const void* vdesc, const HubState& hub, Control* ctl, int num_sms, cudaStream_t st);
 
 // Degrees, tile boundaries and, with hubs, the hub choice (deg then holds orientation keys).
 void launch_prep(const u64* fo, u64 n, u64 nnz, u32* deg, u32* dplus, u64* cnt, u32* tile_i0, const HubState& hub,
@@ -113,7 +119,7 @@ void launch_order_tiles(const u64* fo, const u32* head, const u32* dplus, u64 n,
 
 // The counting kernels of KTRI_METHOD_AUTO.  partials needs count_grid_auto entries.  The hub
 // kernel runs where hub is set (HUB, 32-bit descriptors only).
-constexpr int HUB_WARPS = 23;        // warps of a hub kernel block (one block per SM)
+constexpr int HUB_WARPS = 22;        // warps of a hub kernel block (one block per SM)
 template <typename OffT, bool HUB>
 int count_grid_small(int num_sms);
 template <typename OffT, bool HUB>

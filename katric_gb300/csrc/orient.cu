@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(BLOCK, 4) k_orient(const u64* __restrict__ fo,
 // out-degree threshold.
 template <typename OffT, bool HUB>
 __global__ void k_desc(const u64* __restrict__ fo, u64 n, const u32* __restrict__ dplus, Desc<OffT>* __restrict__ vdesc,
-                       u16* __restrict__ hubp,
+                       u16* __restrict__ hubp, u32* __restrict__ top_info, u32* __restrict__ top_long,
                        uint2* __restrict__ mtiles, uint2* __restrict__ ltiles, u32 small_d, u32 medium_d, u32 seg,
                        Control* ctl) {
     if (ctl->err & DEV_ERR_MASK) return;
@@ -385,13 +385,22 @@ __global__ void k_desc(const u64* __restrict__ fo, u64 n, const u32* __restrict_
             vdesc[v] = ds;
             if constexpr (HUB) {
                 const u64 hs = hub_start(list_start(ds), v);
-                for (u32 k = hub_len<HUB>(d); k & 3u; ++k) hubp[hs + k] = (u16)HUB_PAD;
+                for (u32 k = hub_len<HUB>(d); k & 7u; ++k) hubp[hs + k] = (u16)HUB_PAD;
+                top_info[v] = 0;
             }
             // no tiles at all without tile arrays (the reference strategies pass none)
             const bool tiled = mtiles && ltiles && list_len<HUB>(d) > small_d;
             const u32 nt = tiled ? (u32)((b - a + seg - 1) / seg) : 0u;
             if (list_len<HUB>(d) > medium_d) nl = nt;
             else nm = nt;
+        }
+        if constexpr (HUB) {
+            const bool is_long = v < n && hub_len<HUB>(dplus[v < n ? v : 0]) > HUB_TOP_LIST;
+            const u32 ball = __ballot_sync(0xFFFFFFFFu, is_long);
+            u32 at = 0;
+            if (lane == 0 && ball) at = atomicAdd(&ctl->hub_long, (u32)__popc(ball));
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            if (is_long) top_long[at + __popc(ball & ((1u << lane) - 1))] = (u32)v;
         }
         // warp-aggregated reservation of tile slots, one list per owner class
 #pragma unroll
@@ -412,6 +421,55 @@ __global__ void k_desc(const u64* __restrict__ fo, u64 n, const u32* __restrict_
             for (u32 s = 0; s < mine; ++s) out[my + s] = make_uint2((u32)v, s);
         }
     }
+}
+
+// Top bitmaps of the long hub lists, one warp per list: the entries below HUB_TOP move to a bitmap,
+// the others close up at the front of the list in their order (a row is read before anything is
+// written at or past its start).
+constexpr int TOPS_BLOCK = 256;
+__global__ void __launch_bounds__(TOPS_BLOCK) k_hub_tops(const Desc<u32>* __restrict__ vdesc, u16* __restrict__ hubp,
+                                                         const u32* __restrict__ top_long, u32* __restrict__ top_info,
+                                                         uint2* __restrict__ top_bits, u32 cap, Control* ctl) {
+    __shared__ __align__(8) u32 s_bits[TOPS_BLOCK / 32][HUB_TOP / 32];
+    static_assert(HUB_TOP / 32 == 64, "two words per lane");
+    if (ctl->err & DEV_ERR_MASK) return;
+    const u32 lane = threadIdx.x & 31, lt = (1u << lane) - 1;
+    u32* bits = s_bits[threadIdx.x >> 5];
+    const u32 count = ctl->hub_long;
+    const u32 nwarps = gridDim.x * (TOPS_BLOCK / 32);
+    u32 dup = 0;
+    for (u32 i = (blockIdx.x * TOPS_BLOCK + threadIdx.x) >> 5; i < count; i += nwarps) {
+        const u32 v = top_long[i];
+        const Desc<u32> d = load_desc(vdesc + v);
+        const u32 len = hub_len<true>(d.d);
+        u16* lst = hubp + hub_start(list_start(d), v);
+        u32 tops = 0;
+        for (u32 k = lane; k < len; k += 32) tops += lst[k] < HUB_TOP ? 1u : 0u;
+        tops = __reduce_add_sync(0xFFFFFFFFu, tops);
+        if (tops < HUB_TOP_MIN) continue;
+        u32 slot = 0;
+        if (lane == 0) slot = atomicAdd(&ctl->hub_tops, 1u) + 1;
+        slot = __shfl_sync(0xFFFFFFFFu, slot, 0);
+        if (slot >= cap) continue;
+        bits[lane] = 0;
+        bits[lane + 32] = 0;
+        __syncwarp();
+        u32 out = 0;
+        for (u32 k0 = 0; k0 < len; k0 += 32) {
+            const u32 h = k0 + lane < len ? lst[k0 + lane] : HUB_PAD;
+            const bool other = k0 + lane < len && h >= HUB_TOP;
+            if (h < HUB_TOP && (atomicOr(&bits[h >> 5], 1u << (h & 31u)) & (1u << (h & 31u)))) dup = 1;
+            const u32 ball = __ballot_sync(0xFFFFFFFFu, other);
+            if (other) lst[out + __popc(ball & lt)] = (u16)h;
+            out += __popc(ball);
+        }
+        if (lane < ((8u - out) & 7u)) lst[out + lane] = (u16)HUB_PAD;
+        __syncwarp();
+        top_bits[(u64)slot * 32 + lane] = reinterpret_cast<const uint2*>(bits)[lane];
+        if (lane == 0) top_info[v] = (slot << 12) | tops;
+        __syncwarp();
+    }
+    if (dup) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
 }
 
 // Large-owner tiles in the order of the first vertex each segment streams (a counting sort
@@ -592,6 +650,12 @@ void launch_prep(const u64* fo, u64 n, u64 nnz, u32* deg, u32* dplus, u64* cnt, 
     k_hub_rank<<<HUB_H / 128, 128, 0, st>>>(hub.bins, hub.tmp, hub.ids, deg, ctl);
 }
 
+void launch_hub_tops(const void* vdesc, const HubState& hub, Control* ctl, int num_sms, cudaStream_t st) {
+    cudaMemsetAsync(hub.top_bits, 0, HUB_TOP / 8, st);  // the empty bitmap
+    k_hub_tops<<<num_sms * 8, TOPS_BLOCK, 0, st>>>(reinterpret_cast<const Desc<u32>*>(vdesc), hub.lists, hub.top_long,
+                                                   hub.top_info, hub.top_bits, hub.top_cap, ctl);
+}
+
 u64 hub_bins_words() { return 3ull * HUB_BINS; }
 
 u64 orient_tiles(u64 n, u64 nnz) { return (n + nnz + ORIENT_TILE - 1) / ORIENT_TILE; }
@@ -619,7 +683,7 @@ void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, const HubS
     u64 blocks = (n + 255) / 256;
     u64 cap = (u64)num_sms * 8;
     k_desc<OffT, HUB><<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(
-        fo, n, dplus, reinterpret_cast<Desc<OffT>*>(vdesc), hub.lists, mtiles, ltiles, small_d, medium_d, seg, ctl);
+        fo, n, dplus, reinterpret_cast<Desc<OffT>*>(vdesc), hub.lists, hub.top_info, hub.top_long, mtiles, ltiles, small_d, medium_d, seg, ctl);
 }
 
 #define KTRI_INST(OffT, HUB)                                                                                     \
