@@ -13,17 +13,19 @@
 // table: its hits accumulate in a shared-memory counter next to the key and are flushed once per
 // table.  The streamed endpoint gets its list's hits, the other one its table's total.
 //
-// Three kernels (the bounds are runtime options, at most SMALL_D and MEDIUM_D):
+// The kernels (the bounds are runtime options, at most SMALL_D and MEDIUM_D):
 //   k_count_small: the edges between out-degrees of at most small_outdegree, groups of tails per
 //     warp, one streamed list per lane.  No block barrier.
 //   k_count_medium: owners up to medium_outdegree, one warp per (owner, segment) tile with the
-//     warp's own table, filter and survivor buffer, so tiles need no block barrier.
+//     warp's own table, so tiles need no block barrier.
 //   k_count_large: larger owners, one (owner, segment) tile per block iteration.  Short
 //     streamed lists are handled one per thread while the segment is scanned; longer ones are
 //     queued and taken one at a time by whole warps (one entry per lane, eight loads in
-//     flight), so no block-wide barrier separates the lists.
-// The medium and large kernels test every streamed entry against a one-hash filter of the
-// owner's keys first and look up only the survivors, packed 32 at a time.
+//     flight), so no block-wide barrier separates the lists.  Every streamed entry is tested
+//     against a one-hash filter of the owner's keys first, and only the survivors are looked up,
+//     packed 32 at a time.
+// Graphs with split lists (hubs) have k_count_hub for the hub part of all owner tiles, and
+// k_count_medium takes the other entries of all of them.
 #include "ktri_device.cuh"
 #include "ktri_kernels.h"
 
@@ -383,13 +385,22 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
                 const u32 nb = 3 * t.y, mult = t.z;
                 const uint2* tk = reinterpret_cast<const uint2*>(keys) + 3 * t.x;
                 u32* th = hits + 3 * t.x;
-                auto look = [&](u32 z, bool valid) {
-                    const u32 b = __umulhi(z * mult, nb);
-                    const uint2 kk = tk[b];
-                    const bool h0 = kk.x == z, h1 = kk.y == z;
-                    if ((h0 | h1) & valid) {
-                        atomicAdd(&th[b], h1 ? 0x10000u : 1u);
-                        ++found;
+                auto look4 = [&](u32 z0, u32 z1, u32 z2, u32 z3, int r) {
+                    const u32 z[4] = {z0, z1, z2, z3};
+                    u32 b[4];
+                    uint2 kk[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        b[k] = __umulhi(z[k] * mult, nb);
+                        kk[k] = tk[b[k]];
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const bool h0 = kk[k].x == z[k], h1 = kk[k].y == z[k];
+                        if ((h0 | h1) & (k < r)) {
+                            atomicAdd(&th[b[k]], h1 ? 0x10000u : 1u);
+                            ++found;
+                        }
                     }
                 };
                 if (!HUB || rem > 0) {
@@ -397,10 +408,7 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
                     while (true) {
                         uint4 nxt = cur;
                         if (rem > 4) nxt = ld_in<CG>(++lp);
-                        look(cur.x, true);
-                        look(cur.y, rem > 1);
-                        look(cur.z, rem > 2);
-                        look(cur.w, rem > 3);
+                        look4(cur.x, cur.y, cur.z, cur.w, rem);
                         rem -= 4;
                         if (rem <= 0) break;
                         cur = nxt;
@@ -410,12 +418,11 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
                     const uint4* hp = hubp8 + q_h[q];
                     for (; hrem > 0; hrem -= 8) {
                         const uint4 cur = ld_in<CG>(hp++);
-                        const u32 pair[4] = {cur.x, cur.y, cur.z, cur.w};
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            look(n32 + (pair[k] & 0xFFFFu), 2 * k < hrem);
-                            look(n32 + (pair[k] >> 16), 2 * k + 1 < hrem);
-                        }
+                        look4(n32 + (cur.x & 0xFFFFu), n32 + (cur.x >> 16), n32 + (cur.y & 0xFFFFu), n32 + (cur.y >> 16),
+                              hrem);
+                        if (hrem > 4)
+                            look4(n32 + (cur.z & 0xFFFFu), n32 + (cur.z >> 16), n32 + (cur.w & 0xFFFFu),
+                                  n32 + (cur.w >> 16), hrem - 4);
                     }
                 }
                 if (found) {
@@ -589,7 +596,7 @@ __device__ __forceinline__ void chunk_sizes(u32 klen, u32 max_lg, u32 max_fl, u3
 // One (owner, segment) tile of a large owner, counted by the whole block.  bar is the block's
 // bulk-copy mbarrier, initialised once and kept where no other use of shared memory reaches.
 // Returns true when a bounded wait for a bulk copy ran out (inflight: the second wait ran out too).
-template <int BLOCK, int CAP, typename OffT, bool HUB, bool CG = false>
+template <int BLOCK, int CAP, typename OffT, bool CG = false>
 __device__ __forceinline__ bool large_tile(unsigned char* smem, unsigned long long* bar, uint2 tl,
                                            const u64* __restrict__ fo,
                                            const u32* __restrict__ head, u64 n, const Desc<OffT>* __restrict__ vdesc,
@@ -618,7 +625,7 @@ __device__ __forceinline__ bool large_tile(unsigned char* smem, unsigned long lo
     bool timed_out = false;
     const u64 x = tl.x;
     const Desc<OffT> dxd = ld_desc<CG>(vdesc + x);
-    const u32 dx = rest_len<HUB>(dxd.d), dxt = list_len<HUB>(dxd.d);
+    const u32 dx = dxd.d;
     const u64 fx1 = ld_in<CG>(fo + x + 1);
     const u64 a = ld_in<CG>(fo + x) + (u64)tl.y * seg;
     const u64 b = a + seg < fx1 ? a + seg : fx1;
@@ -677,9 +684,8 @@ __device__ __forceinline__ bool large_tile(unsigned char* smem, unsigned long lo
             if (e < b) {
                 y = ld_in<CG>(head + e);
                 if (y < n) vy = ld_desc<CG>(vdesc + y);
-                const u32 dyt = list_len<HUB>(vy.d), dy = rest_len<HUB>(vy.d);
-                vy.d = dy;
-                if (dy > 0 && key_less(dyt, y, dxt, x)) {
+                const u32 dy = vy.d;
+                if (dy > 0 && key_less(dy, y, dx, x)) {
                     if (dy <= (u32)LONG_LIST) {
                         const u32 hits = lane_stream_short<OffT, CG>(headp4, vy, keys, hitc, lg, filt, fl);
                         if (hits) {
@@ -736,7 +742,7 @@ __device__ __forceinline__ bool large_tile(unsigned char* smem, unsigned long lo
     return timed_out;
 }
 
-template <int BLOCK, int CAP, typename OffT, bool HUB>
+template <int BLOCK, int CAP, typename OffT>
 __global__ void __launch_bounds__(BLOCK) k_count_large(const u64* __restrict__ fo, const u32* __restrict__ head,
                                                        u64 n, const Desc<OffT>* __restrict__ vdesc,
                                                        const u32* __restrict__ headp,
@@ -762,7 +768,7 @@ __global__ void __launch_bounds__(BLOCK) k_count_large(const u64* __restrict__ f
         __syncthreads();
         const u64 t = s_t;
         if (t >= ntiles) break;
-        timed_out = large_tile<BLOCK, CAP, OffT, HUB>(smem, s_bar, ltiles[t], fo, head, n, vdesc, headp, seg, cnt,
+        timed_out = large_tile<BLOCK, CAP, OffT>(smem, s_bar, ltiles[t], fo, head, n, vdesc, headp, seg, cnt,
                                                  first_wait_polls, phase, inflight, local_total, dup);
         if (timed_out) break;
     }
@@ -771,122 +777,231 @@ __global__ void __launch_bounds__(BLOCK) k_count_large(const u64* __restrict__ f
     if (threadIdx.x == 0) partials[blockIdx.x] = local_total;
 }
 
-// Medium owners (small threshold < out-degree <= MEDIUM_D): one warp per (owner, segment)
-// tile, with its own table, filter and buffer in shared memory, so a tile needs no block
-// barrier.  Most owner tiles of skewed graphs are of this kind and carry little work each.
-template <int BLOCK>
-struct MediumLayout {
-    static constexpr int NW = BLOCK / 32;
-    static constexpr int TS = 2 * MEDIUM_D;  // table slots per warp (a quarter to half full)
-    static constexpr int FW = MEDIUM_D / 2;  // filter words per warp (16 bits per key)
-    static constexpr int WBUF = 64;
-    static constexpr int PER_WARP = TS + TS / 2 + FW + WBUF;  // u32 words: keys, 16-bit hits, filter, buffer
-    static constexpr size_t bytes = sizeof(u32) * PER_WARP * NW;
+// Owner tiles counted by single warps (k_count_medium): owners of small_outdegree < out-degree <=
+// medium_outdegree, and with hubs every owner's other entries.  A warp's table holds up to CAP of
+// the owner's keys (owners with more are counted in chunks) in buckets of two; a bucket that
+// overflowed is marked by a cleared top bit of its second key, so a lookup reads one bucket and
+// walks on only past a marked one (about 1 % of them at CAP keys), and a miss in a full bucket ends
+// there.  Streamed lists are cut into units of 32 entries, eight lanes to a unit and four units of
+// any lists to a row; lists of up to four entries go one per lane.
+// What bounds it: instruction issue (71 to 73 %) beside the lookups' shared-memory wavefronts
+// (53 to 62 % of the pipe).  It replaced a one-hash filter with packed survivors and one list per warp
+// iteration, which left most lanes idle on lists below 100 entries: RMAT n = 8191 0.182 -> 0.061 ms
+// (medium + large), 512-graph batch 6.2 -> 5.0 ms, the other entries of RMAT-24 27.6 -> 21 ms.
+// Measured against NB = 768 (24 warps per SM: RMAT-24 +0.8 %, batch +1 %, small graphs -10 %) and
+// CAP = 128 (RMAT-24 +7 %: more owners in two chunks).
+template <typename OffT>
+struct TileLayout {
+    static constexpr u32 NB = 512;   // buckets
+    static constexpr u32 CAP = 192;  // keys per chunk
+    static constexpr int W_KEYS = 0;
+    static constexpr int W_HITS = W_KEYS + 2 * NB;  // two 16-bit counters per bucket, a spare word per lane
+    static constexpr int PER_WARP = W_HITS + NB + 32;
+    static constexpr size_t bytes(int warps) { return sizeof(u32) * PER_WARP * warps; }
 };
+constexpr u32 TILE_MULT = 0x9E3779B1u;
 
-// One (owner, segment) tile of a medium owner, counted by one warp in its slice of shared
-// memory (keys at `keys`, then the hit counters, the filter and the survivor buffer).
-template <int BLOCK, typename OffT, bool HUB, bool CG = false>
-__device__ __forceinline__ void medium_tile(u32* keys, uint2 tl, const u64* __restrict__ fo,
-                                            const u32* __restrict__ head, const Desc<OffT>* __restrict__ vdesc,
-                                            const u32* __restrict__ headp, u32 seg, u64* __restrict__ cnt,
-                                            u64& local_total, u32& dup) {
-    using L = MediumLayout<BLOCK>;
-    constexpr int U = 4;  // medium owners' streamed lists are shorter than 256 entries
-    const int lane = threadIdx.x & 31;
-    u32* hitc = keys + L::TS;
-    u32* filt = hitc + L::TS / 2;
-    u32* wbuf = filt + L::FW;
-    const u32 lt_mask = (1u << lane) - 1;
-    const uint4* headp4 = reinterpret_cast<const uint4*>(headp);
-    const u64 x = tl.x;
-    const Desc<OffT> dxd = ld_desc<CG>(vdesc + x);
-    const u32 dx = rest_len<HUB>(dxd.d), dxt = list_len<HUB>(dxd.d);
-    if (HUB && dx == 0) return;
-    const u64 fx1 = ld_in<CG>(fo + x + 1);
-    const u64 a = ld_in<CG>(fo + x) + (u64)tl.y * seg;
-    const u64 b = a + seg < fx1 ? a + seg : fx1;
-    u32 lg, fl;
-    chunk_sizes(dx, 31 - __clz((u32)L::TS), 31 - __clz((u32)(L::FW * 32)), &lg, &fl);
-    const u32 size = 1u << lg, fwords = (1u << fl) >> 5;
-    for (u32 i = lane; i < size; i += 32) keys[i] = EMPTY_KEY;
-    for (u32 i = lane; i < size / 2; i += 32) hitc[i] = 0;
-    for (u32 i = lane; i < fwords; i += 32) filt[i] = 0;
-    __syncwarp();
-    for (u32 q = lane; q < dx; q += 32) {
-        const u32 w = ld_in<CG>(headp + list_start(dxd) + q);
-        if (!bucket_insert(keys, lg, w)) dup = 1;
-        const u32 h = filter_bit(w, fl);
-        atomicOr(&filt[h >> 5], 1u << (h & 31u));
-    }
-    __syncwarp();
-    u32 T = 0;
-    for (u64 e0 = a; e0 < b; e0 += 32) {
-        const u64 e = e0 + lane;
-        u32 y = 0;
-        Desc<OffT> vy;
-        vy.start = 0;
-        vy.d = 0;
-        bool longl = false;
-        if (e < b) {
-            y = ld_in<CG>(head + e);
-            vy = ld_desc<CG>(vdesc + y);
-            const u32 dyt = list_len<HUB>(vy.d), dy = rest_len<HUB>(vy.d);
-            vy.d = dy;
-            if (dy > 0 && key_less(dyt, y, dxt, x)) {
-                if (dy <= (u32)LONG_LIST) {
-                    const u32 hits = lane_stream_short<OffT, CG>(headp4, vy, keys, hitc, lg, filt, fl);
-                    if (hits) {
-                        atomicAdd(&cnt[y], (u64)hits);
-                        T += hits;
-                    }
-                } else {
-                    longl = true;
-                }
-            }
-        }
-        u32 ball = __ballot_sync(0xFFFFFFFFu, longl);
-        while (ball) {  // the warp streams this chunk's long lists one at a time
-            const int src = __ffs(ball) - 1;
-            ball &= ball - 1;
-            const u32 yy = __shfl_sync(0xFFFFFFFFu, y, src);
-            const u64 ys = (u64)__shfl_sync(0xFFFFFFFFu, (unsigned long long)list_start(vy), src);
-            const u32 yd = __shfl_sync(0xFFFFFFFFu, vy.d, src);
-            u32 hits = warp_stream_list<U, CG>(headp + ys, yd, keys, hitc, lg, filt, fl, wbuf, lane, lt_mask);
-            hits = __reduce_add_sync(0xFFFFFFFFu, hits);
-            if (lane == 0 && hits) {
-                atomicAdd(&cnt[yy], (u64)hits);
-                T += hits;
-            }
-        }
-    }
-    __syncwarp();
-    for (u32 i = lane; i < size; i += 32) {
-        const u32 h = read16(hitc, i);
-        if (h) atomicAdd(&cnt[keys[i]], (u64)h);
-    }
-    const u32 wt = __reduce_add_sync(0xFFFFFFFFu, T);
-    if (lane == 0 && wt) {
-        atomicAdd(&cnt[x], (u64)wt);
-        local_total += wt;
-    }
+// A warp's table is empty between chunks.
+template <typename OffT>
+__device__ __forceinline__ void tile_init(u32* base) {
+    using L = TileLayout<OffT>;
+    const u32 lane = threadIdx.x & 31;
+    for (u32 i = lane; i < 2 * L::NB; i += 32) base[L::W_KEYS + i] = EMPTY_KEY;
+    for (u32 i = lane; i < L::NB + 32; i += 32) base[L::W_HITS + i] = 0;
     __syncwarp();
 }
 
+// One (owner, segment) tile of an owner's out-list (HUB: of its entries that are not hubs), counted by
+// one warp in its slice of shared memory.  top: the bit that marks keys, 0 where ids need all bits
+// (a full bucket is then walked past, marked or not).
+template <typename OffT, bool HUB, bool CG = false>
+__device__ __forceinline__ void medium_tile(u32* base, u32 top, uint2 tl, const u64* __restrict__ fo,
+                                            const u32* __restrict__ head, const Desc<OffT>* __restrict__ vdesc,
+                                            const u32* __restrict__ headp, u32 seg, u64* __restrict__ cnt,
+                                            u64& local_total, u32& dup) {
+    using L = TileLayout<OffT>;
+    constexpr u32 FULL = 0xFFFFFFFFu;
+    const u32 lane = threadIdx.x & 31;
+    u32* keys = base + L::W_KEYS;
+    u32* hits = base + L::W_HITS;
+    const uint2* buckets = reinterpret_cast<const uint2*>(keys);
+    const uint4* headp4 = reinterpret_cast<const uint4*>(headp);
+    const u32 x = tl.x;
+    const Desc<OffT> dx = ld_desc<CG>(vdesc + x);
+    const u32 xr = rest_len<HUB>(dx.d), xt = list_len<HUB>(dx.d);
+    if (xr == 0) return;
+    const u64 a = ld_in<CG>(fo + x) + (u64)tl.y * seg, fx1 = ld_in<CG>(fo + x + 1);
+    const u32 ns = (u32)(a + seg < fx1 ? (u64)seg : fx1 - a);
+    // the first `rem` of four streamed entries: counts their hits at their keys.  One branch for the
+    // four (a lane's misses then count at its spare word), and one for the rare walk.
+    auto look4 = [&](const uint4& w, u32 rem) -> u32 {
+        const u32 z[4] = {w.x, w.y, w.z, w.w};
+        u32 at[4], found = 0;
+        uint2 kk[4];
+#pragma unroll
+        for (u32 k = 0; k < 4; ++k) {
+            at[k] = __umulhi(z[k] * TILE_MULT, L::NB);
+            kk[k] = buckets[at[k]];
+        }
+        u32 walk = 0;
+        u32 one[4];
+#pragma unroll
+        for (u32 k = 0; k < 4; ++k) {
+            const u32 zt = z[k] | top;
+            const bool h0 = kk[k].x == zt, h1 = (kk[k].y | top) == zt;
+            const bool hit = (h0 | h1) & (k < rem);
+            if ((k < rem) & !(h0 | h1) & !(kk[k].y & top)) walk |= 1u << k;
+            one[k] = h0 ? 1u : 0x10000u;
+            at[k] = hit ? at[k] : L::NB + lane;
+            found += hit ? 1u : 0u;
+        }
+        if (found) {
+#pragma unroll
+            for (u32 k = 0; k < 4; ++k) atomicAdd(&hits[at[k]], one[k]);
+        }
+        if (walk) {
+#pragma unroll
+            for (u32 k = 0; k < 4; ++k) {
+                if (!((walk >> k) & 1u)) continue;
+                const u32 zt = z[k] | top;
+                u32 b = __umulhi(z[k] * TILE_MULT, L::NB);
+                uint2 q = buckets[b];
+                while (q.y != EMPTY_KEY && !(q.y & top)) {  // marked (or, without marks, full): the next bucket too
+                    b = b + 1 < L::NB ? b + 1 : 0;
+                    q = buckets[b];
+                    const bool h0 = q.x == zt, h1 = (q.y | top) == zt;
+                    if (h0 | h1) {
+                        atomicAdd(&hits[b], h0 ? 1u : 0x10000u);
+                        ++found;
+                        break;
+                    }
+                }
+            }
+        }
+        return found;
+    };
+    u64 T = 0;
+    for (u32 c0 = 0; c0 < xr; c0 += L::CAP) {
+        const u32 klen = xr - c0 < L::CAP ? xr - c0 : L::CAP;
+        for (u32 k = lane; k < klen; k += 32) {
+            const u32 w = ld_in<CG>(headp + list_start(dx) + c0 + k), wt = w | top;
+            u32 b = __umulhi(w * TILE_MULT, L::NB);
+            while (true) {  // ends: at most CAP of the 2 NB slots are taken
+                const u32 p0 = atomicCAS(&keys[2 * b], EMPTY_KEY, wt);
+                if (p0 == EMPTY_KEY) break;
+                const u32 p1 = p0 == wt ? wt : atomicCAS(&keys[2 * b + 1], EMPTY_KEY, wt);
+                if (p1 == EMPTY_KEY) break;
+                if (p0 == wt || (p1 | top) == wt) {
+                    dup = 1;
+                    break;
+                }
+                if (top) atomicAnd(&keys[2 * b + 1], ~top);
+                b = b + 1 < L::NB ? b + 1 : 0;
+            }
+        }
+        __syncwarp();
+        u32 Tc = 0;
+        // two chunks of slots ahead the neighbours, one ahead their descriptors are in flight
+        auto neighbour = [&](u32 e) { return e + lane < ns ? ld_in<CG>(head + a + e + lane) : x; };
+        u32 y0 = neighbour(0), y1 = neighbour(32);
+        Desc<OffT> v0 = ld_desc<CG>(vdesc + y0);
+        for (u32 e0 = 0; e0 < ns; e0 += 32) {
+            const u32 y = y0;
+            const Desc<OffT> vy = v0;
+            const bool have = e0 + lane < ns;
+            y0 = y1;
+            v0 = ld_desc<CG>(vdesc + y0);
+            y1 = neighbour(e0 + 64);
+            const u32 yr = rest_len<HUB>(vy.d), yt = list_len<HUB>(vy.d);
+            const bool sel = have && yr > 0 && (yt < xt || (yt == xt && y < x));
+            const OffT ys = (OffT)list_group(vy);
+            u32 f = 0;
+            if (sel && yr <= 4) {
+                const uint4 w = ld_in<CG>(headp4 + ys);
+                f = look4(w, yr);
+            }
+            __syncwarp();
+            const u32 units = sel && yr > 4 ? (yr + 31) / 32 : 0u;
+            u32 P = units;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const u32 z = __shfl_up_sync(FULL, P, o);
+                if (lane >= (u32)o) P += z;
+            }
+            const u32 U = __shfl_sync(FULL, P, 31);
+            P = units ? P - units : 0xFFFFFFFFu;  // the list's first unit
+            uint4 nw = make_uint4(0, 0, 0, 0);
+            u32 nrem = 0;                         // entries from this lane's first on
+            int n0 = 0, n1 = 0, n2 = 0, n3 = 0;   // the lanes whose lists the row's units belong to
+            auto fetch = [&](u32 u) {
+                n0 = 31 - __clz(__ballot_sync(FULL, P <= u));
+                n1 = 31 - __clz(__ballot_sync(FULL, P <= u + 1));
+                n2 = 31 - __clz(__ballot_sync(FULL, P <= u + 2));
+                n3 = 31 - __clz(__ballot_sync(FULL, P <= u + 3));
+                const int k = lane < 16 ? (lane < 8 ? n0 : n1) : (lane < 24 ? n2 : n3);
+                const u32 o = (u + (lane >> 3) - __shfl_sync(FULL, P, k)) * 8 + (lane & 7u);
+                const u32 len = __shfl_sync(FULL, yr, k);
+                const uint4* lp = headp4 + (u64)__shfl_sync(FULL, ys, k);
+                nrem = 4 * o < len ? len - 4 * o : 0u;
+                if (nrem) nw = ld_in<CG>(lp + o);
+            };
+            if (U) fetch(0);
+            for (u32 u = 0; u < U; u += 4) {
+                const uint4 w = nw;
+                const u32 rem = nrem;
+                const int k0 = n0, k1 = n1, k2 = n2, k3 = n3;
+                if (u + 4 < U) fetch(u + 4);
+                const u32 g = look4(w, rem);
+                // the four units' hits (at most 32 each) side by side in one sum
+                const u32 s4 = __reduce_add_sync(FULL, g << (lane & 24u));
+                if ((int)lane == k0) f += s4 & 0xFFu;
+                if ((int)lane == k1) f += (s4 >> 8) & 0xFFu;
+                if ((int)lane == k2) f += (s4 >> 16) & 0xFFu;
+                if ((int)lane == k3) f += s4 >> 24;
+            }
+            if (f) {
+                atomicAdd(&cnt[y], (u64)f);
+                Tc += f;
+            }
+        }
+        __syncwarp();
+        // flush and clear
+        for (u32 b = lane; b < L::NB; b += 32) {
+            const u32 h = hits[b];
+            if (h) {
+                const uint2 kk = buckets[b];
+                if (h & 0xFFFFu) atomicAdd(&cnt[kk.x & ~top], (u64)(h & 0xFFFFu));
+                if (h >> 16) atomicAdd(&cnt[kk.y & ~top], (u64)(h >> 16));
+                hits[b] = 0;
+            }
+            reinterpret_cast<uint2*>(keys)[b] = make_uint2(EMPTY_KEY, EMPTY_KEY);
+        }
+        T += __reduce_add_sync(FULL, Tc);
+        __syncwarp();
+    }
+    if (lane == 0 && T) {
+        atomicAdd(&cnt[x], T);
+        local_total += T;
+    }
+}
+
+// HUB: the large owners' tiles come first.
 template <int BLOCK, typename OffT, bool HUB>
-__global__ void __launch_bounds__(BLOCK)
+__global__ void __launch_bounds__(BLOCK, 4)
     k_count_medium(const u64* __restrict__ fo, const u32* __restrict__ head, u64 n,
                    const Desc<OffT>* __restrict__ vdesc, const u32* __restrict__ headp,
-                   const uint2* __restrict__ mtiles, u32 seg, u64* __restrict__ cnt,
-                   u64* __restrict__ partials, Control* ctl) {
-    using L = MediumLayout<BLOCK>;
+                   const uint2* __restrict__ mtiles, const uint2* __restrict__ ltiles, u32 seg,
+                   u64* __restrict__ cnt, u64* __restrict__ partials, Control* ctl) {
+    using L = TileLayout<OffT>;
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ u64 s_red[L::NW];
-    (void)n;
+    __shared__ u64 s_red[BLOCK / 32];
     if (ctl->err & DEV_ERR_MASK) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    u32* keys = reinterpret_cast<u32*>(smem) + warp * L::PER_WARP;
-    const u64 ntiles = *(volatile unsigned long long*)&ctl->medium_tiles;
+    u32* base = reinterpret_cast<u32*>(smem) + warp * L::PER_WARP;
+    tile_init<OffT>(base);
+    const u64 nl = HUB ? *(volatile unsigned long long*)&ctl->large_tiles : 0;
+    const u64 ntiles = nl + *(volatile unsigned long long*)&ctl->medium_tiles;
+    const u32 top = n < 0x7FFFFFFFu ? 0x80000000u : 0u;
     u64 local_total = 0;
     u32 dup = 0;
     while (true) {
@@ -894,7 +1009,8 @@ __global__ void __launch_bounds__(BLOCK)
         if (lane == 0) t = atomicAdd(&ctl->medium_next, 1ull);
         t = __shfl_sync(0xFFFFFFFFu, t, 0);
         if (t >= ntiles) break;
-        medium_tile<BLOCK, OffT, HUB>(keys, mtiles[t], fo, head, vdesc, headp, seg, cnt, local_total, dup);
+        medium_tile<OffT, HUB>(base, top, HUB && t < nl ? ltiles[t] : mtiles[t - nl], fo, head, vdesc, headp, seg, cnt,
+                               local_total, dup);
     }
     if (dup) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
     const u64 bt = block_sum_u64<BLOCK>(local_total, s_red);
@@ -1290,11 +1406,11 @@ __global__ void k_stats(const u64* __restrict__ fo, const u32* __restrict__ head
 // ---- the serving engine ----------------------------------------------------------------
 
 using EngineSmallL = SmallWarpLayout<u32, false>;
-using EngineMediumL = MediumLayout<ENGINE_BLOCK>;
+using EngineMediumL = TileLayout<u32>;
 using EngineLargeL = LargeLayout<ENGINE_BLOCK, LARGE_CAP, u32>;
 constexpr size_t cmax(size_t a, size_t b) { return a > b ? a : b; }
 constexpr size_t ENGINE_SMEM =
-    cmax(cmax(EngineSmallL::bytes(ENGINE_BLOCK / 32), EngineMediumL::bytes), EngineLargeL::bytes);
+    cmax(cmax(EngineSmallL::bytes(ENGINE_BLOCK / 32), EngineMediumL::bytes(ENGINE_BLOCK / 32)), EngineLargeL::bytes);
 static_assert(SMALL_BLOCK == ENGINE_BLOCK && MEDIUM_BLOCK == ENGINE_BLOCK && LARGE_BLOCK == ENGINE_BLOCK,
               "the engine runs every kind of unit with one block shape");
 
@@ -1459,16 +1575,18 @@ __global__ void __launch_bounds__(ENGINE_BLOCK, 4) k_engine(EngineJob* jobs, u32
             }
         } else if (u < jb->units_small + jb->units_medium) {
             const u64 nt = *(volatile unsigned long long*)&ctl->medium_tiles;
+            u32* slice = reinterpret_cast<u32*>(smem) + warp * EngineMediumL::PER_WARP;
+            tile_init<u32>(slice);
+            const u32 top = jb->n < 0x7FFFFFFFu ? 0x80000000u : 0u;
             for (u32 r = 0; r < ENGINE_REPS; ++r) {
                 const u64 t = ((u - jb->units_small) * (ENGINE_BLOCK / 32) + warp) * ENGINE_REPS + r;
                 if (t < nt)
-                    medium_tile<BLOCK, u32, false, true>(reinterpret_cast<u32*>(smem) + warp * EngineMediumL::PER_WARP,
-                                                  __ldcg(jb->mtiles + t), jb->fo, jb->head, vd, jb->headp, jb->seg,
-                                                  jb->cnt, unused_total, dup);
+                    medium_tile<u32, false, true>(slice, top, __ldcg(jb->mtiles + t), jb->fo, jb->head, vd, jb->headp,
+                                                  jb->seg, jb->cnt, unused_total, dup);
             }
         } else {
             const u64 t = u - jb->units_small - jb->units_medium;
-            timed_out = large_tile<BLOCK, LARGE_CAP, u32, false, true>(smem, s_bar, __ldcg(jb->ltiles + t), jb->fo, jb->head,
+            timed_out = large_tile<BLOCK, LARGE_CAP, u32, true>(smem, s_bar, __ldcg(jb->ltiles + t), jb->fo, jb->head,
                                                                 jb->n, vd, jb->headp,
                                                           jb->seg, jb->cnt, COPY_WAIT_POLLS, phase, inflight,
                                                           unused_total, dup);
@@ -1524,7 +1642,6 @@ void launch_engine(EngineJob* jobs, u32 njobs, unsigned long long* done_words, u
 namespace {
 template <typename OffT>
 using LargeL = LargeLayout<LARGE_BLOCK, LARGE_CAP, OffT>;
-using MediumL = MediumLayout<MEDIUM_BLOCK>;
 
 // Resident blocks per SM of a kernel, looked up once; also allows it its dynamic shared memory.
 template <typename Kernel>
@@ -1544,12 +1661,14 @@ int count_grid_small(int num_sms) {
 }
 template <typename OffT, bool HUB>
 int count_grid_medium(int num_sms) {
-    static const int occ = occupancy_of(k_count_medium<MEDIUM_BLOCK, OffT, HUB>, MEDIUM_BLOCK, MediumL::bytes);
+    static const int occ = occupancy_of(k_count_medium<MEDIUM_BLOCK, OffT, HUB>, MEDIUM_BLOCK,
+                                        TileLayout<OffT>::bytes(MEDIUM_BLOCK / 32));
     return num_sms * occ;
 }
 template <typename OffT, bool HUB>
 int count_grid_large(int num_sms) {
-    static const int occ = occupancy_of(k_count_large<LARGE_BLOCK, LARGE_CAP, OffT, HUB>, LARGE_BLOCK, LargeL<OffT>::bytes);
+    if constexpr (HUB) return 0;  // the hub and medium kernels take every tile
+    static const int occ = occupancy_of(k_count_large<LARGE_BLOCK, LARGE_CAP, OffT>, LARGE_BLOCK, LargeL<OffT>::bytes);
     return num_sms * occ;
 }
 template <bool HUB>
@@ -1596,11 +1715,12 @@ cudaError_t launch_count_auto(const u64* fo, const u32* head, u64 n, u64 nnz, co
     if constexpr (HUB)
         k_count_hub<<<count_grid_hub<HUB>(num_sms), 32 * HUB_WARPS, HUB_SMEM, st>>>(
             fo, head, vd, hub.lists, hub.ids, hub.top_info, hub.top_bits, mtiles, ltiles, seg, cnt, partials + cap + gm + gl, ctl);
-    k_count_medium<MEDIUM_BLOCK, OffT, HUB>
-        <<<gm, MEDIUM_BLOCK, MediumL::bytes, st>>>(fo, head, n, vd, headp, mtiles, seg, cnt, partials + cap, ctl);
-    k_count_large<LARGE_BLOCK, LARGE_CAP, OffT, HUB>
-        <<<gl, LARGE_BLOCK, LargeL<OffT>::bytes, st>>>(fo, head, n, vd, headp, ltiles, seg, cnt, partials + cap + gm,
-                                                       ctl, copy_wait_polls);
+    k_count_medium<MEDIUM_BLOCK, OffT, HUB><<<gm, MEDIUM_BLOCK, TileLayout<OffT>::bytes(MEDIUM_BLOCK / 32), st>>>(
+        fo, head, n, vd, headp, mtiles, ltiles, seg, cnt, partials + cap, ctl);
+    if constexpr (!HUB)
+        k_count_large<LARGE_BLOCK, LARGE_CAP, OffT>
+            <<<gl, LARGE_BLOCK, LargeL<OffT>::bytes, st>>>(fo, head, n, vd, headp, ltiles, seg, cnt, partials + cap + gm,
+                                                           ctl, copy_wait_polls);
     if (after_large) cudaEventRecord(after_large, st);
     return cudaGetLastError();
 }
