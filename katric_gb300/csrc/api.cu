@@ -54,6 +54,7 @@ struct ktri_ctx {
     int32_t last_method = KTRI_METHOD_AUTO;
     bool last_collect = false;
     bool hubs = true;          // counts may split their out-lists (more workspace than ktri_workspace_bytes)
+    bool chained = true;       // kernels are launched chained (LaunchStream)
 };
 
 namespace {
@@ -81,11 +82,11 @@ u64 isqrt_ceil(u64 x) {
     return r;
 }
 
-constexpr size_t HUB_WORKSPACE_BYTES = size_t(64) << 20;
+constexpr u64 HUB_MIN_NNZ = 1ull << 21;
 
 // Workspace of one count.  num_sms = 0 sizes the grids for the largest supported part.
 Layout make_layout(u64 n, u64 nnz, int32_t method, int num_sms, bool with_inputs, bool internal_cnt,
-                   bool force_wide = false, u32 small_d = 32, u32 seg = ktri::LARGE_SEG, bool hub = false) {
+                   bool force_wide = false, u32 small_d = 0, u32 seg = 0, bool hub = false) {
     Layout L;
     const u64 cap = ktri::oriented_capacity(n, nnz);
     L.wide = force_wide || cap > ktri::NARROW_CAPACITY;
@@ -96,7 +97,12 @@ Layout make_layout(u64 n, u64 nnz, int32_t method, int num_sms, bool with_inputs
         off = align_up(off + bytes);
         return at;
     };
+    // Hubs pay where the owner tiles outweigh the five short launches they add (RMAT n = 2^18 1.52 ->
+    // 0.60 ms, 2^16 0.36 -> 0.26 ms; +0.03 ms on graphs without hubs).
+    L.hub = hub && method == KTRI_METHOD_AUTO && !L.wide && nnz >= HUB_MIN_NNZ && n < ktri::HUB_MAX_N &&
+            nnz <= ktri::HUB_MAX_NNZ;
     L.ctl = take(sizeof(Control));
+    if (L.hub) L.hub_bins = take(sizeof(u32) * ktri::hub_bins_words());  // its counters are zeroed with ctl
     L.deg = take(sizeof(u32) * (n + 1));
     L.dplus = take(sizeof(u32) * (n + 1));
     L.vdesc = take((L.wide ? 16 : 8) * (n + 1));
@@ -105,10 +111,13 @@ Layout make_layout(u64 n, u64 nnz, int32_t method, int num_sms, bool with_inputs
     L.tile_i0 = take(sizeof(u32) * (ktri::base_tiles(n, nnz) + 2));
     u32 grid = 0;
     if (method == KTRI_METHOD_AUTO) {
-        // medium- and large-owner tiles, and both reordered
-        L.ltiles = take(sizeof(uint2) * 4 * ktri::large_tile_capacity(n, nnz, small_d, seg));
+        // medium- and large-owner tiles, and both reordered (seg = 0: room for the default options)
+        const u64 tcap = seg ? ktri::large_tile_capacity(n, nnz, small_d, seg)
+                             : std::max(ktri::large_tile_capacity(n, nnz, 32, ktri::LARGE_SEG),
+                                        ktri::large_tile_capacity(n, nnz, 32, ktri::default_segment(nnz)));
+        L.ltiles = take(sizeof(uint2) * 4 * tcap);
         L.thist = take(sizeof(u32) * ktri::tile_order_scratch_words());
-        L.tkeys = take(sizeof(u32) * ktri::large_tile_capacity(n, nnz, small_d, seg));
+        L.tkeys = take(sizeof(u32) * tcap);
         grid = (u32)(sms * 48);  // bound on the small + medium + large persistent grids (occupancy <= 16 each)
     } else {
         L.mid = take(sizeof(u32) * (n + 1));
@@ -129,12 +138,7 @@ Layout make_layout(u64 n, u64 nnz, int32_t method, int num_sms, bool with_inputs
         L.in_fo = take(sizeof(u64) * (n + 1));
         L.in_head = take(sizeof(u32) * (nnz + 1));
     }
-    // Hubs pay from the size on where the lists leave L1 and the choice of hubs (three short
-    // launches) is small; every graph the no-allocation array holds stays below the line.
-    if (hub && method == KTRI_METHOD_AUTO && !L.wide && off > HUB_WORKSPACE_BYTES && n < ktri::HUB_MAX_N &&
-        nnz <= ktri::HUB_MAX_NNZ) {
-        L.hub = true;
-        L.hub_bins = take(sizeof(u32) * ktri::hub_bins_words());
+    if (L.hub) {
         L.hub_tmp = take(sizeof(uint2) * ktri::HUB_H);
         L.hub_ids = take(sizeof(u32) * ktri::HUB_H);
         L.hub_lists = take(sizeof(ktri::u16) * ktri::hub_capacity(n, nnz));
@@ -162,8 +166,9 @@ int cuda_fail(ktri_ctx* ctx, cudaError_t e, const char* what) {
         if (e_ != cudaSuccess) return cuda_fail(ctx, e_, #call); \
     } while (0)
 
-ktri::Options resolve(const ktri_opts* o) {
+ktri::Options resolve(const ktri_opts* o, u64 nnz) {
     ktri::Options r;
+    r.segment = ktri::default_segment(nnz);
     if (!o || o->struct_size == 0) return r;
     r.method = o->intersection_method;
     r.collect_stats = o->collect_stats != 0;
@@ -369,10 +374,11 @@ u32 first_wait_polls(uint32_t opt) {
 // no-allocation entry point): errors then carry no message and no events are recorded.
 template <typename OffT, bool HUB>
 int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const u64* fo, const u32* head, u64 n,
-                     u64 nnz, u64* d_total, u64* cnt, const ktri::Options& opt, cudaStream_t st, bool sort_all,
+                     u64 nnz, u64* d_total, u64* cnt, const ktri::Options& opt, cudaStream_t stream, bool sort_all,
                      bool events, ktri::TriangleSink sink = ktri::TriangleSink{}, const HeadChunks* chunks = nullptr,
                      const EnginePublish* publish = nullptr) {
     events = events && ctx;
+    const ktri::LaunchStream st(stream, !ctx || ctx->chained);
     auto* ctl = reinterpret_cast<Control*>(base + L.ctl);
     auto* deg = reinterpret_cast<u32*>(base + L.deg);
     auto* dplus = reinterpret_cast<u32*>(base + L.dplus);
@@ -396,7 +402,8 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     // an error a caller's own failed runtime call left in this thread must not be taken for a
     // failed launch of ours below (errors of kernels that faulted are sticky and stay visible)
     (void)cudaGetLastError();
-    KTRI_CK(ctx, cudaMemsetAsync(ctl, 0, sizeof(Control), st));
+    const size_t zeroed = HUB ? L.hub_bins + ktri::hub_bins_zeroed() - L.ctl : sizeof(Control);
+    KTRI_CK(ctx, cudaMemsetAsync(ctl, 0, zeroed, st));
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[0], st));
     const bool autom = opt.method == KTRI_METHOD_AUTO && !sort_all;
     ktri::launch_prep(fo, n, nnz, deg, dplus, cnt, tile_i0, hub, ctl, sms, st);
@@ -579,6 +586,19 @@ int device_status(ktri_ctx* ctx) {
     return KTRI_OK;
 }
 
+// A new device call may follow one whose status was not read: it replaces that call's status, and
+// its work is ordered after that call's (they share the workspace) on the device, without the host
+// waiting.
+int order_after_pending(ktri_ctx* ctx, cudaStream_t st) {
+    if (!ctx->pending) return KTRI_OK;
+    if (!ctx->have_events) {
+        (void)device_status(ctx);
+        return KTRI_OK;
+    }
+    if (st != ctx->last_stream) KTRI_CK(ctx, cudaStreamWaitEvent(st, ctx->ev[3], 0));
+    return KTRI_OK;
+}
+
 std::mutex g_default_mu;
 std::map<int, ktri_ctx*> g_default;
 
@@ -654,7 +674,7 @@ int noalloc_scratch(int device, void** out) {
 // out-degrees and per-vertex counts; every other region is fully written before it is read.
 int run_noalloc(char* base, const Layout& L, const u64* fo, const u32* head, u64 n, u64 nnz, u64* d_total, u64* cnt,
                 int sms, cudaStream_t st) {
-    const ktri::Options opt;  // AUTO, default owner bins and segment (the layout is sized for them)
+    const ktri::Options opt = resolve(nullptr, nnz);  // AUTO, default options (the layout is sized for them)
     if (enqueue_layout(nullptr, sms, base, L, fo, head, n, nnz, d_total, cnt, opt, st, false, false) != KTRI_OK)
         return KTRI_ERR_CUDA;
     auto* ctl = reinterpret_cast<Control*>(base + L.ctl);
@@ -669,14 +689,14 @@ int run_noalloc(char* base, const Layout& L, const u64* fo, const u32* head, u64
 
 int ktri::ctx_device(const ktri_ctx* ctx) { return ctx->device; }
 
-void ktri::ctx_plain_lists(ktri_ctx* ctx) { ctx->hubs = false; }
+void ktri::ctx_for_server(ktri_ctx* ctx) { ctx->hubs = ctx->chained = false; }
 
 int ktri::ctx_num_sms(const ktri_ctx* ctx) { return ctx->num_sms; }
 
 int ktri::engine_prepare_batch(ktri_ctx* ctx, const uint64_t* d_first_out, const uint32_t* d_head, uint64_t n_total,
                                uint64_t nnz_total, uint64_t* d_per_vertex, void* stream, ktri::EngineJob* job,
                                unsigned long long seq, unsigned long long* done_word, ktri::Control** ctl_out) {
-    ktri::Options opt;  // AUTO with the default bins and segment
+    const ktri::Options opt = resolve(nullptr, nnz_total);  // AUTO with the default options
     int rc = check_common(ctx, d_first_out, d_head, n_total, nnz_total, d_per_vertex, opt);
     if (rc) return rc;
     if (!d_per_vertex || !job || !done_word || n_total == 0) return KTRI_ERR_INVALID_ARGUMENT;
@@ -797,15 +817,13 @@ int ktri_ctx_check(ktri_ctx* ctx) {
 int ktri_count_csr_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint32_t* d_head, uint64_t n,
                           uint64_t nnz, uint64_t* d_total, uint64_t* d_per_vertex, const ktri_opts* opts,
                           void* stream) {
-    const ktri::Options opt = resolve(opts);
+    const ktri::Options opt = resolve(opts, nnz);
     int rc = check_common(ctx, d_first_out, d_head, n, nnz, d_total, opt);
     if (rc) return rc;
     DeviceGuard g(ctx->device);
-    if (ctx->pending) {
-        rc = device_status(ctx);
-        (void)rc;  // the previous call's status was not collected; the new call proceeds
-    }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    rc = order_after_pending(ctx, st);  // the previous call's status was not collected; the new call proceeds
+    if (rc) return rc;
     if (n == 0) {
         KTRI_CK(ctx, cudaMemsetAsync(d_total, 0, sizeof(u64), st));
         ctx->pending = false;
@@ -858,7 +876,7 @@ int ktri_count_csr_device_noalloc(const uint64_t* d_first_out, const uint32_t* d
 int ktri_count_csr_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t* head, uint64_t n, uint64_t nnz,
                        uint64_t* total_out, uint64_t* per_vertex_out, const ktri_opts* opts) {
     const auto t_entry = std::chrono::steady_clock::now();
-    const ktri::Options opt = resolve(opts);
+    const ktri::Options opt = resolve(opts, nnz);
     int rc = check_common(ctx, first_out, head, n, nnz, total_out, opt);
     if (rc) return rc;
     DeviceGuard g(ctx->device);
@@ -964,12 +982,13 @@ int ktri_binary_file_shape(const char* stem, uint64_t* n_out, uint64_t* nnz_out)
 
 int ktri_count_binary_file(ktri_ctx* ctx, const char* stem, uint64_t* total_out, uint64_t* per_vertex_out,
                            const ktri_opts* opts, uint64_t chunk_bytes) {
-    const ktri::Options opt = resolve(opts);
+    ktri::Options opt = resolve(opts, 0);
     if (!ctx) return KTRI_ERR_INVALID_ARGUMENT;
     if (!stem || !total_out) return set_error(ctx, KTRI_ERR_INVALID_ARGUMENT, "stem and total_out are required");
     uint64_t n = 0, nnz = 0;
     int rc = ktri_binary_file_shape(stem, &n, &nnz);
     if (rc) return set_error(ctx, rc, std::string("cannot read ") + stem + ".first_out / .head");
+    opt = resolve(opts, nnz);
     const u64 dummy = 0;
     rc = check_common(ctx, &dummy, &dummy, n, nnz, total_out, opt);
     if (rc) return rc;
@@ -1158,7 +1177,7 @@ int ktri_contract_dag_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32
 int ktri_partition_cost(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t* head, uint64_t n, uint64_t nnz,
                         int32_t cost_function, uint32_t parts, uint64_t* boundaries_out, uint64_t* costs_out,
                         uint64_t* total_cost_out) {
-    ktri::Options opt;
+    ktri::Options opt = resolve(nullptr, 0);
     opt.method = KTRI_METHOD_MERGE;
     int rc = check_common(ctx, first_out, head, n, nnz, total_cost_out, opt);
     if (rc) return rc;
@@ -1210,7 +1229,7 @@ int ktri_partition_cost(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t
 
 int ktri_list_triangles(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t* head, uint64_t n, uint64_t nnz,
                         uint32_t* triples_out, uint64_t capacity, uint64_t* count_out) {
-    ktri::Options opt;
+    ktri::Options opt = resolve(nullptr, 0);
     opt.method = KTRI_METHOD_MERGE;
     int rc = check_common(ctx, first_out, head, n, nnz, count_out, opt);
     if (rc) return rc;
@@ -1258,13 +1277,14 @@ int ktri_list_triangles(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t
 
 int ktri_count_dag_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint32_t* d_head, uint64_t n, uint64_t m,
                           uint64_t* d_total, uint64_t* d_per_vertex, const ktri_opts* opts, void* stream) {
-    const ktri::Options opt = resolve(opts);
+    const ktri::Options opt = resolve(opts, 2 * m);
     int rc = check_common(ctx, d_first_out, d_head, n, m, d_total, opt);
     if (rc) return rc;
     if (m > (1ull << 62)) return set_error(ctx, KTRI_ERR_UNSUPPORTED, "too many edges");
     DeviceGuard g(ctx->device);
-    if (ctx->pending) device_status(ctx);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    rc = order_after_pending(ctx, st);
+    if (rc) return rc;
     if (n == 0) {
         KTRI_CK(ctx, cudaMemsetAsync(d_total, 0, sizeof(u64), st));
         ctx->pending = false;
@@ -1292,7 +1312,7 @@ int ktri_count_dag_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint
 
 int ktri_count_dag_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t* head, uint64_t n, uint64_t m,
                        uint64_t* total_out, uint64_t* per_vertex_out, const ktri_opts* opts) {
-    const ktri::Options opt = resolve(opts);
+    const ktri::Options opt = resolve(opts, 2 * m);
     int rc = check_common(ctx, first_out, head, n, m, total_out, opt);
     if (rc) return rc;
     DeviceGuard g(ctx->device);
@@ -1368,7 +1388,7 @@ int enqueue_batch(ktri_ctx* ctx, char* base, const Layout& L, const u64* fo, con
     int rc = enqueue_layout(ctx, ctx->num_sms, base, L, fo, head, n, nnz, d_total, cnt, opt, st, false, events);
     if (rc) return rc;
     ktri::launch_graph_totals(cnt, graph_first, num_graphs, n, totals, reinterpret_cast<Control*>(base + L.ctl),
-                              ctx->num_sms, st);
+                              ctx->num_sms, ktri::LaunchStream(st, ctx->chained));
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[3], st));  // the call ends after the totals
     KTRI_CK(ctx, cudaGetLastError());
     return KTRI_OK;
@@ -1395,12 +1415,13 @@ extern "C" {
 int ktri_count_batch_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint32_t* d_head, uint64_t n_total,
                             uint64_t nnz_total, const uint64_t* d_graph_first, uint64_t num_graphs, uint64_t* d_totals,
                             uint64_t* d_per_vertex, const ktri_opts* opts, void* stream) {
-    const ktri::Options opt = resolve(opts);
+    const ktri::Options opt = resolve(opts, nnz_total);
     int rc = check_batch(ctx, d_first_out, d_head, n_total, nnz_total, d_graph_first, num_graphs, d_totals, opt);
     if (rc) return rc;
     DeviceGuard g(ctx->device);
-    if (ctx->pending) device_status(ctx);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    rc = order_after_pending(ctx, st);
+    if (rc) return rc;
     if (n_total == 0) {
         if (num_graphs) KTRI_CK(ctx, cudaMemsetAsync(d_totals, 0, sizeof(u64) * num_graphs, st));
         ctx->pending = false;
@@ -1423,7 +1444,7 @@ int ktri_count_batch_device(ktri_ctx* ctx, const uint64_t* d_first_out, const ui
 int ktri_count_batch_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t* head, uint64_t n_total,
                          uint64_t nnz_total, const uint64_t* graph_first, uint64_t num_graphs, uint64_t* totals_out,
                          uint64_t* per_vertex_out, const ktri_opts* opts) {
-    const ktri::Options opt = resolve(opts);
+    const ktri::Options opt = resolve(opts, nnz_total);
     int rc = check_batch(ctx, first_out, head, n_total, nnz_total, graph_first, num_graphs, totals_out, opt);
     if (rc) return rc;
     DeviceGuard g(ctx->device);
@@ -1493,7 +1514,7 @@ int ktri_plan_create_batch(ktri_ctx* ctx, const uint64_t* d_first_out, const uin
                            uint64_t* d_totals, uint64_t* d_per_vertex, const ktri_opts* opts, ktri_plan** out) {
     if (!out) return set_error(ctx, KTRI_ERR_INVALID_ARGUMENT, "out is NULL");
     *out = nullptr;
-    const ktri::Options opt = resolve(opts);
+    const ktri::Options opt = resolve(opts, nnz_total);
     int rc = check_batch(ctx, d_first_out, d_head, n_total, nnz_total, d_graph_first, num_graphs, d_totals, opt);
     if (rc) return rc;
     if (n_total == 0) return set_error(ctx, KTRI_ERR_INVALID_ARGUMENT, "a plan needs at least one vertex");
@@ -1608,7 +1629,7 @@ int ktri_orient_csr(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t* he
     if (n == 0) return KTRI_OK;
     if (first_out[0] != 0 || first_out[n] != nnz)
         return set_error(ctx, KTRI_ERR_INVALID_CSR, "first_out[0] must be 0 and first_out[n] must equal nnz");
-    ktri::Options opt;
+    ktri::Options opt = resolve(nullptr, 0);
     opt.method = KTRI_METHOD_MERGE;
     Layout L = make_layout(n, nnz, KTRI_METHOD_MERGE, ctx->num_sms, true, true);
     // room for the exported CSR: out offsets (u64[n+1]) and out heads (u32[nnz/2])

@@ -460,6 +460,7 @@ __global__ void __launch_bounds__(BLOCK, 4) k_count_small(u64 n, u32 vb, const D
                                                           const u32* __restrict__ hub_ids, u32 sd,
                                                           u64* __restrict__ cnt, u64* __restrict__ partials,
                                                           Control* ctl) {
+    chain_begin();
     using L = SmallWarpLayout<OffT, HUB>;
     constexpr int NW = BLOCK / 32;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -749,18 +750,23 @@ __global__ void __launch_bounds__(BLOCK) k_count_large(const u64* __restrict__ f
                                                        const uint2* __restrict__ ltiles, u32 seg,
                                                        u64* __restrict__ cnt, u64* __restrict__ partials,
                                                        Control* ctl, u32 first_wait_polls) {
+    chain_begin();
     using L = LargeLayout<BLOCK, CAP, OffT>;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ u64 s_t;
     unsigned long long* s_bar = reinterpret_cast<unsigned long long*>(smem + L::off_bar);  // the bulk copy's barrier
 
     if (ctl->err & DEV_ERR_MASK) return;
+    const u64 ntiles = *(volatile unsigned long long*)&ctl->large_tiles;
+    if (ntiles == 0) {
+        if (threadIdx.x == 0) partials[blockIdx.x] = 0;
+        return;
+    }
     if (threadIdx.x == 0) mbar_init(s_bar, 1);
     fence_proxy_async_smem();
     __syncthreads();
     u32 phase = 0;
     bool timed_out = false, inflight = false;
-    const u64 ntiles = *(volatile unsigned long long*)&ctl->large_tiles;
     u64 local_total = 0;
     u32 dup = 0;
     while (true) {
@@ -992,15 +998,20 @@ __global__ void __launch_bounds__(BLOCK, 4)
                    const Desc<OffT>* __restrict__ vdesc, const u32* __restrict__ headp,
                    const uint2* __restrict__ mtiles, const uint2* __restrict__ ltiles, u32 seg,
                    u64* __restrict__ cnt, u64* __restrict__ partials, Control* ctl) {
+    chain_begin();
     using L = TileLayout<OffT>;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ u64 s_red[BLOCK / 32];
     if (ctl->err & DEV_ERR_MASK) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     u32* base = reinterpret_cast<u32*>(smem) + warp * L::PER_WARP;
-    tile_init<OffT>(base);
     const u64 nl = HUB ? *(volatile unsigned long long*)&ctl->large_tiles : 0;
     const u64 ntiles = nl + *(volatile unsigned long long*)&ctl->medium_tiles;
+    if (ntiles == 0) {
+        if (threadIdx.x == 0) partials[blockIdx.x] = 0;
+        return;
+    }
+    tile_init<OffT>(base);
     const u32 top = n < 0x7FFFFFFFu ? 0x80000000u : 0u;
     u64 local_total = 0;
     u32 dup = 0;
@@ -1139,6 +1150,7 @@ __global__ void __launch_bounds__(32 * HUB_WARPS, 1)
                 const uint2* __restrict__ top_bits, const uint2* __restrict__ mtiles,
                 const uint2* __restrict__ ltiles, u32 seg, u64* __restrict__ cnt, u64* __restrict__ partials,
                 Control* ctl) {
+    chain_begin();
     using L = HubLayout;
     constexpr u32 FULL = 0xFFFFFFFFu;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1148,6 +1160,10 @@ __global__ void __launch_bounds__(32 * HUB_WARPS, 1)
     const u32 nh = ctl->hubs;
     const u64 nl = *(volatile unsigned long long*)&ctl->large_tiles;
     const u64 nt = nh ? nl + *(volatile unsigned long long*)&ctl->medium_tiles : 0;
+    if (nt == 0) {
+        if (threadIdx.x == 0) partials[blockIdx.x] = 0;
+        return;
+    }
     unsigned char* sbase = smem + ((L::align - (smem_u32(smem) & (L::align - 1))) & (L::align - 1));
     u32* hcnt = reinterpret_cast<u32*>(sbase + L::off_cnt);
     u32* bits = reinterpret_cast<u32*>(sbase + L::off_bits) + warp * L::BITS;
@@ -1314,6 +1330,7 @@ __global__ void __launch_bounds__(32 * HUB_WARPS, 1)
 // bounded wait that ran out) the partials are incomplete or stale, so the total is written as 0.
 __global__ void __launch_bounds__(1024) k_final(const u64* __restrict__ partials, u32 np, u32 skip0, u32 skip1,
                                                 u64* total, const Control* ctl) {
+    chain_begin();
     __shared__ u64 s_red[32];
     if (*(volatile const u32*)&ctl->err & DEV_ERR_MASK) {
         if (threadIdx.x == 0) *total = 0;
@@ -1331,6 +1348,7 @@ __global__ void __launch_bounds__(1024) k_final(const u64* __restrict__ partials
 // all inside one graph, so a graph's total is the sum of its per-vertex counts over three.
 __global__ void __launch_bounds__(256) k_graph_totals(const u64* __restrict__ cnt, const u64* __restrict__ graph_first,
                                                       u64 num_graphs, u64 n, u64* __restrict__ totals, Control* ctl) {
+    chain_begin();
     __shared__ u64 s_red[8];
     if (ctl->err & DEV_ERR_MASK) return;
     for (u64 g = blockIdx.x; g < num_graphs; g += gridDim.x) {
@@ -1356,6 +1374,7 @@ __global__ void k_stats(const u64* __restrict__ fo, const u32* __restrict__ head
                         const Desc<OffT>* __restrict__ vdesc, const u32* __restrict__ headp,
                         const u16* __restrict__ hubp, const u32* __restrict__ hub_ids, u32 small_d, u32 medium_d,
                         Control* ctl) {
+    chain_begin();
     if (ctl->err & DEV_ERR_MASK) return;
     const int lane = threadIdx.x & 31;
     const u64 gw = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1701,7 +1720,7 @@ int count_grid_auto(int num_sms) {
 template <typename OffT, bool HUB>
 cudaError_t launch_count_auto(const u64* fo, const u32* head, u64 n, u64 nnz, const void* vdesc, const u32* headp,
                               const HubState& hub, const uint2* mtiles, const uint2* ltiles, u32 small_d, u32 seg, u64* cnt, u64* partials,
-                              Control* ctl, int num_sms, cudaStream_t st, cudaEvent_t after_small,
+                              Control* ctl, int num_sms, LaunchStream st, cudaEvent_t after_small,
                               cudaEvent_t after_large, u32 copy_wait_polls) {
     (void)nnz;
     const int cap = count_grid_small<OffT, HUB>(num_sms);
@@ -1709,57 +1728,56 @@ cudaError_t launch_count_auto(const u64* fo, const u32* head, u64 n, u64 nnz, co
     const int gm = count_grid_medium<OffT, HUB>(num_sms);
     const int gl = count_grid_large<OffT, HUB>(num_sms);
     const auto* vd = reinterpret_cast<const Desc<OffT>*>(vdesc);
-    k_count_small<SMALL_BLOCK, OffT, HUB><<<gs, SMALL_BLOCK, SmallWarpLayout<OffT, HUB>::bytes(SMALL_BLOCK / 32), st>>>(
+    launch_chained(k_count_small<SMALL_BLOCK, OffT, HUB>, gs, SMALL_BLOCK, SmallWarpLayout<OffT, HUB>::bytes(SMALL_BLOCK / 32), st, 
         n, small_batch_vertices(n, cap), vd, headp, hub.lists, hub.ids, small_d, cnt, partials, ctl);
     if (after_small) cudaEventRecord(after_small, st);
     if constexpr (HUB)
-        k_count_hub<<<count_grid_hub<HUB>(num_sms), 32 * HUB_WARPS, HUB_SMEM, st>>>(
+        launch_chained(k_count_hub, count_grid_hub<HUB>(num_sms), 32 * HUB_WARPS, HUB_SMEM, st, 
             fo, head, vd, hub.lists, hub.ids, hub.top_info, hub.top_bits, mtiles, ltiles, seg, cnt, partials + cap + gm + gl, ctl);
-    k_count_medium<MEDIUM_BLOCK, OffT, HUB><<<gm, MEDIUM_BLOCK, TileLayout<OffT>::bytes(MEDIUM_BLOCK / 32), st>>>(
+    launch_chained(k_count_medium<MEDIUM_BLOCK, OffT, HUB>, gm, MEDIUM_BLOCK, TileLayout<OffT>::bytes(MEDIUM_BLOCK / 32), st, 
         fo, head, n, vd, headp, mtiles, ltiles, seg, cnt, partials + cap, ctl);
     if constexpr (!HUB)
-        k_count_large<LARGE_BLOCK, LARGE_CAP, OffT>
-            <<<gl, LARGE_BLOCK, LargeL<OffT>::bytes, st>>>(fo, head, n, vd, headp, ltiles, seg, cnt, partials + cap + gm,
+        launch_chained(k_count_large<LARGE_BLOCK, LARGE_CAP, OffT>, gl, LARGE_BLOCK, LargeL<OffT>::bytes, st, fo, head, n, vd, headp, ltiles, seg, cnt, partials + cap + gm,
                                                            ctl, copy_wait_polls);
     if (after_large) cudaEventRecord(after_large, st);
     return cudaGetLastError();
 }
 
 void launch_graph_totals(const u64* cnt, const u64* graph_first, u64 num_graphs, u64 n, u64* totals, Control* ctl,
-                         int num_sms, cudaStream_t st) {
+                         int num_sms, LaunchStream st) {
     if (num_graphs == 0) return;
     u64 blocks = num_graphs < (u64)num_sms * 8 ? num_graphs : (u64)num_sms * 8;
-    k_graph_totals<<<(unsigned)blocks, 256, 0, st>>>(cnt, graph_first, num_graphs, n, totals, ctl);
+    launch_chained(k_graph_totals, (unsigned)blocks, 256, 0, st, cnt, graph_first, num_graphs, n, totals, ctl);
 }
 
-void launch_final(const u64* partials, u32 np, u64* total, Control* ctl, cudaStream_t st) {
-    k_final<<<1, 1024, 0, st>>>(partials, np, 0, 0, total, ctl);
+void launch_final(const u64* partials, u32 np, u64* total, Control* ctl, LaunchStream st) {
+    launch_chained(k_final, 1, 1024, 0, st, partials, np, 0, 0, total, ctl);
 }
 
 template <typename OffT, bool HUB>
-void launch_final_auto(const u64* partials, u64 n, int num_sms, u64* total, Control* ctl, cudaStream_t st) {
+void launch_final_auto(const u64* partials, u64 n, int num_sms, u64* total, Control* ctl, LaunchStream st) {
     const int cap = count_grid_small<OffT, HUB>(num_sms);
-    k_final<<<1, 1024, 0, st>>>(partials, (u32)count_grid_auto<OffT, HUB>(num_sms), (u32)small_grid_launched(n, cap),
+    launch_chained(k_final, 1, 1024, 0, st, partials, (u32)count_grid_auto<OffT, HUB>(num_sms), (u32)small_grid_launched(n, cap),
                                 (u32)cap, total, ctl);
 }
 
 template <typename OffT, bool HUB>
 void launch_stats(const u64* fo, const u32* head, u64 n, const void* vdesc, const u32* headp, const HubState& hub,
-                  u32 small_d, u32 medium_d, Control* ctl, int num_sms, cudaStream_t st) {
+                  u32 small_d, u32 medium_d, Control* ctl, int num_sms, LaunchStream st) {
     if (n == 0) return;
-    k_stats<OffT, HUB><<<num_sms * 8, 256, 0, st>>>(fo, head, n, reinterpret_cast<const Desc<OffT>*>(vdesc), headp,
+    launch_chained(k_stats<OffT, HUB>, num_sms * 8, 256, 0, st, fo, head, n, reinterpret_cast<const Desc<OffT>*>(vdesc), headp,
                                                     hub.lists, hub.ids, small_d, medium_d, ctl);
 }
 
 #define KTRI_INST(OffT, HUB)                                                                                        \
-    template void launch_final_auto<OffT, HUB>(const u64*, u64, int, u64*, Control*, cudaStream_t);                 \
+    template void launch_final_auto<OffT, HUB>(const u64*, u64, int, u64*, Control*, LaunchStream);                 \
     template int count_grid_auto<OffT, HUB>(int);                                                                   \
     template cudaError_t launch_count_auto<OffT, HUB>(const u64*, const u32*, u64, u64, const void*, const u32*,    \
                                                       const HubState&, const uint2*, const uint2*, u32, u32, u64*,  \
-                                                      u64*, Control*, int, cudaStream_t, cudaEvent_t, cudaEvent_t,  \
+                                                      u64*, Control*, int, LaunchStream, cudaEvent_t, cudaEvent_t,  \
                                                       u32);                                                         \
     template void launch_stats<OffT, HUB>(const u64*, const u32*, u64, const void*, const u32*, const HubState&,    \
-                                          u32, u32, Control*, int, cudaStream_t);
+                                          u32, u32, Control*, int, LaunchStream);
 KTRI_INST(u32, false)
 KTRI_INST(u32, true)
 KTRI_INST(u64, false)

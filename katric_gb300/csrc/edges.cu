@@ -32,6 +32,7 @@ constexpr int BIN_STACK = 96;
 template <typename OffT>
 __global__ void k_sort_warp(u64 n, const Desc<OffT>* __restrict__ vdesc, u32* __restrict__ headp, u32* mid_list,
                             u32* big_list, Control* ctl) {
+    chain_begin();
     if (ctl->err & DEV_ERR_MASK) return;
     const int lane = threadIdx.x & 31;
     const u64 gw = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -88,6 +89,7 @@ __device__ void bitonic_block(u32* s, u32 P) {
 template <typename OffT>
 __global__ void __launch_bounds__(SORT_BLOCK) k_sort_block(const Desc<OffT>* __restrict__ vdesc, u32* headp,
                                                            const u32* mid_list, Control* ctl) {
+    chain_begin();
     __shared__ u32 s[SORT_SMEM];
     __shared__ int s_bad;
     const u64 cnt = *(volatile unsigned long long*)&ctl->sort_mid;
@@ -115,6 +117,7 @@ template <typename OffT>
 __global__ void __launch_bounds__(SORT_BLOCK) k_sort_global(const Desc<OffT>* __restrict__ vdesc, u32* headp,
                                                             const u32* big_list, u32* scratch, u64 scratch_per_block,
                                                             Control* ctl) {
+    chain_begin();
     const u64 cnt = *(volatile unsigned long long*)&ctl->sort_big;
     u32* s = scratch + (u64)blockIdx.x * scratch_per_block;
     for (u64 i = blockIdx.x; i < cnt; i += gridDim.x) {
@@ -291,6 +294,7 @@ __global__ void __launch_bounds__(EDGE_BLOCK) k_count_edges(u64 n, const Desc<Of
                                                             double hybrid_scale, u64* __restrict__ cnt,
                                                             u64* __restrict__ partials, Control* ctl,
                                                             TriangleSink sink) {
+    chain_begin();
     __shared__ u64 s_red[EDGE_BLOCK / 32];
     if (ctl->err & DEV_ERR_MASK) return;
     const int lane = threadIdx.x & 31;
@@ -445,20 +449,20 @@ __global__ void __launch_bounds__(PAIR_BLOCK) k_intersect_pairs(int method, cons
 
 template <typename OffT>
 void launch_sort_lists(u64 n, const void* vdesc, u32* headp, u32* mid_list, u32* big_list, u32* scratch,
-                       u64 scratch_per_block, int big_grid, Control* ctl, int num_sms, cudaStream_t st) {
+                       u64 scratch_per_block, int big_grid, Control* ctl, int num_sms, LaunchStream st) {
     if (n == 0) return;
     const auto* vd = reinterpret_cast<const Desc<OffT>*>(vdesc);
-    k_sort_warp<OffT><<<num_sms * 8, 256, 0, st>>>(n, vd, headp, mid_list, big_list, ctl);
-    k_sort_block<OffT><<<num_sms * 4, SORT_BLOCK, 0, st>>>(vd, headp, mid_list, ctl);
-    k_sort_global<OffT><<<big_grid, SORT_BLOCK, 0, st>>>(vd, headp, big_list, scratch, scratch_per_block, ctl);
+    launch_chained(k_sort_warp<OffT>, num_sms * 8, 256, 0, st, n, vd, headp, mid_list, big_list, ctl);
+    launch_chained(k_sort_block<OffT>, num_sms * 4, SORT_BLOCK, 0, st, vd, headp, mid_list, ctl);
+    launch_chained(k_sort_global<OffT>, big_grid, SORT_BLOCK, 0, st, vd, headp, big_list, scratch, scratch_per_block, ctl);
 }
 
 int count_grid_edges(int num_sms) { return num_sms * 8; }
 
 template <typename OffT>
 void launch_count_edges(u64 n, const void* vdesc, const u32* headp, int method, u64 cutoff, double hybrid_scale,
-                        u64* cnt, u64* partials, int grid, Control* ctl, TriangleSink sink, cudaStream_t st) {
-    k_count_edges<OffT><<<grid, EDGE_BLOCK, 0, st>>>(n, reinterpret_cast<const Desc<OffT>*>(vdesc), headp, method,
+                        u64* cnt, u64* partials, int grid, Control* ctl, TriangleSink sink, LaunchStream st) {
+    launch_chained(k_count_edges<OffT>, grid, EDGE_BLOCK, 0, st, n, reinterpret_cast<const Desc<OffT>*>(vdesc), headp, method,
                                                      cutoff, hybrid_scale, cnt, partials, ctl, sink);
 }
 
@@ -488,9 +492,9 @@ void launch_intersect_pairs(int method, const u32* a_vals, const u64* a_off, con
 
 #define KTRI_INST(OffT)                                                                                             \
     template void launch_sort_lists<OffT>(u64, const void*, u32*, u32*, u32*, u32*, u64, int, Control*, int,       \
-                                          cudaStream_t);                                                            \
+                                          LaunchStream);                                                            \
     template void launch_count_edges<OffT>(u64, const void*, const u32*, int, u64, double, u64*, u64*, int,         \
-                                           Control*, TriangleSink, cudaStream_t);                                   \
+                                           Control*, TriangleSink, LaunchStream);                                   \
     template void launch_outdeg<OffT>(u64, const void*, u64*, int, cudaStream_t);                                  \
     template void launch_export<OffT>(u64, const void*, const u32*, const u64*, u32*, int, cudaStream_t);
 KTRI_INST(u32)

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <utility>
 
 #include "ktri_internal.h"
 
@@ -105,6 +106,31 @@ __host__ __device__ __forceinline__ u64 hub_capacity(u64 n, u64 nnz) { return nn
 __device__ __forceinline__ u32 degree_bin(u32 d) {
     const u32 lg = 31 - __clz(d);
     return lg * 128 + (lg >= 7 ? (d >> (lg - 7)) & 0x7Fu : (d << (7 - lg)) & 0x7Fu);
+}
+
+// Chained launches (programmatic dependent launch): a kernel launched with launch_chained starts
+// while its predecessor in the stream still runs, as far as there is room, and chain_begin waits
+// until the predecessor's work is complete and visible, so only the launch latency overlaps (about
+// 2 us per kernel of the small graphs).  Every kernel launched this way calls chain_begin before
+// it touches global memory, and a kernel's successor starts only once all of its own blocks have.
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class Stream, class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, const Stream& ls,
+                                  A&&... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = ls.st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &attr;
+    c.numAttrs = ls.chained ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(std::forward<A>(args))...);
 }
 
 // Total order of the orientation, node_ordering::degree_outward: (deg, id).

@@ -20,7 +20,7 @@ struct Options {
     int32_t method = KTRI_METHOD_AUTO;
     uint32_t small_outdegree = 48;   // owner bins and tile segment of the AUTO kernels
     uint32_t medium_outdegree = 256;
-    uint32_t segment = 1024;
+    uint32_t segment = 0;            // 0: default_segment of the graph, set where its size is known
     bool collect_stats = false;
     uint64_t binary_cutoff = 1000;
     double hybrid_scale = 1.0;
@@ -32,8 +32,9 @@ struct Options {
 // The device a context was created on, and its SM count.
 int ctx_device(const ktri_ctx* ctx);
 int ctx_num_sms(const ktri_ctx* ctx);
-// Keep a context's workspaces at what ktri_workspace_bytes reports (no split out-lists).
-void ctx_plain_lists(ktri_ctx* ctx);
+// A context of one of the server's slots: workspaces as ktri_workspace_bytes reports them (no split
+// out-lists), and kernels that leave their room to the other slots' until they run.
+void ctx_for_server(ktri_ctx* ctx);
 
 struct Control;
 struct EngineJob;

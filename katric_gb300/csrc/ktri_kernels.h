@@ -13,6 +13,16 @@ using u16 = uint16_t;
 using u32 = uint32_t;
 using u64 = unsigned long long;
 
+// A stream, and whether the kernels launched on it are chained (launch_chained): they start while
+// their predecessor still runs.  Not where other streams' kernels should get the room that waiting
+// blocks would hold (the server's slots: 30 requests 7.3 ms chained, 6.9 ms not).
+struct LaunchStream {
+    cudaStream_t st;
+    bool chained;
+    LaunchStream(cudaStream_t s, bool c = true) : st(s), chained(c) {}
+    operator cudaStream_t() const { return st; }
+};
+
 constexpr int ORIENT_BLOCK = 256;   // 8 warps, one merge-path tile each
 constexpr int ORIENT_IPT = 8;       // slots per lane of a tile: tiles of 256 diagonals
 constexpr int SMALL_BLOCK = 256;
@@ -38,6 +48,15 @@ inline u64 large_tile_capacity(u64 n, u64 nnz, u32 small_d, u32 seg) {
     u64 owners = nnz / ((u64)small_d + 1) + 1;
     if (owners > n) owners = n;
     return owners + nnz / seg + 1;
+}
+
+// Default adjacency slots per owner tile: LARGE_SEG where the graph then still has several tiles for
+// every resident warp, fewer below (a power of two): a small graph's longest tile is its critical
+// path (RMAT n = 8191 from host memory 176 -> 157 us).
+inline u32 default_segment(u64 nnz) {
+    u32 seg = LARGE_SEG;
+    while (seg > MIN_SEG && nnz / seg < 8192) seg >>= 1;
+    return seg;
 }
 
 // Optional list of the triangles found by the edge-iterator kernel (debug listing): each
@@ -84,25 +103,26 @@ struct HubState {
     explicit operator bool() const { return lists != nullptr; }
 };
 u64 hub_bins_words();
+size_t hub_bins_zeroed();  // bytes of bins the caller zeroes before launch_prep
 // Top entries of long hub lists into bitmaps (after launch_desc; the lists then hold the others).
-void launch_hub_tops(const void* vdesc, const HubState& hub, Control* ctl, int num_sms, cudaStream_t st);
+void launch_hub_tops(const void* vdesc, const HubState& hub, Control* ctl, int num_sms, LaunchStream st);
 
 // Degrees, tile boundaries and, with hubs, the hub choice (deg then holds orientation keys).
 void launch_prep(const u64* fo, u64 n, u64 nnz, u32* deg, u32* dplus, u64* cnt, u32* tile_i0, const HubState& hub,
-                 Control* ctl, int num_sms, cudaStream_t st);
+                 Control* ctl, int num_sms, LaunchStream st);
 // Orientation over the blocks [tile_begin, tile_end) of ORIENT_TILE diagonals (all by
 // default; a block holds ORIENT_BLOCK / 32 base tiles).  Block t reads adjacency slots below
 // (t + 1) * ORIENT_TILE + 1 only, so it may run as soon as that prefix of head is on the device.
 constexpr u64 ORIENT_TILE = (u64)ORIENT_BLOCK * ORIENT_IPT;
 u64 orient_tiles(u64 n, u64 nnz);
 void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* deg, const u32* tile_i0, u32* headp,
-                   const HubState& hub, u32* dplus, u32* spanning, Control* ctl, cudaStream_t st, u64 tile_begin = 0,
+                   const HubState& hub, u32* dplus, u32* spanning, Control* ctl, LaunchStream st, u64 tile_begin = 0,
                    u64 tile_end = ~0ull);
 // Owner tiles: medium owners' tiles are written to mtiles, large owners' to ltiles (each
 // array holds large_tile_capacity entries).
 template <typename OffT, bool HUB>
 void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, const HubState& hub, uint2* mtiles,
-                 uint2* ltiles, u32 small_d, u32 medium_d, u32 seg, Control* ctl, int num_sms, cudaStream_t st);
+                 uint2* ltiles, u32 small_d, u32 medium_d, u32 seg, Control* ctl, int num_sms, LaunchStream st);
 
 // Owner tiles reordered (*count tiles on the device) by a counting sort on a 12-bit key:
 // TILE_BY_VERTEX, the first vertex each segment streams (tiles that run together then stream
@@ -115,7 +135,7 @@ enum : u32 { TILE_BY_VERTEX = 0, TILE_BY_DEGREE = 1, TILE_BY_COST = 2 };
 u64 tile_order_scratch_words();
 void launch_order_tiles(const u64* fo, const u32* head, const u32* dplus, u64 n, const uint2* tiles,
                         const unsigned long long* count, u32 seg, u32 mode, bool hub, u32* keys, u32* hist,
-                        uint2* sorted, Control* ctl, int num_sms, cudaStream_t st);
+                        uint2* sorted, Control* ctl, int num_sms, LaunchStream st);
 
 // The counting kernels of KTRI_METHOD_AUTO.  partials needs count_grid_auto entries.  The hub
 // kernel runs where hub is set (HUB, 32-bit descriptors only).
@@ -131,13 +151,13 @@ int count_grid_auto(int num_sms);  // small + medium + large + hub
 template <typename OffT, bool HUB>
 cudaError_t launch_count_auto(const u64* fo, const u32* head, u64 n, u64 nnz, const void* vdesc, const u32* headp,
                               const HubState& hub, const uint2* mtiles, const uint2* ltiles, u32 small_d, u32 seg,
-                              u64* cnt, u64* partials, Control* ctl, int num_sms, cudaStream_t st,
+                              u64* cnt, u64* partials, Control* ctl, int num_sms, LaunchStream st,
                               cudaEvent_t after_small, cudaEvent_t after_large, u32 copy_wait_polls = COPY_WAIT_POLLS);
-void launch_final(const u64* partials, u32 np, u64* total, Control* ctl, cudaStream_t st);
+void launch_final(const u64* partials, u32 np, u64* total, Control* ctl, LaunchStream st);
 // The total of an AUTO count (the small kernel's grid depends on n).
 int small_grid_launched(u64 n, int cap);
 template <typename OffT, bool HUB>
-void launch_final_auto(const u64* partials, u64 n, int num_sms, u64* total, Control* ctl, cudaStream_t st);
+void launch_final_auto(const u64* partials, u64 n, int num_sms, u64* total, Control* ctl, LaunchStream st);
 
 // ---- the serving engine ------------------------------------------------------------------
 // A prepared batch (orientation, descriptors and owner tiles done on its slot's stream) is
@@ -208,22 +228,22 @@ void launch_contract(const u64* fo, const u32* head, u64 n, u64 n_local, u64* cn
 void launch_dag_symmetrize(const u64* fo, const u32* head, u64 n, u64* fs, u32* hs, u32* cursor, u64* sums,
                            int num_sms, cudaStream_t st);
 void launch_graph_totals(const u64* cnt, const u64* graph_first, u64 num_graphs, u64 n, u64* totals, Control* ctl,
-                         int num_sms, cudaStream_t st);
+                         int num_sms, LaunchStream st);
 
 // Work counters of the reference (wedge_checks, intersection_size_local) and of the AUTO
 // kernels, accumulated into the control block.
 template <typename OffT, bool HUB>
 void launch_stats(const u64* fo, const u32* head, u64 n, const void* vdesc, const u32* headp, const HubState& hub,
-                  u32 small_d, u32 medium_d, Control* ctl, int num_sms, cudaStream_t st);
+                  u32 small_d, u32 medium_d, Control* ctl, int num_sms, LaunchStream st);
 
 // Sorted-list strategies (merge, binary search, binary, hybrid): sort out-lists by id, then
 // one warp per oriented edge.
 template <typename OffT>
 void launch_sort_lists(u64 n, const void* vdesc, u32* headp, u32* mid_list, u32* big_list, u32* scratch,
-                       u64 scratch_per_block, int big_grid, Control* ctl, int num_sms, cudaStream_t st);
+                       u64 scratch_per_block, int big_grid, Control* ctl, int num_sms, LaunchStream st);
 template <typename OffT>
 void launch_count_edges(u64 n, const void* vdesc, const u32* headp, int method, u64 cutoff, double hybrid_scale,
-                        u64* cnt, u64* partials, int grid, Control* ctl, TriangleSink sink, cudaStream_t st);
+                        u64* cnt, u64* partials, int grid, Control* ctl, TriangleSink sink, LaunchStream st);
 int count_grid_edges(int num_sms);
 
 // Oriented CSR export: compact copy of the out-lists (after sorting).

@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(PREP_BLOCK) k_prep(const u64* __restrict__ fo,
                                                      u32* __restrict__ dplus, u64* __restrict__ cnt,
                                                      u32* __restrict__ tile_i0, u32* __restrict__ hub_bins,
                                                      Control* ctl) {
+    chain_begin();
     __shared__ u32 s_bins[HUB ? HUB_BINS : 1];
     if constexpr (HUB) {
         for (u32 b = threadIdx.x; b < HUB_BINS; b += PREP_BLOCK) s_bins[b] = 0;
@@ -110,6 +111,7 @@ __global__ void __launch_bounds__(PREP_BLOCK) k_prep(const u64* __restrict__ fo,
 // overwrites deg).
 __global__ void k_hub_place(u64 n, const u32* __restrict__ deg, u32* __restrict__ hub_bins, uint2* __restrict__ hub_tmp,
                             const Control* ctl) {
+    chain_begin();
     if (ctl->hubs == 0 || (ctl->err & DEV_ERR_MASK)) return;
     const u32 low = ctl->hub_bin;
     const u64 stride = (u64)gridDim.x * blockDim.x;
@@ -126,6 +128,7 @@ __global__ void k_hub_place(u64 n, const u32* __restrict__ deg, u32* __restrict_
 // one gather gives a neighbour's place in the order and its hub index.
 __global__ void k_hub_rank(const u32* __restrict__ hub_bins, const uint2* __restrict__ hub_tmp, u32* __restrict__ hub_ids,
                            u32* __restrict__ key, const Control* ctl) {
+    chain_begin();
     const u32 p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= ctl->hubs || (ctl->err & DEV_ERR_MASK)) return;
     const uint2 me = hub_tmp[p];
@@ -346,6 +349,7 @@ __global__ void __launch_bounds__(BLOCK, 4) k_orient(const u64* __restrict__ fo,
                                                      const u32* __restrict__ tile_i0, u32* __restrict__ headp,
                                                      u16* __restrict__ hubp, u32* __restrict__ dplus,
                                                      u32* __restrict__ spanning, Control* ctl, u64 tile_begin) {
+    chain_begin();
     // at a piece's first slot: (window index + 1, key)
     __shared__ uint2 s_info_all[BLOCK / 32][32 * IPT];
     // at a piece's first slot: the tile ranks (at its first slot, past its last slot), then the
@@ -368,6 +372,7 @@ __global__ void k_desc(const u64* __restrict__ fo, u64 n, const u32* __restrict_
                        u16* __restrict__ hubp, u32* __restrict__ top_info, u32* __restrict__ top_long,
                        uint2* __restrict__ mtiles, uint2* __restrict__ ltiles, u32 small_d, u32 medium_d, u32 seg,
                        Control* ctl) {
+    chain_begin();
     if (ctl->err & DEV_ERR_MASK) return;
     const int lane = threadIdx.x & 31;
     const u64 warp_global = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -430,11 +435,13 @@ constexpr int TOPS_BLOCK = 256;
 __global__ void __launch_bounds__(TOPS_BLOCK) k_hub_tops(const Desc<u32>* __restrict__ vdesc, u16* __restrict__ hubp,
                                                          const u32* __restrict__ top_long, u32* __restrict__ top_info,
                                                          uint2* __restrict__ top_bits, u32 cap, Control* ctl) {
+    chain_begin();
     __shared__ __align__(8) u32 s_bits[TOPS_BLOCK / 32][HUB_TOP / 32];
     static_assert(HUB_TOP / 32 == 64, "two words per lane");
     if (ctl->err & DEV_ERR_MASK) return;
     const u32 lane = threadIdx.x & 31, lt = (1u << lane) - 1;
     u32* bits = s_bits[threadIdx.x >> 5];
+    if (blockIdx.x == 0 && threadIdx.x < 32) top_bits[threadIdx.x] = make_uint2(0, 0);  // the empty bitmap
     const u32 count = ctl->hub_long;
     const u32 nwarps = gridDim.x * (TOPS_BLOCK / 32);
     u32 dup = 0;
@@ -503,6 +510,7 @@ __device__ __forceinline__ u32 tile_key(const u64* fo, const u32* head, const u3
 __global__ void k_tile_cost(const u64* __restrict__ fo, const u32* __restrict__ head, const u32* __restrict__ dplus,
                             const uint2* __restrict__ tiles, const unsigned long long* count, u32 seg,
                             bool hub, u32* __restrict__ keys, Control* ctl) {
+    chain_begin();
     if (ctl->err & DEV_ERR_MASK) return;
     const u64 nt = *(volatile const unsigned long long*)count;
     const int lane = threadIdx.x & 31;
@@ -550,6 +558,7 @@ __global__ void __launch_bounds__(TILE_ORDER_BLOCK) k_tile_hist(const u64* __res
                                                                 const unsigned long long* count, u32 seg, u32 shift,
                                                                 u32 mode, bool hub, u32* __restrict__ keys, u32* hist,
                                                                 Control* ctl) {
+    chain_begin();
     __shared__ u32 s_cnt[TILE_BUCKETS];
     if (ctl->err & DEV_ERR_MASK) return;
     const u64 nt = *(volatile const unsigned long long*)count;
@@ -571,6 +580,7 @@ __global__ void __launch_bounds__(TILE_ORDER_BLOCK) k_tile_hist(const u64* __res
 // 256 threads: a block this small also fits beside the serving engine's resident blocks.
 constexpr int TILE_SCAN_BLOCK = 256;
 __global__ void __launch_bounds__(TILE_SCAN_BLOCK) k_tile_scan(u32* hist, Control* ctl) {
+    chain_begin();
     constexpr int PER = TILE_BUCKETS / TILE_SCAN_BLOCK;
     __shared__ u32 s_warp[TILE_SCAN_BLOCK / 32];
     if (ctl->err & DEV_ERR_MASK) return;
@@ -596,6 +606,7 @@ __global__ void __launch_bounds__(TILE_ORDER_BLOCK) k_tile_scatter(const uint2* 
                                                                    const unsigned long long* count,
                                                                    const u32* __restrict__ keys, u32* cursor,
                                                                    uint2* __restrict__ sorted, Control* ctl) {
+    chain_begin();
     __shared__ u32 s_pos[TILE_BUCKETS];
     if (ctl->err & DEV_ERR_MASK) return;
     const u64 nt = *(volatile const unsigned long long*)count;
@@ -620,48 +631,47 @@ u64 tile_order_scratch_words() { return TILE_BUCKETS; }
 
 void launch_order_tiles(const u64* fo, const u32* head, const u32* dplus, u64 n, const uint2* tiles,
                         const unsigned long long* count, u32 seg, u32 mode, bool hub, u32* keys, u32* hist,
-                        uint2* sorted, Control* ctl, int num_sms, cudaStream_t st) {
+                        uint2* sorted, Control* ctl, int num_sms, LaunchStream st) {
     if (n == 0) return;
     u32 bits = 0;
     while ((1ull << bits) < n) ++bits;
     const u32 shift = bits > 12 ? bits - 12 : 0;
     cudaMemsetAsync(hist, 0, sizeof(u32) * TILE_BUCKETS, st);
     if (mode == TILE_BY_COST)
-        k_tile_cost<<<num_sms * 8, 256, 0, st>>>(fo, head, dplus, tiles, count, seg, hub, keys, ctl);
-    k_tile_hist<<<num_sms * 4, TILE_ORDER_BLOCK, 0, st>>>(fo, head, dplus, tiles, count, seg, shift, mode, hub, keys,
+        launch_chained(k_tile_cost, num_sms * 8, 256, 0, st, fo, head, dplus, tiles, count, seg, hub, keys, ctl);
+    launch_chained(k_tile_hist, num_sms * 4, TILE_ORDER_BLOCK, 0, st, fo, head, dplus, tiles, count, seg, shift, mode, hub, keys,
                                                           hist, ctl);
-    k_tile_scan<<<1, TILE_SCAN_BLOCK, 0, st>>>(hist, ctl);
-    k_tile_scatter<<<num_sms * 4, TILE_ORDER_BLOCK, 0, st>>>(tiles, count, keys, hist, sorted, ctl);
+    launch_chained(k_tile_scan, 1, TILE_SCAN_BLOCK, 0, st, hist, ctl);
+    launch_chained(k_tile_scatter, num_sms * 4, TILE_ORDER_BLOCK, 0, st, tiles, count, keys, hist, sorted, ctl);
 }
 
 void launch_prep(const u64* fo, u64 n, u64 nnz, u32* deg, u32* dplus, u64* cnt, u32* tile_i0, const HubState& hub,
-                 Control* ctl, int num_sms, cudaStream_t st) {
+                 Control* ctl, int num_sms, LaunchStream st) {
     if (n == 0) return;
     const u64 blocks = (n + PREP_BLOCK - 1) / PREP_BLOCK;
     const u64 cap = (u64)num_sms * 8;
     const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
     if (!hub) {
-        k_prep<false><<<grid, PREP_BLOCK, 0, st>>>(fo, n, nnz, deg, dplus, cnt, tile_i0, nullptr, ctl);
+        launch_chained(k_prep<false>, grid, PREP_BLOCK, 0, st, fo, n, nnz, deg, dplus, cnt, tile_i0, nullptr, ctl);
         return;
     }
-    cudaMemsetAsync(hub.bins, 0, sizeof(u32) * HUB_BINS, st);
-    k_prep<true><<<grid, PREP_BLOCK, 0, st>>>(fo, n, nnz, deg, dplus, cnt, tile_i0, hub.bins, ctl);
-    k_hub_place<<<grid, 256, 0, st>>>(n, deg, hub.bins, hub.tmp, ctl);
-    k_hub_rank<<<HUB_H / 128, 128, 0, st>>>(hub.bins, hub.tmp, hub.ids, deg, ctl);
+    launch_chained(k_prep<true>, grid, PREP_BLOCK, 0, st, fo, n, nnz, deg, dplus, cnt, tile_i0, hub.bins, ctl);
+    launch_chained(k_hub_place, grid, 256, 0, st, n, deg, hub.bins, hub.tmp, ctl);
+    launch_chained(k_hub_rank, HUB_H / 128, 128, 0, st, hub.bins, hub.tmp, hub.ids, deg, ctl);
 }
 
-void launch_hub_tops(const void* vdesc, const HubState& hub, Control* ctl, int num_sms, cudaStream_t st) {
-    cudaMemsetAsync(hub.top_bits, 0, HUB_TOP / 8, st);  // the empty bitmap
-    k_hub_tops<<<num_sms * 8, TOPS_BLOCK, 0, st>>>(reinterpret_cast<const Desc<u32>*>(vdesc), hub.lists, hub.top_long,
+void launch_hub_tops(const void* vdesc, const HubState& hub, Control* ctl, int num_sms, LaunchStream st) {
+    launch_chained(k_hub_tops, num_sms * 8, TOPS_BLOCK, 0, st, reinterpret_cast<const Desc<u32>*>(vdesc), hub.lists, hub.top_long,
                                                    hub.top_info, hub.top_bits, hub.top_cap, ctl);
 }
 
 u64 hub_bins_words() { return 3ull * HUB_BINS; }
+size_t hub_bins_zeroed() { return sizeof(u32) * HUB_BINS; }
 
 u64 orient_tiles(u64 n, u64 nnz) { return (n + nnz + ORIENT_TILE - 1) / ORIENT_TILE; }
 
 void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* deg, const u32* tile_i0, u32* headp,
-                   const HubState& hub, u32* dplus, u32* spanning, Control* ctl, cudaStream_t st, u64 tile_begin,
+                   const HubState& hub, u32* dplus, u32* spanning, Control* ctl, LaunchStream st, u64 tile_begin,
                    u64 tile_end) {
     constexpr int BLOCK = ORIENT_BLOCK, IPT = ORIENT_IPT;
     const u64 tiles = orient_tiles(n, nnz);
@@ -669,26 +679,26 @@ void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* de
     if (tile_begin >= tile_end) return;
     const unsigned grid = (unsigned)(tile_end - tile_begin);
     if (hub)
-        k_orient<BLOCK, IPT, true><<<grid, BLOCK, 0, st>>>(fo, head, n, nnz, deg, tile_i0, headp, hub.lists, dplus,
+        launch_chained(k_orient<BLOCK, IPT, true>, grid, BLOCK, 0, st, fo, head, n, nnz, deg, tile_i0, headp, hub.lists, dplus,
                                                            spanning, ctl, tile_begin);
     else
-        k_orient<BLOCK, IPT, false><<<grid, BLOCK, 0, st>>>(fo, head, n, nnz, deg, tile_i0, headp, nullptr, dplus,
+        launch_chained(k_orient<BLOCK, IPT, false>, grid, BLOCK, 0, st, fo, head, n, nnz, deg, tile_i0, headp, nullptr, dplus,
                                                             spanning, ctl, tile_begin);
 }
 
 template <typename OffT, bool HUB>
 void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, const HubState& hub, uint2* mtiles, uint2* ltiles, u32 small_d,
-                 u32 medium_d, u32 seg, Control* ctl, int num_sms, cudaStream_t st) {
+                 u32 medium_d, u32 seg, Control* ctl, int num_sms, LaunchStream st) {
     if (n == 0) return;
     u64 blocks = (n + 255) / 256;
     u64 cap = (u64)num_sms * 8;
-    k_desc<OffT, HUB><<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(
+    launch_chained(k_desc<OffT, HUB>, (unsigned)(blocks < cap ? blocks : cap), 256, 0, st, 
         fo, n, dplus, reinterpret_cast<Desc<OffT>*>(vdesc), hub.lists, hub.top_info, hub.top_long, mtiles, ltiles, small_d, medium_d, seg, ctl);
 }
 
 #define KTRI_INST(OffT, HUB)                                                                                     \
     template void launch_desc<OffT, HUB>(const u64*, u64, const u32*, void*, const HubState&, uint2*, uint2*,    \
-                                         u32, u32, u32, Control*, int, cudaStream_t);
+                                         u32, u32, u32, Control*, int, LaunchStream);
 KTRI_INST(u32, false)
 KTRI_INST(u32, true)
 KTRI_INST(u64, false)

@@ -530,7 +530,7 @@ int finish_engine_batch(ktri_server* s, Slot& sl) {
     char* d = static_cast<char*>(sl.dev);
     ktri::launch_graph_totals(reinterpret_cast<const u64*>(d + sl.off_pv), reinterpret_cast<const u64*>(d + sl.off_vf),
                               sl.reqs.size(), sl.n_total, reinterpret_cast<u64*>(d + sl.off_tot), sl.ctl,
-                              ktri::ctx_num_sms(sl.ctx), sl.stream);
+                              ktri::ctx_num_sms(sl.ctx), ktri::LaunchStream(sl.stream, false));
     return enqueue_readback(s, sl);
 }
 
@@ -916,7 +916,7 @@ int ktri_server_create(int device, const ktri_server_opts* opts, ktri_server** o
     int rc = KTRI_OK;
     for (Slot& sl : s->slots) {
         rc = ktri_ctx_create(device, &sl.ctx);
-        if (rc == KTRI_OK) ktri::ctx_plain_lists(sl.ctx);  // the budget counts ktri_workspace_bytes per batch
+        if (rc == KTRI_OK) ktri::ctx_for_server(sl.ctx);  // the budget counts ktri_workspace_bytes per batch
         if (rc) break;
         cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking);
         cudaEventCreate(&sl.start);
