@@ -448,7 +448,7 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     if (!autom) {
         ktri::launch_sort_lists<OffT>(n, vdesc, headp, reinterpret_cast<u32*>(base + L.mid),
                                       reinterpret_cast<u32*>(base + L.big), reinterpret_cast<u32*>(base + L.scratch),
-                                      L.scratch_per_block, L.big_grid, ctl, sms, st);
+                                      L.scratch_per_block, L.big_grid, spanning, ctl, sms, st);
     }
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[1], st));
     if (opt.collect_stats)
@@ -471,7 +471,7 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     } else {
         const int grid = ktri::count_grid_edges(sms);
         ktri::launch_count_edges<OffT>(n, vdesc, headp, opt.method, opt.binary_cutoff, opt.hybrid_scale, cnt, partials,
-                                       grid, ctl, sink, st);
+                                       grid, reinterpret_cast<u32*>(base + L.mid), ctl, sink, st);
         ktri::launch_final(partials, (u32)grid, d_total, ctl, st);
     }
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[3], st));
@@ -1153,7 +1153,7 @@ int ktri_contract_dag_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32
     // sorted by id, as preprocessing_global does after compact (cetric.h:916-930)
     ktri::launch_sort_lists<u64>(n_local, base + x_desc, d_ohead, reinterpret_cast<u32*>(base + x_mid),
                                  reinterpret_cast<u32*>(base + x_big), reinterpret_cast<u32*>(base + x_scr), P, big_grid,
-                                 ctl, ctx->num_sms, st);
+                                 nullptr, ctl, ctx->num_sms, st);
     KTRI_CK(ctx, cudaGetLastError());
     u64 ke[2] = {0, 0};
     KTRI_CK(ctx, cudaMemcpyAsync(&ke[0], d_keep + n_local, 8, cudaMemcpyDeviceToHost, st));

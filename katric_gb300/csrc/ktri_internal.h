@@ -78,6 +78,7 @@ struct Control {
     unsigned long long medium_tiles;     // number of (owner, segment) tiles for medium owners
     unsigned long long medium_next;      // dynamic tile cursor of the medium-owner kernel
     unsigned long long stat_chunked;     // collect_stats: streamed entries times the owner's table chunks
+    unsigned long long edge_tails;       // tails left to the warp-per-edge kernel
     unsigned long long hub_next;         // dynamic tile cursor of the hub kernel
     uint32_t hubs;                       // number of hubs
     uint32_t hub_bin;                    // smallest degree bin of the hubs

@@ -237,13 +237,15 @@ void launch_stats(const u64* fo, const u32* head, u64 n, const void* vdesc, cons
                   u32 small_d, u32 medium_d, Control* ctl, int num_sms, LaunchStream st);
 
 // Sorted-list strategies (merge, binary search, binary, hybrid): sort out-lists by id, then
-// one warp per oriented edge.
+// intersect per oriented edge.  spanning: the lists the orientation put together from several
+// pieces (the only ones to sort where ctl says that the input is sorted), or null to look at all.
 template <typename OffT>
 void launch_sort_lists(u64 n, const void* vdesc, u32* headp, u32* mid_list, u32* big_list, u32* scratch,
-                       u64 scratch_per_block, int big_grid, Control* ctl, int num_sms, LaunchStream st);
+                       u64 scratch_per_block, int big_grid, const u32* spanning, Control* ctl, int num_sms, LaunchStream st);
 template <typename OffT>
 void launch_count_edges(u64 n, const void* vdesc, const u32* headp, int method, u64 cutoff, double hybrid_scale,
-                        u64* cnt, u64* partials, int grid, Control* ctl, TriangleSink sink, LaunchStream st);
+                        u64* cnt, u64* partials, int grid, u32* tails, Control* ctl, TriangleSink sink,
+                        LaunchStream st);  // tails: n entries of scratch
 int count_grid_edges(int num_sms);
 
 // Oriented CSR export: compact copy of the out-lists (after sorting).
