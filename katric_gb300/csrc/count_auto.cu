@@ -15,7 +15,7 @@
 //
 // The kernels (the bounds are runtime options, at most SMALL_D and MEDIUM_D):
 //   k_count_small: the edges between out-degrees of at most small_outdegree, groups of tails per
-//     warp, one streamed list per lane.  No block barrier.
+//     warp, one streamed list per pair of lanes.  No block barrier.
 //   k_count_medium: owners up to medium_outdegree, one warp per (owner, segment) tile with the
 //     warp's own table, so tiles need no block barrier.
 //   k_count_large: larger owners, one (owner, segment) tile per block iteration.  Short
@@ -146,16 +146,20 @@ __device__ __forceinline__ u32 bucket_probe16_flat(const u32* keys, u32* hits32,
 // QCAP keys together.  A key is both an entry of its tail's table and an edge whose head's list
 // is streamed through that table, so one pass over the keys builds the tables and the queue, and
 // neither the input adjacency nor the lower neighbours are read.  The queue is counting-sorted
-// by list length and streamed one list per lane, longest first.  Only __syncwarp orders the
+// by list length and streamed longest first, a list per pair of lanes.  Only __syncwarp orders the
 // phases: the warps of a block never wait for one another.
 //
-// What bounds it: instruction issue and shared-memory wavefronts of the lookups.  A lookup reads
-// one bucket of two keys (8 bytes) and never walks: a table of 3 d buckets for d keys is rebuilt
-// with another multiplier until no bucket holds more than two (about 0.013 d overfull buckets
-// expected, so most tables of d <= 32 succeed at once), and a table that never does is searched
-// entry by entry.  Against one table per owner in buckets of four with early exits, streamed over
-// the whole adjacency (the form before), 1.0x to 1.05x the entries are streamed on uniform and
-// geometric graphs (the head's list instead of the shorter one) at a quarter of the instructions.
+// What bounds it: the shared-memory pipe (89 % busy on RGG n = 2^20, where half of the lookups hit;
+// issue 68 %).  A lookup reads one bucket of two keys (8 bytes, about six wavefronts per 32 random
+// buckets) and never walks: a table of 3 d buckets for d keys is rebuilt with another multiplier
+// until no bucket holds more than two (about 0.013 d overfull buckets expected, so most tables of
+// d <= 32 succeed at once), and a table that never does is searched entry by entry.
+// Measured (this kernel, RGG 2^20 / RGG-24 / G(n,m) n = 10^6 of degree 60): one table per owner in
+// buckets of four with early exits, streamed over the whole adjacency 0.915 / 13.2 ms / -; tails
+// with a list per lane 0.514 / 7.55 / 3.22 ms; with keys placed by stores instead of
+// compare-and-swap, the queue sorted by ballots and a list per pair of lanes 0.508 / 7.43 / 2.21 ms.
+// The head's list is streamed instead of the shorter one: 1.0x to 1.05x the entries on uniform and
+// geometric graphs.
 template <typename OffT, bool HUB>
 struct SmallWarpLayout {
     static constexpr int GROUP = 16;             // tails per group
@@ -192,16 +196,18 @@ __device__ __forceinline__ void small_init(u32* base) {
 }
 
 // One batch: the tails among the vertices [bi * vb, (bi + 1) * vb), vb <= 32, counted by one warp in
-// its slice of shared memory.  HUB: lists are split, and hub i is the key n + i of a table.
+// its slice of shared memory.  distinct: no list holds an entry twice (the input lists ascend), so
+// the tables need no compare-and-swap to find duplicates.  HUB: lists are split, and hub i is the
+// key n + i of a table.
 template <typename OffT, bool HUB, bool CG = false>
 __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, const Desc<OffT>* __restrict__ vdesc,
                                             const u32* __restrict__ headp, const u16* __restrict__ hubp,
-                                            const u32* __restrict__ hub_ids, u32 sd, u64* __restrict__ cnt,
-                                            u64& local_total, u32& dup) {
+                                            const u32* __restrict__ hub_ids, u32 sd, bool distinct,
+                                            u64* __restrict__ cnt, u64& local_total, u32& dup) {
     using L = SmallWarpLayout<OffT, HUB>;
     constexpr u32 FULL = 0xFFFFFFFFu;
     static_assert(SMALL_D < 64 && SMALL_D <= L::QCAP && L::GROUP <= 16, "field widths of the queue entries");
-    static_assert(2 * L::NB <= (int)NO_SLOT && (SMALL_D + 3) / 4 < 32, "slots and length bins");
+    static_assert(2 * L::NB <= (int)NO_SLOT && (SMALL_D + 3) / 4 + 1 < 16, "slots and length bins");
     const u32 lane = threadIdx.x & 31;
     const u32 lt_mask = (1u << lane) - 1, le_mask = lt_mask | (1u << lane);
     u32* keys = base + L::W_KEYS;
@@ -287,6 +293,34 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
             for (int r = 0; r < L::ROWS; ++r) need |= (w[r] != EMPTY_KEY ? 1u : 0u) << r;
             for (int attempt = 0;; ++attempt) {
                 u32 failed = 0;
+                if (distinct) {
+                    // all keys are written to their bucket's first slot and read back; who lost tries the
+                    // second slot the same way (a third of a compare-and-swap's wavefronts)
+                    u32 lost = 0;
+#pragma unroll
+                    for (int r = 0; r < L::ROWS; ++r) {
+                        if (!((need >> r) & 1u)) continue;
+                        const uint4 t = rec[gi[r]];
+                        slot[r] = 2 * (3 * t.x + __umulhi(w[r] * t.z, 3 * t.y));
+                        keys[slot[r]] = w[r];
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int r = 0; r < L::ROWS; ++r)
+                        if (((need >> r) & 1u) && keys[slot[r]] != w[r]) lost |= 1u << r;
+                    __syncwarp();
+#pragma unroll
+                    for (int r = 0; r < L::ROWS; ++r)
+                        if ((lost >> r) & 1u) keys[++slot[r]] = w[r];
+                    __syncwarp();
+#pragma unroll
+                    for (int r = 0; r < L::ROWS; ++r)
+                        if (((lost >> r) & 1u) && keys[slot[r]] != w[r]) {
+                            slot[r] = NO_SLOT;
+                            failed |= 1u << gi[r];
+                        }
+                    need = 0;
+                }
 #pragma unroll
                 for (int r = 0; r < L::ROWS; ++r) {
                     if (!((need >> r) & 1u)) continue;
@@ -331,7 +365,24 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
             q_s[q] = (OffT)list_group(dw[r]);
             if constexpr (HUB) q_h[q] = (u32)(hub_start(list_start(dw[r]), vertex_of(w[r])) >> 3);
             q_m[q] = (slot[r] << 16) | (gi[r] << 12) | (dh << 6) | dr;
-            atomicAdd(&bins[(dr + 3) / 4 + (dh + 7) / 8], 1u);
+        }
+        // counting sort by length in 16-byte groups: lanes of a row with the same length are found by
+        // ballots, and their first lane adds for all of them
+        u32 same[L::ROWS], len[L::ROWS];
+#pragma unroll
+        for (int r = 0; r < L::ROWS; ++r) {
+            const u32 d = list_len<HUB>(dw[r].d);
+            const bool sel = d != 0 && d <= sd;
+            len[r] = sel ? (rest_len<HUB>(dw[r].d) + 3) / 4 + (hub_len<HUB>(dw[r].d) + 7) / 8 : 0u;
+            same[r] = 0;
+            if (32u * r >= K) continue;
+            same[r] = __ballot_sync(FULL, sel);
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const u32 set = __ballot_sync(FULL, (len[r] >> b) & 1u);
+                same[r] &= (len[r] >> b) & 1u ? set : ~set;
+            }
+            if (sel && !(same[r] & lt_mask)) atomicAdd(&bins[len[r]], (u32)__popc(same[r]));
         }
         __syncwarp();
         u32 qn;
@@ -350,19 +401,26 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
         __syncwarp();
 #pragma unroll
         for (int r = 0; r < L::ROWS; ++r) {
-            const u32 d = list_len<HUB>(dw[r].d), dr = rest_len<HUB>(dw[r].d), dh = hub_len<HUB>(dw[r].d);
-            if (d != 0 && d <= sd)
-                q_ord[atomicAdd(&bins[(dr + 3) / 4 + (dh + 7) / 8], 1u)] = (unsigned short)(32 * r + lane);
+            if (32u * r >= K) continue;
+            const u32 first = same[r] & lt_mask;
+            u32 at = 0;
+            if (len[r] && !first) at = atomicAdd(&bins[len[r]], (u32)__popc(same[r]));
+            at = __shfl_sync(FULL, at, __ffs(same[r] | (1u << lane)) - 1);
+            if (len[r]) q_ord[at + __popc(first)] = (unsigned short)(32 * r + lane);
         }
         __syncwarp();
-        // stream the queued lists, one per lane, longest first; the next 16-byte group of a list is
-        // in flight while the current one is looked up (groups are padded, so the load stays inside
-        // the list's slots)
-        for (u32 i = lane; i < qn; i += 32) {
-            const u32 q = q_ord[i];
-            const u32 m = q_m[q];
+        // stream the queued lists, longest first, one per pair of lanes that take turns at its 16-byte
+        // groups (a pair's reads share a 32-byte sector: half the wavefronts of one list per lane); the
+        // next group is in flight while the current one is looked up (groups are padded, so the load
+        // stays inside the list's slots)
+        const u32 half = lane & 1u;
+        for (u32 i0 = 0; i0 < qn; i0 += 16) {
+            const u32 i = i0 + (lane >> 1);
+            const bool have = i < qn;
+            const u32 q = have ? q_ord[i] : 0u;
+            const u32 m = have ? q_m[q] : 0u;
             const u32 g = (m >> 12) & 15u;
-            const uint4* lp = headp4 + (u64)q_s[q];
+            const uint4* lp = headp4 + (have ? (u64)q_s[q] : 0ull);
             const uint4 t = rec[g];
             int rem = (int)(m & 63u), hrem = HUB ? (int)((m >> 6) & 63u) : 0;
             u32 found = 0;
@@ -371,7 +429,7 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
                 auto own_key = [&](u32 k) {
                     return !HUB || k < t.w ? ld_in<CG>(headp + own + k) : n32 + ld_in<CG>(hubp + hown + (k - t.w));
                 };
-                for (int e = 0; e < rem + hrem; ++e) {
+                for (int e = (int)half; e < rem + hrem; e += 2) {
                     const u32 z = e < rem ? ld_in<CG>(reinterpret_cast<const u32*>(lp) + e)
                                           : n32 + ld_in<CG>(reinterpret_cast<const u16*>(hubp8 + q_h[q]) + (e - rem));
                     for (u32 k = 0; k < t.y; ++k)
@@ -381,6 +439,8 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
                         }
                 }
                 if (found) atomicAdd(&cnt[vertex_of(own_key(q - t.x))], (u64)found);
+                if (found) atomicAdd(&tot[g], found);
+                found = 0;
             } else {
                 const u32 nb = 3 * t.y, mult = t.z;
                 const uint2* tk = reinterpret_cast<const uint2*>(keys) + 3 * t.x;
@@ -403,21 +463,23 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
                         }
                     }
                 };
-                if (!HUB || rem > 0) {
+                rem -= 4 * (int)half;
+                if (rem > 0) {
+                    lp += half;
                     uint4 cur = ld_in<CG>(lp);
                     while (true) {
                         uint4 nxt = cur;
-                        if (rem > 4) nxt = ld_in<CG>(++lp);
+                        if (rem > 8) nxt = ld_in<CG>(lp += 2);
                         look4(cur.x, cur.y, cur.z, cur.w, rem);
-                        rem -= 4;
+                        rem -= 8;
                         if (rem <= 0) break;
                         cur = nxt;
                     }
                 }
                 if constexpr (HUB) {
-                    const uint4* hp = hubp8 + q_h[q];
-                    for (; hrem > 0; hrem -= 8) {
-                        const uint4 cur = ld_in<CG>(hp++);
+                    const uint4* hp = hubp8 + (have ? q_h[q] : 0u) + half;
+                    for (hrem -= 8 * (int)half; hrem > 0; hrem -= 16, hp += 2) {
+                        const uint4 cur = ld_in<CG>(hp);
                         look4(n32 + (cur.x & 0xFFFFu), n32 + (cur.x >> 16), n32 + (cur.y & 0xFFFFu), n32 + (cur.y >> 16),
                               hrem);
                         if (hrem > 4)
@@ -425,12 +487,14 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
                                   n32 + (cur.w >> 16), hrem - 4);
                     }
                 }
-                if (found) {
-                    const u32 s = m >> 16;
-                    atomicAdd(&hits[s >> 1], found << ((s & 1u) << 4));  // the edge's head
-                }
             }
-            if (found) atomicAdd(&tot[g], found);
+            __syncwarp();
+            found += __shfl_xor_sync(FULL, found, 1);
+            if (found && !half) {
+                const u32 s = m >> 16;
+                atomicAdd(&hits[s >> 1], found << ((s & 1u) << 4));  // the edge's head
+                atomicAdd(&tot[g], found);
+            }
         }
         __syncwarp();
         // flush and clear: every key's hits (as the third corner and as the head of its edge), then
@@ -469,6 +533,7 @@ __global__ void __launch_bounds__(BLOCK, 4) k_count_small(u64 n, u32 vb, const D
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     u32* base = reinterpret_cast<u32*>(smem) + warp * L::PER_WARP;
     small_init<OffT, HUB>(base);
+    const bool distinct = !(ctl->err & DEV_FLAG_UNSORTED);
     const bool split = HUB && ctl->hubs != 0;  // without hubs the plain body reads the same lists
     const u64 nbatch = (n + vb - 1) / vb;
     u64 local_total = 0;
@@ -479,9 +544,10 @@ __global__ void __launch_bounds__(BLOCK, 4) k_count_small(u64 n, u32 vb, const D
         bi = __shfl_sync(0xFFFFFFFFu, bi, 0);
         if (bi >= nbatch) break;
         if (split)
-            small_batch<OffT, HUB>(base, bi, vb, n, vdesc, headp, hubp, hub_ids, sd, cnt, local_total, dup);
+            small_batch<OffT, HUB>(base, bi, vb, n, vdesc, headp, hubp, hub_ids, sd, distinct, cnt, local_total, dup);
         else
-            small_batch<OffT, false>(base, bi, vb, n, vdesc, headp, nullptr, nullptr, sd, cnt, local_total, dup);
+            small_batch<OffT, false>(base, bi, vb, n, vdesc, headp, nullptr, nullptr, sd, distinct, cnt, local_total,
+                                     dup);
     }
     if (dup) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
     const u64 bt = block_sum_u64<BLOCK>(local_total, s_red);
@@ -1585,12 +1651,13 @@ __global__ void __launch_bounds__(ENGINE_BLOCK, 4) k_engine(EngineJob* jobs, u32
         if (u < jb->units_small) {
             const u64 nb = (jb->n + 31) / 32;
             u32* slice = reinterpret_cast<u32*>(smem) + warp * EngineSmallL::PER_WARP;
+            const bool distinct = !(*(volatile u32*)&ctl->err & DEV_FLAG_UNSORTED);
             small_init<u32, false>(slice);  // other kinds of unit use the same shared memory
             for (u32 r = 0; r < ENGINE_REPS; ++r) {
                 const u64 bi = (u * (ENGINE_BLOCK / 32) + warp) * ENGINE_REPS + r;
                 if (bi < nb)
                     small_batch<u32, false, true>(slice, bi, 32, jb->n, vd, jb->headp, nullptr, nullptr, jb->small_d,
-                                                  jb->cnt, unused_total, dup);
+                                                  distinct, jb->cnt, unused_total, dup);
             }
         } else if (u < jb->units_small + jb->units_medium) {
             const u64 nt = *(volatile unsigned long long*)&ctl->medium_tiles;
