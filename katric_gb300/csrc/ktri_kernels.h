@@ -24,6 +24,7 @@ struct LaunchStream {
 };
 
 constexpr int ORIENT_BLOCK = 256;   // 8 warps, one merge-path tile each
+constexpr int ORIENT_BLOCKS = 4;   // blocks per SM
 constexpr int ORIENT_IPT = 8;       // slots per lane of a tile: tiles of 256 diagonals
 constexpr int SMALL_BLOCK = 256;
 constexpr int SMALL_D = 48;          // largest (and default) out-degree bound of the small kernel's edges

@@ -145,17 +145,18 @@ __global__ void k_hub_rank(const u32* __restrict__ hub_bins, const uint2* __rest
 
 // Orientation of one merge-path tile of W = 32 * IPT diagonals per warp.  The tile holds the
 // window vertices i0..i1 and the adjacency slots [j0, j1); every list with slots in the tile
-// has one piece there.  Slots are taken 32 at a time, one per lane, so the owner of a slot,
-// the rank of a kept entry among the tile's kept entries and the rank at a piece's ends all
-// come from warp ballots and population counts: no block barrier, no per-thread path walk.
+// has one piece there, numbered in slot order.  Slots are taken 32 at a time, one per lane: the
+// gathers, and the writes of what is kept, then touch the fewest lines.  All per-list work is done
+// once per piece by the window's lanes, and a slot finds its piece by one population count over
+// the bits of the pieces' first slots.
 // Inside the tile all arithmetic is 32-bit (ids are below 2^32, slots relative to j0).
-//   vertex pass  at the slot where each piece starts: (window index + 1, degree of its vertex)
-//   pass 1       per slot: owner (the last piece start at or below the lane), deg[y] gather,
-//                the (deg, id) decision, input checks; the tile rank at each piece's first
-//                and past its last slot
-//   piece pass   per window vertex, lanes in parallel: the piece's out-degree share (a plain
-//                store, or an atomic reservation for a piece of a split list) and the
-//                gapped-array index of its first kept entry
+//   vertex pass  per window vertex with slots here: its piece's first slot as a bit of s_start, the
+//                slot before it as a bit of s_stop, (key, id) of its vertex in s_piece
+//   pass 1       per slot: its piece, the (key, id) decision, input checks; per row of 32 the kept
+//                slots' mask and the kept slots before the row
+//   piece pass   per window vertex: the tile ranks at the piece's ends (from the rows' masks), its
+//                out-degree share (a plain store, or an atomic reservation for a piece of a split
+//                list) and the gapped-array index of tile rank 0 for its entries
 //   pass 2       kept entries written from registers, in slot order
 // A list held by one tile keeps its input order.  A split list's pieces reserve their ranges
 // with one atomic each and are recorded in the spanning list by the tile that holds the list's
@@ -163,136 +164,146 @@ __global__ void k_hub_rank(const u32* __restrict__ hub_bins, const uint2* __rest
 // HUB: deg holds orientation keys (the degree, or a hub's key above every degree), a kept entry that
 // is a hub goes to the hub array as its index and the others to headp, so a piece has two ranks
 // and two shares of its out-list's length word (hubs << 16 | others, as everywhere with hubs).
-template <int BLOCK, int IPT, bool HUB>
-__device__ __forceinline__ void orient_tile(uint2 (*s_info_all)[32 * IPT], u64 (*s_base_all)[32 * IPT],
-                                            const u64* __restrict__ fo, const u32* __restrict__ head, u64 n, u64 nnz,
+// What bounds it: latency (a tile's offset, its slots, their keys, one after the other: half of the
+// issue slots are taken with 32 warps per SM, 64 registers) and instruction issue.  Measured (kernel
+// under ncu, RGG n = 2^20 of 33 M slots): 187 us with 112 instructions per row of 32 slots, against
+// 229 us with 172 when every slot carried its piece's ends and rank; the orientation phase of
+// RGG-24 3.7 -> 3.2 ms, of RMAT n = 10^6 0.42 -> 0.32 ms.  Five or six blocks per SM spill: 3.4 and
+// 3.6 ms.
+template <int IPT>
+struct OrientWarp {
+    static constexpr int W = 32 * IPT;
+    union {
+        uint2 piece[W];  // until the piece pass: key and id of the piece's vertex
+        // then: the headp index of tile rank 0 for its entries (HUB: the indices in both arrays
+        // relative to where the tile's first vertex would start, 32 bits each)
+        u64 base[W];
+    };
+    uint4 row[IPT + 1];  // kept slots (others, hubs) of the row and the tile rank before it
+    u32 start[IPT];      // a piece starts at this slot
+    u32 stop[IPT];       // the next slot is another piece's or past the tile
+};
+
+template <int IPT, bool HUB>
+__device__ __forceinline__ void orient_tile(OrientWarp<IPT>& sw, const u64* __restrict__ fo,
+                                            const u32* __restrict__ head, u64 n, u64 nnz,
                                             const u32* __restrict__ deg, const u32* __restrict__ tile_i0,
                                             u32* __restrict__ headp, u16* __restrict__ hubp, u32* __restrict__ dplus,
-                                            u32* __restrict__ spanning, Control* ctl, u64 tile_begin) {
+                                            u32* __restrict__ spanning, Control* ctl, u64 tile) {
     constexpr int W = 32 * IPT;
-    constexpr int WARPS = BLOCK / 32;
     constexpr u32 FULL = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    static_assert(W <= 256 && IPT % 4 == 0, "piece numbers in bytes");
+    const u32 lane = threadIdx.x & 31;
     const u64 total = n + nnz;
-    const u64 tile = (tile_begin + blockIdx.x) * WARPS + wid;
     const u64 d0 = tile * W;
     if (d0 >= total) return;
     const u64 d1 = d0 + W < total ? d0 + W : total;
-    uint2* s_info = s_info_all[wid];
-    u64* s_base = s_base_all[wid];
-    uint2* s_rank = reinterpret_cast<uint2*>(s_base);
     // tile_i0 holds base_tiles + 1 entries (the last is n), and tile + 1 <= base_tiles here
     const u64 i0 = tile_i0[tile], i1 = tile_i0[tile + 1];
     const u64 j0 = d0 - i0, j1 = d1 - i1;
     const u32 ns = (u32)(j1 - j0);
     if (ns == 0) return;  // only vertex ends: those lists have no slots here (out-degrees start at 0)
     const u32 n32 = (u32)n;  // n < 2^32: every id fits
-    // every slot's neighbour and its degree, all in flight before the window is read
+    // every slot's neighbour and its key, all in flight before the window is read
     u32 y_r[IPT], dy_r[IPT];
+    const u32* hl = head + j0 + lane;
+#pragma unroll
+    for (int it = 0; it < IPT; ++it) y_r[it] = (u32)it * 32 + lane < ns ? __ldcs(hl + it * 32) : 0u;
+    u32 y_max = 0;
 #pragma unroll
     for (int it = 0; it < IPT; ++it) {
-        const u32 s = (u32)it * 32 + lane;
-        y_r[it] = s < ns ? __ldcs(head + j0 + s) : 0u;
+        y_max = y_r[it] > y_max ? y_r[it] : y_max;
+        // 0 past the tile and for an id out of range: below every owner's key, so never kept
+        dy_r[it] = ((u32)it * 32 + lane < ns && y_r[it] < n32) ? __ldg(deg + y_r[it]) : 0u;
     }
-#pragma unroll
-    for (int it = 0; it < IPT; ++it) {
-        const u32 s = (u32)it * 32 + lane;
-        dy_r[it] = (s < ns && y_r[it] < n32) ? __ldg(deg + y_r[it]) : 0u;
+    if (lane < IPT) {
+        sw.start[lane] = 0;
+        const u32 used = ns - 1;  // slots with a next one in the tile
+        sw.stop[lane] = used >= (lane + 1) * 32 ? 0u : used <= lane * 32 ? FULL : FULL << (used - lane * 32);
     }
-    for (u32 s = lane; s < ns; s += 32) s_info[s] = make_uint2(0u, 0u);
     __syncwarp();
     const u64 last_v = i1 < n ? i1 : n - 1;
     const u32 nwin = (u32)(last_v - i0) + 1;  // window vertices (at most W + 1)
+    const u32 lt = (1u << lane) - 1u, le = lt | (1u << lane);
+    u32 end_y = 0, end_nx = 1;  // the neighbours on both sides of the tile's end, when one list has both
+    // the window vertex' piece starts at slot s0 and has the number q
+    auto enter = [&](u64 v, u32 s0, u32 q, u32 key, u64 b) {
+        if (b > j1) {
+            end_y = head[j1 - 1];
+            end_nx = head[j1];
+        }
+        atomicOr(&sw.start[s0 >> 5], 1u << (s0 & 31u));
+        if (s0) atomicOr(&sw.stop[(s0 - 1) >> 5], 1u << ((s0 - 1) & 31u));
+        sw.piece[q] = make_uint2(key, (u32)v);
+    };
     // the first 32 window vertices with every lane present (lane 0's list may begin before the
     // tile); their bounds stay in registers for the piece pass
-    const bool have0 = (u32)lane < nwin;
+    const bool have0 = lane < nwin;
     const u64 a0 = have0 ? fo[i0 + lane] : 0, b0 = have0 ? fo[i0 + lane + 1] : 0;
-    if (have0 && b0 > a0 && a0 < j1 && b0 > j0)
-        s_info[a0 > j0 ? a0 - j0 : 0] = make_uint2((u32)lane + 1, HUB ? __ldg(deg + i0 + lane) : (u32)(b0 - a0));
-    for (u32 k = 32 + lane; k < nwin; k += 32) {
-        const u64 v = i0 + k;
-        const u64 a = fo[v], b = fo[v + 1];
-        if (b > a && a < j1 && b > j0) s_info[a - j0] = make_uint2(k + 1, HUB ? __ldg(deg + v) : (u32)(b - a));
+    const bool in0 = have0 && b0 > a0 && a0 < j1 && b0 > j0;
+    const u32 ball0 = __ballot_sync(FULL, in0);
+    if (in0) enter(i0 + lane, a0 > j0 ? (u32)(a0 - j0) : 0u, __popc(ball0 & lt), HUB ? __ldg(deg + i0 + lane) : (u32)(b0 - a0), b0);
+    for (u32 k0 = 32, q0 = __popc(ball0); k0 < nwin; k0 += 32) {
+        const u64 v = i0 + k0 + lane;
+        const bool have = k0 + lane < nwin;
+        const u64 a = have ? fo[v] : 0, b = have ? fo[v + 1] : 0;
+        const bool in = b > a && a < j1 && b > j0;
+        const u32 ball = __ballot_sync(FULL, in);
+        if (in) enter(v, (u32)(a - j0), q0 + __popc(ball & lt), HUB ? __ldg(deg + v) : (u32)(b - a), b);
+        q0 += __popc(ball);
     }
     __syncwarp();
-    // the tile's last list continues past the tile
-    const bool last_past = fo[last_v] < j1 && fo[last_v + 1] > j1;
-    const u32 lt = (1u << lane) - 1u, le = lt | (1u << lane);
-    const u32 i0_32 = (u32)i0;
-
-    u32 s0_r[IPT], km_r[IPT], hm_r[HUB ? IPT : 1];
-    u32 rank = 0;                // kept entries of the tile before this iteration (HUB: hubs << 16 | others)
-    u32 s0c = 0, kc = 0, dc = 0;  // the piece open at the end of the previous iteration
-    bool bad_id = false, self_loop = false, dup = false, unsorted = false;
+    bool dup = false, unsorted = false, self_loop = false;
+    u32 q_r[IPT / 4];        // the slots' pieces, a byte each
+    u32 rank = 0;            // kept entries of the tile before this row (HUB: hubs << 16 | others)
+    u32 q_row = 0u - 1u;     // the last piece that starts before this row
 #pragma unroll
     for (int it = 0; it < IPT; ++it) {
-        s0_r[it] = 0;
-        km_r[it] = 0;
-        if constexpr (HUB) hm_r[it] = 0;
+        if (it % 4 == 0) q_r[it / 4] = 0;
         if ((u32)it * 32 >= ns) continue;
-        const u32 s = (u32)it * 32 + lane;
-        const bool valid = s < ns;
-        const uint2 info = valid ? s_info[s] : make_uint2(0u, 0u);
-        const u32 starts = __ballot_sync(FULL, info.x != 0);
-        const u32 below = starts & le;
-        const int src = 31 - __clz(below);  // -1 when no piece starts at or below this lane
-        const u32 kx = __shfl_sync(FULL, info.x, src & 31);
-        const u32 dxs = __shfl_sync(FULL, info.y, src & 31);
-        const bool here = below != 0;
-        const u32 s0 = here ? (u32)it * 32 + (u32)src : s0c;
-        const u32 k1 = here ? kx : kc;
-        const u32 dx = here ? dxs : dc;
-        const u32 y = y_r[it];
-        const u32 x = i0_32 + k1 - 1;
-        const bool in_range = y < n32;
-        bad_id |= valid && !in_range;
-        self_loop |= valid && in_range && y == x;
-        const u32 dy = dy_r[it];
-        const bool kept = valid && in_range && y != x && (dx < dy || (dx == dy && x < y));
+        const u32 starts = sw.start[it], stop = sw.stop[it];
+        const u32 q = q_row + __popc(starts & le);
+        q_row += __popc(starts);
+        q_r[it / 4] |= q << (8 * (it % 4));
+        const uint2 px = sw.piece[q];
+        const u32 y = y_r[it], dy = dy_r[it];
+        const bool tie = dy == px.x;
+        const bool kept = dy > px.x || (tie && y > px.y);
+        self_loop |= tie && y == px.y;  // a slot past the tile has the key 0: no tie
         u32 km = __ballot_sync(FULL, kept), hm = 0;
         if constexpr (HUB) {
             hm = __ballot_sync(FULL, kept && dy >= HUB_FLAG);
             km &= ~hm;
         }
-        const bool last_slot = s + 1 == ns;
-        bool next_start;
-        if (lane < 31) next_start = (starts >> (lane + 1)) & 1u;
-        else next_start = valid && !last_slot && s_info[s + 1].x != 0;
-        // tile ranks at the piece's first slot and past its last slot
-        if (valid && info.x != 0) s_rank[s].x = rank + __popc(km & lt) + (HUB ? __popc(hm & lt) << 16 : 0u);
-        if (valid && (last_slot || next_start))
-            s_rank[s0].y = rank + __popc(km & le) + (HUB ? __popc(hm & le) << 16 : 0u);
-        // the next slot's neighbour (the next lane's, or lane 0's of the next iteration) when it
-        // belongs to the same list: adjacent duplicates and order
-        const u32 nd = __shfl_down_sync(FULL, y, 1);
-        const u32 nn = __shfl_sync(FULL, y_r[it + 1 < IPT ? it + 1 : it], 0);
-        const bool same = valid && (last_slot ? last_past : !next_start);
-        if (same) {
-            const u32 nx = last_slot ? __ldcs(head + j1) : (lane < 31 ? nd : nn);
+        // the next slot's neighbour (the next lane's, or lane 0's of the next row) when it belongs
+        // to the same list: adjacent duplicates and order
+        const u32 nx = __shfl_sync(FULL, (lane == 0 && it + 1 < IPT) ? y_r[it + 1 < IPT ? it + 1 : it] : y, lane + 1);
+        if (!(stop & (le ^ lt))) {
             unsorted |= nx < y;
             dup |= nx == y;
         }
-        s0c = __shfl_sync(FULL, s0, 31);
-        kc = __shfl_sync(FULL, k1, 31);
-        dc = __shfl_sync(FULL, dx, 31);
+        if (lane == 0) sw.row[it] = make_uint4(km, hm, rank, 0);
         rank += __popc(km) + (HUB ? __popc(hm) << 16 : 0u);
-        s0_r[it] = s0;
-        km_r[it] = km;
-        if constexpr (HUB) hm_r[it] = hm;
     }
-    const u32 err = (bad_id ? DEV_ERR_ID_RANGE : 0u) | (self_loop ? DEV_ERR_SELF_LOOP : 0u) |
-                    (dup ? DEV_ERR_DUPLICATE : 0u);
+    // the row after the last slot: where a piece that fills the tile ends
+    if (lane == 0 && (ns & 31u) == 0) sw.row[ns >> 5] = make_uint4(0, 0, rank, 0);
+    dup |= end_nx == end_y;
+    unsorted |= end_nx < end_y;
+    const u32 err = (y_max >= n32 ? DEV_ERR_ID_RANGE : 0u) | (self_loop ? DEV_ERR_SELF_LOOP : 0u) |
+                    (dup ? DEV_ERR_DUPLICATE : 0u) | (unsorted ? DEV_FLAG_UNSORTED : 0u);
     if (err) atomicOr(&ctl->err, err);
-    if (unsorted) atomicOr(&ctl->err, DEV_FLAG_UNSORTED);
     __syncwarp();
     // piece pass: out-degree shares and where each piece's kept entries go
     const u64 ref = oriented_start(j0, i0), href = hub_start(ref, i0);  // HUB: origins of the 32-bit indices
     {
-        auto settle = [&](u64 v, u64 a, u64 b) {
-            if (!(b > a && a < j1 && b > j0)) return;
-            const u32 s0 = a > j0 ? (u32)(a - j0) : 0u;
-            const uint2 rk = s_rank[s0];
-            const u32 cnt = rk.y - rk.x;
+        auto rank_at = [&](u32 s) {
+            const uint4 r = sw.row[s >> 5];
+            const u32 m = (1u << (s & 31u)) - 1u;
+            return r.z + __popc(r.x & m) + (HUB ? __popc(r.y & m) << 16 : 0u);
+        };
+        auto settle = [&](u64 v, u64 a, u64 b, u32 q) {
+            const u32 first = rank_at(a > j0 ? (u32)(a - j0) : 0u);
+            const u32 cnt = rank_at(b < j1 ? (u32)(b - j0) : ns) - first;
             u32 carry = 0;
             if (a < j0 || b > j1) {
                 if (cnt) carry = atomicAdd(&dplus[v], cnt);
@@ -303,40 +314,43 @@ __device__ __forceinline__ void orient_tile(uint2 (*s_info_all)[32 * IPT], u64 (
             const u64 start = oriented_start(a, v);
             if constexpr (HUB) {
                 // differences stay below 2^31: a list begins at most its degree before the tile
-                const u32 to = (u32)(start - ref) + (carry & 0xFFFFu) - (rk.x & 0xFFFFu);
-                const u32 hto = (u32)(hub_start(start, v) - href) + (carry >> 16) - (rk.x >> 16);
-                s_base[s0] = (u64)to | ((u64)hto << 32);
+                const u32 to = (u32)(start - ref) + (carry & 0xFFFFu) - (first & 0xFFFFu);
+                const u32 hto = (u32)(hub_start(start, v) - href) + (carry >> 16) - (first >> 16);
+                sw.base[q] = (u64)to | ((u64)hto << 32);
             } else {
-                s_base[s0] = start + carry - rk.x;
+                sw.base[q] = start + carry - first;
             }
         };
-        if (have0) settle(i0 + lane, a0, b0);
-        for (u32 k = 32 + lane; k < nwin; k += 32) {
-            const u64 v = i0 + k;
-            settle(v, fo[v], fo[v + 1]);
+        if (in0) settle(i0 + lane, a0, b0, __popc(ball0 & lt));
+        for (u32 k0 = 32, q0 = __popc(ball0); k0 < nwin; k0 += 32) {
+            const u64 v = i0 + k0 + lane;
+            const bool have = k0 + lane < nwin;
+            const u64 a = have ? fo[v] : 0, b = have ? fo[v + 1] : 0;
+            const bool in = b > a && a < j1 && b > j0;
+            const u32 ball = __ballot_sync(FULL, in);
+            if (in) settle(v, a, b, q0 + __popc(ball & lt));
+            q0 += __popc(ball);
         }
     }
     __syncwarp();
-    rank = 0;
 #pragma unroll
     for (int it = 0; it < IPT; ++it) {
-        const u32 km = km_r[it];
+        if ((u32)it * 32 >= ns) continue;
+        const uint4 r = sw.row[it];
+        const u32 q = (q_r[it / 4] >> (8 * (it % 4))) & 0xFFu;
         if constexpr (HUB) {
-            const u32 hm = hm_r[it];
-            if (((km | hm) >> lane) & 1u) {
-                const u64 base = s_base[s0_r[it]];
-                if ((km >> lane) & 1u) {
-                    const u32 at = (u32)base + (rank & 0xFFFFu) + __popc(km & lt);
+            if (((r.x | r.y) >> lane) & 1u) {
+                const u64 base = sw.base[q];
+                if ((r.x >> lane) & 1u) {
+                    const u32 at = (u32)base + (r.z & 0xFFFFu) + __popc(r.x & lt);
                     __stcs(headp + ref + (long long)(int)at, y_r[it]);
                 } else {
-                    const u32 at = (u32)(base >> 32) + (rank >> 16) + __popc(hm & lt);
+                    const u32 at = (u32)(base >> 32) + (r.z >> 16) + __popc(r.y & lt);
                     __stcs(hubp + href + (long long)(int)at, (u16)(HUB_H - 1 - (dy_r[it] & ~HUB_FLAG)));
                 }
             }
-            rank += __popc(km) + (__popc(hm) << 16);
         } else {
-            if ((km >> lane) & 1u) __stcs(headp + s_base[s0_r[it]] + rank + __popc(km & lt), y_r[it]);
-            rank += __popc(km);
+            if ((r.x >> lane) & 1u) __stcs(headp + sw.base[q] + (r.z + __popc(r.x & lt)), y_r[it]);
         }
     }
 }
@@ -344,25 +358,20 @@ __device__ __forceinline__ void orient_tile(uint2 (*s_info_all)[32 * IPT], u64 (
 // One tile per warp.  HUB: a graph without hubs (hubs = 0) runs the plain body, whose lists and
 // length words are then the same.
 template <int BLOCK, int IPT, bool HUB>
-__global__ void __launch_bounds__(BLOCK, 4) k_orient(const u64* __restrict__ fo, const u32* __restrict__ head, u64 n,
+__global__ void __launch_bounds__(BLOCK, ORIENT_BLOCKS) k_orient(const u64* __restrict__ fo, const u32* __restrict__ head, u64 n,
                                                      u64 nnz, const u32* __restrict__ deg,
                                                      const u32* __restrict__ tile_i0, u32* __restrict__ headp,
                                                      u16* __restrict__ hubp, u32* __restrict__ dplus,
                                                      u32* __restrict__ spanning, Control* ctl, u64 tile_begin) {
     chain_begin();
-    // at a piece's first slot: (window index + 1, key)
-    __shared__ uint2 s_info_all[BLOCK / 32][32 * IPT];
-    // at a piece's first slot: the tile ranks (at its first slot, past its last slot), then the
-    // headp index of tile rank 0 for its entries (HUB: the indices in both arrays relative to where
-    // the tile's first vertex would start, 32 bits each)
-    __shared__ u64 s_base_all[BLOCK / 32][32 * IPT];
+    __shared__ OrientWarp<IPT> s_warp[BLOCK / 32];
     if (ctl->err & DEV_ERR_MASK) return;
+    const int wid = threadIdx.x >> 5;
+    const u64 tile = (tile_begin + blockIdx.x) * (BLOCK / 32) + wid;
     if (HUB && ctl->hubs)
-        orient_tile<BLOCK, IPT, true>(s_info_all, s_base_all, fo, head, n, nnz, deg, tile_i0, headp, hubp, dplus,
-                                      spanning, ctl, tile_begin);
+        orient_tile<IPT, true>(s_warp[wid], fo, head, n, nnz, deg, tile_i0, headp, hubp, dplus, spanning, ctl, tile);
     else
-        orient_tile<BLOCK, IPT, false>(s_info_all, s_base_all, fo, head, n, nnz, deg, tile_i0, headp, nullptr, dplus,
-                                       spanning, ctl, tile_begin);
+        orient_tile<IPT, false>(s_warp[wid], fo, head, n, nnz, deg, tile_i0, headp, nullptr, dplus, spanning, ctl, tile);
 }
 
 // Out-list descriptors, and the (owner, segment) tiles of owners above the small
