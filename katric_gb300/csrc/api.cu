@@ -64,7 +64,6 @@ inline size_t align_up(size_t x) { return (x + ALIGN - 1) & ~(ALIGN - 1); }
 
 struct Layout {
     size_t ctl = 0, deg = 0, dplus = 0, tile_i0 = 0, vdesc = 0, headp = 0, ltiles = 0, thist = 0, tkeys = 0,
-           spanning = 0,
            partials = 0, cnt = 0,
            total = 0, mid = 0, big = 0, scratch = 0, in_fo = 0, in_head = 0, hub_bins = 0, hub_tmp = 0,
            hub_ids = 0, hub_lists = 0, top_info = 0, top_long = 0, top_bits = 0, bytes = 0;
@@ -107,7 +106,6 @@ Layout make_layout(u64 n, u64 nnz, int32_t method, int num_sms, bool with_inputs
     L.dplus = take(sizeof(u32) * (n + 1));
     L.vdesc = take((L.wide ? 16 : 8) * (n + 1));
     L.headp = take(sizeof(u32) * cap);
-    L.spanning = take(sizeof(u32) * ktri::spanning_capacity(n, nnz));
     L.tile_i0 = take(sizeof(u32) * (ktri::base_tiles(n, nnz) + 2));
     u32 grid = 0;
     if (method == KTRI_METHOD_AUTO) {
@@ -384,7 +382,6 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     auto* dplus = reinterpret_cast<u32*>(base + L.dplus);
     void* vdesc = base + L.vdesc;
     auto* headp = reinterpret_cast<u32*>(base + L.headp);
-    auto* spanning = reinterpret_cast<u32*>(base + L.spanning);
     auto* partials = reinterpret_cast<u64*>(base + L.partials);
     auto* tile_i0 = reinterpret_cast<u32*>(base + L.tile_i0);
     ktri::HubState hub;
@@ -408,7 +405,7 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     const bool autom = opt.method == KTRI_METHOD_AUTO && !sort_all;
     ktri::launch_prep(fo, n, nnz, deg, dplus, cnt, tile_i0, hub, ctl, sms, st);
     if (!chunks) {
-        ktri::launch_orient(fo, head, n, nnz, deg, tile_i0, headp, hub, dplus, spanning, ctl, st);
+        ktri::launch_orient(fo, head, n, nnz, deg, tile_i0, headp, hub, dplus, ctl, st);
     } else {
         // tile t reads slots below (t + 1) * ORIENT_TILE + 1: launch each tile once its slots are in
         u64 done = 0;
@@ -417,7 +414,7 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
             const u64 upto = c + 1 == chunks->count ? ktri::orient_tiles(n, nnz)
                                                     : (chunks->ends[c] - 1) / ktri::ORIENT_TILE;
             if (upto > done) {
-                ktri::launch_orient(fo, head, n, nnz, deg, tile_i0, headp, hub, dplus, spanning, ctl, st, done, upto);
+                ktri::launch_orient(fo, head, n, nnz, deg, tile_i0, headp, hub, dplus, ctl, st, done, upto);
                 done = upto;
             }
         }
@@ -448,7 +445,8 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     if (!autom) {
         ktri::launch_sort_lists<OffT>(n, vdesc, headp, reinterpret_cast<u32*>(base + L.mid),
                                       reinterpret_cast<u32*>(base + L.big), reinterpret_cast<u32*>(base + L.scratch),
-                                      L.scratch_per_block, L.big_grid, spanning, ctl, sms, st);
+                                      L.scratch_per_block, L.big_grid, {fo, tile_i0, ktri::base_tiles(n, nnz)}, ctl,
+                                      sms, st);
     }
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[1], st));
     if (opt.collect_stats)
@@ -1153,7 +1151,7 @@ int ktri_contract_dag_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32
     // sorted by id, as preprocessing_global does after compact (cetric.h:916-930)
     ktri::launch_sort_lists<u64>(n_local, base + x_desc, d_ohead, reinterpret_cast<u32*>(base + x_mid),
                                  reinterpret_cast<u32*>(base + x_big), reinterpret_cast<u32*>(base + x_scr), P, big_grid,
-                                 nullptr, ctl, ctx->num_sms, st);
+                                 {}, ctl, ctx->num_sms, st);
     KTRI_CK(ctx, cudaGetLastError());
     u64 ke[2] = {0, 0};
     KTRI_CK(ctx, cudaMemcpyAsync(&ke[0], d_keep + n_local, 8, cudaMemcpyDeviceToHost, st));

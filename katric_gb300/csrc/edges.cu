@@ -32,32 +32,27 @@ constexpr int BIN_STACK = 96;
 
 template <typename OffT>
 __global__ void k_sort_warp(u64 n, const Desc<OffT>* __restrict__ vdesc, u32* __restrict__ headp, u32* mid_list,
-                            u32* big_list, const u32* __restrict__ spanning, Control* ctl) {
+                            u32* big_list, SplitLists split, Control* ctl) {
     chain_begin();
     if (ctl->err & DEV_ERR_MASK) return;
     const int lane = threadIdx.x & 31;
     const u64 gw = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
-    // spanning: the lists are pieces of the input's; where that is sorted, only those put together
-    // from several pieces can be out of order (RGG n = 2^18: 25 -> 3 us)
-    const bool few = spanning && !(ctl->err & DEV_FLAG_UNSORTED);
-    const u64 lists = few ? *(volatile unsigned long long*)&ctl->spanning : n;
-    for (u64 i = gw; i < lists; i += nwarps) {
-        const u64 v = few ? spanning[i] : i;
+    auto sort_list = [&](u64 v) {
         const Desc<OffT> d = load_desc(vdesc + v);
-        if (d.d <= 1) continue;
+        if (d.d <= 1) return;
         if (d.d > 32) {
             if (lane == 0) {
                 if (d.d <= (u32)SORT_SMEM) mid_list[atomicAdd(&ctl->sort_mid, 1ull)] = (u32)v;
                 else big_list[atomicAdd(&ctl->sort_big, 1ull)] = (u32)v;
             }
-            continue;
+            return;
         }
         u32* p = headp + list_start(d);
         u32 x = lane < (int)d.d ? p[lane] : EMPTY_KEY;
         const u32 nx = __shfl_down_sync(0xFFFFFFFFu, x, 1);
         const bool bad = lane + 1 < (int)d.d && nx < x;
-        if (!__any_sync(0xFFFFFFFFu, bad)) continue;
+        if (!__any_sync(0xFFFFFFFFu, bad)) return;
 #pragma unroll
         for (int k = 2; k <= 32; k <<= 1) {
 #pragma unroll
@@ -69,6 +64,30 @@ __global__ void k_sort_warp(u64 n, const Desc<OffT>* __restrict__ vdesc, u32* __
             }
         }
         if (lane < (int)d.d) p[lane] = x;
+    };
+    if (!split.tile_i0 || (ctl->err & DEV_FLAG_UNSORTED)) {
+        for (u64 v = gw; v < n; v += nwarps) sort_list(v);
+        return;
+    }
+    // The lists are pieces of the input's; where that is sorted, only those put together from
+    // several tiles' pieces can be out of order (RGG n = 2^18: 25 -> 3 us): at most one list
+    // starts in a tile and ends past it, the last of its window.
+    const u64 even = (split.tiles + nwarps - 1) / nwarps;
+    const u32 per = even < 32 ? (u32)even : 32u;  // tiles a warp looks at together
+    for (u64 t0 = gw * per; t0 < split.tiles; t0 += nwarps * per) {
+        const u64 t = t0 + lane;
+        u32 v = 0;
+        bool is_split = false;
+        if ((u32)lane < per && t < split.tiles) {
+            v = split.tile_i0[t + 1];
+            if (v < n) {
+                const u64 a = split.fo[v], b = split.fo[v + 1];
+                const u64 j0 = t * TILE_BASE - split.tile_i0[t], j1 = (t + 1) * TILE_BASE - v;
+                is_split = a >= j0 && a < j1 && b > j1;
+            }
+        }
+        for (u32 ball = __ballot_sync(0xFFFFFFFFu, is_split); ball; ball &= ball - 1)
+            sort_list(__shfl_sync(0xFFFFFFFFu, v, __ffs(ball) - 1));
     }
 }
 
@@ -676,11 +695,11 @@ __global__ void __launch_bounds__(PAIR_BLOCK) k_intersect_pairs(int method, cons
 
 template <typename OffT>
 void launch_sort_lists(u64 n, const void* vdesc, u32* headp, u32* mid_list, u32* big_list, u32* scratch,
-                       u64 scratch_per_block, int big_grid, const u32* spanning, Control* ctl, int num_sms,
+                       u64 scratch_per_block, int big_grid, SplitLists split, Control* ctl, int num_sms,
                        LaunchStream st) {
     if (n == 0) return;
     const auto* vd = reinterpret_cast<const Desc<OffT>*>(vdesc);
-    launch_chained(k_sort_warp<OffT>, num_sms * 8, 256, 0, st, n, vd, headp, mid_list, big_list, spanning, ctl);
+    launch_chained(k_sort_warp<OffT>, num_sms * 8, 256, 0, st, n, vd, headp, mid_list, big_list, split, ctl);
     launch_chained(k_sort_block<OffT>, num_sms * 4, SORT_BLOCK, 0, st, vd, headp, mid_list, ctl);
     launch_chained(k_sort_global<OffT>, big_grid, SORT_BLOCK, 0, st, vd, headp, big_list, scratch, scratch_per_block, ctl);
 }
@@ -732,7 +751,7 @@ void launch_intersect_pairs(int method, const u32* a_vals, const u64* a_off, con
 }
 
 #define KTRI_INST(OffT)                                                                                             \
-    template void launch_sort_lists<OffT>(u64, const void*, u32*, u32*, u32*, u32*, u64, int, const u32*,          \
+    template void launch_sort_lists<OffT>(u64, const void*, u32*, u32*, u32*, u32*, u64, int, SplitLists,          \
                                           Control*, int, LaunchStream);                                            \
     template void launch_count_edges<OffT>(u64, const void*, const u32*, int, u64, double, u64*, u64*, int, u32*,   \
                                            Control*, TriangleSink, LaunchStream);                                   \

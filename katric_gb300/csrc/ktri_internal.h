@@ -67,7 +67,6 @@ struct Control {
     unsigned long long large_tiles;      // number of (owner, segment) tiles for large owners
     unsigned long long small_next;       // dynamic tile cursor of the small-owner kernel
     unsigned long long large_next;       // dynamic tile cursor of the large-owner kernel
-    unsigned long long spanning;         // number of vertices whose out-list was assembled by several tiles
     unsigned long long edge_next;        // dynamic cursor of the per-edge kernels
     unsigned long long stat_wedge;       // collect_stats: sum of |N+(u)| over oriented (v,u)
     unsigned long long stat_isz;         // collect_stats: sum of |N+(v)|+|N+(u)|

@@ -41,8 +41,6 @@ constexpr u32 COPY_WAIT_POLLS = 1u << 22;  // polls of a bounded wait for a bulk
 // the vertex where diagonal k * TILE_BASE crosses the path.  One warp orients one base tile.
 constexpr u64 TILE_BASE = 32ull * ORIENT_IPT;
 inline u64 base_tiles(u64 n, u64 nnz) { return (n + nnz + TILE_BASE - 1) / TILE_BASE; }
-// Each base tile records at most one split list (the one that starts in it and ends past it).
-inline u64 spanning_capacity(u64 n, u64 nnz) { return base_tiles(n, nnz) + 2; }
 // Owners above small_d hold more than small_d adjacency entries each; every owner has at most
 // deg / seg + 1 tiles.
 inline u64 large_tile_capacity(u64 n, u64 nnz, u32 small_d, u32 seg) {
@@ -117,7 +115,7 @@ void launch_prep(const u64* fo, u64 n, u64 nnz, u32* deg, u32* dplus, u64* cnt, 
 constexpr u64 ORIENT_TILE = (u64)ORIENT_BLOCK * ORIENT_IPT;
 u64 orient_tiles(u64 n, u64 nnz);
 void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* deg, const u32* tile_i0, u32* headp,
-                   const HubState& hub, u32* dplus, u32* spanning, Control* ctl, LaunchStream st, u64 tile_begin = 0,
+                   const HubState& hub, u32* dplus, Control* ctl, LaunchStream st, u64 tile_begin = 0,
                    u64 tile_end = ~0ull);
 // Owner tiles: medium owners' tiles are written to mtiles, large owners' to ltiles (each
 // array holds large_tile_capacity entries).
@@ -238,11 +236,17 @@ void launch_stats(const u64* fo, const u32* head, u64 n, const void* vdesc, cons
                   u32 small_d, u32 medium_d, Control* ctl, int num_sms, LaunchStream st);
 
 // Sorted-list strategies (merge, binary search, binary, hybrid): sort out-lists by id, then
-// intersect per oriented edge.  spanning: the lists the orientation put together from several
-// pieces (the only ones to sort where ctl says that the input is sorted), or null to look at all.
+// intersect per oriented edge.  split: the orientation's tiles, from which follow the lists that were
+// put together from several pieces (the only ones to sort where ctl says that the input is sorted);
+// none to look at all.
+struct SplitLists {
+    const u64* fo = nullptr;
+    const u32* tile_i0 = nullptr;
+    u64 tiles = 0;
+};
 template <typename OffT>
 void launch_sort_lists(u64 n, const void* vdesc, u32* headp, u32* mid_list, u32* big_list, u32* scratch,
-                       u64 scratch_per_block, int big_grid, const u32* spanning, Control* ctl, int num_sms, LaunchStream st);
+                       u64 scratch_per_block, int big_grid, SplitLists split, Control* ctl, int num_sms, LaunchStream st);
 template <typename OffT>
 void launch_count_edges(u64 n, const void* vdesc, const u32* headp, int method, u64 cutoff, double hybrid_scale,
                         u64* cnt, u64* partials, int grid, u32* tails, Control* ctl, TriangleSink sink,

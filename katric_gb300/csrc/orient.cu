@@ -6,9 +6,8 @@
 // out-list of v iff (deg(v), v) < (deg(u), u).  The reference partitions each list in place;
 // here the input CSR is read-only and the out-lists are written to a separate gapped array.
 // A list that one merge-path tile holds entirely keeps its input order.  A list that spans
-// tiles is assembled from per-tile pieces and is recorded in the spanning list; the id sort
-// (sort_neighborhoods, distributed_graph.h:578-593) runs only where a strategy needs sorted
-// lists.
+// tiles is assembled from per-tile pieces; the id sort (sort_neighborhoods,
+// distributed_graph.h:578-593) runs only where a strategy needs sorted lists.
 #include "ktri_device.cuh"
 #include "ktri_kernels.h"
 
@@ -159,17 +158,18 @@ __global__ void k_hub_rank(const u32* __restrict__ hub_bins, const uint2* __rest
 //                list) and the gapped-array index of tile rank 0 for its entries
 //   pass 2       kept entries written from registers, in slot order
 // A list held by one tile keeps its input order.  A split list's pieces reserve their ranges
-// with one atomic each and are recorded in the spanning list by the tile that holds the list's
-// start.
+// with one atomic each; which lists are split follows from the tiles' bounds (SplitLists): a list
+// of them kept with one counter took an atomic of one address per tile (130 k of them on RGG
+// n = 2^20), which bounded the kernel: orientation of RGG-24 3.2 -> 2.4 ms without it.
 // HUB: deg holds orientation keys (the degree, or a hub's key above every degree), a kept entry that
 // is a hub goes to the hub array as its index and the others to headp, so a piece has two ranks
 // and two shares of its out-list's length word (hubs << 16 | others, as everywhere with hubs).
-// What bounds it: latency (a tile's offset, its slots, their keys, one after the other: half of the
-// issue slots are taken with 32 warps per SM, 64 registers) and instruction issue.  Measured (kernel
-// under ncu, RGG n = 2^20 of 33 M slots): 187 us with 112 instructions per row of 32 slots, against
-// 229 us with 172 when every slot carried its piece's ends and rank; the orientation phase of
-// RGG-24 3.7 -> 3.2 ms, of RMAT n = 10^6 0.42 -> 0.32 ms.  Five or six blocks per SM spill: 3.4 and
-// 3.6 ms.
+// What bounds it: latency (a tile's offset, its slots, their keys, one after the other, with 32
+// warps per SM of 64 registers) and instruction issue: 112 instructions per row of 32 slots, 172 when
+// every slot carried its piece's ends and rank.  Measured (orientation phase, RGG-24 / RMAT n = 10^6
+// / 512-graph batch): 3.7 / 0.42 / 3.5 ms in that form, 2.44 / 0.31 / 2.2 ms now.  Five blocks per SM
+// spill: 2.29 / 0.33 / 2.25 ms.  Copying the next tile's slots to shared memory while one is at work
+// (a persistent grid) takes the L1 cache that the keys' gathers use: 2.50 / 0.31 / 3.0 ms.
 template <int IPT>
 struct OrientWarp {
     static constexpr int W = 32 * IPT;
@@ -189,7 +189,7 @@ __device__ __forceinline__ void orient_tile(OrientWarp<IPT>& sw, const u64* __re
                                             const u32* __restrict__ head, u64 n, u64 nnz,
                                             const u32* __restrict__ deg, const u32* __restrict__ tile_i0,
                                             u32* __restrict__ headp, u16* __restrict__ hubp, u32* __restrict__ dplus,
-                                            u32* __restrict__ spanning, Control* ctl, u64 tile) {
+                                            Control* ctl, u64 tile) {
     constexpr int W = 32 * IPT;
     constexpr u32 FULL = 0xFFFFFFFFu;
     static_assert(W <= 256 && IPT % 4 == 0, "piece numbers in bytes");
@@ -291,7 +291,7 @@ __device__ __forceinline__ void orient_tile(OrientWarp<IPT>& sw, const u64* __re
     unsorted |= end_nx < end_y;
     const u32 err = (y_max >= n32 ? DEV_ERR_ID_RANGE : 0u) | (self_loop ? DEV_ERR_SELF_LOOP : 0u) |
                     (dup ? DEV_ERR_DUPLICATE : 0u) | (unsorted ? DEV_FLAG_UNSORTED : 0u);
-    if (err) atomicOr(&ctl->err, err);
+    if (err & ~*(volatile u32*)&ctl->err) atomicOr(&ctl->err, err);
     __syncwarp();
     // piece pass: out-degree shares and where each piece's kept entries go
     const u64 ref = oriented_start(j0, i0), href = hub_start(ref, i0);  // HUB: origins of the 32-bit indices
@@ -307,7 +307,6 @@ __device__ __forceinline__ void orient_tile(OrientWarp<IPT>& sw, const u64* __re
             u32 carry = 0;
             if (a < j0 || b > j1) {
                 if (cnt) carry = atomicAdd(&dplus[v], cnt);
-                if (a >= j0) spanning[atomicAdd(&ctl->spanning, 1ull)] = (u32)v;
             } else {
                 dplus[v] = cnt;
             }
@@ -362,16 +361,16 @@ __global__ void __launch_bounds__(BLOCK, ORIENT_BLOCKS) k_orient(const u64* __re
                                                      u64 nnz, const u32* __restrict__ deg,
                                                      const u32* __restrict__ tile_i0, u32* __restrict__ headp,
                                                      u16* __restrict__ hubp, u32* __restrict__ dplus,
-                                                     u32* __restrict__ spanning, Control* ctl, u64 tile_begin) {
+                                                     Control* ctl, u64 tile_begin) {
     chain_begin();
     __shared__ OrientWarp<IPT> s_warp[BLOCK / 32];
     if (ctl->err & DEV_ERR_MASK) return;
     const int wid = threadIdx.x >> 5;
     const u64 tile = (tile_begin + blockIdx.x) * (BLOCK / 32) + wid;
     if (HUB && ctl->hubs)
-        orient_tile<IPT, true>(s_warp[wid], fo, head, n, nnz, deg, tile_i0, headp, hubp, dplus, spanning, ctl, tile);
+        orient_tile<IPT, true>(s_warp[wid], fo, head, n, nnz, deg, tile_i0, headp, hubp, dplus, ctl, tile);
     else
-        orient_tile<IPT, false>(s_warp[wid], fo, head, n, nnz, deg, tile_i0, headp, nullptr, dplus, spanning, ctl, tile);
+        orient_tile<IPT, false>(s_warp[wid], fo, head, n, nnz, deg, tile_i0, headp, nullptr, dplus, ctl, tile);
 }
 
 // Out-list descriptors, and the (owner, segment) tiles of owners above the small
@@ -680,7 +679,7 @@ size_t hub_bins_zeroed() { return sizeof(u32) * HUB_BINS; }
 u64 orient_tiles(u64 n, u64 nnz) { return (n + nnz + ORIENT_TILE - 1) / ORIENT_TILE; }
 
 void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* deg, const u32* tile_i0, u32* headp,
-                   const HubState& hub, u32* dplus, u32* spanning, Control* ctl, LaunchStream st, u64 tile_begin,
+                   const HubState& hub, u32* dplus, Control* ctl, LaunchStream st, u64 tile_begin,
                    u64 tile_end) {
     constexpr int BLOCK = ORIENT_BLOCK, IPT = ORIENT_IPT;
     const u64 tiles = orient_tiles(n, nnz);
@@ -689,10 +688,10 @@ void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* de
     const unsigned grid = (unsigned)(tile_end - tile_begin);
     if (hub)
         launch_chained(k_orient<BLOCK, IPT, true>, grid, BLOCK, 0, st, fo, head, n, nnz, deg, tile_i0, headp, hub.lists, dplus,
-                                                           spanning, ctl, tile_begin);
+                                                           ctl, tile_begin);
     else
         launch_chained(k_orient<BLOCK, IPT, false>, grid, BLOCK, 0, st, fo, head, n, nnz, deg, tile_i0, headp, nullptr, dplus,
-                                                            spanning, ctl, tile_begin);
+                                                            ctl, tile_begin);
 }
 
 template <typename OffT, bool HUB>
