@@ -1273,6 +1273,20 @@ int ktri_list_triangles(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t
 
 // ---- oriented lists (the katric local phase) ---------------------------------------------
 
+namespace {
+
+// The scratch of the symmetrisation lies in regions that are free until orientation starts: the
+// counters in deg and dplus (n + 1 each, one after the other), the entries' places behind the first
+// 3 n + 8 entries of the out-list array.
+void symmetrize(ktri_ctx* ctx, char* base, const Layout& L, const u64* fo, const u32* head, u64 n, u64 m, u64* fs,
+                u32* hs, u64* sums, cudaStream_t st) {
+    ktri::launch_dag_symmetrize(fo, head, n, m, fs, hs, reinterpret_cast<u32*>(base + L.deg),
+                                reinterpret_cast<u64*>(base + L.vdesc),
+                                reinterpret_cast<u32*>(base + L.headp) + (3 * n + 8), sums, ctx->num_sms, st);
+}
+
+}  // namespace
+
 int ktri_count_dag_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint32_t* d_head, uint64_t n, uint64_t m,
                           uint64_t* d_total, uint64_t* d_per_vertex, const ktri_opts* opts, void* stream) {
     const ktri::Options opt = resolve(opts, 2 * m);
@@ -1296,12 +1310,10 @@ int ktri_count_dag_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint
     char* base = static_cast<char*>(ctx->ws);
     auto* fs = reinterpret_cast<u64*>(base + L.in_fo);
     auto* hs = reinterpret_cast<u32*>(base + L.in_head);
-    // the out-list and descriptor regions are free until orientation starts: in-list cursors
-    // and scan sums live there meanwhile
-    auto* cursor = reinterpret_cast<u32*>(base + L.deg);
+    // the out-list array (2 m + 3 n + 8 entries) is free until orientation starts: the scan sums are
+    // at its start meanwhile
     auto* sums = reinterpret_cast<u64*>(base + L.headp);
-    ktri::launch_dag_symmetrize(reinterpret_cast<const u64*>(d_first_out), d_head, n, fs, hs, cursor, sums,
-                                ctx->num_sms, st);
+    symmetrize(ctx, base, L, reinterpret_cast<const u64*>(d_first_out), d_head, n, m, fs, hs, sums, st);
     KTRI_CK(ctx, cudaGetLastError());
     u64* cnt = d_per_vertex ? reinterpret_cast<u64*>(d_per_vertex) : reinterpret_cast<u64*>(base + L.cnt);
     auto* tot = reinterpret_cast<u64*>(d_total);
@@ -1342,13 +1354,12 @@ int ktri_count_dag_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t*
     auto* sums = reinterpret_cast<u64*>(base + x_sums);
     auto* fs = reinterpret_cast<u64*>(base + L.in_fo);
     auto* hs = reinterpret_cast<u32*>(base + L.in_head);
-    auto* cursor = reinterpret_cast<u32*>(base + L.deg);
     auto* d_cnt = reinterpret_cast<u64*>(base + L.cnt);
     auto* d_total = reinterpret_cast<u64*>(base + L.total);
     cudaStream_t st = ctx->stream;
     KTRI_CK(ctx, copy_host(ctx, dfo, first_out, sizeof(u64) * (n + 1), true, st));
     if (m) KTRI_CK(ctx, copy_host(ctx, dhead, head, sizeof(u32) * m, true, st));
-    ktri::launch_dag_symmetrize(dfo, dhead, n, fs, hs, cursor, sums, ctx->num_sms, st);
+    symmetrize(ctx, base, L, dfo, dhead, n, m, fs, hs, sums, st);
     KTRI_CK(ctx, cudaGetLastError());
     rc = run_pipeline(ctx, L, fs, hs, n, nnz, d_total, d_cnt, opt, st, false);
     if (rc) return rc;

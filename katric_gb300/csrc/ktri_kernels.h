@@ -209,8 +209,8 @@ void launch_narrow_ids(const u64* src, u64 count, u32* dst, int num_sms, cudaStr
 bool copy_by_kernel_ok(const void* src, const void* dst);
 bool launch_copy(const void* src, void* dst, u64 bytes, int num_sms, cudaStream_t st);
 
-// Oriented out-lists -> undirected CSR of their edges (fs: n + 1 offsets, hs: 2m ids).  cursor
-// needs n u32 and sums dag_scan_chunks(n) u64 of scratch.
+// Oriented out-lists -> undirected CSR of their edges (fs: n + 1 offsets, hs: 2m ids).  Scratch:
+// in_deg 2 n u32 (a power of two of at least n of them is used), in_start n u64, pos m u32, sums dag_scan_chunks(n) u64.
 u64 dag_scan_chunks(u64 n);
 void launch_scan_u64(u64* x, u64 len, u64* sums, cudaStream_t st);  // exclusive, in place
 // Per-vertex cost (KTRI_COST_*) into cost[0..n), its exclusive prefix in place (cost[n] = total),
@@ -224,8 +224,8 @@ void launch_cost_partition(const u64* fo, const u32* head, u64 n, const u32* deg
 void launch_contract(const u64* fo, const u32* head, u64 n, u64 n_local, u64* cnt, u64* keep, u64* sums,
                      unsigned long long* maxlen, u32* kept, u64* out_fo, u32* out_head, void* desc, int num_sms,
                      cudaStream_t st);
-void launch_dag_symmetrize(const u64* fo, const u32* head, u64 n, u64* fs, u32* hs, u32* cursor, u64* sums,
-                           int num_sms, cudaStream_t st);
+void launch_dag_symmetrize(const u64* fo, const u32* head, u64 n, u64 m, u64* fs, u32* hs, u32* in_deg, u64* in_start,
+                           u32* pos, u64* sums, int num_sms, cudaStream_t st);
 void launch_graph_totals(const u64* cnt, const u64* graph_first, u64 num_graphs, u64 n, u64* totals, Control* ctl,
                          int num_sms, LaunchStream st);
 
