@@ -465,12 +465,12 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
             fo, head, n, nnz, vdesc, headp, hub, mrun, lrun, opt.small_outdegree, opt.segment, cnt, partials, ctl, sms,
             st, events ? ctx->ev[4] : nullptr, events ? ctx->ev[5] : nullptr, first_wait_polls(opt.copy_wait_polls));
         if (e != cudaSuccess) return cuda_fail(ctx, e, "launch of the counting kernels");
-        ktri::launch_final_auto<OffT, HUB>(partials, n, sms, d_total, ctl, st);
+        if (d_total) ktri::launch_final_auto<OffT, HUB>(partials, n, sms, d_total, ctl, st);
     } else {
         const int grid = ktri::count_grid_edges(sms);
         ktri::launch_count_edges<OffT>(n, vdesc, headp, opt.method, opt.binary_cutoff, opt.hybrid_scale, cnt, partials,
                                        grid, reinterpret_cast<u32*>(base + L.mid), ctl, sink, st);
-        ktri::launch_final(partials, (u32)grid, d_total, ctl, st);
+        if (d_total) ktri::launch_final(partials, (u32)grid, d_total, ctl, st);
     }
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[3], st));
     KTRI_CK(ctx, cudaGetLastError());
@@ -1393,8 +1393,8 @@ int check_batch(ktri_ctx* ctx, const void* fo, const void* head, u64 n, u64 nnz,
 int enqueue_batch(ktri_ctx* ctx, char* base, const Layout& L, const u64* fo, const u32* head, u64 n, u64 nnz,
                   const u64* graph_first, u64 num_graphs, u64* totals, u64* cnt, const ktri::Options& opt,
                   cudaStream_t st, bool events) {
-    auto* d_total = reinterpret_cast<u64*>(base + L.total);
-    int rc = enqueue_layout(ctx, ctx->num_sms, base, L, fo, head, n, nnz, d_total, cnt, opt, st, false, events);
+    // no total over all graphs
+    int rc = enqueue_layout(ctx, ctx->num_sms, base, L, fo, head, n, nnz, nullptr, cnt, opt, st, false, events);
     if (rc) return rc;
     ktri::launch_graph_totals(cnt, graph_first, num_graphs, n, totals, reinterpret_cast<Control*>(base + L.ctl),
                               ctx->num_sms, ktri::LaunchStream(st, ctx->chained));
