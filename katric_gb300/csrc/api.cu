@@ -688,6 +688,11 @@ int run_noalloc(char* base, const Layout& L, const u64* fo, const u32* head, u64
 int ktri::ctx_device(const ktri_ctx* ctx) { return ctx->device; }
 
 void ktri::ctx_for_server(ktri_ctx* ctx) { ctx->hubs = ctx->chained = false; }
+void ktri::ctx_allow_hubs(ktri_ctx* ctx, bool allow) { ctx->hubs = allow; }
+size_t ktri::hub_bytes(uint64_t n, uint64_t nnz) {
+    return make_layout(n, nnz, KTRI_METHOD_AUTO, 0, false, true, false, 0, 0, true).bytes -
+           make_layout(n, nnz, KTRI_METHOD_AUTO, 0, false, true).bytes;
+}
 
 int ktri::ctx_num_sms(const ktri_ctx* ctx) { return ctx->num_sms; }
 

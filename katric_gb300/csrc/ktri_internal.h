@@ -32,9 +32,12 @@ struct Options {
 // The device a context was created on, and its SM count.
 int ctx_device(const ktri_ctx* ctx);
 int ctx_num_sms(const ktri_ctx* ctx);
-// A context of one of the server's slots: workspaces as ktri_workspace_bytes reports them (no split
-// out-lists), and kernels that leave their room to the other slots' until they run.
+// A context of one of the server's slots: kernels that leave their room to the other slots' until
+// they run, and split out-lists only in the counts that ctx_allow_hubs allows them.
 void ctx_for_server(ktri_ctx* ctx);
+void ctx_allow_hubs(ktri_ctx* ctx, bool allow);
+// What split out-lists add to ktri_workspace_bytes (0 where a count of this size has none).
+size_t hub_bytes(uint64_t n, uint64_t nnz);
 
 struct Control;
 struct EngineJob;

