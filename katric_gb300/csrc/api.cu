@@ -83,6 +83,11 @@ u64 isqrt_ceil(u64 x) {
 
 constexpr u64 HUB_MIN_NNZ = 1ull << 21;
 
+// Tile orders (large tiles by the vertex range they stream, for L2 reuse; medium tiles
+// longest owner first, so the warps' last tiles are short).  Below 2^20 adjacency entries
+// everything fits L2 and the few tiles are not worth the three extra launches.
+constexpr u64 TILE_ORDER_MIN_NNZ = 1ull << 20;
+
 // Workspace of one count.  num_sms = 0 sizes the grids for the largest supported part.
 Layout make_layout(u64 n, u64 nnz, int32_t method, int num_sms, bool with_inputs, bool internal_cnt,
                    bool force_wide = false, u32 small_d = 0, u32 seg = 0, bool hub = false) {
@@ -109,13 +114,15 @@ Layout make_layout(u64 n, u64 nnz, int32_t method, int num_sms, bool with_inputs
     L.tile_i0 = take(sizeof(u32) * (ktri::base_tiles(n, nnz) + 2));
     u32 grid = 0;
     if (method == KTRI_METHOD_AUTO) {
-        // medium- and large-owner tiles, and both reordered (seg = 0: room for the default options)
+        // owner tiles and both kinds reordered (seg = 0: room for the default options)
         const u64 tcap = seg ? ktri::large_tile_capacity(n, nnz, small_d, seg)
                              : std::max(ktri::large_tile_capacity(n, nnz, 32, ktri::LARGE_SEG),
                                         ktri::large_tile_capacity(n, nnz, 32, ktri::default_segment(nnz)));
-        L.ltiles = take(sizeof(uint2) * 4 * tcap);
-        L.thist = take(sizeof(u32) * ktri::tile_order_scratch_words());
-        L.tkeys = take(sizeof(u32) * tcap);
+        L.ltiles = take(sizeof(uint2) * (nnz >= TILE_ORDER_MIN_NNZ ? 2 : 1) * tcap);
+        if (nnz >= TILE_ORDER_MIN_NNZ) {
+            L.thist = take(sizeof(u32) * ktri::tile_order_scratch_words());
+            L.tkeys = take(sizeof(u32) * tcap);
+        }
         grid = (u32)(sms * 48);  // bound on the small + medium + large persistent grids (occupancy <= 16 each)
     } else {
         L.mid = take(sizeof(u32) * (n + 1));
@@ -422,25 +429,22 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     auto* mtiles = autom ? reinterpret_cast<uint2*>(base + L.ltiles) : nullptr;
     const u64 tcap = ktri::large_tile_capacity(n, nnz, opt.small_outdegree, opt.segment);
     auto* ltiles = autom ? mtiles + tcap : nullptr;
+    const bool order = autom && nnz >= TILE_ORDER_MIN_NNZ;
+    auto* hist = order ? reinterpret_cast<u32*>(base + L.thist) : nullptr;
     ktri::launch_desc<OffT, HUB>(fo, n, dplus, vdesc, hub, mtiles, ltiles, autom ? opt.small_outdegree : 0xFFFFFFFFu,
-                            opt.medium_outdegree, opt.segment, ctl, sms, st);
-    // Tile orders (large tiles by the vertex range they stream, for L2 reuse; medium tiles
-    // longest owner first, so the warps' last tiles are short).  Below 2^20 adjacency entries
-    // everything fits L2 and the few tiles are not worth the four extra launches.
-    const bool order = autom && nnz >= (1ull << 20);
+                            opt.medium_outdegree, opt.segment, hist, ctl, sms, st);
     uint2* lrun = ltiles;
     uint2* mrun = mtiles;
     if (order) {
+        mrun = ltiles;
         lrun = ltiles + tcap;
-        mrun = lrun + tcap;
         const bool by_cost = opt.tile_order == KTRI_TILE_ORDER_COST;
         auto* keys = reinterpret_cast<u32*>(base + L.tkeys);
-        ktri::launch_order_tiles(fo, head, dplus, n, ltiles, &ctl->large_tiles, opt.segment,
-                                 by_cost ? ktri::TILE_BY_COST : ktri::TILE_BY_VERTEX, HUB, keys,
-                                 reinterpret_cast<u32*>(base + L.thist), lrun, ctl, sms, st);
-        ktri::launch_order_tiles(fo, head, dplus, n, mtiles, &ctl->medium_tiles, opt.segment,
-                                 by_cost ? ktri::TILE_BY_COST : ktri::TILE_BY_DEGREE, HUB, keys,
-                                 reinterpret_cast<u32*>(base + L.thist), mrun, ctl, sms, st);
+        ktri::launch_order_tiles(
+            fo, head, dplus, n,
+            {{{true, ltiles, &ctl->large_tiles, by_cost ? ktri::TILE_BY_COST : ktri::TILE_BY_VERTEX, keys + tcap, lrun},
+              {false, mtiles, &ctl->medium_tiles, by_cost ? ktri::TILE_BY_COST : ktri::TILE_BY_DEGREE, keys, mrun}}},
+            opt.segment, HUB, hist, ctl, sms, st);
     }
     if (!autom) {
         ktri::launch_sort_lists<OffT>(n, vdesc, headp, reinterpret_cast<u32*>(base + L.mid),

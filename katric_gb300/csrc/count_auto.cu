@@ -840,7 +840,7 @@ __global__ void __launch_bounds__(BLOCK) k_count_large(const u64* __restrict__ f
         __syncthreads();
         const u64 t = s_t;
         if (t >= ntiles) break;
-        timed_out = large_tile<BLOCK, CAP, OffT>(smem, s_bar, ltiles[t], fo, head, n, vdesc, headp, seg, cnt,
+        timed_out = large_tile<BLOCK, CAP, OffT>(smem, s_bar, ltiles[tile_at(true, t)], fo, head, n, vdesc, headp, seg, cnt,
                                                  first_wait_polls, phase, inflight, local_total, dup);
         if (timed_out) break;
     }
@@ -1086,7 +1086,7 @@ __global__ void __launch_bounds__(BLOCK, 4)
         if (lane == 0) t = atomicAdd(&ctl->medium_next, 1ull);
         t = __shfl_sync(0xFFFFFFFFu, t, 0);
         if (t >= ntiles) break;
-        medium_tile<OffT, HUB>(base, top, HUB && t < nl ? ltiles[t] : mtiles[t - nl], fo, head, vdesc, headp, seg, cnt,
+        medium_tile<OffT, HUB>(base, top, HUB && t < nl ? ltiles[tile_at(true, t)] : mtiles[t - nl], fo, head, vdesc, headp, seg, cnt,
                                local_total, dup);
     }
     if (dup) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
@@ -1249,7 +1249,7 @@ __global__ void __launch_bounds__(32 * HUB_WARPS, 1)
         if (lane == 0) t = atomicAdd(&ctl->hub_next, 1ull);
         t = __shfl_sync(FULL, t, 0);
         if (t >= nt) break;
-        const uint2 tl = t < nl ? ltiles[t] : mtiles[t - nl];
+        const uint2 tl = t < nl ? ltiles[tile_at(true, t)] : mtiles[t - nl];
         const u32 x = tl.x;
         const Desc<u32> dx = load_desc(vdesc + x);
         const u32 xh = hub_len<true>(dx.d), xt = list_len<true>(dx.d);
@@ -1684,7 +1684,7 @@ __global__ void __launch_bounds__(ENGINE_BLOCK, 4) k_engine(EngineJob* jobs, u32
             }
         } else {
             const u64 t = u - jb->units_small - jb->units_medium;
-            timed_out = large_tile<BLOCK, LARGE_CAP, u32, true>(smem, s_bar, __ldcg(jb->ltiles + t), jb->fo, jb->head,
+            timed_out = large_tile<BLOCK, LARGE_CAP, u32, true>(smem, s_bar, __ldcg(jb->ltiles + tile_at(true, t)), jb->fo, jb->head,
                                                                 jb->n, vd, jb->headp,
                                                           jb->seg, jb->cnt, COPY_WAIT_POLLS, phase, inflight,
                                                           unused_total, dup);

@@ -118,10 +118,10 @@ __device__ __forceinline__ void chain_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <class Stream, class... P, class... A>
-inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, const Stream& ls,
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, const Stream& ls,
                                   A&&... args) {
     cudaLaunchConfig_t c{};
-    c.gridDim = dim3(grid);
+    c.gridDim = grid;
     c.blockDim = dim3(block);
     c.dynamicSmemBytes = smem;
     c.stream = ls.st;

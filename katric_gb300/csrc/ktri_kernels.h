@@ -117,24 +117,38 @@ u64 orient_tiles(u64 n, u64 nnz);
 void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* deg, const u32* tile_i0, u32* headp,
                    const HubState& hub, u32* dplus, Control* ctl, LaunchStream st, u64 tile_begin = 0,
                    u64 tile_end = ~0ull);
-// Owner tiles: medium owners' tiles are written to mtiles, large owners' to ltiles (each
-// array holds large_tile_capacity entries).
+// Owner tiles: medium owners' tiles are written from mtiles on, large owners' from ltiles backwards
+// (mtiles + large_tile_capacity: an owner has one kind, so both fit one array).  order_hist: the histograms launch_order_tiles uses next,
+// or null.
 template <typename OffT, bool HUB>
 void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, const HubState& hub, uint2* mtiles,
-                 uint2* ltiles, u32 small_d, u32 medium_d, u32 seg, Control* ctl, int num_sms, LaunchStream st);
+                 uint2* ltiles, u32 small_d, u32 medium_d, u32 seg, u32* order_hist, Control* ctl, int num_sms,
+                 LaunchStream st);
 
-// Owner tiles reordered (*count tiles on the device) by a counting sort on a 12-bit key:
-// TILE_BY_VERTEX, the first vertex each segment streams (tiles that run together then stream
-// from the same region of the list array); TILE_BY_DEGREE, the owner's out-degree, largest
-// first; TILE_BY_COST, the tile's streamed entries (k_tile_cost writes them, log-scaled, into
-// keys), heaviest first.  keys holds every tile's key between the two passes, so it needs the
-// tiles' capacity in u32; hist needs tile_order_scratch_words() u32, sorted the same capacity
-// as tiles.
+// Both lists of owner tiles reordered (*count tiles on the device) by a counting sort on a 12-bit
+// key, in the same launches: TILE_BY_VERTEX, the first vertex each segment streams (tiles that run
+// together then stream from the same region of the list array); TILE_BY_DEGREE, the owner's
+// out-degree, largest first; TILE_BY_COST (of both lists or none), the tile's streamed entries
+// (k_tile_cost writes them, log-scaled, into keys), heaviest first.  keys holds every tile's key
+// between the passes (laid out as the tiles are, in u32), sorted receives them (as they are too);
+// hist needs tile_order_scratch_words() u32, which launch_desc zeroes.
 enum : u32 { TILE_BY_VERTEX = 0, TILE_BY_DEGREE = 1, TILE_BY_COST = 2 };
+// Where entry t of a list is, for lists that run backwards from the address of their end.
+__host__ __device__ __forceinline__ long long tile_at(bool back, u64 t) { return back ? -1 - (long long)t : (long long)t; }
+struct TileOrder {
+    bool back;  // tiles, keys and sorted run backwards
+    const uint2* tiles;
+    const unsigned long long* count;
+    u32 mode;
+    u32* keys;
+    uint2* sorted;
+};
+struct TileOrders {
+    TileOrder of[2];
+};
 u64 tile_order_scratch_words();
-void launch_order_tiles(const u64* fo, const u32* head, const u32* dplus, u64 n, const uint2* tiles,
-                        const unsigned long long* count, u32 seg, u32 mode, bool hub, u32* keys, u32* hist,
-                        uint2* sorted, Control* ctl, int num_sms, LaunchStream st);
+void launch_order_tiles(const u64* fo, const u32* head, const u32* dplus, u64 n, const TileOrders& orders, u32 seg,
+                        bool hub, u32* hist, Control* ctl, int num_sms, LaunchStream st);
 
 // The counting kernels of KTRI_METHOD_AUTO.  partials needs count_grid_auto entries.  The hub
 // kernel runs where hub is set (HUB, 32-bit descriptors only).

@@ -13,6 +13,8 @@
 
 namespace ktri {
 
+constexpr u32 TILE_BUCKETS = 4096;  // keys of a tile order
+
 // deg[v] = first_out[v+1] - first_out[v]; zero the out-degrees and the per-vertex counts.
 // Also tabulates the merge-path tile boundaries: vertex v covers the diagonals
 // [first_out[v] + v, first_out[v+1] + v] (its slots and its end event), so every boundary
@@ -128,18 +130,21 @@ __global__ void k_hub_place(u64 n, const u32* __restrict__ deg, u32* __restrict_
 __global__ void k_hub_rank(const u32* __restrict__ hub_bins, const uint2* __restrict__ hub_tmp, u32* __restrict__ hub_ids,
                            u32* __restrict__ key, const Control* ctl) {
     chain_begin();
-    const u32 p = blockIdx.x * blockDim.x + threadIdx.x;
+    const u32 p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (p >= ctl->hubs || (ctl->err & DEV_ERR_MASK)) return;
     const uint2 me = hub_tmp[p];
     const u32 b = degree_bin(me.y);
     const u32 first = hub_bins[2 * HUB_BINS + b], count = hub_bins[b];
-    u32 r = first;
-    for (u32 q = first; q < first + count; ++q) {
+    u32 higher = 0;
+    for (u32 q = first + lane; q < first + count; q += 32) {
         const uint2 o = hub_tmp[q];
-        if (o.y > me.y || (o.y == me.y && o.x > me.x)) ++r;
+        if (o.y > me.y || (o.y == me.y && o.x > me.x)) ++higher;
     }
-    hub_ids[r] = me.x;
-    key[me.x] = HUB_FLAG | (HUB_H - 1 - r);
+    const u32 r = first + __reduce_add_sync(0xFFFFFFFFu, higher);
+    if (lane == 0) {
+        hub_ids[r] = me.x;
+        key[me.x] = HUB_FLAG | (HUB_H - 1 - r);
+    }
 }
 
 // Orientation of one merge-path tile of W = 32 * IPT diagonals per warp.  The tile holds the
@@ -374,20 +379,30 @@ __global__ void __launch_bounds__(BLOCK, ORIENT_BLOCKS) k_orient(const u64* __re
 }
 
 // Out-list descriptors, and the (owner, segment) tiles of owners above the small
-// out-degree threshold.
+// out-degree threshold.  The slots in the tile lists and in the list of long hub lists are reserved
+// once per block and 256 vertices: with an atomic per warp the counters' L2 slice was 70 % busy (RMAT
+// n = 2^24: 470 us, 338 us so).  order_hist: the tile orders' histograms, zeroed here.
+constexpr int DESC_BLOCK = 256;
 template <typename OffT, bool HUB>
-__global__ void k_desc(const u64* __restrict__ fo, u64 n, const u32* __restrict__ dplus, Desc<OffT>* __restrict__ vdesc,
-                       u16* __restrict__ hubp, u32* __restrict__ top_info, u32* __restrict__ top_long,
-                       uint2* __restrict__ mtiles, uint2* __restrict__ ltiles, u32 small_d, u32 medium_d, u32 seg,
-                       Control* ctl) {
+__global__ void __launch_bounds__(DESC_BLOCK) k_desc(const u64* __restrict__ fo, u64 n, const u32* __restrict__ dplus,
+                                                     Desc<OffT>* __restrict__ vdesc, u16* __restrict__ hubp,
+                                                     u32* __restrict__ top_info, u32* __restrict__ top_long,
+                                                     uint2* __restrict__ mtiles, uint2* __restrict__ ltiles,
+                                                     u32 small_d, u32 medium_d, u32 seg, u32* __restrict__ order_hist,
+                                                     Control* ctl) {
     chain_begin();
+    constexpr int WARPS = DESC_BLOCK / 32;
+    __shared__ u32 s_sum[3][WARPS];  // of each warp: medium tiles, large tiles, long hub lists
+    __shared__ u64 s_at[3][WARPS];   // where its entries go
     if (ctl->err & DEV_ERR_MASK) return;
-    const int lane = threadIdx.x & 31;
-    const u64 warp_global = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
-    for (u64 base = warp_global * 32; base < n; base += nwarps * 32) {
-        const u64 v = base + lane;
-        u32 nm = 0, nl = 0;
+    const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const u64 stride = (u64)gridDim.x * DESC_BLOCK;
+    if (order_hist)
+        for (u64 k = (u64)blockIdx.x * DESC_BLOCK + threadIdx.x; k < 2 * TILE_BUCKETS; k += stride) order_hist[k] = 0;
+    for (u64 base = (u64)blockIdx.x * DESC_BLOCK; base < n; base += stride) {
+        const u64 v = base + threadIdx.x;
+        u32 nt = 0;
+        bool large = false, is_long = false;
         if (v < n) {
             const u64 a = fo[v], b = fo[v + 1];
             const u32 d = dplus[v];
@@ -400,39 +415,46 @@ __global__ void k_desc(const u64* __restrict__ fo, u64 n, const u32* __restrict_
                 const u64 hs = hub_start(list_start(ds), v);
                 for (u32 k = hub_len<HUB>(d); k & 7u; ++k) hubp[hs + k] = (u16)HUB_PAD;
                 top_info[v] = 0;
+                is_long = hub_len<HUB>(d) > HUB_TOP_LIST;
             }
             // no tiles at all without tile arrays (the reference strategies pass none)
-            const bool tiled = mtiles && ltiles && list_len<HUB>(d) > small_d;
-            const u32 nt = tiled ? (u32)((b - a + seg - 1) / seg) : 0u;
-            if (list_len<HUB>(d) > medium_d) nl = nt;
-            else nm = nt;
+            if (mtiles && ltiles && list_len<HUB>(d) > small_d) nt = (u32)((b - a + seg - 1) / seg);
+            large = list_len<HUB>(d) > medium_d;
         }
-        if constexpr (HUB) {
-            const bool is_long = v < n && hub_len<HUB>(dplus[v < n ? v : 0]) > HUB_TOP_LIST;
-            const u32 ball = __ballot_sync(0xFFFFFFFFu, is_long);
-            u32 at = 0;
-            if (lane == 0 && ball) at = atomicAdd(&ctl->hub_long, (u32)__popc(ball));
-            at = __shfl_sync(0xFFFFFFFFu, at, 0);
-            if (is_long) top_long[at + __popc(ball & ((1u << lane) - 1))] = (u32)v;
-        }
-        // warp-aggregated reservation of tile slots, one list per owner class
+        if (!__syncthreads_or(nt || is_long)) continue;
+        u32 before[2], mine[2] = {large ? 0 : nt, large ? nt : 0};
 #pragma unroll
         for (int cls = 0; cls < 2; ++cls) {
-            const u32 mine = cls == 0 ? nm : nl;
-            u32 incl = mine;
+            u32 incl = mine[cls];
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                u32 y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                const u32 y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
                 if (lane >= o) incl += y;
             }
-            const u32 wsum = __shfl_sync(0xFFFFFFFFu, incl, 31);
-            u64 wbase = 0;
-            if (lane == 31 && wsum) wbase = atomicAdd(cls == 0 ? &ctl->medium_tiles : &ctl->large_tiles, (u64)wsum);
-            wbase = __shfl_sync(0xFFFFFFFFu, wbase, 31);
-            const u64 my = wbase + incl - mine;
-            uint2* out = cls == 0 ? mtiles : ltiles;
-            for (u32 s = 0; s < mine; ++s) out[my + s] = make_uint2((u32)v, s);
+            if (lane == 31) s_sum[cls][wid] = incl;
+            before[cls] = incl - mine[cls];
         }
+        const u32 longs = __ballot_sync(0xFFFFFFFFu, is_long);
+        if (lane == 0) s_sum[2][wid] = __popc(longs);
+        __syncthreads();
+        if (threadIdx.x < 3) {
+            u64 total = 0;
+            for (int w = 0; w < WARPS; ++w) {
+                s_at[threadIdx.x][w] = total;
+                total += s_sum[threadIdx.x][w];
+            }
+            u64 at = 0;
+            if (total)
+                at = threadIdx.x == 0   ? atomicAdd(&ctl->medium_tiles, total)
+                     : threadIdx.x == 1 ? atomicAdd(&ctl->large_tiles, total)
+                                        : atomicAdd(&ctl->hub_long, (u32)total);
+            for (int w = 0; w < WARPS; ++w) s_at[threadIdx.x][w] += at;
+        }
+        __syncthreads();
+        if (HUB && is_long) top_long[s_at[2][wid] + __popc(longs & ((1u << lane) - 1))] = (u32)v;
+        const u64 my = s_at[large][wid] + (large ? before[1] : before[0]);
+        uint2* out = large ? ltiles : mtiles;
+        for (u32 s = 0; s < nt; ++s) out[tile_at(large, my + s)] = make_uint2((u32)v, s);
     }
 }
 
@@ -491,16 +513,15 @@ __global__ void __launch_bounds__(TOPS_BLOCK) k_hub_tops(const Desc<u32>* __rest
 // on the top id bits).  Input adjacency lists are mostly in id order, so tiles that run at the
 // same time then stream out-lists from the same region of the list array, and the L2 cache
 // serves the repeats.  Counts do not depend on the order.
-constexpr u32 TILE_BUCKETS = 4096;
 
 // Sort key of a tile (TILE_BY_VERTEX): the top id bits of the first vertex its segment
 // streams; (TILE_BY_DEGREE): the owner's out-degree, largest first (longest tiles first);
-// (TILE_BY_COST): the key k_tile_cost left in keys[t].
+// (TILE_BY_COST): the key k_tile_cost left.
 __device__ __forceinline__ u32 tile_key(const u64* fo, const u32* head, const u32* dplus, uint2 tl, u32 seg,
-                                        u32 shift, u32 mode, bool hub, const u32* keys, u64 t) {
+                                        u32 shift, u32 mode, bool hub, u32 cost_key) {
     u32 key;
     if (mode == TILE_BY_COST) {
-        key = keys[t];
+        key = cost_key;
     } else if (mode == TILE_BY_DEGREE) {
         const u32 d = hub ? list_len<true>(dplus[tl.x]) : dplus[tl.x];
         key = d >= TILE_BUCKETS ? 0u : TILE_BUCKETS - 1 - d;
@@ -516,15 +537,15 @@ __device__ __forceinline__ u32 tile_key(const u64* fo, const u32* head, const u3
 // restated for owner-side tiles.  One warp per tile; the key orders heaviest first on a
 // log scale (7 fractional bits).
 __global__ void k_tile_cost(const u64* __restrict__ fo, const u32* __restrict__ head, const u32* __restrict__ dplus,
-                            const uint2* __restrict__ tiles, const unsigned long long* count, u32 seg,
-                            bool hub, u32* __restrict__ keys, Control* ctl) {
+                            TileOrders orders, u32 seg, bool hub, Control* ctl) {
     chain_begin();
     if (ctl->err & DEV_ERR_MASK) return;
-    const u64 nt = *(volatile const unsigned long long*)count;
+    const TileOrder& o = orders.of[blockIdx.y];
+    const u64 nt = *(volatile const unsigned long long*)o.count;
     const int lane = threadIdx.x & 31;
     const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
     for (u64 t = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += nwarps) {
-        const uint2 tl = tiles[t];
+        const uint2 tl = o.tiles[tile_at(o.back, t)];
         const u64 x = tl.x;
         const u32 dx = hub ? list_len<true>(dplus[x]) : dplus[x];
         const u64 a = fo[x] + (u64)tl.y * seg, e1 = fo[x + 1], b = a + seg < e1 ? a + seg : e1;
@@ -535,13 +556,13 @@ __global__ void k_tile_cost(const u64* __restrict__ fo, const u32* __restrict__ 
             if (dy > 0 && key_less(dy, y, dx, x)) cost += dy;
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) cost += __shfl_down_sync(0xFFFFFFFFu, cost, o);
+        for (int k = 16; k > 0; k >>= 1) cost += __shfl_down_sync(0xFFFFFFFFu, cost, k);
         if (lane == 0) {
             const u32 c = cost > 0xFFFFFFFFull ? 0xFFFFFFFFu : (u32)cost;
             const u32 lg = 31 - __clz(c | 1u);
             const u32 frac = lg >= 7 ? (c >> (lg - 7)) & 0x7Fu : (c << (7 - lg)) & 0x7Fu;
             const u32 bucket = lg * 128 + frac;  // < 32 * 128 = TILE_BUCKETS
-            keys[t] = TILE_BUCKETS - 1 - bucket;
+            o.keys[tile_at(o.back, t)] = TILE_BUCKETS - 1 - bucket;
         }
     }
 }
@@ -561,23 +582,24 @@ __device__ __forceinline__ void tile_chunk(u64 nt, u64& t0, u64& t1) {
 constexpr int TILE_ORDER_BLOCK = 256;
 __global__ void __launch_bounds__(TILE_ORDER_BLOCK) k_tile_hist(const u64* __restrict__ fo,
                                                                 const u32* __restrict__ head,
-                                                                const u32* __restrict__ dplus,
-                                                                const uint2* __restrict__ tiles,
-                                                                const unsigned long long* count, u32 seg, u32 shift,
-                                                                u32 mode, bool hub, u32* __restrict__ keys, u32* hist,
+                                                                const u32* __restrict__ dplus, TileOrders orders,
+                                                                u32 seg, u32 shift, bool hub, u32* hist,
                                                                 Control* ctl) {
     chain_begin();
     __shared__ u32 s_cnt[TILE_BUCKETS];
     if (ctl->err & DEV_ERR_MASK) return;
-    const u64 nt = *(volatile const unsigned long long*)count;
+    const TileOrder& o = orders.of[blockIdx.y];
+    hist += blockIdx.y * TILE_BUCKETS;
+    const u64 nt = *(volatile const unsigned long long*)o.count;
     u64 t0, t1;
     tile_chunk(nt, t0, t1);
     if (t0 == t1) return;
     for (u32 k = threadIdx.x; k < TILE_BUCKETS; k += TILE_ORDER_BLOCK) s_cnt[k] = 0;
     __syncthreads();
     for (u64 t = t0 + threadIdx.x; t < t1; t += TILE_ORDER_BLOCK) {
-        const u32 key = tile_key(fo, head, dplus, tiles[t], seg, shift, mode, hub, keys, t);
-        if (mode != TILE_BY_COST) keys[t] = key;
+        const long long at = tile_at(o.back, t);
+        const u32 key = tile_key(fo, head, dplus, o.tiles[at], seg, shift, o.mode, hub, o.keys[at]);
+        if (o.mode != TILE_BY_COST) o.keys[at] = key;
         atomicAdd(&s_cnt[key], 1u);
     }
     __syncthreads();
@@ -592,6 +614,7 @@ __global__ void __launch_bounds__(TILE_SCAN_BLOCK) k_tile_scan(u32* hist, Contro
     constexpr int PER = TILE_BUCKETS / TILE_SCAN_BLOCK;
     __shared__ u32 s_warp[TILE_SCAN_BLOCK / 32];
     if (ctl->err & DEV_ERR_MASK) return;
+    hist += blockIdx.x * TILE_BUCKETS;
     u32 v[PER], t = 0;
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
@@ -610,47 +633,46 @@ __global__ void __launch_bounds__(TILE_SCAN_BLOCK) k_tile_scan(u32* hist, Contro
 // Scatter of the tiles into key order (cursor = the scanned histogram).  Each block counts its
 // chunk's keys again, reserves one range per key present with one atomic, and hands out the
 // positions inside its ranges with shared-memory atomics.
-__global__ void __launch_bounds__(TILE_ORDER_BLOCK) k_tile_scatter(const uint2* __restrict__ tiles,
-                                                                   const unsigned long long* count,
-                                                                   const u32* __restrict__ keys, u32* cursor,
-                                                                   uint2* __restrict__ sorted, Control* ctl) {
+__global__ void __launch_bounds__(TILE_ORDER_BLOCK) k_tile_scatter(TileOrders orders, u32* cursor, Control* ctl) {
     chain_begin();
     __shared__ u32 s_pos[TILE_BUCKETS];
     if (ctl->err & DEV_ERR_MASK) return;
-    const u64 nt = *(volatile const unsigned long long*)count;
+    const TileOrder& o = orders.of[blockIdx.y];
+    cursor += blockIdx.y * TILE_BUCKETS;
+    const u64 nt = *(volatile const unsigned long long*)o.count;
     u64 t0, t1;
     tile_chunk(nt, t0, t1);
     if (t0 == t1) return;
     for (u32 k = threadIdx.x; k < TILE_BUCKETS; k += TILE_ORDER_BLOCK) s_pos[k] = 0;
     __syncthreads();
-    for (u64 t = t0 + threadIdx.x; t < t1; t += TILE_ORDER_BLOCK) atomicAdd(&s_pos[keys[t]], 1u);
+    for (u64 t = t0 + threadIdx.x; t < t1; t += TILE_ORDER_BLOCK) atomicAdd(&s_pos[o.keys[tile_at(o.back, t)]], 1u);
     __syncthreads();
     for (u32 k = threadIdx.x; k < TILE_BUCKETS; k += TILE_ORDER_BLOCK) {
         const u32 c = s_pos[k];
         if (c) s_pos[k] = atomicAdd(&cursor[k], c);
     }
     __syncthreads();
-    for (u64 t = t0 + threadIdx.x; t < t1; t += TILE_ORDER_BLOCK) sorted[atomicAdd(&s_pos[keys[t]], 1u)] = tiles[t];
+    for (u64 t = t0 + threadIdx.x; t < t1; t += TILE_ORDER_BLOCK) {
+        const long long at = tile_at(o.back, t);
+        o.sorted[tile_at(o.back, atomicAdd(&s_pos[o.keys[at]], 1u))] = o.tiles[at];
+    }
 }
 
 // ---- launchers ------------------------------------------------------------------------
 
-u64 tile_order_scratch_words() { return TILE_BUCKETS; }
+u64 tile_order_scratch_words() { return 2ull * TILE_BUCKETS; }
 
-void launch_order_tiles(const u64* fo, const u32* head, const u32* dplus, u64 n, const uint2* tiles,
-                        const unsigned long long* count, u32 seg, u32 mode, bool hub, u32* keys, u32* hist,
-                        uint2* sorted, Control* ctl, int num_sms, LaunchStream st) {
+void launch_order_tiles(const u64* fo, const u32* head, const u32* dplus, u64 n, const TileOrders& orders, u32 seg,
+                        bool hub, u32* hist, Control* ctl, int num_sms, LaunchStream st) {
     if (n == 0) return;
     u32 bits = 0;
     while ((1ull << bits) < n) ++bits;
     const u32 shift = bits > 12 ? bits - 12 : 0;
-    cudaMemsetAsync(hist, 0, sizeof(u32) * TILE_BUCKETS, st);
-    if (mode == TILE_BY_COST)
-        launch_chained(k_tile_cost, num_sms * 8, 256, 0, st, fo, head, dplus, tiles, count, seg, hub, keys, ctl);
-    launch_chained(k_tile_hist, num_sms * 4, TILE_ORDER_BLOCK, 0, st, fo, head, dplus, tiles, count, seg, shift, mode, hub, keys,
-                                                          hist, ctl);
-    launch_chained(k_tile_scan, 1, TILE_SCAN_BLOCK, 0, st, hist, ctl);
-    launch_chained(k_tile_scatter, num_sms * 4, TILE_ORDER_BLOCK, 0, st, tiles, count, keys, hist, sorted, ctl);
+    if (orders.of[0].mode == TILE_BY_COST)
+        launch_chained(k_tile_cost, dim3(num_sms * 8, 2), 256, 0, st, fo, head, dplus, orders, seg, hub, ctl);
+    launch_chained(k_tile_hist, dim3(num_sms * 4, 2), TILE_ORDER_BLOCK, 0, st, fo, head, dplus, orders, seg, shift, hub, hist, ctl);
+    launch_chained(k_tile_scan, 2, TILE_SCAN_BLOCK, 0, st, hist, ctl);
+    launch_chained(k_tile_scatter, dim3(num_sms * 4, 2), TILE_ORDER_BLOCK, 0, st, orders, hist, ctl);
 }
 
 void launch_prep(const u64* fo, u64 n, u64 nnz, u32* deg, u32* dplus, u64* cnt, u32* tile_i0, const HubState& hub,
@@ -665,7 +687,7 @@ void launch_prep(const u64* fo, u64 n, u64 nnz, u32* deg, u32* dplus, u64* cnt, 
     }
     launch_chained(k_prep<true>, grid, PREP_BLOCK, 0, st, fo, n, nnz, deg, dplus, cnt, tile_i0, hub.bins, ctl);
     launch_chained(k_hub_place, grid, 256, 0, st, n, deg, hub.bins, hub.tmp, ctl);
-    launch_chained(k_hub_rank, HUB_H / 128, 128, 0, st, hub.bins, hub.tmp, hub.ids, deg, ctl);
+    launch_chained(k_hub_rank, HUB_H / 8, 256, 0, st, hub.bins, hub.tmp, hub.ids, deg, ctl);
 }
 
 void launch_hub_tops(const void* vdesc, const HubState& hub, Control* ctl, int num_sms, LaunchStream st) {
@@ -696,17 +718,17 @@ void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* de
 
 template <typename OffT, bool HUB>
 void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, const HubState& hub, uint2* mtiles, uint2* ltiles, u32 small_d,
-                 u32 medium_d, u32 seg, Control* ctl, int num_sms, LaunchStream st) {
+                 u32 medium_d, u32 seg, u32* order_hist, Control* ctl, int num_sms, LaunchStream st) {
     if (n == 0) return;
-    u64 blocks = (n + 255) / 256;
+    u64 blocks = (n + DESC_BLOCK - 1) / DESC_BLOCK;
     u64 cap = (u64)num_sms * 8;
-    launch_chained(k_desc<OffT, HUB>, (unsigned)(blocks < cap ? blocks : cap), 256, 0, st, 
-        fo, n, dplus, reinterpret_cast<Desc<OffT>*>(vdesc), hub.lists, hub.top_info, hub.top_long, mtiles, ltiles, small_d, medium_d, seg, ctl);
+    launch_chained(k_desc<OffT, HUB>, (unsigned)(blocks < cap ? blocks : cap), DESC_BLOCK, 0, st,
+        fo, n, dplus, reinterpret_cast<Desc<OffT>*>(vdesc), hub.lists, hub.top_info, hub.top_long, mtiles, ltiles, small_d, medium_d, seg, order_hist, ctl);
 }
 
 #define KTRI_INST(OffT, HUB)                                                                                     \
     template void launch_desc<OffT, HUB>(const u64*, u64, const u32*, void*, const HubState&, uint2*, uint2*,    \
-                                         u32, u32, u32, Control*, int, LaunchStream);
+                                         u32, u32, u32, u32*, Control*, int, LaunchStream);
 KTRI_INST(u32, false)
 KTRI_INST(u32, true)
 KTRI_INST(u64, false)
