@@ -57,9 +57,10 @@ KERNELS_PER_STEP = 7  # k_prep, k_orient, k_desc, k_count_small, k_count_medium,
 
 
 def kernels_per_count(nnz: int) -> int:
-    """Kernels of one AUTO count: the seven above, plus k_tile_hist / k_tile_scan /
-    k_tile_scatter for the large and the medium tiles from 2^20 adjacency entries on."""
-    return KERNELS_PER_STEP + (6 if nnz >= (1 << 20) else 0)
+    """Kernels of one AUTO count: the seven above, plus k_tile_hist / k_tile_scan / k_tile_scatter from
+    2^20 adjacency entries on; from 2^21 on k_hub_place, k_hub_rank, k_hub_tops and k_count_hub
+    run and k_count_large does not."""
+    return KERNELS_PER_STEP + (3 if nnz >= (1 << 20) else 0) + (3 if nnz >= (1 << 21) else 0)
 
 
 def make_graph(name: str):
@@ -416,7 +417,7 @@ def run_batch(args, steps: int, warmup: int, plain_passes: int = 3) -> dict:
         "autotune": tune,
         "triangles_total": int(totals.sum()),
         "totals_match_oracle_fixture": pinned,
-        "gpu_launches": (kernels_per_count(nnz) + 1) * steps,  # the pipeline + k_graph_totals per replay
+        "gpu_launches": kernels_per_count(nnz) * steps,  # per replay, k_graph_totals for k_final
         "clocks": clk,
     }
 
@@ -710,7 +711,7 @@ def main():
                       "count_medium_large": statistics.mean(large_ms), "count_total": k_ms},
         "work": {"wedge_checks": wedge_checks, "oriented_edges": m_oriented, "streamed_entries": streamed},
         "roofline": {"bound": "hbm",
-                     "kernel": "intersection phase (k_count_small + k_count_medium + k_count_large + k_final)",
+                     "kernel": "intersection phase (k_count_small, k_count_hub + k_count_medium or k_count_medium + k_count_large, k_final)",
                      "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
                      "peak_kind": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
                      else "fallback 6.8 TB/s",
