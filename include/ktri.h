@@ -119,7 +119,9 @@ int ktri_ctx_destroy(ktri_ctx* ctx);
 /* Cap on the workspace this context may hold (bytes; 0 = no cap).  Over-budget calls fail
  * with KTRI_ERR_OUT_OF_MEMORY before launching anything. */
 int ktri_ctx_set_memory_budget(ktri_ctx* ctx, uint64_t bytes);
-/* Device bytes a count of a graph with n vertices and nnz entries needs in the workspace. */
+/* Device bytes a count of a graph with n vertices and nnz entries needs in the workspace.  AUTO counts
+ * from 2^21 entries on take about 2.4 bytes per entry and 18 per vertex more (split out-lists) where
+ * the budget and the free memory have room for them. */
 uint64_t ktri_workspace_bytes(uint64_t n, uint64_t nnz, int32_t intersection_method);
 const char* ktri_last_error(const ktri_ctx* ctx);
 int ktri_ctx_stats(ktri_ctx* ctx, ktri_run_stats* out); /* synchronises the context's last stream */

@@ -597,7 +597,15 @@ int order_after_pending(ktri_ctx* ctx, cudaStream_t st) {
         (void)device_status(ctx);
         return KTRI_OK;
     }
-    if (st != ctx->last_stream) KTRI_CK(ctx, cudaStreamWaitEvent(st, ctx->ev[3], 0));
+    // what is captured now runs later, maybe on another stream: the pending call ends first, as seen
+    // from the host
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    const bool asked = cudaStreamIsCapturing(st, &capturing) == cudaSuccess;
+    if (asked && capturing == cudaStreamCaptureStatusNone &&
+        (st == ctx->last_stream || cudaStreamWaitEvent(st, ctx->ev[3], 0) == cudaSuccess))
+        return KTRI_OK;
+    (void)cudaGetLastError();
+    (void)device_status(ctx);
     return KTRI_OK;
 }
 

@@ -812,7 +812,7 @@ void worker_main(ktri_server* s) {
                 s->cv_done.notify_all();
             } else {
                 // Split out-lists where the budget has room beside what is resident: they cost no
-                // graph its place.  (A burst of 30 graphs, 8.3 M entries in its largest batch:
+                // graph its place.  (A burst of 30 graphs, 16 M entries in its largest batch:
                 // 6.7 -> 5.8 ms; the owner tiles of its two large batches took 2.5 ms without, 0.66 ms with.)
                 ktri::ctx_allow_hubs(free_slot->ctx, need + ktri::hub_bytes(n, nnz) + inflight + s->resident_bytes <=
                                                          s->opts.memory_budget);
