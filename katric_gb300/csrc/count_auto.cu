@@ -1414,8 +1414,9 @@ __global__ void __launch_bounds__(1024) k_final(const u64* __restrict__ partials
 // all inside one graph, so a graph's total is the sum of its per-vertex counts over three.
 // `parts` blocks share a graph (totals are zeroed by the caller when there are several): few graphs
 // would otherwise leave the largest to one block (11 graphs with one of 2.7 M vertices: 711 us by
-// one block each, 52 us by 64).  A part's sum need not be a multiple of three, but the sum of all is,
-// so each part is multiplied by the inverse of three modulo 2^64.
+// one block each, 21 us by 64 with eight loads in flight per thread; 512 graphs 57 -> 46 us).  A part's
+// sum need not be a multiple of three, but the sum of all is, so each part is multiplied by the
+// inverse of three modulo 2^64.
 __global__ void __launch_bounds__(256) k_graph_totals(const u64* __restrict__ cnt, const u64* __restrict__ graph_first,
                                                       u64 num_graphs, u64 n, u64* __restrict__ totals, u32 parts,
                                                       Control* ctl) {
@@ -1429,9 +1430,15 @@ __global__ void __launch_bounds__(256) k_graph_totals(const u64* __restrict__ cn
         const bool ok = a <= b && b <= n;
         u64 s = 0;
         if (ok) {
+            // eight loads in flight per thread
             const u64 step = 256 * (u64)parts;
-#pragma unroll 4
-            for (u64 v = a + part * 256 + threadIdx.x; v < b; v += step) s += cnt[v];
+            for (u64 v = a + part * 256 + threadIdx.x; v < b; v += 8 * step) {
+                u64 c[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) c[k] = v + k * step < b ? cnt[v + k * step] : 0;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) s += c[k];
+            }
         }
         s = block_sum_u64<256>(s, s_red);
         if (threadIdx.x == 0) {
