@@ -590,7 +590,8 @@ int device_status(ktri_ctx* ctx) {
 
 // A new device call may follow one whose status was not read: it replaces that call's status, and
 // its work is ordered after that call's (they share the workspace) on the device, without the host
-// waiting.
+// waiting.  The event is waited for on equal stream handles too: cudaStreamPerThread is one handle for
+// another stream in every thread, and a destroyed stream's handle may come back for a new one.
 int order_after_pending(ktri_ctx* ctx, cudaStream_t st) {
     if (!ctx->pending) return KTRI_OK;
     if (!ctx->have_events) {
@@ -601,8 +602,7 @@ int order_after_pending(ktri_ctx* ctx, cudaStream_t st) {
     // from the host
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     const bool asked = cudaStreamIsCapturing(st, &capturing) == cudaSuccess;
-    if (asked && capturing == cudaStreamCaptureStatusNone &&
-        (st == ctx->last_stream || cudaStreamWaitEvent(st, ctx->ev[3], 0) == cudaSuccess))
+    if (asked && capturing == cudaStreamCaptureStatusNone && cudaStreamWaitEvent(st, ctx->ev[3], 0) == cudaSuccess)
         return KTRI_OK;
     (void)cudaGetLastError();
     (void)device_status(ctx);
