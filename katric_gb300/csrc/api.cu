@@ -609,6 +609,13 @@ int order_after_pending(ktri_ctx* ctx, cudaStream_t st) {
     return KTRI_OK;
 }
 
+// A call that starts nothing on the workspace leaves nothing behind for the next call to wait for, so
+// it ends the pending call from the host.
+void end_pending(ktri_ctx* ctx) {
+    if (ctx->pending) (void)device_status(ctx);
+    ctx->pending = false;
+}
+
 std::mutex g_default_mu;
 std::map<int, ktri_ctx*> g_default;
 
@@ -840,8 +847,8 @@ int ktri_count_csr_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint
     rc = order_after_pending(ctx, st);  // the previous call's status was not collected; the new call proceeds
     if (rc) return rc;
     if (n == 0) {
+        end_pending(ctx);
         KTRI_CK(ctx, cudaMemsetAsync(d_total, 0, sizeof(u64), st));
-        ctx->pending = false;
         ctx->stats = ktri_run_stats{};
         return KTRI_OK;
     }
@@ -1315,8 +1322,8 @@ int ktri_count_dag_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint
     rc = order_after_pending(ctx, st);
     if (rc) return rc;
     if (n == 0) {
+        end_pending(ctx);
         KTRI_CK(ctx, cudaMemsetAsync(d_total, 0, sizeof(u64), st));
-        ctx->pending = false;
         ctx->stats = ktri_run_stats{};
         return KTRI_OK;
     }
@@ -1449,8 +1456,8 @@ int ktri_count_batch_device(ktri_ctx* ctx, const uint64_t* d_first_out, const ui
     rc = order_after_pending(ctx, st);
     if (rc) return rc;
     if (n_total == 0) {
+        end_pending(ctx);
         if (num_graphs) KTRI_CK(ctx, cudaMemsetAsync(d_totals, 0, sizeof(u64) * num_graphs, st));
-        ctx->pending = false;
         return KTRI_OK;
     }
     const Layout L = pick_layout(ctx, n_total, nnz_total, opt, false, true);
