@@ -210,12 +210,16 @@ int ensure_chunk_events(ktri_ctx* ctx, size_t count) {
     return KTRI_OK;
 }
 
+int device_status(ktri_ctx* ctx);
+
 int ensure_ws(ktri_ctx* ctx, size_t bytes) {
     if (ctx->budget && bytes > ctx->budget)
         return set_error(ctx, KTRI_ERR_OUT_OF_MEMORY,
                          "workspace of " + std::to_string(bytes) + " bytes exceeds the memory budget of " +
                              std::to_string(ctx->budget));
     if (bytes <= ctx->ws_bytes) return KTRI_OK;
+    if (ctx->pending) (void)device_status(ctx);  // its control block goes with the old workspace
+    ctx->pending = false;
     if (ctx->ws) {
         KTRI_CK(ctx, cudaStreamSynchronize(ctx->stream));
         cudaFree(ctx->ws);  // waits for the work still using the old workspace

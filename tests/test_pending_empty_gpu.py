@@ -1,10 +1,11 @@
-"""A graph without vertices after an unread device call (needs a GB300): it starts nothing on the
-context's workspace, and the unread call still ends before the next one takes it."""
+"""Calls after an unread device call that start nothing on the context's workspace (needs a GB300): a
+graph without vertices, and a call that is refused for its size.  The unread call still ends before
+the next one takes the workspace, and its status is not read from a workspace that is gone."""
 import numpy as np
 import pytest
 import torch
 
-from katric_gb300 import Graph, TriangleCounter
+from katric_gb300 import Graph, KtriError, TriangleCounter
 
 pytestmark = pytest.mark.gpu
 
@@ -55,3 +56,17 @@ def test_empty_call_between_two_counts(graphs, empty):
                 assert np.array_equal(dev[i][3].cpu().numpy().view(np.uint64), pv)
                 dev[i][3].zero_()
             assert host[0] == graphs[2][1][0] and np.array_equal(host[1], graphs[2][1][1])
+
+
+def test_refused_size_after_an_unread_call(graphs):
+    (g, (total, pv)), (fo, hd, t, p) = graphs[1], on_device(graphs[1][0])
+    torch.cuda.synchronize()
+    with TriangleCounter(0) as ctr:
+        ctr.count_device(fo.data_ptr(), hd.data_ptr(), g.n, g.nnz, t.data_ptr(), p.data_ptr())
+        with pytest.raises(KtriError):  # a workspace of terabytes
+            ctr.count_device(fo.data_ptr(), hd.data_ptr(), g.n, 1 << 41, t.data_ptr(), p.data_ptr())
+        ctr.check()
+        assert int(t[0]) == total and np.array_equal(p.cpu().numpy().view(np.uint64), pv)
+        ctr.count_device(fo.data_ptr(), hd.data_ptr(), g.n, g.nnz, t.data_ptr(), p.data_ptr())
+        ctr.check()
+        assert int(t[0]) == total
