@@ -8,8 +8,9 @@
 // ordinary pipeline, under its own (degree, id) orientation.
 //
 // Vertex v's undirected list is its out-list (in the given order) followed by its in-list
-// (in arrival order).  Entries that are out of range or self-loops are copied into the out
-// part as they are, so the pipeline's validation reports them; they get no in-list entry.
+// (in arrival order).  Entries that are out of range or self-loops are copied into the out part as
+// they are, so the pipeline's validation reports them (out of range: without an in-list entry).
+// Offsets that do not hold m entries read none: their lists come out too long, which it reports.
 #include <algorithm>
 
 #include "ktri.h"
@@ -31,11 +32,15 @@ constexpr u64 SCAN_CHUNK = (u64)SCAN_BLOCK * SCAN_IPT;
 // whole count of a uniform graph.)
 __device__ __forceinline__ u32 count_slot(u32 u, u32 mask) { return (u * 0x9E3779B1u) & mask; }
 
+// Do the offsets hold m entries?  (Any first offset: the lists may lie inside a larger buffer.)
+__device__ __forceinline__ bool holds(const u64* fo, u64 n, u64 m) { return fo[n] - fo[0] == m; }
+
 // Arrivals: pos[e] = the place of entry e among the entries that name the same vertex, in_deg[slot of
 // u] = the number of entries that name u (zeroed by the caller).  The only atomics of the symmetrisation; an
 // entry needs no owner here (a self-loop gets a place like any other and is reported as what it is).
 __global__ void k_dag_arrive(const u64* __restrict__ fo, const u32* __restrict__ head, u64 n, u64 m,
                              u32* __restrict__ in_deg, u32 mask, u32* __restrict__ pos) {
+    if (!holds(fo, n, m)) return;
     const u32* h = head + fo[0];
     const u64 stride = (u64)gridDim.x * blockDim.x;
     for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += 4 * stride) {
@@ -48,10 +53,11 @@ __global__ void k_dag_arrive(const u64* __restrict__ fo, const u32* __restrict__
     }
 }
 
-// |out(v)|; descending offsets give a length that no graph of m edges has.
-__device__ __forceinline__ u64 out_length(const u64* fo, u64 v, u64 m) {
+// |out(v)|; descending offsets, and vertex 0 of offsets that do not hold m entries, give a length that
+// no graph of m edges has.
+__device__ __forceinline__ u64 out_length(const u64* fo, u64 v, u64 n, u64 m) {
     const u64 a = fo[v], b = fo[v + 1];
-    return b >= a ? b - a : 2 * m + 1;
+    return b >= a && (v || holds(fo, n, m)) ? b - a : 2 * m + 1;
 }
 
 // In-place exclusive scan of x[0..len), pass 1: every chunk scanned locally, its sum to sums.
@@ -64,8 +70,12 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_chunks(u64* x, u64 len, u64
     u64 v[SCAN_IPT], t = 0;
 #pragma unroll
     for (int k = 0; k < SCAN_IPT; ++k) {
-        if constexpr (DAG) v[k] = c0 + k + 1 < len ? out_length(fo, c0 + k, m) + in_deg[count_slot((u32)(c0 + k), mask)] : 0ull;
-        else v[k] = c0 + k < len ? x[c0 + k] : 0ull;
+        if constexpr (DAG) {
+            v[k] = 0;
+            if (c0 + k + 1 < len) v[k] = out_length(fo, c0 + k, len - 1, m) + in_deg[count_slot((u32)(c0 + k), mask)];
+        } else {
+            v[k] = c0 + k < len ? x[c0 + k] : 0ull;
+        }
         t += v[k];
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -133,7 +143,7 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_add(u64* x, u64 len, const 
         const u64 s = x[k] + off;
         x[k] = s;
         if constexpr (DAG)
-            if (k + 1 < len) in_start[k] = s + out_length(fo, k, m);
+            if (k + 1 < len) in_start[k] = s + out_length(fo, k, len - 1, m);
     }
 }
 
@@ -160,7 +170,7 @@ constexpr u32 DAG_TILE = 128;
 __global__ void k_dag_scatter(const u64* __restrict__ fo, const u32* __restrict__ head, u64 n, u64 m,
                               const u64* __restrict__ fs, const u64* __restrict__ in_start,
                               const u32* __restrict__ pos, u32* __restrict__ hs) {
-    if (fs[n] != 2 * m) return;
+    if (fs[n] != 2 * m || !holds(fo, n, m)) return;
     const u32 lane = threadIdx.x & 31;
     const u64 warp = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
