@@ -72,7 +72,8 @@ __device__ __forceinline__ Desc<u64> load_desc<u64>(const Desc<u64>* p) {
 // Split out-lists (hubs).  With hubs, an out-list is kept in two parts: the entries that are
 // not hubs (u32 ids, in the gapped array above) and the hubs (u16 hub indices, in a gapped array
 // of their own whose lists start on 16-byte boundaries).  The length word of a descriptor then
-// packs both: hubs in the high half, the others in the low half (both below 2^16, see HUB_MAX_NNZ).
+// packs both: hubs in the high half, the others in the low half (both below 2^16 where no list holds
+// a neighbour twice, see HUB_MAX_NNZ; the orientation reports a half that overflows as a duplicate).
 // The region of x in the hub array starts at align8(oriented start + 4x) and has room for deg(x)
 // entries; the array holds nnz + 7n + 32 entries.  A list is filled up to a
 // multiple of eight entries with HUB_PAD, an index no hub has, so it can be read eight at a time.

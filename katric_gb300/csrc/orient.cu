@@ -312,6 +312,11 @@ __device__ __forceinline__ void orient_tile(OrientWarp<IPT>& sw, const u64* __re
             u32 carry = 0;
             if (a < j0 || b > j1) {
                 if (cnt) carry = atomicAdd(&dplus[v], cnt);
+                if constexpr (HUB) {
+                    // a half of the length word that overflows counts some neighbour twice (HUB_MAX_NNZ)
+                    if ((carry & 0xFFFFu) + (cnt & 0xFFFFu) > 0xFFFFu || (carry >> 16) + (cnt >> 16) > 0xFFFFu)
+                        atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
+                }
             } else {
                 dplus[v] = cnt;
             }
@@ -412,6 +417,8 @@ __global__ void __launch_bounds__(DESC_BLOCK) k_desc(const u64* __restrict__ fo,
             if constexpr (sizeof(OffT) == 8) ds.pad = 0;
             vdesc[v] = ds;
             if constexpr (HUB) {
+                // oriented without hubs: a count past the low half is of a list with duplicates, too
+                if (d > 0xFFFFu && ctl->hubs == 0) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
                 const u64 hs = hub_start(list_start(ds), v);
                 for (u32 k = hub_len<HUB>(d); k & 7u; ++k) hubp[hs + k] = (u16)HUB_PAD;
                 top_info[v] = 0;
