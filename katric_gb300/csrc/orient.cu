@@ -53,6 +53,9 @@ __global__ void __launch_bounds__(PREP_BLOCK) k_prep(const u64* __restrict__ fo,
         if (cnt) cnt[v] = 0;
         if constexpr (HUB) {
             if (d >= HUB_MIN_DEGREE) atomicAdd(&s_bins[degree_bin(d)], 1u);
+            // n is below HUB_MAX_N, so such a list repeats a neighbour; the orientation counts on shorter
+            // ones (keys below HUB_FLAG, list starts at most 2^31 entries before a tile)
+            if (d >= HUB_MAX_N) err |= DEV_ERR_DUPLICATE;
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {

@@ -4,7 +4,7 @@ list is refused as one with duplicates, also where the part's length would wrap 
 import numpy as np
 import pytest
 
-from katric_gb300 import KtriError
+from katric_gb300 import KtriError, TriangleCounter
 
 pytestmark = pytest.mark.gpu
 
@@ -28,3 +28,22 @@ def test_lists_past_the_length_word(counter, k):
     assert len(hd) >= 1 << 21
     with pytest.raises(KtriError, match="duplicate"):
         counter.count(fo, hd)
+
+
+def test_list_longer_than_any_vertex_count():
+    """A list of 2^30 entries and more has none but repeated neighbours: refused before orientation."""
+    torch = pytest.importorskip("torch")
+    d = (1 << 30) + 1000
+    if torch.cuda.mem_get_info()[0] < 24 << 30:
+        pytest.skip("needs 24 GiB of device memory")
+    fo = torch.tensor([0, d, d + 1, d + 2], dtype=torch.int64, device="cuda")
+    head = torch.zeros(d + 2, dtype=torch.int32, device="cuda")
+    head[0:d:2] = 1
+    head[1:d:2] = 2
+    total = torch.zeros(1, dtype=torch.int64, device="cuda")
+    with TriangleCounter(0) as ctr:
+        ctr.count_device(fo.data_ptr(), head.data_ptr(), 3, d + 2, total.data_ptr())
+        with pytest.raises(KtriError, match="duplicate"):
+            ctr.check()
+    del head
+    torch.cuda.empty_cache()
