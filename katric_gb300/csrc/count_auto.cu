@@ -885,12 +885,15 @@ __device__ __forceinline__ void tile_init(u32* base) {
 
 // One (owner, segment) tile of an owner's out-list (HUB: of its entries that are not hubs), counted by
 // one warp in its slice of shared memory.  top: the bit that marks keys, 0 where ids need all bits
-// (a full bucket is then walked past, marked or not).
+// (a full bucket is then walked past, marked or not).  Where some input list does not ascend, the
+// tables are the only check for entries that a list holds twice, so the owner's first tile also looks
+// the keys of later chunks up in each chunk's table (its conditions are read again there: kept in
+// registers they made the kernel spill).
 template <typename OffT, bool HUB, bool CG = false>
 __device__ __forceinline__ void medium_tile(u32* base, u32 top, uint2 tl, const u64* __restrict__ fo,
                                             const u32* __restrict__ head, const Desc<OffT>* __restrict__ vdesc,
                                             const u32* __restrict__ headp, u32 seg, u64* __restrict__ cnt,
-                                            u64& local_total, u32& dup) {
+                                            const Control* ctl, u64& local_total, u32& dup) {
     using L = TileLayout<OffT>;
     constexpr u32 FULL = 0xFFFFFFFFu;
     const u32 lane = threadIdx.x & 31;
@@ -972,6 +975,18 @@ __device__ __forceinline__ void medium_tile(u32* base, u32 top, uint2 tl, const 
             }
         }
         __syncwarp();
+        if (c0 + L::CAP < xr && a == ld_in<CG>(fo + x) && (__ldcg(&ctl->err) & DEV_FLAG_UNSORTED)) {
+            for (u32 k = c0 + L::CAP + lane; k < xr; k += 32) {
+                const u32 wt = ld_in<CG>(headp + list_start(dx) + k) | top;
+                u32 b = __umulhi((wt & ~top) * TILE_MULT, L::NB);
+                while (true) {  // ends: a bucket without a second key, or without a mark
+                    const uint2 q = buckets[b];
+                    if (q.x == wt || (q.y | top) == wt) dup = 1;
+                    if (q.y == EMPTY_KEY || (q.y & top)) break;
+                    b = b + 1 < L::NB ? b + 1 : 0;
+                }
+            }
+        }
         u32 Tc = 0;
         // two chunks of slots ahead the neighbours, one ahead their descriptors are in flight
         auto neighbour = [&](u32 e) { return e + lane < ns ? ld_in<CG>(head + a + e + lane) : x; };
@@ -1086,8 +1101,8 @@ __global__ void __launch_bounds__(BLOCK, 4)
         if (lane == 0) t = atomicAdd(&ctl->medium_next, 1ull);
         t = __shfl_sync(0xFFFFFFFFu, t, 0);
         if (t >= ntiles) break;
-        medium_tile<OffT, HUB>(base, top, HUB && t < nl ? ltiles[tile_at(true, t)] : mtiles[t - nl], fo, head, vdesc, headp, seg, cnt,
-                               local_total, dup);
+        const uint2 tl = HUB && t < nl ? ltiles[tile_at(true, t)] : mtiles[t - nl];
+        medium_tile<OffT, HUB>(base, top, tl, fo, head, vdesc, headp, seg, cnt, ctl, local_total, dup);
     }
     if (dup) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
     const u64 bt = block_sum_u64<BLOCK>(local_total, s_red);
@@ -1687,7 +1702,7 @@ __global__ void __launch_bounds__(ENGINE_BLOCK, 4) k_engine(EngineJob* jobs, u32
                 const u64 t = ((u - jb->units_small) * (ENGINE_BLOCK / 32) + warp) * ENGINE_REPS + r;
                 if (t < nt)
                     medium_tile<u32, false, true>(slice, top, __ldcg(jb->mtiles + t), jb->fo, jb->head, vd, jb->headp,
-                                                  jb->seg, jb->cnt, unused_total, dup);
+                                                  jb->seg, jb->cnt, ctl, unused_total, dup);
             }
         } else {
             const u64 t = u - jb->units_small - jb->units_medium;
