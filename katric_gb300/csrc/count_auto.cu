@@ -853,7 +853,7 @@ __global__ void __launch_bounds__(BLOCK) k_count_large(const u64* __restrict__ f
 // medium_outdegree, and with hubs every owner's other entries.  A warp's table holds up to CAP of
 // the owner's keys (owners with more are counted in chunks) in buckets of two; a bucket that
 // overflowed is marked by a cleared top bit of its second key, so a lookup reads one bucket and
-// walks on only past a marked one (about 1 % of them at CAP keys), and a miss in a full bucket ends
+// walks on only past a marked one (about 1.5 % of them at CAP keys), and a miss in a full bucket ends
 // there.  Streamed lists are cut into units of 32 entries, eight lanes to a unit and four units of
 // any lists to a row; lists of up to four entries go one per lane.
 // What bounds it: instruction issue (71 to 73 %) beside the lookups' shared-memory wavefronts
@@ -861,11 +861,12 @@ __global__ void __launch_bounds__(BLOCK) k_count_large(const u64* __restrict__ f
 // iteration, which left most lanes idle on lists below 100 entries: RMAT n = 8191 0.182 -> 0.061 ms
 // (medium + large), 512-graph batch 6.2 -> 5.0 ms, the other entries of RMAT-24 27.6 -> 21 ms.
 // Measured against NB = 768 (24 warps per SM: RMAT-24 +0.8 %, batch +1 %, small graphs -10 %) and
-// CAP = 128 (RMAT-24 +7 %: more owners in two chunks).
+// fewer keys per chunk (more owners in two chunks: RMAT-24 66.3 ms, CAP = 192 68.0, CAP = 128 +7 %; a
+// lattice of out-degree 200 without hubs 1.41 ms, CAP = 192 2.49).  All of a medium owner's keys fit one chunk.
 template <typename OffT>
 struct TileLayout {
     static constexpr u32 NB = 512;   // buckets
-    static constexpr u32 CAP = 192;  // keys per chunk
+    static constexpr u32 CAP = MEDIUM_D;  // keys per chunk
     static constexpr int W_KEYS = 0;
     static constexpr int W_HITS = W_KEYS + 2 * NB;  // two 16-bit counters per bucket, a spare word per lane
     static constexpr int PER_WARP = W_HITS + NB + 32;
