@@ -87,7 +87,7 @@ struct Control {
     uint32_t prep_blocks;                // blocks of k_prep that have finished
     uint32_t hub_long;                   // vertices with a hub list above HUB_TOP_LIST
     uint32_t hub_tops;                   // hub lists whose top entries became bitmaps
-    uint32_t pad1;
+    uint32_t hub_crowd;                  // most hubs in one degree bin
 };
 
 }  // namespace ktri

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(PREP_BLOCK) k_prep(const u64* __restrict__ fo,
     if constexpr (HUB) {
         __shared__ u32 s_last;
         __shared__ u32 s_warp[PREP_BLOCK / 32];
-        __shared__ u32 s_bin, s_hubs;
+        __shared__ u32 s_bin, s_hubs, s_crowd;
         __syncthreads();
         for (u32 b = threadIdx.x; b < HUB_BINS; b += PREP_BLOCK)
             if (s_bins[b]) atomicAdd(&hub_bins[b], s_bins[b]);
@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(PREP_BLOCK) k_prep(const u64* __restrict__ fo,
         constexpr int PER = HUB_BINS / PREP_BLOCK;
         if (threadIdx.x == 0) {
             s_bin = HUB_BINS;
-            s_hubs = 0;
+            s_hubs = s_crowd = 0;
         }
         u32 c[PER];
         unsigned long long sum = 0;
@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(PREP_BLOCK) k_prep(const u64* __restrict__ fo,
         // counts above 2 HUB_H do not matter: saturate, so that 32 bits hold every prefix
         u32 total;
         u32 run = block_exclusive_scan<PREP_BLOCK>(sum > 2 * HUB_H ? 2 * HUB_H : (u32)sum, s_warp, &total);
+        u32 bin = HUB_BINS, upto = 0, crowd = 0;  // of this thread's bins: the last hub bin, hubs down to it, largest
 #pragma unroll
         for (int k = 0; k < PER; ++k) {
             const u32 b = HUB_BINS - 1 - (threadIdx.x * PER + k);
@@ -98,15 +99,25 @@ __global__ void __launch_bounds__(PREP_BLOCK) k_prep(const u64* __restrict__ fo,
             hub_bins[2 * HUB_BINS + b] = run;
             const u32 next = run + (c[k] > 2 * HUB_H ? 2 * HUB_H : c[k]);
             if (next < HUB_H) {
-                atomicMin(&s_bin, b);
-                atomicMax(&s_hubs, next);
+                bin = b;
+                upto = next;
+                crowd = c[k] > crowd ? c[k] : crowd;
             }
             run = next < 4 * HUB_H ? next : 4 * HUB_H;
+        }
+        bin = __reduce_min_sync(0xFFFFFFFFu, bin);
+        upto = __reduce_max_sync(0xFFFFFFFFu, upto);
+        crowd = __reduce_max_sync(0xFFFFFFFFu, crowd);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&s_bin, bin);
+            atomicMax(&s_hubs, upto);
+            atomicMax(&s_crowd, crowd);
         }
         __syncthreads();
         if (threadIdx.x == 0) {
             ctl->hub_bin = s_bin;
             ctl->hubs = s_hubs;
+            ctl->hub_crowd = s_crowd;
         }
     }
 }
@@ -127,26 +138,65 @@ __global__ void k_hub_place(u64 n, const u32* __restrict__ deg, u32* __restrict_
     }
 }
 
+// Where a bin holds more than HUB_CROWD hubs: the hubs by (degree, id), highest first, inside each chunk
+// of HUB_CHUNK places (a bitonic network in shared memory; the places are in bin order already, so no
+// hub leaves its bin).
+constexpr u32 HUB_CHUNK = HUB_H / 32;  // k_hub_rank: a chunk per lane
+constexpr u32 HUB_CROWD = 4096;        // reading a bin of this many takes 7 us, the sort of all chunks 9 us
+__global__ void __launch_bounds__(HUB_CHUNK / 2) k_hub_sort(u64* hub_tmp, const Control* ctl) {
+    chain_begin();
+    __shared__ u64 s[HUB_CHUNK];  // degree << 32 | id, as hub_tmp holds them
+    const u32 hubs = ctl->hubs, base = blockIdx.x * HUB_CHUNK;
+    if (base >= hubs || ctl->hub_crowd <= HUB_CROWD || (ctl->err & DEV_ERR_MASK)) return;
+    const u32 len = hubs - base < HUB_CHUNK ? hubs - base : HUB_CHUNK;
+    for (u32 i = threadIdx.x; i < HUB_CHUNK; i += HUB_CHUNK / 2) s[i] = i < len ? hub_tmp[base + i] : 0ull;
+    for (u32 k = 2; k <= HUB_CHUNK; k <<= 1) {
+        for (u32 j = k >> 1; j > 0; j >>= 1) {
+            __syncthreads();
+            const u32 i = 2 * threadIdx.x - (threadIdx.x & (j - 1));
+            const u64 a = s[i], b = s[i + j];
+            if ((a < b) == ((i & k) == 0)) {
+                s[i] = b;
+                s[i + j] = a;
+            }
+        }
+    }
+    __syncthreads();
+    for (u32 i = threadIdx.x; i < len; i += HUB_CHUNK / 2) hub_tmp[base + i] = s[i];
+}
+
 // Hub index = rank by (degree, id) from the top: the hubs above the bin plus those of the bin that
 // order higher.  key[v] (the degree of every other vertex) becomes the hub's orientation key, so
 // one gather gives a neighbour's place in the order and its hub index.
-__global__ void k_hub_rank(const u32* __restrict__ hub_bins, const uint2* __restrict__ hub_tmp, u32* __restrict__ hub_ids,
+// A warp per hub, which reads its bin whole, or, where the bin is crowded, searches the sorted chunks the
+// bin reaches into, one per lane.  With 31 000 vertices of one degree, reading the bin
+// took 430 us (by blocks of 128 hubs that share their reads 260 us), sort and search take 45 us.
+__global__ void k_hub_rank(const u32* __restrict__ hub_bins, const u64* hub_tmp, u32* __restrict__ hub_ids,
                            u32* __restrict__ key, const Control* ctl) {
     chain_begin();
     const u32 p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (p >= ctl->hubs || (ctl->err & DEV_ERR_MASK)) return;
-    const uint2 me = hub_tmp[p];
-    const u32 b = degree_bin(me.y);
-    const u32 first = hub_bins[2 * HUB_BINS + b], count = hub_bins[b];
+    const u64 me = hub_tmp[p];
+    const u32 b = degree_bin((u32)(me >> 32));
+    const u32 first = hub_bins[2 * HUB_BINS + b], count = hub_bins[b], end = first + count;
     u32 higher = 0;
-    for (u32 q = first + lane; q < first + count; q += 32) {
-        const uint2 o = hub_tmp[q];
-        if (o.y > me.y || (o.y == me.y && o.x > me.x)) ++higher;
+    if (count <= HUB_CROWD) {
+        for (u32 q = first + lane; q < end; q += 32) higher += hub_tmp[q] > me ? 1u : 0u;
+    } else {
+        const u32 at = lane * HUB_CHUNK;  // the chunk's part of the bin, highest first
+        const u32 from = at > first ? at : first, to = at + HUB_CHUNK < end ? at + HUB_CHUNK : end;
+        u32 lo = from, hi = to > from ? to : from;
+        while (lo < hi) {
+            const u32 mid = (lo + hi) >> 1;
+            if (hub_tmp[mid] > me) lo = mid + 1;
+            else hi = mid;
+        }
+        higher = lo - from;
     }
     const u32 r = first + __reduce_add_sync(0xFFFFFFFFu, higher);
     if (lane == 0) {
-        hub_ids[r] = me.x;
-        key[me.x] = HUB_FLAG | (HUB_H - 1 - r);
+        hub_ids[r] = (u32)me;
+        key[(u32)me] = HUB_FLAG | (HUB_H - 1 - r);
     }
 }
 
@@ -403,6 +453,7 @@ __global__ void __launch_bounds__(DESC_BLOCK) k_desc(const u64* __restrict__ fo,
     __shared__ u32 s_sum[3][WARPS];  // of each warp: medium tiles, large tiles, long hub lists
     __shared__ u64 s_at[3][WARPS];   // where its entries go
     if (ctl->err & DEV_ERR_MASK) return;
+    const bool plain = HUB && ctl->hubs == 0;
     const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const u64 stride = (u64)gridDim.x * DESC_BLOCK;
     if (order_hist)
@@ -421,7 +472,7 @@ __global__ void __launch_bounds__(DESC_BLOCK) k_desc(const u64* __restrict__ fo,
             vdesc[v] = ds;
             if constexpr (HUB) {
                 // oriented without hubs: a count past the low half is of a list with duplicates, too
-                if (d > 0xFFFFu && ctl->hubs == 0) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
+                if (plain && d > 0xFFFFu) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
                 const u64 hs = hub_start(list_start(ds), v);
                 for (u32 k = hub_len<HUB>(d); k & 7u; ++k) hubp[hs + k] = (u16)HUB_PAD;
                 top_info[v] = 0;
@@ -697,7 +748,9 @@ void launch_prep(const u64* fo, u64 n, u64 nnz, u32* deg, u32* dplus, u64* cnt, 
     }
     launch_chained(k_prep<true>, grid, PREP_BLOCK, 0, st, fo, n, nnz, deg, dplus, cnt, tile_i0, hub.bins, ctl);
     launch_chained(k_hub_place, grid, 256, 0, st, n, deg, hub.bins, hub.tmp, ctl);
-    launch_chained(k_hub_rank, HUB_H / 8, 256, 0, st, hub.bins, hub.tmp, hub.ids, deg, ctl);
+    auto* tmp = reinterpret_cast<u64*>(hub.tmp);  // {id, degree} as one number
+    launch_chained(k_hub_sort, HUB_H / HUB_CHUNK, HUB_CHUNK / 2, 0, st, tmp, ctl);
+    launch_chained(k_hub_rank, HUB_H / 8, 256, 0, st, hub.bins, tmp, hub.ids, deg, ctl);
 }
 
 void launch_hub_tops(const void* vdesc, const HubState& hub, Control* ctl, int num_sms, LaunchStream st) {
