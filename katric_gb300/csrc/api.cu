@@ -712,6 +712,14 @@ int ktri::ctx_device(const ktri_ctx* ctx) { return ctx->device; }
 
 void ktri::ctx_for_server(ktri_ctx* ctx) { ctx->hubs = ctx->chained = false; }
 void ktri::ctx_allow_hubs(ktri_ctx* ctx, bool allow) { ctx->hubs = allow; }
+size_t ktri::ctx_ws_bytes(const ktri_ctx* ctx) { return ctx->ws_bytes; }
+void ktri::ctx_release_ws(ktri_ctx* ctx) {
+    DeviceGuard g(ctx->device);
+    end_pending(ctx);
+    if (ctx->ws) cudaFree(ctx->ws);
+    ctx->ws = nullptr;
+    ctx->ws_bytes = 0;
+}
 size_t ktri::hub_bytes(uint64_t n, uint64_t nnz) {
     return make_layout(n, nnz, KTRI_METHOD_AUTO, 0, false, true, false, 0, 0, true).bytes -
            make_layout(n, nnz, KTRI_METHOD_AUTO, 0, false, true).bytes;

@@ -36,6 +36,9 @@ int ctx_num_sms(const ktri_ctx* ctx);
 // they run, and split out-lists only in the counts that ctx_allow_hubs allows them.
 void ctx_for_server(ktri_ctx* ctx);
 void ctx_allow_hubs(ktri_ctx* ctx, bool allow);
+// The workspace a context holds, and its return (once the work on it has ended).
+size_t ctx_ws_bytes(const ktri_ctx* ctx);
+void ctx_release_ws(ktri_ctx* ctx);
 // What split out-lists add to ktri_workspace_bytes (0 where a count of this size has none).
 size_t hub_bytes(uint64_t n, uint64_t nnz);
 

@@ -213,6 +213,7 @@ struct Slot {
     bool counting = false;
     ktri::Control* ctl = nullptr;
     double t_published = 0;
+    bool split = false;  // the context's workspace was grown for split out-lists
 };
 
 size_t al(size_t x) { return (x + 255) & ~size_t(255); }
@@ -287,6 +288,24 @@ bool make_room(ktri_server* s, size_t need, size_t inflight) {
     return s->resident_bytes + inflight + need <= s->opts.memory_budget;
 }
 
+// Device bytes the server holds: resident graphs, and the slots' unions and counting workspaces.
+size_t held_bytes(const ktri_server* s) {
+    size_t sum = s->resident_bytes;
+    for (const Slot& o : s->slots) sum += o.dev_bytes + ktri::ctx_ws_bytes(o.ctx);
+    return sum;
+}
+
+// Where `more` bytes do not fit the budget beside all that is held, the workspaces that split out-lists
+// have grown in idle slots (and in `done`, whose batch has ended) are given back.  Called with s->mu held.
+void release_split(ktri_server* s, const Slot* done, size_t more) {
+    if (held_bytes(s) + more <= s->opts.memory_budget) return;
+    for (Slot& o : s->slots) {
+        if (!o.split || (o.busy && &o != done)) continue;
+        ktri::ctx_release_ws(o.ctx);
+        o.split = false;
+    }
+}
+
 void finish(ktri_server* s, Request* r, int status) {
     r->status = status;
     r->t_done = now_s();
@@ -347,6 +366,7 @@ void keep_resident(ktri_server* s, Request* r, const Slot& sl, u64 vbase, u64 eb
     }
     const size_t bytes = al(8 * (r->n + 1)) + al(4 * (r->nnz + 1)) + al(8 * (r->n + 1));
     if (bytes > s->opts.memory_budget / 4) return;
+    release_split(s, &sl, bytes);
     if (!make_room(s, bytes, inflight)) return;
     void* mem = nullptr;
     if (cudaMallocAsync(&mem, bytes, s->aux) != cudaSuccess) {
@@ -811,11 +831,19 @@ void worker_main(ktri_server* s) {
                 for (Request* r : batch) finish(s, r, KTRI_ERR_OUT_OF_MEMORY);
                 s->cv_done.notify_all();
             } else {
-                // Split out-lists where the budget has room beside what is resident: they cost no
-                // graph its place.  (A burst of 30 graphs, 16 M entries in its largest batch:
-                // 6.7 -> 5.8 ms; the owner tiles of its two large batches took 2.5 ms without, 0.66 ms with.)
-                ktri::ctx_allow_hubs(free_slot->ctx, need + ktri::hub_bytes(n, nnz) + inflight + s->resident_bytes <=
-                                                         s->opts.memory_budget);
+                // Split out-lists where the budget has room beside all that is held, with the headroom that
+                // buffers grow by: they cost no graph its place.  (A burst of 30 graphs, 16 M entries in
+                // its largest batch: 6.7 -> 5.8 ms; the owner tiles of its two large batches took 2.5 ms
+                // without, 0.66 ms with.)
+                const size_t plain = (size_t)ktri_workspace_bytes(n, nnz, KTRI_METHOD_AUTO);
+                const size_t split = ktri::hub_bytes(n, nnz), ws = ktri::ctx_ws_bytes(free_slot->ctx);
+                const size_t rest = held_bytes(s) - free_slot->dev_bytes - ws +
+                                    std::max(free_slot->dev_bytes, (need - plain) + (need - plain) / 4);
+                auto with = [&](size_t bytes) { return rest + std::max(ws, bytes + bytes / 8); };
+                const bool allow = split && !s->engine && with(plain + split) <= s->opts.memory_budget;
+                ktri::ctx_allow_hubs(free_slot->ctx, allow);
+                if (allow) free_slot->split = true;
+                else release_split(s, nullptr, with(plain) - held_bytes(s));
                 for (Request* r : batch) r->pv_wanted = r->want_pv || r->follower_pv;
                 free_slot->reqs = batch;
                 free_slot->busy = true;
