@@ -53,6 +53,7 @@ struct ktri_ctx {
     bool have_events = false;
     int32_t last_method = KTRI_METHOD_AUTO;
     bool last_collect = false;
+    size_t refused_bytes = ~size_t(0);  // smallest workspace for split out-lists that could not be allocated
     bool hubs = true;          // counts may split their out-lists (more workspace than ktri_workspace_bytes)
     bool chained = true;       // kernels are launched chained (LaunchStream)
 };
@@ -242,29 +243,37 @@ int ensure_ws(ktri_ctx* ctx, size_t bytes) {
     return KTRI_OK;
 }
 
-// The layout of a count on a context, with extra bytes behind it: split out-lists (hubs) where the
-// larger workspace is within the memory budget and, when the workspace has to grow, within what
-// the device has free; otherwise the plain one, which any accepted call can have.
+// The layout of a count on a context, and the workspace for it with extra bytes behind it: split
+// out-lists (hubs) where the larger workspace is there already, or is within the memory budget and what
+// the device has free and can be allocated; otherwise the plain layout, which any accepted call can
+// have.
 template <class Extra>
-Layout pick_layout(ktri_ctx* ctx, u64 n, u64 nnz, const ktri::Options& opt, bool with_inputs, bool internal_cnt,
-                   Extra extra) {
-    const Layout L = make_layout(n, nnz, opt.method, ctx->num_sms, with_inputs, internal_cnt, opt.force_wide,
-                                 opt.small_outdegree, opt.segment, ctx->hubs);
-    if (L.hub) {
-        const size_t bytes = extra(L.bytes);
-        bool fits = !ctx->budget || bytes <= ctx->budget;
-        if (fits && bytes > ctx->ws_bytes) {
-            size_t free_bytes = 0, total_bytes = 0;
-            fits = cudaMemGetInfo(&free_bytes, &total_bytes) == cudaSuccess && bytes <= free_bytes + ctx->ws_bytes;
+int take_workspace(ktri_ctx* ctx, u64 n, u64 nnz, const ktri::Options& opt, bool with_inputs, bool internal_cnt,
+                   Layout* L, Extra extra) {
+    auto layout = [&](bool hub) {
+        return make_layout(n, nnz, opt.method, ctx->num_sms, with_inputs, internal_cnt, opt.force_wide,
+                           opt.small_outdegree, opt.segment, hub);
+    };
+    auto can_grow = [&](size_t bytes) {
+        if (bytes >= ctx->refused_bytes) return false;
+        size_t free_bytes = 0, total_bytes = 0;
+        return cudaMemGetInfo(&free_bytes, &total_bytes) == cudaSuccess && bytes <= free_bytes + ctx->ws_bytes;
+    };
+    *L = layout(ctx->hubs);
+    if (L->hub) {
+        const size_t bytes = extra(L->bytes);
+        if ((!ctx->budget || bytes <= ctx->budget) && (bytes <= ctx->ws_bytes || can_grow(bytes))) {
+            if (ensure_ws(ctx, bytes) == KTRI_OK) return KTRI_OK;
+            ctx->refused_bytes = bytes;  // not tried again: it costs the workspace that is there
+            ctx->last_error.clear();
         }
-        if (!fits)
-            return make_layout(n, nnz, opt.method, ctx->num_sms, with_inputs, internal_cnt, opt.force_wide,
-                               opt.small_outdegree, opt.segment, false);
+        *L = layout(false);
     }
-    return L;
+    return ensure_ws(ctx, extra(L->bytes));
 }
-Layout pick_layout(ktri_ctx* ctx, u64 n, u64 nnz, const ktri::Options& opt, bool with_inputs, bool internal_cnt) {
-    return pick_layout(ctx, n, nnz, opt, with_inputs, internal_cnt, [](size_t b) { return b; });
+int take_workspace(ktri_ctx* ctx, u64 n, u64 nnz, const ktri::Options& opt, bool with_inputs, bool internal_cnt,
+                   Layout* L) {
+    return take_workspace(ctx, n, nnz, opt, with_inputs, internal_cnt, L, [](size_t b) { return b; });
 }
 
 struct DeviceGuard {
@@ -864,8 +873,8 @@ int ktri_count_csr_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint
         ctx->stats = ktri_run_stats{};
         return KTRI_OK;
     }
-    const Layout L = pick_layout(ctx, n, nnz, opt, false, d_per_vertex == nullptr);
-    rc = ensure_ws(ctx, L.bytes);
+    Layout L;
+    rc = take_workspace(ctx, n, nnz, opt, false, d_per_vertex == nullptr, &L);
     if (rc) return rc;
     u64* cnt = d_per_vertex ? reinterpret_cast<u64*>(d_per_vertex)
                             : reinterpret_cast<u64*>(static_cast<char*>(ctx->ws) + L.cnt);
@@ -921,8 +930,8 @@ int ktri_count_csr_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t*
     }
     if (first_out[0] != 0 || first_out[n] != nnz)
         return set_error(ctx, KTRI_ERR_INVALID_CSR, "first_out[0] must be 0 and first_out[n] must equal nnz");
-    const Layout L = pick_layout(ctx, n, nnz, opt, true, true);
-    rc = ensure_ws(ctx, L.bytes);
+    Layout L;
+    rc = take_workspace(ctx, n, nnz, opt, true, true, &L);
     if (rc) return rc;
     char* base = static_cast<char*>(ctx->ws);
     auto* d_fo = reinterpret_cast<u64*>(base + L.in_fo);
@@ -1052,12 +1061,12 @@ int ktri_count_binary_file(ktri_ctx* ctx, const char* stem, uint64_t* total_out,
         *total_out = 0;
         return cleanup(nnz ? set_error(ctx, KTRI_ERR_INVALID_CSR, "edges without vertices") : KTRI_OK);
     }
-    Layout L = pick_layout(ctx, n, nnz, opt, true, true, [&](size_t b) { return align_up(b + 2 * chunk_bytes); });
     // two device staging chunks for u64 ids follow the count's workspace
-    const size_t x_stage = L.bytes;
-    L.bytes = align_up(x_stage + 2 * chunk_bytes);
-    rc = ensure_ws(ctx, L.bytes);
+    Layout L;
+    rc = take_workspace(ctx, n, nnz, opt, true, true, &L,
+                        [&](size_t b) { return align_up(b + 2 * chunk_bytes); });
     if (rc) return cleanup(rc);
+    const size_t x_stage = L.bytes;
     for (int i = 0; i < 2; ++i) {
         if (cudaHostAlloc(&pinned[i], chunk_bytes, cudaHostAllocDefault) != cudaSuccess ||
             cudaEventCreateWithFlags(&freed[i], cudaEventDisableTiming) != cudaSuccess) {
@@ -1340,8 +1349,8 @@ int ktri_count_dag_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint
         return KTRI_OK;
     }
     const u64 nnz = 2 * m;
-    const Layout L = pick_layout(ctx, n, nnz, opt, true, d_per_vertex == nullptr);
-    rc = ensure_ws(ctx, L.bytes);
+    Layout L;
+    rc = take_workspace(ctx, n, nnz, opt, true, d_per_vertex == nullptr, &L);
     if (rc) return rc;
     char* base = static_cast<char*>(ctx->ws);
     auto* fs = reinterpret_cast<u64*>(base + L.in_fo);
@@ -1374,16 +1383,15 @@ int ktri_count_dag_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t*
             return set_error(ctx, KTRI_ERR_INVALID_CSR, "first_out is not monotone");
     if (m > (1ull << 62)) return set_error(ctx, KTRI_ERR_UNSUPPORTED, "too many edges");
     const u64 nnz = 2 * m;
-    Layout L = pick_layout(ctx, n, nnz, opt, true, true, [&](size_t b) {
+    // the caller's lists and the scan sums follow the count's workspace
+    Layout L;
+    rc = take_workspace(ctx, n, nnz, opt, true, true, &L, [&](size_t b) {
         return align_up(align_up(align_up(b + sizeof(u64) * (n + 1)) + sizeof(u32) * m) +
                         sizeof(u64) * (ktri::dag_scan_chunks(n) + 1));
     });
-    // the caller's lists and the scan sums follow the count's workspace
+    if (rc) return rc;
     const size_t x_fo = L.bytes, x_head = align_up(x_fo + sizeof(u64) * (n + 1)),
                  x_sums = align_up(x_head + sizeof(u32) * m);
-    L.bytes = align_up(x_sums + sizeof(u64) * (ktri::dag_scan_chunks(n) + 1));
-    rc = ensure_ws(ctx, L.bytes);
-    if (rc) return rc;
     char* base = static_cast<char*>(ctx->ws);
     auto* dfo = reinterpret_cast<u64*>(base + x_fo);
     auto* dhead = reinterpret_cast<u32*>(base + x_head);
@@ -1472,8 +1480,8 @@ int ktri_count_batch_device(ktri_ctx* ctx, const uint64_t* d_first_out, const ui
         if (num_graphs) KTRI_CK(ctx, cudaMemsetAsync(d_totals, 0, sizeof(u64) * num_graphs, st));
         return KTRI_OK;
     }
-    const Layout L = pick_layout(ctx, n_total, nnz_total, opt, false, true);
-    rc = ensure_ws(ctx, L.bytes);
+    Layout L;
+    rc = take_workspace(ctx, n_total, nnz_total, opt, false, true, &L);
     if (rc) return rc;
     char* base = static_cast<char*>(ctx->ws);
     u64* cnt = d_per_vertex ? reinterpret_cast<u64*>(d_per_vertex) : reinterpret_cast<u64*>(base + L.cnt);
@@ -1505,13 +1513,12 @@ int ktri_count_batch_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_
     }
     if (first_out[0] != 0 || first_out[n_total] != nnz_total)
         return set_error(ctx, KTRI_ERR_INVALID_CSR, "first_out[0] must be 0 and first_out[n] must equal nnz");
-    const Layout L = pick_layout(ctx, n_total, nnz_total, opt, true, true, [&](size_t b) {
+    Layout L;
+    rc = take_workspace(ctx, n_total, nnz_total, opt, true, true, &L, [&](size_t b) {
         return align_up(align_up(b + sizeof(u64) * (num_graphs + 1)) + sizeof(u64) * (num_graphs + 1));
     });
-    const size_t off_gf = L.bytes, off_tot = align_up(off_gf + sizeof(u64) * (num_graphs + 1));
-    const size_t total_bytes = align_up(off_tot + sizeof(u64) * (num_graphs + 1));
-    rc = ensure_ws(ctx, total_bytes);
     if (rc) return rc;
+    const size_t off_gf = L.bytes, off_tot = align_up(off_gf + sizeof(u64) * (num_graphs + 1));
     char* base = static_cast<char*>(ctx->ws);
     auto* d_fo = reinterpret_cast<u64*>(base + L.in_fo);
     auto* d_head = reinterpret_cast<u32*>(base + L.in_head);
