@@ -246,18 +246,23 @@ int ensure_ws(ktri_ctx* ctx, size_t bytes) {
 // The layout of a count on a context, and the workspace for it with extra bytes behind it: split
 // out-lists (hubs) where the larger workspace is there already, or is within the memory budget and what
 // the device has free and can be allocated; otherwise the plain layout, which any accepted call can
-// have.
+// have.  While the stream captures nothing grows for split lists: an allocation would end the capture.
 template <class Extra>
 int take_workspace(ktri_ctx* ctx, u64 n, u64 nnz, const ktri::Options& opt, bool with_inputs, bool internal_cnt,
-                   Layout* L, Extra extra) {
+                   cudaStream_t st, Layout* L, Extra extra) {
     auto layout = [&](bool hub) {
         return make_layout(n, nnz, opt.method, ctx->num_sms, with_inputs, internal_cnt, opt.force_wide,
                            opt.small_outdegree, opt.segment, hub);
     };
     auto can_grow = [&](size_t bytes) {
         if (bytes >= ctx->refused_bytes) return false;
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         size_t free_bytes = 0, total_bytes = 0;
-        return cudaMemGetInfo(&free_bytes, &total_bytes) == cudaSuccess && bytes <= free_bytes + ctx->ws_bytes;
+        if (cudaStreamIsCapturing(st, &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone &&
+            cudaMemGetInfo(&free_bytes, &total_bytes) == cudaSuccess)
+            return bytes <= free_bytes + ctx->ws_bytes;
+        (void)cudaGetLastError();
+        return false;
     };
     *L = layout(ctx->hubs);
     if (L->hub) {
@@ -272,8 +277,8 @@ int take_workspace(ktri_ctx* ctx, u64 n, u64 nnz, const ktri::Options& opt, bool
     return ensure_ws(ctx, extra(L->bytes));
 }
 int take_workspace(ktri_ctx* ctx, u64 n, u64 nnz, const ktri::Options& opt, bool with_inputs, bool internal_cnt,
-                   Layout* L) {
-    return take_workspace(ctx, n, nnz, opt, with_inputs, internal_cnt, L, [](size_t b) { return b; });
+                   cudaStream_t st, Layout* L) {
+    return take_workspace(ctx, n, nnz, opt, with_inputs, internal_cnt, st, L, [](size_t b) { return b; });
 }
 
 struct DeviceGuard {
@@ -874,7 +879,7 @@ int ktri_count_csr_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint
         return KTRI_OK;
     }
     Layout L;
-    rc = take_workspace(ctx, n, nnz, opt, false, d_per_vertex == nullptr, &L);
+    rc = take_workspace(ctx, n, nnz, opt, false, d_per_vertex == nullptr, st, &L);
     if (rc) return rc;
     u64* cnt = d_per_vertex ? reinterpret_cast<u64*>(d_per_vertex)
                             : reinterpret_cast<u64*>(static_cast<char*>(ctx->ws) + L.cnt);
@@ -931,7 +936,7 @@ int ktri_count_csr_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t*
     if (first_out[0] != 0 || first_out[n] != nnz)
         return set_error(ctx, KTRI_ERR_INVALID_CSR, "first_out[0] must be 0 and first_out[n] must equal nnz");
     Layout L;
-    rc = take_workspace(ctx, n, nnz, opt, true, true, &L);
+    rc = take_workspace(ctx, n, nnz, opt, true, true, ctx->stream, &L);
     if (rc) return rc;
     char* base = static_cast<char*>(ctx->ws);
     auto* d_fo = reinterpret_cast<u64*>(base + L.in_fo);
@@ -1063,7 +1068,7 @@ int ktri_count_binary_file(ktri_ctx* ctx, const char* stem, uint64_t* total_out,
     }
     // two device staging chunks for u64 ids follow the count's workspace
     Layout L;
-    rc = take_workspace(ctx, n, nnz, opt, true, true, &L,
+    rc = take_workspace(ctx, n, nnz, opt, true, true, ctx->stream, &L,
                         [&](size_t b) { return align_up(b + 2 * chunk_bytes); });
     if (rc) return cleanup(rc);
     const size_t x_stage = L.bytes;
@@ -1350,7 +1355,7 @@ int ktri_count_dag_device(ktri_ctx* ctx, const uint64_t* d_first_out, const uint
     }
     const u64 nnz = 2 * m;
     Layout L;
-    rc = take_workspace(ctx, n, nnz, opt, true, d_per_vertex == nullptr, &L);
+    rc = take_workspace(ctx, n, nnz, opt, true, d_per_vertex == nullptr, st, &L);
     if (rc) return rc;
     char* base = static_cast<char*>(ctx->ws);
     auto* fs = reinterpret_cast<u64*>(base + L.in_fo);
@@ -1385,7 +1390,7 @@ int ktri_count_dag_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t*
     const u64 nnz = 2 * m;
     // the caller's lists and the scan sums follow the count's workspace
     Layout L;
-    rc = take_workspace(ctx, n, nnz, opt, true, true, &L, [&](size_t b) {
+    rc = take_workspace(ctx, n, nnz, opt, true, true, ctx->stream, &L, [&](size_t b) {
         return align_up(align_up(align_up(b + sizeof(u64) * (n + 1)) + sizeof(u32) * m) +
                         sizeof(u64) * (ktri::dag_scan_chunks(n) + 1));
     });
@@ -1481,7 +1486,7 @@ int ktri_count_batch_device(ktri_ctx* ctx, const uint64_t* d_first_out, const ui
         return KTRI_OK;
     }
     Layout L;
-    rc = take_workspace(ctx, n_total, nnz_total, opt, false, true, &L);
+    rc = take_workspace(ctx, n_total, nnz_total, opt, false, true, st, &L);
     if (rc) return rc;
     char* base = static_cast<char*>(ctx->ws);
     u64* cnt = d_per_vertex ? reinterpret_cast<u64*>(d_per_vertex) : reinterpret_cast<u64*>(base + L.cnt);
@@ -1514,7 +1519,7 @@ int ktri_count_batch_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_
     if (first_out[0] != 0 || first_out[n_total] != nnz_total)
         return set_error(ctx, KTRI_ERR_INVALID_CSR, "first_out[0] must be 0 and first_out[n] must equal nnz");
     Layout L;
-    rc = take_workspace(ctx, n_total, nnz_total, opt, true, true, &L, [&](size_t b) {
+    rc = take_workspace(ctx, n_total, nnz_total, opt, true, true, ctx->stream, &L, [&](size_t b) {
         return align_up(align_up(b + sizeof(u64) * (num_graphs + 1)) + sizeof(u64) * (num_graphs + 1));
     });
     if (rc) return rc;

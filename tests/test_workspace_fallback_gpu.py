@@ -1,15 +1,16 @@
 """Counts that could split their out-lists but have no room for the larger workspace (needs a GB300): an
-allocation that fails although the device reports the memory as free.  They are counted with plain
-lists."""
+allocation that fails although the device reports the memory as free, and a call captured on a
+context whose workspace only holds the plain lists.  Both are counted with plain lists."""
 import glob
 import os
 import subprocess
 import sys
 import textwrap
 
+import numpy as np
 import pytest
 
-from katric_gb300 import build
+from katric_gb300 import Graph, TriangleCounter, _native, build
 
 pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -95,3 +96,33 @@ def test_allocation_that_fails(tmp_path):
     r = subprocess.run([sys.executable, "-c", textwrap.dedent(CHILD), str(lib)], cwd=ROOT, capture_output=True,
                        text=True, timeout=300)
     assert r.returncode == 0 and "counted" in r.stdout, r.stdout + r.stderr
+
+
+def test_capture_grows_no_workspace(oracle):
+    import torch
+    g = Graph.rmat(16, 24, seed=9)
+    total, pv, _ = oracle.count(g.first_out, g.head, num_threads=8)
+    fo = torch.from_numpy(g.first_out.view(np.int64).copy()).cuda()
+    hd = torch.from_numpy(g.head.view(np.int32).copy()).cuda()
+    t = torch.zeros(1, dtype=torch.int64, device="cuda")
+    p = torch.zeros(g.n, dtype=torch.int64, device="cuda")
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with TriangleCounter(0) as ctr:
+        def count():
+            ctr.count_device(fo.data_ptr(), hd.data_ptr(), g.n, g.nnz, t.data_ptr(), p.data_ptr(),
+                             stream=side.cuda_stream)
+
+        ctr.set_memory_budget(int(_native.load().ktri_workspace_bytes(g.n, g.nnz, 0)) + 4096)  # plain lists only
+        count()
+        ctr.check()
+        ctr.set_memory_budget(0)
+        captured = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(captured, stream=side):
+            count()
+        for _ in range(2):
+            t.zero_()
+            p.zero_()
+            captured.replay()
+            torch.cuda.synchronize()
+            assert int(t[0]) == total and np.array_equal(p.cpu().numpy().view(np.uint64), pv)
