@@ -280,7 +280,8 @@ int ktri_partition_cost(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t
  * intersection strategy, small_outdegree, medium_outdegree and segment, and writes the fastest
  * into *opts (other fields are kept).  With a cache_path the choice is looked up first and, when
  * timed, appended as one JSON line keyed by the input's shape class (compute capability, SM
- * count, floor log2 of graphs, n, nnz and the largest degree).  The call synchronises `stream`. */
+ * count, floor log2 of graphs, n, nnz and the largest degree) and the library's version (a line of
+ * another version is passed over).  The call synchronises `stream`. */
 typedef struct ktri_tuning {
     uint32_t struct_size;
     int32_t intersection_method; /* the chosen configuration */

@@ -781,7 +781,7 @@ int ktri::engine_prepare_batch(ktri_ctx* ctx, const uint64_t* d_first_out, const
 
 extern "C" {
 
-const char* ktri_version(void) { return "katric_gb300 1.0 (sm_103a)"; }
+const char* ktri_version(void) { return "katric_gb300 1.1 (sm_103a)"; }
 
 int ktri_ctx_create(int device, ktri_ctx** out) {
     if (!out) return KTRI_ERR_INVALID_ARGUMENT;

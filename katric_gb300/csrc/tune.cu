@@ -1,11 +1,11 @@
 // Autotuner of the counting configuration: intersection strategy, owner-bin thresholds and
 // the owner tile segment.  It times candidate configurations of one count (a single graph or
 // a packed batch) on the caller's device buffers, keeps the fastest, and persists the choice
-// per shape class in a JSON-lines cache file, so later runs on inputs of the same class read
-// it back without timing.
+// per shape class in a JSON-lines cache file, so later runs of the same library version on inputs of
+// the same class read it back without timing (another version's kernels give the options other times).
 //
-// Search: the library default (KTRI_METHOD_AUTO with bins 48 / 256, segment 1024) is timed
-// first; then the reference's strategies (hybrid first; merge, binary search and binary only
+// Search: the library default (KTRI_METHOD_AUTO with bins 48 / 256, the segment of the input's size)
+// is timed first; then the reference's strategies (hybrid first; merge, binary search and binary only
 // when hybrid comes within 1.5x of the best); then, if an AUTO configuration is best, one pass
 // of coordinate descent over small_outdegree, medium_outdegree and segment, and last the tile
 // order by streamed work (KTRI_TILE_ORDER_COST).  A candidate replaces the best configuration so
@@ -21,14 +21,14 @@
 
 #include "ktri.h"
 
-#include "ktri_internal.h"
+#include "ktri_kernels.h"
 
 namespace {
 
 // Relative gain a candidate must show over the best configuration so far to replace it.
 constexpr double kMinGain = 0.02;
 
-using u64 = unsigned long long;
+using ktri::u64;
 
 __global__ void k_max_degree(const u64* __restrict__ fo, u64 n, u64* __restrict__ out) {
     u64 m = 0;
@@ -53,17 +53,18 @@ int floor_log2(u64 x) {
 
 struct Cand {
     int32_t method = KTRI_METHOD_AUTO;
-    uint32_t small = 48, medium = 256, seg = 1024, order = 0;
+    uint32_t small = ktri::SMALL_D, medium = ktri::MEDIUM_D, seg = ktri::LARGE_SEG, order = 0;
     bool operator==(const Cand& o) const {
         return method == o.method && small == o.small && medium == o.medium && seg == o.seg && order == o.order;
     }
 };
 
-// Reads the last line of the cache whose signature matches.
+// Reads the last line of the cache whose signature and library version match.
 bool read_cache(const char* path, const std::string& sig, Cand* c, double* ms) {
     std::ifstream f(path);
     if (!f) return false;
     const std::string key = "\"signature\": \"" + sig + "\"";
+    const std::string version = std::string("\"version\": \"") + ktri_version() + "\"";
     std::string line;
     bool found = false;
     auto field = [](const std::string& l, const char* name, double* v) {
@@ -74,12 +75,12 @@ bool read_cache(const char* path, const std::string& sig, Cand* c, double* ms) {
         return true;
     };
     while (std::getline(f, line)) {
-        if (line.find(key) == std::string::npos) continue;
-        double m, s, md, sg, t, to = 0;
+        if (line.find(key) == std::string::npos || line.find(version) == std::string::npos) continue;
+        double m, s, md, sg, t, to;
         if (!field(line, "method", &m) || !field(line, "small_outdegree", &s) ||
-            !field(line, "medium_outdegree", &md) || !field(line, "segment", &sg) || !field(line, "ms", &t))
+            !field(line, "medium_outdegree", &md) || !field(line, "segment", &sg) || !field(line, "ms", &t) ||
+            !field(line, "tile_order", &to))
             continue;
-        field(line, "tile_order", &to);  // absent in lines written before the option existed
         c->method = (int32_t)m;
         c->small = (uint32_t)s;
         c->medium = (uint32_t)md;
@@ -91,15 +92,16 @@ bool read_cache(const char* path, const std::string& sig, Cand* c, double* ms) {
     return found;
 }
 
-bool append_cache(const char* path, const std::string& sig, const Cand& c, double ms, double default_ms,
-                  uint32_t candidates) {
+bool append_cache(const char* path, const std::string& sig, const Cand& c, double ms, const Cand& def,
+                  double default_ms, uint32_t candidates) {
     FILE* f = std::fopen(path, "a");
     if (!f) return false;
     std::fprintf(f,
                  "{\"signature\": \"%s\", \"method\": %d, \"small_outdegree\": %u, \"medium_outdegree\": %u, "
-                 "\"segment\": %u, \"tile_order\": %u, \"ms\": %.6f, \"default_ms\": %.6f, \"candidates\": %u, "
-                 "\"version\": \"%s\"}\n",
-                 sig.c_str(), c.method, c.small, c.medium, c.seg, c.order, ms, default_ms, candidates, ktri_version());
+                 "\"segment\": %u, \"tile_order\": %u, \"ms\": %.6f, \"default_segment\": %u, \"default_ms\": %.6f, "
+                 "\"candidates\": %u, \"version\": \"%s\"}\n",
+                 sig.c_str(), c.method, c.small, c.medium, c.seg, c.order, ms, def.seg, default_ms, candidates,
+                 ktri_version());
     return std::fclose(f) == 0;
 }
 
@@ -208,6 +210,8 @@ extern "C" int ktri_autotune(ktri_ctx* ctx, const uint64_t* d_first_out, const u
             // noise (and the difference between the tuning sample and the full input)
             auto clearly_faster = [](double t, double incumbent) { return t < (1.0 - kMinGain) * incumbent; };
             Cand def;
+            def.seg = ktri::default_segment(nnz);
+            best = def;
             double t = 0;
             rc = timed(def, &best_ms);
             if (rc) break;
@@ -258,7 +262,7 @@ extern "C" int ktri_autotune(ktri_ctx* ctx, const uint64_t* d_first_out, const u
                     }
                 }
                 if (rc) break;
-                for (uint32_t g : {256u, 512u, 1024u}) {
+                for (uint32_t g = ktri::MIN_SEG; g <= ktri::LARGE_SEG; g *= 2) {
                     Cand c = best;
                     c.seg = g;
                     rc = timed(c, &t);
@@ -281,7 +285,7 @@ extern "C" int ktri_autotune(ktri_ctx* ctx, const uint64_t* d_first_out, const u
                 }
             }
             res.ms = best_ms;
-            if (cache_path && !append_cache(cache_path, sig, best, best_ms, res.default_ms, res.candidates)) {
+            if (cache_path && !append_cache(cache_path, sig, best, best_ms, def, res.default_ms, res.candidates)) {
                 rc = KTRI_ERR_IO;
                 break;
             }
