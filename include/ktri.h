@@ -105,7 +105,8 @@ typedef struct ktri_run_stats {
     float host_ms_call;               /* host-buffer calls: host time of the whole call */
     uint64_t streamed_chunked;        /* entries the AUTO kernels stream, counted once per owner-table chunk
                                          that streams them (collect_stats); above streamed_entries only when
-                                         some owner has more than 2048 out-neighbours */
+                                         some owner has more than 2048 out-neighbours or, where lists are split,
+                                         more than 256 that are not hubs */
 } ktri_run_stats;
 
 typedef struct ktri_ctx ktri_ctx;

@@ -473,7 +473,7 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[1], st));
     if (opt.collect_stats)
         ktri::launch_stats<OffT, HUB>(fo, head, n, vdesc, headp, hub, opt.small_outdegree,
-                                 autom ? opt.medium_outdegree : 0xFFFFFFFFu, ctl, sms, st);
+                                 autom ? opt.medium_outdegree : 0, ctl, sms, st);
     if (events) KTRI_CK(ctx, cudaEventRecord(ctx->ev[2], st));
     if (HUB) ktri::launch_hub_tops(vdesc, hub, ctl, sms, st);  // after the work counters, which read whole lists
     if (sort_all) {

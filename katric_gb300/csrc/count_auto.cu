@@ -1468,8 +1468,8 @@ __global__ void __launch_bounds__(256) k_graph_totals(const u64* __restrict__ cn
 
 // collect_stats: wedge_checks = sum over oriented (v,u) of |N+(u)|, the reference's counter
 // (cetric_edge_iterator.h:279-281), plus the entries streamed by the AUTO kernels, also counted
-// once per table chunk of their owner (owners above medium_d keep at most LARGE_CAP keys per
-// chunk and stream their segment once per chunk).
+// once per table chunk of their owner: LARGE_CAP keys for owners above medium_d, TileLayout's CAP for the
+// others and, with hubs, for what no owner's hubs take.  medium_d = 0: a strategy without tables.
 template <typename OffT, bool HUB>
 __global__ void k_stats(const u64* __restrict__ fo, const u32* __restrict__ head, u64 n,
                         const Desc<OffT>* __restrict__ vdesc, const u32* __restrict__ headp,
@@ -1484,7 +1484,8 @@ __global__ void k_stats(const u64* __restrict__ fo, const u32* __restrict__ head
     for (u64 v = gw; v < n; v += nwarps) {
         const Desc<OffT> dv = load_desc(vdesc + v);
         const u32 lv = list_len<HUB>(dv.d), rv = rest_len<HUB>(dv.d);
-        const u64 chunks = lv > medium_d ? (rv + LARGE_CAP - 1) / LARGE_CAP : 1;
+        const u32 keys = medium_d == 0 ? ~0u : !HUB && lv > medium_d ? (u32)LARGE_CAP : TileLayout<OffT>::CAP;
+        const u64 chunks = rv > keys ? ((u64)rv + keys - 1) / keys : 1;
         if (lane == 0) oriented += lv;
         for (u32 k = lane; k < lv; k += 32) {
             const u32 u = k < rv ? headp[list_start(dv) + k]
@@ -1502,7 +1503,7 @@ __global__ void k_stats(const u64* __restrict__ fo, const u32* __restrict__ head
             const u32 word = load_desc(vdesc + y).d, dy = list_len<HUB>(word);
             if (dy > 0 && lv > small_d && key_less(dy, y, lv, v)) {
                 streamed += dy;
-                chunked += hub_len<HUB>(word) + rest_len<HUB>(word) * (chunks ? chunks : 1);
+                chunked += hub_len<HUB>(word) + rest_len<HUB>(word) * chunks;
             }
         }
     }
