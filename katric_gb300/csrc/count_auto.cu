@@ -1431,8 +1431,9 @@ __global__ void __launch_bounds__(1024) k_final(const u64* __restrict__ partials
 // `parts` blocks share a graph (totals are zeroed by the caller when there are several): few graphs
 // would otherwise leave the largest to one block (11 graphs with one of 2.7 M vertices: 711 us by
 // one block each, 21 us by 64 with eight loads in flight per thread; 512 graphs 57 -> 46 us).  A part's
-// sum need not be a multiple of three, but the sum of all is, so each part is multiplied by the
-// inverse of three modulo 2^64.
+// sum need not be a multiple of three, so the parts add up their sums, and the last to arrive (the top
+// bits of totals[g] count them: the sum of all per-vertex counts of 2^36 entries is below 2^57) divides.
+constexpr int GRAPH_PARTS = 64;  // most blocks of a graph
 __global__ void __launch_bounds__(256) k_graph_totals(const u64* __restrict__ cnt, const u64* __restrict__ graph_first,
                                                       u64 num_graphs, u64 n, u64* __restrict__ totals, u32 parts,
                                                       Control* ctl) {
@@ -1458,9 +1459,14 @@ __global__ void __launch_bounds__(256) k_graph_totals(const u64* __restrict__ cn
         }
         s = block_sum_u64<256>(s, s_red);
         if (threadIdx.x == 0) {
-            const u64 t = s * 0xAAAAAAAAAAAAAAABull;
-            if (parts == 1) totals[g] = ok ? t : 0;
-            else if (t) atomicAdd(&totals[g], t);
+            if (parts == 1) {
+                totals[g] = s / 3;
+            } else if (ok) {
+                constexpr u64 ARRIVED = 1ull << 57;
+                static_assert(GRAPH_PARTS < (1 << 7), "arrivals fit above the sum");
+                const u64 before = atomicAdd(&totals[g], s + ARRIVED);
+                if (before / ARRIVED + 1 == parts) totals[g] = (before + s) % ARRIVED / 3;
+            }
             if (!ok) atomicOr(&ctl->err, DEV_ERR_DEGREE);
         }
     }
@@ -1853,7 +1859,7 @@ void launch_graph_totals(const u64* cnt, const u64* graph_first, u64 num_graphs,
     const u64 blocks = num_graphs < cap ? num_graphs : cap;
     // as many parts as fill the chip, none smaller than 4096 vertices if one graph has them all
     const u64 fill = cap / blocks < n / 4096 ? cap / blocks : n / 4096;
-    const u64 parts = fill < 1 ? 1 : fill < 64 ? fill : 64;
+    const u64 parts = fill < 1 ? 1 : fill < GRAPH_PARTS ? fill : GRAPH_PARTS;
     if (parts > 1) cudaMemsetAsync(totals, 0, sizeof(u64) * num_graphs, st.st);
     launch_chained(k_graph_totals, (unsigned)(blocks * parts), 256, 0, st, cnt, graph_first, num_graphs, n, totals,
                    (u32)parts, ctl);
