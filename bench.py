@@ -58,9 +58,9 @@ KERNELS_PER_STEP = 7  # k_prep, k_orient, k_desc, k_count_small, k_count_medium,
 
 def kernels_per_count(nnz: int) -> int:
     """Kernels of one AUTO count: the seven above, plus k_tile_hist / k_tile_scan / k_tile_scatter from
-    2^20 adjacency entries on; from 2^21 on k_hub_place, k_hub_rank, k_hub_tops and k_count_hub
-    run and k_count_large does not."""
-    return KERNELS_PER_STEP + (3 if nnz >= (1 << 20) else 0) + (3 if nnz >= (1 << 21) else 0)
+    2^20 adjacency entries on; from 2^21 to 2^32 - 1 k_hub_place, k_hub_sort, k_hub_rank, k_hub_tops and
+    k_count_hub run and k_count_large does not."""
+    return KERNELS_PER_STEP + (3 if nnz >= (1 << 20) else 0) + (4 if 1 << 21 <= nnz < 1 << 32 else 0)
 
 
 def make_graph(name: str):

@@ -40,7 +40,8 @@ extern "C" {
  * selected by shmetric's --intersection-method, apps/parse_parameters.h:156-158).
  * KTRI_METHOD_AUTO is the GPU default: owner-side shared-memory hash tables that stream the
  * shorter out-list of every edge.  The other four run the reference's strategies on
- * id-sorted out-lists, one warp per oriented edge.  All five give identical counts. */
+ * id-sorted out-lists, one warp per oriented edge, or one lane where both lists have at most 48
+ * entries (merged there, or searched by the strategies that search).  All five give identical counts. */
 #define KTRI_METHOD_AUTO 0
 #define KTRI_METHOD_MERGE 1         /* merge_intersection, include/cetric/counters/intersection.h:82-96 */
 #define KTRI_METHOD_BINARY_SEARCH 2 /* binary_search_intersection, intersection.h:99-117 */
@@ -54,20 +55,23 @@ typedef struct ktri_opts {
                                       kernel, the rest by owner tiles: 1..48 (0 = default: 48, or medium_outdegree
                                       where that is set lower) */
     uint32_t collect_stats;        /* 1: also compute wedge_checks / intersection work counters */
-    uint64_t binary_intersection_cutoff; /* Config::binary_intersection_cutoff (config.h:173), default 1000 */
+    uint64_t binary_intersection_cutoff; /* Config::binary_intersection_cutoff (config.h:173), default 1000; no
+                                      effect on edges of two out-lists of at most 48, which are merged */
     double hybrid_cutoff_scale;    /* Config::hybrid_cutoff_scale (config.h:174), default 1.0 */
     uint32_t force_wide_offsets;   /* 1: 64-bit out-list offsets even where 32 bits suffice (the path
                                       graphs with nnz + 3n > 2^32 take; exposed for testing) */
     uint32_t medium_outdegree;     /* owners above small_outdegree and at most this use the warp-per-tile
-                                      kernel, larger ones the block-per-tile kernel: small_outdegree..256
+                                      kernel, larger ones the block-per-tile kernel (the warp-per-tile and hub
+                                      kernels where out-lists are split): small_outdegree..256
                                       (0 = default 256; at least 32 with small_outdegree 0) */
-    uint32_t segment;              /* adjacency slots per owner tile of those two kernels: a power of two
-                                      in 64..1024 (0 = default 1024) */
-    uint32_t copy_wait_polls;      /* bound on the polls of the large-owner kernel's first wait for each
+    uint32_t segment;              /* adjacency slots per owner tile of those kernels: a power of two
+                                      in 64..1024 (0 = default: by the graph's size, the largest of them that
+                                      leaves 8192 tiles, or 64) */
+    uint32_t copy_wait_polls;      /* bound on the polls of the block-per-tile kernel's first wait for each
                                       bulk copy into shared memory (0 = default 2^22).  A wait that runs
                                       out makes the call fail with KTRI_ERR_TIMEOUT and a total of 0.
                                       KTRI_COPY_WAIT_NONE gives up at once (tests of that path). */
-    uint32_t tile_order;           /* order in which the medium- and large-owner kernels take their tiles:
+    uint32_t tile_order;           /* order in which the owner kernels take their tiles:
                                       0 (default) large tiles by the first vertex they stream (tiles that run
                                       together read nearby out-lists), medium tiles longest owner first;
                                       KTRI_TILE_ORDER_COST both by the entries each tile streams, heaviest first
@@ -94,8 +98,9 @@ typedef struct ktri_run_stats {
     float ms_orient;                  /* device time of orientation (+ sort when one ran) */
     float ms_count;                   /* device time of intersection + reduction */
     float ms_total;                   /* device time of the whole call */
-    float ms_count_small;             /* AUTO: device time of the small-owner tile kernel */
-    float ms_count_large;             /* AUTO: device time of the large-owner vertex kernel */
+    float ms_count_small;             /* AUTO: device time of the edges counted at their tail (and, with split
+                                         out-lists, of the bitmaps of their densest parts) */
+    float ms_count_large;             /* AUTO: device time of the owner tiles, all kernels */
     float ms_h2d;                     /* host-buffer calls: device time from the first input copy until the
                                          last piece of head has landed (orientation overlaps it) */
     float ms_d2h;                     /* host-buffer calls: device time of the read-back of the results */
@@ -121,8 +126,8 @@ int ktri_ctx_destroy(ktri_ctx* ctx);
  * with KTRI_ERR_OUT_OF_MEMORY before launching anything. */
 int ktri_ctx_set_memory_budget(ktri_ctx* ctx, uint64_t bytes);
 /* Device bytes a count of a graph with n vertices and nnz entries needs in the workspace.  AUTO counts
- * from 2^21 entries on take about 2.4 bytes per entry and 18 per vertex more (split out-lists) where
- * the budget and the free memory have room for them. */
+ * from 2^21 entries on take about 3.1 bytes per entry (above 2^28 entries 2.1, and 256 MiB) and 18 per
+ * vertex more (split out-lists) where the budget and the free memory have room for them. */
 uint64_t ktri_workspace_bytes(uint64_t n, uint64_t nnz, int32_t intersection_method);
 const char* ktri_last_error(const ktri_ctx* ctx);
 int ktri_ctx_stats(ktri_ctx* ctx, ktri_run_stats* out); /* synchronises the context's last stream */

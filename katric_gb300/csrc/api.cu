@@ -484,7 +484,7 @@ int enqueue_pipeline(ktri_ctx* ctx, int sms, char* base, const Layout& L, const 
                              opt.small_outdegree, opt.segment, publish->done_word, st);
     } else if (autom) {
         const cudaError_t e = ktri::launch_count_auto<OffT, HUB>(
-            fo, head, n, nnz, vdesc, headp, hub, mrun, lrun, opt.small_outdegree, opt.segment, cnt, partials, ctl, sms,
+            fo, head, n, vdesc, headp, hub, mrun, lrun, opt.small_outdegree, opt.segment, cnt, partials, ctl, sms,
             st, events ? ctx->ev[4] : nullptr, events ? ctx->ev[5] : nullptr, first_wait_polls(opt.copy_wait_polls));
         if (e != cudaSuccess) return cuda_fail(ctx, e, "launch of the counting kernels");
         if (d_total) ktri::launch_final_auto<OffT, HUB>(partials, n, sms, d_total, ctl, st);
@@ -513,7 +513,8 @@ int run_pipeline(ktri_ctx* ctx, const Layout& L, const u64* fo, const u32* head,
                  ktri::TriangleSink sink = ktri::TriangleSink{}, const HeadChunks* chunks = nullptr) {
     char* base = static_cast<char*>(ctx->ws);
     const int rc =
-        enqueue_layout(ctx, ctx->num_sms, base, L, fo, head, n, nnz, d_total, cnt, opt, st, sort_all, true, sink, chunks);
+        enqueue_layout(ctx, ctx->num_sms, base, L, fo, head, n, nnz, d_total, cnt, opt, st, sort_all, true, sink,
+                       chunks);
     if (rc) return rc;
     ctx->ctl = reinterpret_cast<Control*>(base + L.ctl);
     ctx->last_stream = st;
@@ -761,9 +762,10 @@ int ktri::engine_prepare_batch(ktri_ctx* ctx, const uint64_t* d_first_out, const
     pub.job = job;
     pub.seq = seq;
     pub.done_word = done_word;
-    rc = enqueue_pipeline<u32, false>(ctx, ctx->num_sms, base, L, reinterpret_cast<const u64*>(d_first_out), d_head, n_total,
-                               nnz_total, reinterpret_cast<u64*>(base + L.total), reinterpret_cast<u64*>(d_per_vertex),
-                               opt, st, false, false, ktri::TriangleSink{}, nullptr, &pub);
+    rc = enqueue_pipeline<u32, false>(ctx, ctx->num_sms, base, L, reinterpret_cast<const u64*>(d_first_out), d_head,
+                                      n_total, nnz_total, reinterpret_cast<u64*>(base + L.total),
+                                      reinterpret_cast<u64*>(d_per_vertex), opt, st, false, false,
+                                      ktri::TriangleSink{}, nullptr, &pub);
     if (rc) return rc;
     ctx->ctl = reinterpret_cast<Control*>(base + L.ctl);
     ctx->last_stream = st;
@@ -974,7 +976,8 @@ int ktri_count_csr_ctx(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t*
         if (nnz) KTRI_CK(ctx, copy_host(ctx, d_head, head, head_bytes, true, st));
         KTRI_CK(ctx, cudaEventRecord(ctx->ev_io[1], st));
     }
-    rc = run_pipeline(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, false, {}, chunks.count ? &chunks : nullptr);
+    rc = run_pipeline(ctx, L, d_fo, d_head, n, nnz, d_total, d_cnt, opt, st, false, {},
+                      chunks.count ? &chunks : nullptr);
     if (rc) return rc;
     KTRI_CK(ctx, cudaEventRecord(ctx->ev_io[2], st));
     KTRI_CK(ctx, copy_host(ctx, total_out, d_total, sizeof(u64), false, st));
@@ -1255,7 +1258,8 @@ int ktri_partition_cost(ktri_ctx* ctx, const uint64_t* first_out, const uint32_t
     KTRI_CK(ctx, cudaMemcpyAsync(d_fo, first_out, 8 * (n + 1), cudaMemcpyHostToDevice, st));
     if (nnz) KTRI_CK(ctx, cudaMemcpyAsync(d_head, head, 4 * nnz, cudaMemcpyHostToDevice, st));
     // degrees and out-degrees come from the orientation stage of the pipeline
-    rc = run_pipeline(ctx, L, d_fo, d_head, n, nnz, reinterpret_cast<u64*>(base + L.total), reinterpret_cast<u64*>(base + L.cnt), opt, st, true);
+    rc = run_pipeline(ctx, L, d_fo, d_head, n, nnz, reinterpret_cast<u64*>(base + L.total),
+                      reinterpret_cast<u64*>(base + L.cnt), opt, st, true);
     if (rc) return rc;
     ktri::launch_cost_partition(d_fo, d_head, n, reinterpret_cast<const u32*>(base + L.deg),
                                 reinterpret_cast<const u32*>(base + L.dplus), cost_function, parts, d_cost,

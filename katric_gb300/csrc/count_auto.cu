@@ -96,7 +96,8 @@ __device__ __forceinline__ Desc<OffT> ld_desc(const Desc<OffT>* p) {
 __device__ __forceinline__ void hit16(u32* hits32, u32 slot) { atomicAdd(&hits32[slot >> 1], 1u << ((slot & 1u) << 4)); }
 __device__ __forceinline__ u32 read16(const u32* hits32, u32 slot) { return (hits32[slot >> 1] >> ((slot & 1u) << 4)) & 0xFFFFu; }
 
-// Lookup with a 16-bit hit counter (same table layout as bucket_probe).
+// Count a lookup of w in a table of buckets of four: on a hit, add one to the slot's 16-bit counter and
+// return 1.
 __device__ __forceinline__ u32 bucket_probe16(const u32* keys, u32* hits32, u32 lg, u32 w) {
     const u32 nb_mask = (1u << (lg - 2)) - 1;
     u32 b = bucket_home(w, lg);
@@ -173,9 +174,10 @@ struct SmallWarpLayout {
     static constexpr int W_REC = W_HITS + NB;                           // tail records (uint4)
     static constexpr int W_QS = W_REC + 4 * GROUP;                      // list starts (OffT), by key
     static constexpr int W_OS = W_QS + QCAP * (int)(sizeof(OffT) / 4);  // tails' list starts (OffT)
-    static constexpr int W_QM = W_OS + GROUP * (int)(sizeof(OffT) / 4); // by key: slot << 16 | tail << 12 | hubs << 6 | others
+    // by key: slot << 16 | tail << 12 | hubs << 6 | others
+    static constexpr int W_QM = W_OS + GROUP * (int)(sizeof(OffT) / 4);
     static constexpr int W_QH = W_QM + QCAP;                            // HUB: hub list starts (16-byte groups), by key
-    static constexpr int W_TOT = W_QH + (HUB ? QCAP : 0);                         // tails' hit totals
+    static constexpr int W_TOT = W_QH + (HUB ? QCAP : 0);               // tails' hit totals
     static constexpr int W_VTX = W_TOT + GROUP;                         // tails' vertices
     static constexpr int W_BIN = W_VTX + GROUP;                         // lists by length in 16-byte groups
     static constexpr int W_ORD = W_BIN + 32;                            // queue order (u16)
@@ -480,8 +482,8 @@ __device__ __forceinline__ void small_batch(u32* base, u64 bi, u32 vb, u64 n, co
                     const uint4* hp = hubp8 + (have ? q_h[q] : 0u) + half;
                     for (hrem -= 8 * (int)half; hrem > 0; hrem -= 16, hp += 2) {
                         const uint4 cur = ld_in<CG>(hp);
-                        look4(n32 + (cur.x & 0xFFFFu), n32 + (cur.x >> 16), n32 + (cur.y & 0xFFFFu), n32 + (cur.y >> 16),
-                              hrem);
+                        look4(n32 + (cur.x & 0xFFFFu), n32 + (cur.x >> 16), n32 + (cur.y & 0xFFFFu),
+                              n32 + (cur.y >> 16), hrem);
                         if (hrem > 4)
                             look4(n32 + (cur.z & 0xFFFFu), n32 + (cur.z >> 16), n32 + (cur.w & 0xFFFFu),
                                   n32 + (cur.w >> 16), hrem - 4);
@@ -840,8 +842,8 @@ __global__ void __launch_bounds__(BLOCK) k_count_large(const u64* __restrict__ f
         __syncthreads();
         const u64 t = s_t;
         if (t >= ntiles) break;
-        timed_out = large_tile<BLOCK, CAP, OffT>(smem, s_bar, ltiles[tile_at(true, t)], fo, head, n, vdesc, headp, seg, cnt,
-                                                 first_wait_polls, phase, inflight, local_total, dup);
+        timed_out = large_tile<BLOCK, CAP, OffT>(smem, s_bar, ltiles[tile_at(true, t)], fo, head, n, vdesc, headp, seg,
+                                                 cnt, first_wait_polls, phase, inflight, local_total, dup);
         if (timed_out) break;
     }
     if (dup) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
@@ -1714,10 +1716,9 @@ __global__ void __launch_bounds__(ENGINE_BLOCK, 4) k_engine(EngineJob* jobs, u32
             }
         } else {
             const u64 t = u - jb->units_small - jb->units_medium;
-            timed_out = large_tile<BLOCK, LARGE_CAP, u32, true>(smem, s_bar, __ldcg(jb->ltiles + tile_at(true, t)), jb->fo, jb->head,
-                                                                jb->n, vd, jb->headp,
-                                                          jb->seg, jb->cnt, COPY_WAIT_POLLS, phase, inflight,
-                                                          unused_total, dup);
+            timed_out = large_tile<BLOCK, LARGE_CAP, u32, true>(smem, s_bar, __ldcg(jb->ltiles + tile_at(true, t)), jb->fo,
+                                                                jb->head, jb->n, vd, jb->headp, jb->seg, jb->cnt,
+                                                                COPY_WAIT_POLLS, phase, inflight, unused_total, dup);
         }
         if (dup) atomicOr(&ctl->err, DEV_ERR_DUPLICATE);
         if (timed_out && threadIdx.x == 0)
@@ -1827,27 +1828,29 @@ int count_grid_auto(int num_sms) {
 }
 
 template <typename OffT, bool HUB>
-cudaError_t launch_count_auto(const u64* fo, const u32* head, u64 n, u64 nnz, const void* vdesc, const u32* headp,
-                              const HubState& hub, const uint2* mtiles, const uint2* ltiles, u32 small_d, u32 seg, u64* cnt, u64* partials,
-                              Control* ctl, int num_sms, LaunchStream st, cudaEvent_t after_small,
-                              cudaEvent_t after_large, u32 copy_wait_polls) {
-    (void)nnz;
+cudaError_t launch_count_auto(const u64* fo, const u32* head, u64 n, const void* vdesc, const u32* headp,
+                              const HubState& hub, const uint2* mtiles, const uint2* ltiles, u32 small_d, u32 seg,
+                              u64* cnt, u64* partials, Control* ctl, int num_sms, LaunchStream st,
+                              cudaEvent_t after_small, cudaEvent_t after_large, u32 copy_wait_polls) {
     const int cap = count_grid_small<OffT, HUB>(num_sms);
     const int gs = small_grid_launched(n, cap);
     const int gm = count_grid_medium<OffT, HUB>(num_sms);
     const int gl = count_grid_large<OffT, HUB>(num_sms);
     const auto* vd = reinterpret_cast<const Desc<OffT>*>(vdesc);
-    launch_chained(k_count_small<SMALL_BLOCK, OffT, HUB>, gs, SMALL_BLOCK, SmallWarpLayout<OffT, HUB>::bytes(SMALL_BLOCK / 32), st, 
-        n, small_batch_vertices(n, cap), vd, headp, hub.lists, hub.ids, small_d, cnt, partials, ctl);
+    launch_chained(k_count_small<SMALL_BLOCK, OffT, HUB>, gs, SMALL_BLOCK,
+                   SmallWarpLayout<OffT, HUB>::bytes(SMALL_BLOCK / 32), st, n, small_batch_vertices(n, cap), vd, headp,
+                   hub.lists, hub.ids, small_d, cnt, partials, ctl);
     if (after_small) cudaEventRecord(after_small, st);
     if constexpr (HUB)
-        launch_chained(k_count_hub, count_grid_hub<HUB>(num_sms), 32 * HUB_WARPS, HUB_SMEM, st, 
-            fo, head, vd, hub.lists, hub.ids, hub.top_info, hub.top_bits, mtiles, ltiles, seg, cnt, partials + cap + gm + gl, ctl);
-    launch_chained(k_count_medium<MEDIUM_BLOCK, OffT, HUB>, gm, MEDIUM_BLOCK, TileLayout<OffT>::bytes(MEDIUM_BLOCK / 32), st, 
-        fo, head, n, vd, headp, mtiles, ltiles, seg, cnt, partials + cap, ctl);
+        launch_chained(k_count_hub, count_grid_hub<HUB>(num_sms), 32 * HUB_WARPS, HUB_SMEM, st, fo, head, vd,
+                       hub.lists, hub.ids, hub.top_info, hub.top_bits, mtiles, ltiles, seg, cnt,
+                       partials + cap + gm + gl, ctl);
+    launch_chained(k_count_medium<MEDIUM_BLOCK, OffT, HUB>, gm, MEDIUM_BLOCK,
+                   TileLayout<OffT>::bytes(MEDIUM_BLOCK / 32), st, fo, head, n, vd, headp, mtiles, ltiles, seg, cnt,
+                   partials + cap, ctl);
     if constexpr (!HUB)
-        launch_chained(k_count_large<LARGE_BLOCK, LARGE_CAP, OffT>, gl, LARGE_BLOCK, LargeL<OffT>::bytes, st, fo, head, n, vd, headp, ltiles, seg, cnt, partials + cap + gm,
-                                                           ctl, copy_wait_polls);
+        launch_chained(k_count_large<LARGE_BLOCK, LARGE_CAP, OffT>, gl, LARGE_BLOCK, LargeL<OffT>::bytes, st, fo, head,
+                       n, vd, headp, ltiles, seg, cnt, partials + cap + gm, ctl, copy_wait_polls);
     if (after_large) cudaEventRecord(after_large, st);
     return cudaGetLastError();
 }
@@ -1872,22 +1875,22 @@ void launch_final(const u64* partials, u32 np, u64* total, Control* ctl, LaunchS
 template <typename OffT, bool HUB>
 void launch_final_auto(const u64* partials, u64 n, int num_sms, u64* total, Control* ctl, LaunchStream st) {
     const int cap = count_grid_small<OffT, HUB>(num_sms);
-    launch_chained(k_final, 1, 1024, 0, st, partials, (u32)count_grid_auto<OffT, HUB>(num_sms), (u32)small_grid_launched(n, cap),
-                                (u32)cap, total, ctl);
+    launch_chained(k_final, 1, 1024, 0, st, partials, (u32)count_grid_auto<OffT, HUB>(num_sms),
+                   (u32)small_grid_launched(n, cap), (u32)cap, total, ctl);
 }
 
 template <typename OffT, bool HUB>
 void launch_stats(const u64* fo, const u32* head, u64 n, const void* vdesc, const u32* headp, const HubState& hub,
                   u32 small_d, u32 medium_d, Control* ctl, int num_sms, LaunchStream st) {
     if (n == 0) return;
-    launch_chained(k_stats<OffT, HUB>, num_sms * 8, 256, 0, st, fo, head, n, reinterpret_cast<const Desc<OffT>*>(vdesc), headp,
-                                                    hub.lists, hub.ids, small_d, medium_d, ctl);
+    launch_chained(k_stats<OffT, HUB>, num_sms * 8, 256, 0, st, fo, head, n,
+                   reinterpret_cast<const Desc<OffT>*>(vdesc), headp, hub.lists, hub.ids, small_d, medium_d, ctl);
 }
 
 #define KTRI_INST(OffT, HUB)                                                                                        \
     template void launch_final_auto<OffT, HUB>(const u64*, u64, int, u64*, Control*, LaunchStream);                 \
     template int count_grid_auto<OffT, HUB>(int);                                                                   \
-    template cudaError_t launch_count_auto<OffT, HUB>(const u64*, const u32*, u64, u64, const void*, const u32*,    \
+    template cudaError_t launch_count_auto<OffT, HUB>(const u64*, const u32*, u64, const void*, const u32*,         \
                                                       const HubState&, const uint2*, const uint2*, u32, u32, u64*,  \
                                                       u64*, Control*, int, LaunchStream, cudaEvent_t, cudaEvent_t,  \
                                                       u32);                                                         \

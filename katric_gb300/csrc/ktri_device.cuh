@@ -241,24 +241,6 @@ __device__ __forceinline__ bool bucket_insert(u32* keys, u32 lg, u32 w) {
     return true;  // unreachable: tables are at most half full
 }
 
-// Count a lookup of w: on a hit, add one to the slot's hit counter and return 1.
-__device__ __forceinline__ u32 bucket_probe(const u32* keys, u32* hits, u32 lg, u32 w) {
-    const u32 nb_mask = (1u << (lg - 2)) - 1;
-    u32 b = bucket_home(w, lg);
-    for (u32 it = 0; it <= nb_mask; ++it) {
-        const uint4 q = *reinterpret_cast<const uint4*>(keys + 4 * b);
-        const bool m0 = q.x == w, m1 = q.y == w, m2 = q.z == w, m3 = q.w == w;
-        if (m0 | m1 | m2 | m3) {
-            const u32 i = m0 ? 0u : (m1 ? 1u : (m2 ? 2u : 3u));
-            atomicAdd(&hits[4 * b + i], 1u);
-            return 1u;
-        }
-        if (q.w == EMPTY_KEY) return 0u;
-        b = (b + 1) & nb_mask;
-    }
-    return 0u;
-}
-
 __host__ __device__ __forceinline__ u32 ceil_log2(u32 v) {
     u32 lg = 0;
     while ((1u << lg) < v) ++lg;

@@ -118,8 +118,8 @@ void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* de
                    const HubState& hub, u32* dplus, Control* ctl, LaunchStream st, u64 tile_begin = 0,
                    u64 tile_end = ~0ull);
 // Owner tiles: medium owners' tiles are written from mtiles on, large owners' from ltiles backwards
-// (mtiles + large_tile_capacity: an owner has one kind, so both fit one array).  order_hist: the histograms launch_order_tiles uses next,
-// or null.
+// (mtiles + large_tile_capacity: an owner has one kind, so both fit one array).  order_hist: the
+// histograms launch_order_tiles uses next, or null.
 template <typename OffT, bool HUB>
 void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, const HubState& hub, uint2* mtiles,
                  uint2* ltiles, u32 small_d, u32 medium_d, u32 seg, u32* order_hist, Control* ctl, int num_sms,
@@ -134,7 +134,9 @@ void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, const HubS
 // hist needs tile_order_scratch_words() u32, which launch_desc zeroes.
 enum : u32 { TILE_BY_VERTEX = 0, TILE_BY_DEGREE = 1, TILE_BY_COST = 2 };
 // Where entry t of a list is, for lists that run backwards from the address of their end.
-__host__ __device__ __forceinline__ long long tile_at(bool back, u64 t) { return back ? -1 - (long long)t : (long long)t; }
+__host__ __device__ __forceinline__ long long tile_at(bool back, u64 t) {
+    return back ? -1 - (long long)t : (long long)t;
+}
 struct TileOrder {
     bool back;  // tiles, keys and sorted run backwards
     const uint2* tiles;
@@ -162,7 +164,7 @@ int count_grid_large(int num_sms);
 template <typename OffT, bool HUB>
 int count_grid_auto(int num_sms);  // small + medium + large + hub
 template <typename OffT, bool HUB>
-cudaError_t launch_count_auto(const u64* fo, const u32* head, u64 n, u64 nnz, const void* vdesc, const u32* headp,
+cudaError_t launch_count_auto(const u64* fo, const u32* head, u64 n, const void* vdesc, const u32* headp,
                               const HubState& hub, const uint2* mtiles, const uint2* ltiles, u32 small_d, u32 seg,
                               u64* cnt, u64* partials, Control* ctl, int num_sms, LaunchStream st,
                               cudaEvent_t after_small, cudaEvent_t after_large, u32 copy_wait_polls = COPY_WAIT_POLLS);
@@ -224,7 +226,8 @@ bool copy_by_kernel_ok(const void* src, const void* dst);
 bool launch_copy(const void* src, void* dst, u64 bytes, int num_sms, cudaStream_t st);
 
 // Oriented out-lists -> undirected CSR of their edges (fs: n + 1 offsets, hs: 2m ids).  Scratch:
-// in_deg 2 n u32 (a power of two of at least n of them is used), in_start n u64, pos m u32, sums dag_scan_chunks(n) u64.
+// in_deg 2 n u32 (a power of two of at least n of them is used), in_start n u64, pos m u32, sums
+// dag_scan_chunks(n) u64.
 u64 dag_scan_chunks(u64 n);
 void launch_scan_u64(u64* x, u64 len, u64* sums, cudaStream_t st);  // exclusive, in place
 // Per-vertex cost (KTRI_COST_*) into cost[0..n), its exclusive prefix in place (cost[n] = total),
@@ -260,7 +263,8 @@ struct SplitLists {
 };
 template <typename OffT>
 void launch_sort_lists(u64 n, const void* vdesc, u32* headp, u32* mid_list, u32* big_list, u32* scratch,
-                       u64 scratch_per_block, int big_grid, SplitLists split, Control* ctl, int num_sms, LaunchStream st);
+                       u64 scratch_per_block, int big_grid, SplitLists split, Control* ctl, int num_sms,
+                       LaunchStream st);
 template <typename OffT>
 void launch_count_edges(u64 n, const void* vdesc, const u32* headp, int method, u64 cutoff, double hybrid_scale,
                         u64* cnt, u64* partials, int grid, u32* tails, Control* ctl, TriangleSink sink,

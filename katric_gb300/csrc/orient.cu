@@ -300,7 +300,9 @@ __device__ __forceinline__ void orient_tile(OrientWarp<IPT>& sw, const u64* __re
     const u64 a0 = have0 ? fo[i0 + lane] : 0, b0 = have0 ? fo[i0 + lane + 1] : 0;
     const bool in0 = have0 && b0 > a0 && a0 < j1 && b0 > j0;
     const u32 ball0 = __ballot_sync(FULL, in0);
-    if (in0) enter(i0 + lane, a0 > j0 ? (u32)(a0 - j0) : 0u, __popc(ball0 & lt), HUB ? __ldg(deg + i0 + lane) : (u32)(b0 - a0), b0);
+    if (in0)
+        enter(i0 + lane, a0 > j0 ? (u32)(a0 - j0) : 0u, __popc(ball0 & lt),
+              HUB ? __ldg(deg + i0 + lane) : (u32)(b0 - a0), b0);
     for (u32 k0 = 32, q0 = __popc(ball0); k0 < nwin; k0 += 32) {
         const u64 v = i0 + k0 + lane;
         const bool have = k0 + lane < nwin;
@@ -420,11 +422,10 @@ __device__ __forceinline__ void orient_tile(OrientWarp<IPT>& sw, const u64* __re
 // One tile per warp.  HUB: a graph without hubs (hubs = 0) runs the plain body, whose lists and
 // length words are then the same.
 template <int BLOCK, int IPT, bool HUB>
-__global__ void __launch_bounds__(BLOCK, ORIENT_BLOCKS) k_orient(const u64* __restrict__ fo, const u32* __restrict__ head, u64 n,
-                                                     u64 nnz, const u32* __restrict__ deg,
-                                                     const u32* __restrict__ tile_i0, u32* __restrict__ headp,
-                                                     u16* __restrict__ hubp, u32* __restrict__ dplus,
-                                                     Control* ctl, u64 tile_begin) {
+__global__ void __launch_bounds__(BLOCK, ORIENT_BLOCKS)
+    k_orient(const u64* __restrict__ fo, const u32* __restrict__ head, u64 n, u64 nnz, const u32* __restrict__ deg,
+             const u32* __restrict__ tile_i0, u32* __restrict__ headp, u16* __restrict__ hubp, u32* __restrict__ dplus,
+             Control* ctl, u64 tile_begin) {
     chain_begin();
     __shared__ OrientWarp<IPT> s_warp[BLOCK / 32];
     if (ctl->err & DEV_ERR_MASK) return;
@@ -731,7 +732,8 @@ void launch_order_tiles(const u64* fo, const u32* head, const u32* dplus, u64 n,
     const u32 shift = bits > 12 ? bits - 12 : 0;
     if (orders.of[0].mode == TILE_BY_COST)
         launch_chained(k_tile_cost, dim3(num_sms * 8, 2), 256, 0, st, fo, head, dplus, orders, seg, hub, ctl);
-    launch_chained(k_tile_hist, dim3(num_sms * 4, 2), TILE_ORDER_BLOCK, 0, st, fo, head, dplus, orders, seg, shift, hub, hist, ctl);
+    launch_chained(k_tile_hist, dim3(num_sms * 4, 2), TILE_ORDER_BLOCK, 0, st, fo, head, dplus, orders, seg, shift,
+                   hub, hist, ctl);
     launch_chained(k_tile_scan, 2, TILE_SCAN_BLOCK, 0, st, hist, ctl);
     launch_chained(k_tile_scatter, dim3(num_sms * 4, 2), TILE_ORDER_BLOCK, 0, st, orders, hist, ctl);
 }
@@ -754,8 +756,8 @@ void launch_prep(const u64* fo, u64 n, u64 nnz, u32* deg, u32* dplus, u64* cnt, 
 }
 
 void launch_hub_tops(const void* vdesc, const HubState& hub, Control* ctl, int num_sms, LaunchStream st) {
-    launch_chained(k_hub_tops, num_sms * 8, TOPS_BLOCK, 0, st, reinterpret_cast<const Desc<u32>*>(vdesc), hub.lists, hub.top_long,
-                                                   hub.top_info, hub.top_bits, hub.top_cap, ctl);
+    launch_chained(k_hub_tops, num_sms * 8, TOPS_BLOCK, 0, st, reinterpret_cast<const Desc<u32>*>(vdesc), hub.lists,
+                   hub.top_long, hub.top_info, hub.top_bits, hub.top_cap, ctl);
 }
 
 u64 hub_bins_words() { return 3ull * HUB_BINS; }
@@ -772,21 +774,23 @@ void launch_orient(const u64* fo, const u32* head, u64 n, u64 nnz, const u32* de
     if (tile_begin >= tile_end) return;
     const unsigned grid = (unsigned)(tile_end - tile_begin);
     if (hub)
-        launch_chained(k_orient<BLOCK, IPT, true>, grid, BLOCK, 0, st, fo, head, n, nnz, deg, tile_i0, headp, hub.lists, dplus,
-                                                           ctl, tile_begin);
+        launch_chained(k_orient<BLOCK, IPT, true>, grid, BLOCK, 0, st, fo, head, n, nnz, deg, tile_i0, headp, hub.lists,
+                       dplus, ctl, tile_begin);
     else
-        launch_chained(k_orient<BLOCK, IPT, false>, grid, BLOCK, 0, st, fo, head, n, nnz, deg, tile_i0, headp, nullptr, dplus,
-                                                            ctl, tile_begin);
+        launch_chained(k_orient<BLOCK, IPT, false>, grid, BLOCK, 0, st, fo, head, n, nnz, deg, tile_i0, headp, nullptr,
+                       dplus, ctl, tile_begin);
 }
 
 template <typename OffT, bool HUB>
-void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, const HubState& hub, uint2* mtiles, uint2* ltiles, u32 small_d,
-                 u32 medium_d, u32 seg, u32* order_hist, Control* ctl, int num_sms, LaunchStream st) {
+void launch_desc(const u64* fo, u64 n, const u32* dplus, void* vdesc, const HubState& hub, uint2* mtiles,
+                 uint2* ltiles, u32 small_d, u32 medium_d, u32 seg, u32* order_hist, Control* ctl, int num_sms,
+                 LaunchStream st) {
     if (n == 0) return;
     u64 blocks = (n + DESC_BLOCK - 1) / DESC_BLOCK;
     u64 cap = (u64)num_sms * 8;
-    launch_chained(k_desc<OffT, HUB>, (unsigned)(blocks < cap ? blocks : cap), DESC_BLOCK, 0, st,
-        fo, n, dplus, reinterpret_cast<Desc<OffT>*>(vdesc), hub.lists, hub.top_info, hub.top_long, mtiles, ltiles, small_d, medium_d, seg, order_hist, ctl);
+    launch_chained(k_desc<OffT, HUB>, (unsigned)(blocks < cap ? blocks : cap), DESC_BLOCK, 0, st, fo, n, dplus,
+                   reinterpret_cast<Desc<OffT>*>(vdesc), hub.lists, hub.top_info, hub.top_long, mtiles, ltiles, small_d,
+                   medium_d, seg, order_hist, ctl);
 }
 
 #define KTRI_INST(OffT, HUB)                                                                                     \
