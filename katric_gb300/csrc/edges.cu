@@ -709,7 +709,12 @@ void launch_sort_lists(u64 n, const void* vdesc, u32* headp, u32* mid_list, u32*
     const auto* vd = reinterpret_cast<const Desc<OffT>*>(vdesc);
     launch_chained(k_sort_warp<OffT>, num_sms * 8, 256, 0, st, n, vd, headp, mid_list, big_list, split, ctl);
     launch_chained(k_sort_block<OffT>, num_sms * 4, SORT_BLOCK, 0, st, vd, headp, mid_list, ctl);
-    launch_chained(k_sort_global<OffT>, big_grid, SORT_BLOCK, 0, st, vd, headp, big_list, scratch, scratch_per_block, ctl);
+    // Chained, its blocks start beside the block sort's and get the small L1 cache that leaves, where a
+    // list of its own needs 128 KB and more (60 lists of 25 000: 1.9 -> 2.8 ms).  So it is only where there
+    // is room for no such list.
+    const LaunchStream alone(st.st, st.chained && scratch_per_block <= (u64)SORT_SMEM);
+    launch_chained(k_sort_global<OffT>, big_grid, SORT_BLOCK, 0, alone, vd, headp, big_list, scratch, scratch_per_block,
+                   ctl);
 }
 
 // Blocks of both edge kernels (half of them each).
