@@ -1506,10 +1506,11 @@ __global__ void k_stats(const u64* __restrict__ fo, const u32* __restrict__ head
                 chunked += du;
             }
         }
+        if (lv <= small_d) continue;  // no owner
         for (u64 e = fo[v] + lane; e < fo[v + 1]; e += 32) {
             const u32 y = head[e];
             const u32 word = load_desc(vdesc + y).d, dy = list_len<HUB>(word);
-            if (dy > 0 && lv > small_d && key_less(dy, y, lv, v)) {
+            if (dy > 0 && key_less(dy, y, lv, v)) {
                 streamed += dy;
                 chunked += hub_len<HUB>(word) + rest_len<HUB>(word) * chunks;
             }
