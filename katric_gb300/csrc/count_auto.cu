@@ -861,7 +861,7 @@ __global__ void __launch_bounds__(BLOCK) k_count_large(const u64* __restrict__ f
 // What bounds it: instruction issue (71 to 73 %) beside the lookups' shared-memory wavefronts
 // (53 to 62 % of the pipe).  It replaced a one-hash filter with packed survivors and one list per warp
 // iteration, which left most lanes idle on lists below 100 entries: RMAT n = 8191 0.182 -> 0.061 ms
-// (medium + large), 512-graph batch 6.2 -> 5.0 ms, the other entries of RMAT-24 27.6 -> 21 ms.
+// (medium + large), 512-graph batch 6.2 -> 5.0 ms, the other entries of RMAT-24 27.6 -> 18 ms.
 // Measured against NB = 768 (24 warps per SM: RMAT-24 +0.8 %, batch +1 %, small graphs -10 %) and
 // fewer keys per chunk (more owners in two chunks: RMAT-24 66.3 ms, CAP = 192 68.0, CAP = 128 +7 %; a
 // lattice of out-degree 200 without hubs 1.41 ms, CAP = 192 2.49).  All of a medium owner's keys fit one chunk.
@@ -1127,7 +1127,7 @@ __global__ void __launch_bounds__(BLOCK, 4)
 // AND, a population count and 3.5 additions per word count 32 of them (TopCounters).
 // Measured (medium and large tiles, RMAT n = 10^6 / RMAT-24): ids through filters and hash tables
 // 4.31 / 119.4 ms; hub lists, one list per warp 1.90 / 74.7 ms; with the top bitmaps and units
-// 1.50 / 71.6 ms, of which this kernel takes 1.4 / 43 ms.  What is left: on RMAT-24 the lists'
+// 1.50 / 71.6 ms, of which this kernel takes 1.4 / 44 ms.  What is left: on RMAT-24 the lists'
 // reads (2.9 TB/s from L2 at a 70 % hit rate, 22 warps per SM beside 128 KB of counters), on
 // smaller graphs instruction issue.
 struct HubLayout {
